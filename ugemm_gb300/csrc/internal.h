@@ -89,6 +89,12 @@ struct Gemm {
 };
 
 #ifdef __CUDACC__
+// The epilogue with the row's bias already in hand (0 without one).
+__device__ __forceinline__ float epilogue_value(float v, float bias, const Epilogue& e) {
+  v += bias;
+  if (e.act) v = v > 0.f ? v : v * e.slope;
+  return v;
+}
 __device__ __forceinline__ float epilogue_apply(float v, const Epilogue& e, int row) {
   if (e.bias) v += e.bias[row];
   if (e.act) v = v > 0.f ? v : v * e.slope;

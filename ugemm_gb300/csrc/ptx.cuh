@@ -41,6 +41,19 @@ __device__ __forceinline__ bool error_raised(const int* err) {
   return err && *reinterpret_cast<const volatile int*>(err) != 0;
 }
 
+// Registers handed back by, or granted to, every thread of a warpgroup
+// (all four warps execute it).  The warpgroups' shares of a kernel must add
+// up to no more than threads x registers at its launch, or the grant waits
+// for ever.
+template <int kRegs>
+__device__ __forceinline__ void setmaxnreg_dec() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+template <int kRegs>
+__device__ __forceinline__ void setmaxnreg_inc() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

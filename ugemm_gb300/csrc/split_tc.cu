@@ -28,14 +28,14 @@
 //   1. split kernel: reads op(A)/op(B) in any transpose and leading
 //      dimension, writes the pieces as K-major bf16 planes [pieces][rows][Kp]
 //      (Kp = K rounded up to 32, zero padded);
-//   2. GEMM kernel, 10 warps:
+//   2. GEMM kernel, 12 warps (a fused launch: 10 or 16, without idle ones):
 //        warp 0   TMA producer: one 3-D TMA per operand per stage brings all
 //                 pieces of a 32-deep k slice (64-byte swizzle; TF32
 //                 pieces: 128-byte rows and swizzle) into a 3-4 stage ring
 //                 (mbarrier full/empty pairs);
 //        warp 1   allocates TMEM (2 x BN columns: main + corrections) and,
 //                 from one thread, issues the tcgen05.mma stream;
-//        warps 2-9  epilogue: chunk drains, then alpha/beta and the store of
+//        warps 4-11 epilogue: chunk drains, then alpha/beta and the store of
 //                 the 128 x BN tile (one TMEM lane per row; two warps per
 //                 lane quarter, each owning half of the columns).
 // All mbarrier waits are bounded (ptx.cuh); on a timeout the kernel records
@@ -110,17 +110,22 @@ __device__ __forceinline__ TileCoord tile_coord(const TcProblem& single, const T
   return tc;
 }
 
+// alpha * sum + beta * old (old is not looked at when beta == 0), rounded the
+// same way in every epilogue.
+__device__ __forceinline__ float scaled_sum(const TcProblem& P, float sum, float old) {
+  return P.beta != 0.f ? fmaf(P.alpha, sum, P.beta * old) : P.alpha * sum;
+}
+
 // The end of a tile's epilogue once acc holds its sums (this warp's HALF
 // columns of its lane quarter's 32 rows): the FP16x3 scales, alpha/beta (C is
 // read only when beta != 0), the bias / activation (EPI instantiations only)
 // and the stores.  stage_base: the shared-memory staging area after the ring.
 template <int NP, int BN, bool GROUPED, bool EPI>
 __device__ __forceinline__ void epi_store(const TcProblem& P, const TileCoord& tc,
-                                          float (&acc)[BN / 2], int warp, int lane,
+                                          float (&acc)[BN / 2], int ew, int warp, int lane,
                                           float* stage_base) {
-  using S = TcShape<NP, BN, false>;  // only its BN-dependent staging is read here
+  using S = TcShape<NP, BN, false>;  // only its staging, the same for WIDE, is read here
   constexpr int HALF = BN / 2;
-  const int ew = warp - 2;
   const int q = warp & 3;
   const int col_off = (ew >> 2) * HALF;
   const int n_live = GROUPED ? P.N - tc.n0 - col_off : HALF;
@@ -148,125 +153,124 @@ __device__ __forceinline__ void epi_store(const TcProblem& P, const TileCoord& t
   const bool has_epi = EPI && (P.epi.bias != nullptr || P.epi.act != 0);
   if (GROUPED && P.swap) {
     // transposed problem: this lane's kernel row is a C column, so for a
-    // fixed register the warp writes 32 consecutive floats of one C row
+    // fixed register the warp writes 32 consecutive floats of one C row.
+    // Old values and biases are read 32 columns ahead of the stores.
     const int r = tc.m0 + q * 32 + lane;
-    if (r < P.M) {
-#pragma unroll
-      for (int j = 0; j < HALF; ++j) {
-        const int c = tc.n0 + col_off + j;
-        if (c < P.N) {
-          float* cp = P.C + static_cast<size_t>(c) * P.ldc + r;
-          float v = P.alpha * acc[j];
-          if (P.beta != 0.f) v += P.beta * *cp;
-          if (has_epi) v = epilogue_apply(v, P.epi, c);
-          *cp = v;
-        }
-      }
-    }
-    return;
-  }
-  if constexpr (GROUPED && S::STAGE_C8) {
-    // 256-wide tiles: each 32 x 32 block goes through shared memory 8
-    // rows at a time (lanes 8p..8p+7 hold rows 8p..8p+7), so every store
-    // instruction still writes one 128-byte row segment
-    float* stage = stage_base + ew * 8 * 33;
-    const int col = tc.n0 + col_off + lane;
 #pragma unroll
     for (int c32 = 0; c32 < HALF / 32; ++c32) {
       if (c32 * 32 >= n_live) break;
-      const int cc = col + c32 * 32;
+      const int c0 = tc.n0 + col_off + c32 * 32;
+      float bl = 0.f;  // lane l: the bias of column c0 + l
+      if constexpr (EPI) {
+        if (P.epi.bias != nullptr && c0 + lane < P.N) bl = __ldg(P.epi.bias + c0 + lane);
+      }
+      if (P.beta != 0.f) {
+        float old[32];
 #pragma unroll
-      for (int pass = 0; pass < 4; ++pass) {
-        if ((lane >> 3) == pass) {
+        for (int j = 0; j < 32; ++j)
+          old[j] = r < P.M && c0 + j < P.N ? P.C[static_cast<size_t>(c0 + j) * P.ldc + r] : 0.f;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) stage[(lane & 7) * 33 + j] = acc[c32 * 32 + j];
+        for (int j = 0; j < 32; ++j)
+          acc[c32 * 32 + j] = scaled_sum(P, acc[c32 * 32 + j], old[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[c32 * 32 + j] *= P.alpha;
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        float v = acc[c32 * 32 + j];
+        if constexpr (EPI) {
+          const float b = __shfl_sync(0xffffffffu, bl, j);
+          if (has_epi) v = epilogue_value(v, b, P.epi);
         }
-        __syncwarp();
-        if (cc < P.N) {
-          for (int rr = 0; rr < 8; ++rr) {
-            const int row = tc.m0 + q * 32 + pass * 8 + rr;
-            if (row >= P.M) break;
-            float* cp = P.C + static_cast<size_t>(row) * P.ldc + cc;
-            float v = P.alpha * stage[rr * 33 + lane];
-            if (P.beta != 0.f) v += P.beta * *cp;
-            if (has_epi) v = epilogue_apply(v, P.epi, row);
-            *cp = v;
-          }
-        }
-        __syncwarp();
+        if (r < P.M && c0 + j < P.N) P.C[static_cast<size_t>(c0 + j) * P.ldc + r] = v;
       }
     }
     return;
   }
-  if constexpr (S::STAGE_C) {
-    // transpose each 32 x 32 block through shared memory: lane = column,
-    // one 128-byte row segment per store instruction
-    float* stage = stage_base + ew * 32 * 33;
-    const int col = tc.n0 + col_off + lane;
-#pragma unroll
-    for (int c32 = 0; c32 < HALF / 32; ++c32) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) stage[lane * 33 + j] = acc[c32 * 32 + j];
-      __syncwarp();
-      const int cc = col + c32 * 32;
-      if (cc < P.N) {
-        if (has_epi) {
-          for (int rr = 0; rr < 32; ++rr) {
-            const int row = tc.m0 + q * 32 + rr;
-            if (row >= P.M) break;
-            float* cp = P.C + static_cast<size_t>(row) * P.ldc + cc;
-            float v = P.alpha * stage[rr * 33 + lane];
-            if (P.beta != 0.f) v += P.beta * *cp;
-            *cp = epilogue_apply(v, P.epi, row);
-          }
-        } else {
-          for (int rr = 0; rr < 32; ++rr) {
-            const int row = tc.m0 + q * 32 + rr;
-            if (row >= P.M) break;
-            float* cp = P.C + static_cast<size_t>(row) * P.ldc + cc;
-            float v = P.alpha * stage[rr * 33 + lane];
-            if (P.beta != 0.f) v += P.beta * *cp;
-            *cp = v;
-          }
-        }
-      }
-      __syncwarp();
-    }
-    return;
+  // Each 32 x 32 block is transposed through shared memory, so that a store
+  // instruction writes one 128-byte row segment: all 32 rows at once where
+  // the ring leaves 32 x 33 floats a warp (STAGE_C), else 8 rows at a time
+  // (lanes 8p..8p+7 hold rows 8p..8p+7).  A batch of rows' old values is read
+  // together before any store: one at a time, each read waited for the store
+  // before it (C may alias itself as far as the compiler knows), and storing
+  // straight from registers, a row per lane, touched 32 lines per instruction
+  // (4095 x 4097 x 1023, beta = 0.5: 459 -> 166 us of GEMM kernel).  Grouped
+  // launches keep the row loops rolled: their tiles are short, and unrolled
+  // this code, which runs once a tile, missed the instruction cache (5 to 10
+  // us a tile); one GEMM's long tiles rather want many reads in flight
+  // (8192^3 FP16x3: 1.84 ms unrolled, 1.97 rolled).
+  constexpr int SROWS = S::STAGE_C ? 32 : 8, BATCH = GROUPED || SROWS == 8 ? 8 : 16;
+  constexpr int kUnroll = GROUPED ? 1 : 4;
+  float* stage = stage_base + ew * SROWS * 33;
+  const int row0 = tc.m0 + q * 32;
+  float bl = 0.f;  // lane l: the bias of row row0 + l
+  if constexpr (EPI) {
+    if (P.epi.bias != nullptr && row0 + lane < P.M) bl = __ldg(P.epi.bias + row0 + lane);
   }
-  const int row = tc.m0 + q * 32 + lane;
-  if (row < P.M) {
-    float* crow = P.C + static_cast<size_t>(row) * P.ldc;
-    const int col0 = tc.n0 + col_off;
-    const bool vec = ((P.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(P.C) & 15) == 0);
-    if (has_epi) {
 #pragma unroll
-      for (int j = 0; j < HALF; ++j)
-        if (col0 + j < P.N) {
-          float v = P.alpha * acc[j];
-          if (P.beta != 0.f) v += P.beta * crow[col0 + j];
-          crow[col0 + j] = epilogue_apply(v, P.epi, row);
-        }
-    } else if (vec && col0 + HALF <= P.N) {
+  for (int c32 = 0; c32 < HALF / 32; ++c32) {
+    if (GROUPED && c32 * 32 >= n_live) break;
+    const int cc = tc.n0 + col_off + c32 * 32 + lane;
+    const bool live = cc < P.N;
+#pragma unroll kUnroll
+    for (int pass = 0; pass < 32 / SROWS; ++pass) {
+      if (row0 + pass * SROWS >= P.M) break;
+      float old[BATCH];
+      auto load_old = [&](int lr) {
+        const int rows = P.M - (row0 + lr);
+        const float* cp = P.C + static_cast<size_t>(row0 + lr) * P.ldc + cc;
 #pragma unroll
-      for (int j = 0; j < HALF; j += 4) {
-        float4 v = make_float4(P.alpha * acc[j], P.alpha * acc[j + 1], P.alpha * acc[j + 2],
-                               P.alpha * acc[j + 3]);
+        for (int rr = 0; rr < BATCH; ++rr) old[rr] = 0.f;
         if (P.beta != 0.f) {
-          const float4 o = *reinterpret_cast<const float4*>(crow + col0 + j);
-          v.x += P.beta * o.x; v.y += P.beta * o.y; v.z += P.beta * o.z; v.w += P.beta * o.w;
-        }
-        *reinterpret_cast<float4*>(crow + col0 + j) = v;
-      }
-    } else {
 #pragma unroll
-      for (int j = 0; j < HALF; ++j)
-        if (col0 + j < P.N) {
-          float v = P.alpha * acc[j];
-          if (P.beta != 0.f) v += P.beta * crow[col0 + j];
-          crow[col0 + j] = v;
+          for (int rr = 0; rr < BATCH; ++rr)
+            if (live && rr < rows) old[rr] = cp[static_cast<size_t>(rr) * P.ldc];
         }
+      };
+      if (!GROUPED && BATCH == SROWS) load_old(pass * SROWS);
+      if (SROWS == 32 || (lane >> 3) == pass) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) stage[(lane & (SROWS - 1)) * 33 + j] = acc[c32 * 32 + j];
+      }
+      __syncwarp();
+#pragma unroll kUnroll
+      for (int g = 0; g < SROWS; g += BATCH) {
+        const int lr = pass * SROWS + g, rows = P.M - (row0 + lr);
+        if (rows <= 0) break;
+        if (GROUPED || BATCH != SROWS) load_old(lr);
+        float* cp = P.C + static_cast<size_t>(row0 + lr) * P.ldc + cc;
+#pragma unroll
+        for (int rr = 0; rr < BATCH; ++rr) {
+          float x = scaled_sum(P, stage[(g + rr) * 33 + lane], old[rr]);
+          if constexpr (EPI) {
+            const float b = __shfl_sync(0xffffffffu, bl, lr + rr);
+            if (has_epi) x = epilogue_value(x, b, P.epi);
+          }
+          if (live && rr < rows) cp[static_cast<size_t>(rr) * P.ldc] = x;
+        }
+      }
+      __syncwarp();
     }
+  }
+}
+
+// Brings the old values of this warp's part of a tile of C (beta != 0) into
+// L2 when the tile starts, so that the epilogue, which cannot hold them in
+// registers, does not wait for DRAM once per block of rows (8192^3 FP16x3
+// with beta = 0.5: 2% of the step).
+template <int BN, bool GROUPED>
+__device__ __forceinline__ void prefetch_old_c(const TcProblem& P, const TileCoord& tc, int ew,
+                                               int warp, int lane) {
+  constexpr int HALF = BN / 2;
+  const int c0 = tc.n0 + (ew >> 2) * HALF, r = tc.m0 + (warp & 3) * 32;
+  auto pf = [](const float* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); };
+  if (GROUPED && P.swap) {
+    for (int j = lane; j < HALF && c0 + j < P.N; j += 32)
+      if (r < P.M) pf(P.C + static_cast<size_t>(c0 + j) * P.ldc + r);
+  } else if (r + lane < P.M) {
+    for (int j = 0; j < HALF && c0 + j < P.N; j += 32)
+      pf(P.C + static_cast<size_t>(r + lane) * P.ldc + c0 + j);
   }
 }
 
@@ -482,7 +486,7 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
 // rows, 64-byte swizzle), so the MMA issuer and the epilogue run unchanged
 // and the results are the same bits.
 template <int NP, int BN, bool GROUPED, bool EPI, bool TF32 = false, bool FUSED = false>
-__global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcThreads, 1)
+__global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1)
     split_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ TcProblem single, const CUtensorMap* __restrict__ maps,
                     const TcProblem* __restrict__ probs, const int4* __restrict__ tiles,
@@ -550,113 +554,123 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  // A 256-wide tile's epilogue holds 128 sums a thread: the four control
+  // warps (producer, issuer, two idle) give registers to the eight epilogue
+  // warps, instead of 168 each (at 168 the
+  // epilogue spilled 100 to 600 bytes a thread).  The hand-over opens each
+  // role's own branch: the compiler budgets the code it dominates.
+  constexpr int EW0 = FUSED ? 2 : 4;  // first epilogue warp
+  constexpr bool REGSPLIT = !FUSED && BN == 256;
 
-  if (FUSED && !DUAL && warp >= 2 + kTcEpiWarps) {
-    // ------------------------------------------------- fused converters
-    // threads of warps 12 and 13 first (see fused_convert)
-    static_assert(kTcConvWarps == 6 && 2 + kTcEpiWarps == 10, "converter warps 10-15");
-    if constexpr (FUSED && !DUAL)
-      fused_convert<NP, BN>(probs, tiles, smem, smem + NST * S::STAGE_BYTES, full, empty,
-                            raw_full, raw_empty, ((warp - 2 - kTcEpiWarps + 4) % 6) * 32 + lane,
-                            err);
-  } else if (FUSED && warp == 0) {
-    // ------------------------------------------- fused raw TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
-      uint8_t* raw = smem + NST * S::STAGE_BYTES;
-      for (int t = tr.first; ok && t < tr.end; t += tr.step) {
-        TcProblem P;
-        const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
-        const CUtensorMap* ma = &maps[2 * P.map];
-        const CUtensorMap* mb = &maps[2 * P.map + 1];
-        fence_tensormap(ma);
-        fence_tensormap(mb);
-        // each piece stage from kTcKB / RAW_K raw stages
-        for (int kr = 0; ok && kr < P.nkb * (kTcKB / S::RAW_K); ++kr, ++it) {
-          const int s = it % RST;
-          const uint32_t ph = (it / RST) & 1;
-          if (!mbar_wait(&raw_empty[s], ph ^ 1, err, kDevTimeoutEmpty)) { ok = false; break; }
-          uint8_t* ra = raw + s * S::RAW_BYTES;
-          const int k0 = P.kb0 * kTcKB + kr * S::RAW_K;
-          mbar_arrive_expect_tx(&raw_full[s], S::RAW_BYTES);
-          if (P.kc_a) tma_load_2d(ra, ma, &raw_full[s], k0, tc.m0);
-          else tma_load_2d(ra, ma, &raw_full[s], tc.m0, k0);
-          if (P.kc_b) tma_load_2d(ra + S::RAW_A, mb, &raw_full[s], k0, tc.n0);
-          else tma_load_2d(ra + S::RAW_A, mb, &raw_full[s], tc.n0, k0);
-        }
-      }
-      if (!ok) {  // let copies still in flight land before the CTA exits
-        for (uint32_t j = (it > uint32_t(RST) ? it - RST : 0); j < it; ++j)
-          mbar_wait(&raw_full[j % RST], (j / RST) & 1, nullptr, 0);
-      }
-    }
-  } else if (warp == 0) {
-    // ------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      if (!GROUPED) {
-        tma_prefetch_desc(&tmA);
-        tma_prefetch_desc(&tmB);
-      }
-      uint32_t it = 0;
-      bool ok = true;
-      const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
-      for (int t = tr.first; ok && t < tr.end; t += tr.step) {
-        TcProblem P;
-        const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
-        const CUtensorMap* ma = GROUPED ? &maps[2 * P.map] : &tmA;
-        const CUtensorMap* mb = GROUPED ? &maps[2 * P.map + 1] : &tmB;
-        if (GROUPED) {
+  auto control_and_converters = [&] {
+    if (FUSED && !DUAL && warp >= 2 + kTcEpiWarps) {
+      // ------------------------------------------------- fused converters
+      // threads of warps 12 and 13 first (see fused_convert)
+      static_assert(kTcConvWarps == 6 && 2 + kTcEpiWarps == 10, "converter warps 10-15");
+      if constexpr (FUSED && !DUAL)
+        fused_convert<NP, BN>(probs, tiles, smem, smem + NST * S::STAGE_BYTES, full, empty,
+                              raw_full, raw_empty, ((warp - 2 - kTcEpiWarps + 4) % 6) * 32 + lane,
+                              err);
+    } else if (FUSED && warp == 0) {
+      // ------------------------------------------- fused raw TMA producer
+      if (lane == 0) {
+        uint32_t it = 0;
+        bool ok = true;
+        const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
+        uint8_t* raw = smem + NST * S::STAGE_BYTES;
+        for (int t = tr.first; ok && t < tr.end; t += tr.step) {
+          TcProblem P;
+          const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+          const CUtensorMap* ma = &maps[2 * P.map];
+          const CUtensorMap* mb = &maps[2 * P.map + 1];
           fence_tensormap(ma);
           fence_tensormap(mb);
+          // each piece stage from kTcKB / RAW_K raw stages
+          for (int kr = 0; ok && kr < P.nkb * (kTcKB / S::RAW_K); ++kr, ++it) {
+            const int s = it % RST;
+            const uint32_t ph = (it / RST) & 1;
+            if (!mbar_wait(&raw_empty[s], ph ^ 1, err, kDevTimeoutEmpty)) { ok = false; break; }
+            uint8_t* ra = raw + s * S::RAW_BYTES;
+            const int k0 = P.kb0 * kTcKB + kr * S::RAW_K;
+            mbar_arrive_expect_tx(&raw_full[s], S::RAW_BYTES);
+            if (P.kc_a) tma_load_2d(ra, ma, &raw_full[s], k0, tc.m0);
+            else tma_load_2d(ra, ma, &raw_full[s], tc.m0, k0);
+            if (P.kc_b) tma_load_2d(ra + S::RAW_A, mb, &raw_full[s], k0, tc.n0);
+            else tma_load_2d(ra + S::RAW_A, mb, &raw_full[s], tc.n0, k0);
+          }
         }
-        const int kb0 = GROUPED ? P.kb0 : 0;  // first k-block of a split-K slice
-        constexpr int kx = TF32 ? KB / 2 : KB;  // elements of k per stage
-        for (int kb = 0; kb < P.nkb; ++kb, ++it) {
-          const int s = it % S::STAGES;
-          const uint32_t ph = (it / S::STAGES) & 1;
-          if (!mbar_wait(&empty[s], ph ^ 1, err, kDevTimeoutEmpty)) { ok = false; break; }
-          uint8_t* sa = smem + s * S::STAGE_BYTES;
-          mbar_arrive_expect_tx(&full[s], S::STAGE_BYTES);
-          tma_load_3d(sa, ma, &full[s], (kb0 + kb) * kx, tc.m0, 0);
-          tma_load_3d(sa + S::A_BYTES, mb, &full[s], (kb0 + kb) * kx, tc.n0, 0);
+        if (!ok) {  // let copies still in flight land before the CTA exits
+          for (uint32_t j = (it > uint32_t(RST) ? it - RST : 0); j < it; ++j)
+            mbar_wait(&raw_full[j % RST], (j / RST) & 1, nullptr, 0);
         }
       }
-      if (!ok) {  // let copies still in flight land before the CTA exits
-        for (uint32_t j = (it > uint32_t(S::STAGES) ? it - S::STAGES : 0); j < it; ++j)
-          mbar_wait(&full[j % S::STAGES], (j / S::STAGES) & 1, nullptr, 0);
+    } else if (warp == 0) {
+      // ------------------------------------------------------ TMA producer
+      if (lane == 0) {
+        if (!GROUPED) {
+          tma_prefetch_desc(&tmA);
+          tma_prefetch_desc(&tmB);
+        }
+        uint32_t it = 0;
+        bool ok = true;
+        const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
+        for (int t = tr.first; ok && t < tr.end; t += tr.step) {
+          TcProblem P;
+          const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+          const CUtensorMap* ma = GROUPED ? &maps[2 * P.map] : &tmA;
+          const CUtensorMap* mb = GROUPED ? &maps[2 * P.map + 1] : &tmB;
+          if (GROUPED) {
+            fence_tensormap(ma);
+            fence_tensormap(mb);
+          }
+          const int kb0 = GROUPED ? P.kb0 : 0;  // first k-block of a split-K slice
+          constexpr int kx = TF32 ? KB / 2 : KB;  // elements of k per stage
+          for (int kb = 0; kb < P.nkb; ++kb, ++it) {
+            const int s = it % S::STAGES;
+            const uint32_t ph = (it / S::STAGES) & 1;
+            if (!mbar_wait(&empty[s], ph ^ 1, err, kDevTimeoutEmpty)) { ok = false; break; }
+            uint8_t* sa = smem + s * S::STAGE_BYTES;
+            mbar_arrive_expect_tx(&full[s], S::STAGE_BYTES);
+            tma_load_3d(sa, ma, &full[s], (kb0 + kb) * kx, tc.m0, 0);
+            tma_load_3d(sa + S::A_BYTES, mb, &full[s], (kb0 + kb) * kx, tc.n0, 0);
+          }
+        }
+        if (!ok) {  // let copies still in flight land before the CTA exits
+          for (uint32_t j = (it > uint32_t(S::STAGES) ? it - S::STAGES : 0); j < it; ++j)
+            mbar_wait(&full[j % S::STAGES], (j / S::STAGES) & 1, nullptr, 0);
+        }
       }
+    } else if (warp == 1) {
+      // ------------------------------------------------------ MMA issuer
+      if (lane == 0) {
+        // the product count as a compile-time constant: two-piece forms have
+        // three products, three-piece ones six (BF16x6) or nine (BF16x9)
+        if constexpr (NP == 2)
+          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 3>(single, probs, tiles, total_tiles, smem,
+                                                          tmem, full, empty, main_full, main_empty,
+                                                          tile_full, tmem_empty, chunk_kb, fmt, err);
+        else if (nprod == 9)
+          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 9>(single, probs, tiles, total_tiles, smem,
+                                                          tmem, full, empty, main_full, main_empty,
+                                                          tile_full, tmem_empty, chunk_kb, fmt, err);
+        else
+          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 6>(single, probs, tiles, total_tiles, smem,
+                                                          tmem, full, empty, main_full, main_empty,
+                                                          tile_full, tmem_empty, chunk_kb, fmt, err);
+      }
+      __syncwarp();
+    } else if (DUAL) {
+      // ---------------------------------- epilogue warps that also convert
+      if constexpr (DUAL)
+        fused_dual<NP, BN, EPI>(probs, tiles, single.chunk_sums, smem, tmem, full, empty,
+                                raw_full, raw_empty, main_full, main_empty, tile_full, tmem_empty,
+                                stage_free, chunk_kb, warp, lane, err);
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      // the product count as a compile-time constant: two-piece forms have
-      // three products, three-piece ones six (BF16x6) or nine (BF16x9)
-      if constexpr (NP == 2)
-        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 3>(single, probs, tiles, total_tiles, smem,
-                                                        tmem, full, empty, main_full, main_empty,
-                                                        tile_full, tmem_empty, chunk_kb, fmt, err);
-      else if (nprod == 9)
-        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 9>(single, probs, tiles, total_tiles, smem,
-                                                        tmem, full, empty, main_full, main_empty,
-                                                        tile_full, tmem_empty, chunk_kb, fmt, err);
-      else
-        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 6>(single, probs, tiles, total_tiles, smem,
-                                                        tmem, full, empty, main_full, main_empty,
-                                                        tile_full, tmem_empty, chunk_kb, fmt, err);
-    }
-    __syncwarp();
-  } else if (DUAL) {
-    // ---------------------------------- epilogue warps that also convert
-    if constexpr (DUAL)
-      fused_dual<NP, BN, EPI>(probs, tiles, single.chunk_sums, smem, tmem, full, empty,
-                              raw_full, raw_empty, main_full, main_empty, tile_full, tmem_empty,
-                              stage_free, chunk_kb, warp, lane, err);
-  } else if (warp < 2 + kTcEpiWarps) {
+  };
+  auto epilogue = [&] {
     // ------------------------------------------------------ epilogue warps
     constexpr int HALF = BN / 2;  // columns per epilogue warp
-    const int ew = warp - 2;
+    const int ew = warp - EW0;
     const int q = warp & 3;       // TMEM lane quarter this warp may access
     const int col_off = (ew >> 2) * HALF;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
@@ -669,6 +683,7 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcThreads, 1)
       const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
       const uint32_t buf = ntile % NB, use = ntile / NB;
       const uint32_t t_buf = tmem + buf * 2 * BN + lane_base + col_off;
+      if (P.beta != 0.f) prefetch_old_c<BN, GROUPED>(P, tc, ew, warp, lane);
       float acc[HALF];
 #pragma unroll
       for (int j = 0; j < HALF; ++j) acc[j] = 0.f;
@@ -698,9 +713,16 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcThreads, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-      epi_store<NP, BN, GROUPED, EPI>(P, tc, acc, warp, lane,
+      epi_store<NP, BN, GROUPED, EPI>(P, tc, acc, ew, warp, lane,
                                       reinterpret_cast<float*>(smem + RING + 256));
     }
+  };
+  if (!DUAL && warp >= EW0 && warp < EW0 + kTcEpiWarps) {
+    if constexpr (REGSPLIT) setmaxnreg_inc<kTcEpilogueRegs<GROUPED>>();
+    epilogue();
+  } else {
+    if constexpr (REGSPLIT) setmaxnreg_dec<kTcControlRegs<GROUPED>>();
+    control_and_converters();
   }
 
   tc_fence_before();
@@ -1485,8 +1507,7 @@ __device__ __forceinline__ bool fused_dual_finish(const TcProblem P, const TileC
           const int c = c_base + j;
           if (c < P.N) {
             float* cp = P.C + static_cast<size_t>(c) * P.ldc + r;
-            float v = P.alpha * stage[lane * 65 + j];
-            if (P.beta != 0.f) v += P.beta * *cp;
+            float v = scaled_sum(P, stage[lane * 65 + j], P.beta != 0.f ? *cp : 0.f);
             if (has_epi) v = epilogue_apply(v, P.epi, c);
             *cp = v;
           }
@@ -1502,8 +1523,7 @@ __device__ __forceinline__ bool fused_dual_finish(const TcProblem P, const TileC
           const int row = row0 + rr;
           if (row >= P.M) break;
           float* cp = P.C + static_cast<size_t>(row) * P.ldc + c;
-          float v = P.alpha * stage[rr * 65 + c32 * 32 + lane];
-          if (P.beta != 0.f) v += P.beta * *cp;
+          float v = scaled_sum(P, stage[rr * 65 + c32 * 32 + lane], P.beta != 0.f ? *cp : 0.f);
           if (has_epi) v = epilogue_apply(v, P.epi, row);
           *cp = v;
         }
@@ -1732,10 +1752,18 @@ ugemm_status launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const T
   static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
   constexpr size_t kSmem = FUSED ? S::SMEM_FUSED : S::SMEM;
   static_assert(kSmem <= 232448, "shared memory budget");
+  if (!(attr_done.load(std::memory_order_acquire)) && !FUSED && BN == 256) {
+    // the kernel's register hand-over needs this many registers at launch
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kern) != cudaSuccess ||
+        (fa.numRegs + 7) / 8 * 8 * kTcSplitThreads <
+            128 * kTcControlRegs<GROUPED> + kTcEpiWarps * 32 * kTcEpilogueRegs<GROUPED>)
+      return UGEMM_ERR_CUDA;
+  }
   if (!smem_attr_once(kern, kSmem, attr_done)) return UGEMM_ERR_CUDA;
   const int grid = std::max(1, std::min(total_tiles, max_ctas > 0 ? max_ctas : sm_count()));
   prof_begin(st);
-  kern<<<grid, FUSED ? fused_threads(BN) : kTcThreads, kSmem, st>>>(
+  kern<<<grid, FUSED ? fused_threads(BN) : kTcSplitThreads, kSmem, st>>>(
       ta, tb, single, maps, probs, tiles, total_tiles, nprod, chunk_kb, fmt, dev_err);
   prof_end(st, GROUPED ? kProfGrouped : kProfSplitGemm);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;

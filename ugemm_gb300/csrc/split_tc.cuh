@@ -14,7 +14,17 @@ namespace ugemm {
 constexpr int kTcBM = 128;       // rows of C per CTA tile (UMMA M)
 constexpr int kTcKB = 32;        // k depth of one pipeline stage (64-byte bf16 rows)
 constexpr int kTcEpiWarps = 8;   // two per TMEM lane quarter
-constexpr int kTcThreads = (2 + kTcEpiWarps) * 32;
+constexpr int kTcThreads = (2 + kTcEpiWarps) * 32;       // 256-wide fused launches
+constexpr int kTcSplitThreads = (4 + kTcEpiWarps) * 32;  // launches on pieces: whole warpgroups,
+                                                         // so that registers can be shared out
+// 256-wide tiles: registers of a control and of an epilogue thread, 62,464 in
+// all of the launch's 384 x 168 = 64,512.  A grouped launch's producer and
+// issuer read problem records and want 72 (256-problem group: 125 us, 137 at
+// 40); one GEMM's need 40, and its epilogue reads C in larger batches.
+template <bool GROUPED>
+constexpr int kTcControlRegs = GROUPED ? 72 : 40;
+template <bool GROUPED>
+constexpr int kTcEpilogueRegs = GROUPED ? 208 : 224;
 // Fused launches (the operands split inside the GEMM kernel): warp 0's TMA
 // copies bring raw FP32 tiles of the operands into a ring of kTcRawStages
 // stages, which converter threads split into the three bf16 pieces of a
@@ -105,17 +115,14 @@ struct TcShape {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int FIT = (224 * 1024) / STAGE_BYTES;
   static constexpr int STAGES = FIT > 4 ? 4 : FIT;
-  // 128-wide tiles stage each epilogue warp's 32 x 32 output block in shared
-  // memory (padded rows) so C is written row by row, coalesced; 256-wide
-  // tiles have no room left and store straight from registers.
-  static constexpr bool STAGE_C = (BN == 128);
-  static constexpr size_t STAGE_C_BYTES = STAGE_C ? size_t(kTcEpiWarps) * 32 * 33 * 4 : 0;
-  // 256-wide tiles of grouped launches stage 8 rows x 32 columns per warp
-  // at a time: what the stage ring leaves of shared memory
-  static constexpr bool STAGE_C8 = (BN == 256);
-  static constexpr size_t STAGE_C8_BYTES = STAGE_C8 ? size_t(kTcEpiWarps) * 8 * 33 * 4 : 0;
+  // Each epilogue warp's 32 x 32 output blocks pass through shared memory so
+  // that C is written by rows: whole blocks (padded rows) where the stage
+  // ring leaves room -- 128-wide tiles, and 256-wide ones of two pieces --,
+  // 8 rows at a time for 256-wide tiles of three pieces.
+  static constexpr bool STAGE_C = (BN == 128 || NP == 2);
+  static constexpr size_t STAGE_C_BYTES = size_t(kTcEpiWarps) * (STAGE_C ? 32 : 8) * 33 * 4;
   static constexpr size_t SMEM =
-      1024 + size_t(STAGES) * STAGE_BYTES + 256 + STAGE_C_BYTES + STAGE_C8_BYTES;
+      1024 + size_t(STAGES) * STAGE_BYTES + 256 + STAGE_C_BYTES;
   // fused launches: kTcFusedPieceStages piece stages, then kTcRawStages raw
   // FP32 stages (the a tile, then the b tile, RAW_K deep)
   static constexpr int RAW_K = fused_raw_k(BN);
@@ -123,7 +130,7 @@ struct TcShape {
   static constexpr int RAW_BYTES = RAW_A + BN * RAW_K * 4;
   static constexpr size_t FUSED_RING =
       size_t(kTcFusedPieceStages) * STAGE_BYTES + size_t(kTcRawStages) * RAW_BYTES;
-  static constexpr size_t SMEM_FUSED = 1024 + FUSED_RING + 256 + STAGE_C_BYTES + STAGE_C8_BYTES;
+  static constexpr size_t SMEM_FUSED = 1024 + FUSED_RING + 256 + STAGE_C_BYTES;
   // main + correction accumulators, double-buffered across tiles when they fit
   static constexpr int ACC_BUFS = (4 * BN <= 512) ? 2 : 1;
   static constexpr uint32_t TMEM_COLS = ACC_BUFS * 2 * BN;
