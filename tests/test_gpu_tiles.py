@@ -1,0 +1,51 @@
+"""Tile choices and epilogues of the single-GEMM kernels at the sizes where
+they change: SIMT outputs of wide and narrow tiles mixed, split-form outputs
+whose rows of C are unaligned and updated (beta != 0), against the FP64 oracle.
+
+Normwise bound: a depth-K FP32 accumulation is within about sqrt(K) 2^-24 of
+FP64 (5e-7 at K = 70); 2e-6 is the suite's bound for both forms."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+import ugemm_gb300 as ug  # noqa: E402
+
+
+@pytest.fixture(scope="module", autouse=True)
+def gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    ug.build()
+    ug.load()
+
+
+def check(ta, tb, M, N, K, prec, beta=0.5, pad=0):
+    g = torch.Generator(device="cuda").manual_seed(M + 7 * N + 13 * K)
+    mat = lambda r, c: torch.rand((r, c), device="cuda", generator=g) * 2 - 1  # noqa: E731
+    A = mat(M, K) if ta == "N" else mat(K, M)
+    B = mat(K, N) if tb == "N" else mat(N, K)
+    buf = mat(M, N + pad)
+    C = buf[:, :N]
+    ref = ug.ref64(ta, tb, A, B, C.contiguous(), 1.5, beta)
+    rest = buf[:, N:].clone()
+    ug.gemm(A, B, C, ta=ta, tb=tb, alpha=1.5, beta=beta, precision=prec)
+    torch.cuda.synchronize()
+    assert float(torch.linalg.norm(C.double() - ref) / torch.linalg.norm(ref)) < 2e-6
+    assert torch.equal(buf[:, N:], rest)
+
+
+@pytest.mark.parametrize("ta,tb", ["NN", "NT", "TN", "TT"])
+@pytest.mark.parametrize("M,N,K", [(2500, 2300, 70),    # 180 wide tiles: 152, then 28 as 56 narrow
+                                   (20000, 129, 33),    # one and a bit narrow columns
+                                   (2049, 2561, 40),    # last wide tile row and column nearly empty
+                                   (19457, 300, 32)])   # 153 x 2 wide tiles: two left over
+def test_simt_wide_and_narrow_tiles(ta, tb, M, N, K):
+    check(ta, tb, M, N, K, "simt", pad=3)
+
+
+@pytest.mark.parametrize("prec", ["bf16x6", "fp16x3", "tf32x3"])
+@pytest.mark.parametrize("M,N,K,pad", [(257, 513, 96, 0), (129, 300, 33, 1), (300, 131, 64, 2),
+                                       (2049, 4097, 64, 0)])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_split_epilogue_unaligned_rows(prec, M, N, K, pad, beta):
+    check("T", "N", M, N, K, prec, beta, pad)

@@ -135,14 +135,15 @@ struct Scratch {
 };
 
 // Tile configurations of the SIMT kernel (rows x cols of C per CTA).
-// 128x128 and 64x64 use 8 compute warps plus a TMA producer warp; the "np"
-// configurations drop the producer warp (thread 0 issues the copies), which
-// lifts the per-thread register limit from 168 to 255.
+// 64x64 uses 8 compute warps plus a TMA producer warp; the others drop the
+// producer warp (thread 0 issues the copies), which lifts the per-thread
+// register limit from 168 to 255.  Grouped launches: 64x64 or 128x128, with a
+// producer warp.
 enum SimtTile : int {
-  kSimt128x128 = 0,
+  kSimt128x128 = 0,  // 8 x 8 per thread
   kSimt64x64 = 1,
-  kSimt128x256 = 2,    // 8 x 16 per thread, producer-less
-  kSimt128x128np = 3,  // 8 x 8 per thread, producer-less
+  kSimt128x256 = 2,  // 8 x 16 per thread
+  kSimtMixed = 3,    // 128x256, the last of them as 128x128 where that fills the SMs better
   kSimtTileCount = 4
 };
 

@@ -35,140 +35,169 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 // by TMA with CU_TENSOR_MAP_SWIZZLE_128B (address bits [4,7) ^= bits [7,10)).
 __device__ __forceinline__ int swz_chunk(int r, int q) { return q ^ (r & 7); }
 
-// One BM x BN tile's k loop, consuming the TMA ring from stage counter `it`
-// (which keeps running across the tiles of a persistent CTA).  AK: op(A) rows
-// are k-contiguous (ta == 'N').  BKM: op(B) columns are k-contiguous (tb == 'T').
+// Two FP32 accumulators side by side in one 64-bit register, and the packed
+// FMA that updates both (fma.rn.f32x2: each half rounds as fmaf does).  A
+// packed FMA takes one issue slot and one set of register reads for two
+// products, which leaves the issue slots that the fragment loads and the
+// moves need; scalar FMAs stalled at dispatch at 68% of the FMA pipe.
+using Acc2 = unsigned long long;
+__device__ __forceinline__ Acc2 pack2(float lo, float hi) {
+  Acc2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpack2(Acc2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma2(Acc2& acc, Acc2 a, Acc2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// Which dimension a pair of accumulators spans.  The operand whose fragment
+// already lies in register pairs (float4 loads of consecutive rows or columns)
+// is the paired one, and the other is broadcast, which costs nothing; pairs
+// assembled from two loads cost a move each (4096^3 NT: 35 TFLOP/s).  Where
+// both operands are k-contiguous, a pair is an even and an odd k of the same
+// element, added at the end: no moves, but twice the accumulators, so an 8 x 8
+// block is the largest.
+enum class Pair { kN, kM, kK };
+template <bool AK, bool BKM>
+constexpr Pair pair_of() { return !BKM ? Pair::kN : !AK ? Pair::kM : Pair::kK; }
+
+template <int TM, int TN, Pair P>
+struct AccTile {
+  static constexpr int R = P == Pair::kM ? TM / 2 : TM, C = P == Pair::kN ? TN / 2 : TN;
+  Acc2 v[R][C];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < C; ++j) v[i][j] = 0;
+  }
+  __device__ __forceinline__ float get(int i, int j) const {
+    float lo, hi;
+    unpack2(v[P == Pair::kM ? i / 2 : i][P == Pair::kN ? j / 2 : j], lo, hi);
+    if (P == Pair::kK) return lo + hi;
+    return ((P == Pair::kM ? i : j) & 1) ? hi : lo;
+  }
+};
+
+// One k-slice (kBK deep) of the register-blocked product, consumed from a
+// staged tile pair.  AK: op(A) rows are k-contiguous (ta == 'N').  BKM: op(B)
+// columns are k-contiguous (tb == 'T').  k-contiguous operands are read as
+// float4 of 4 k, eight columns of B at a time; the other layout is read per
+// k, so few fragment values are live beside the accumulators.
 template <int TM, int TN, bool AK, bool BKM>
-__device__ __forceinline__ bool simt_mainloop(const uint8_t* smem, uint64_t* full, uint64_t* empty,
-                                              int nkt, uint32_t& it, float (&acc)[TM][TN],
-                                              int* err) {
-  using S = SimtShape<TM, TN>;
-  constexpr int BM = S::BM, BN = S::BN;
-  const int tid = threadIdx.x, lane = tid & 31;
+__device__ __forceinline__ void simt_consume(const float* As, const float* Bs,
+                                             AccTile<TM, TN, pair_of<AK, BKM>()>& acc) {
+  constexpr Pair P = pair_of<AK, BKM>();
+  constexpr int BM = 16 * TM, BW = TN > 8 ? 128 : 16 * TN;  // BW: columns of a B box
+  constexpr int JG = BKM && TN > 8 ? 8 : TN;  // columns of a B fragment
+  constexpr bool A4 = AK || BKM;              // A's fragment covers the 4 k of a step
+  const int tid = threadIdx.x;
   const int ty = tid >> 4, tx = tid & 15;
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+  for (int q = 0; q < kBK / 4; ++q) {
+    float4 a4[A4 ? TM : 1];   // AK: [row] of 4 k; else [k][TM / 4] of 4 rows
+    auto load_a = [&](int kk, float4* v) {  // [32][BM]: rows 64 g + 4 ty + {0..3}
 #pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+      for (int g = 0; g < TM / 4; ++g)
+        v[g] = *reinterpret_cast<const float4*>(As + (4 * q + kk) * BM + 64 * g + 4 * ty);
+    };
+    if constexpr (AK) {  // [BM][32], 128-byte swizzled rows; thread rows ty + 16 i
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const int r = ty + 16 * i;
+        a4[i] = *reinterpret_cast<const float4*>(As + r * kBK + 4 * swz_chunk(ty, q));
+      }
+    } else if constexpr (A4) {
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) load_a(kk, a4 + kk * (TM / 4));
+    }
+    auto el = [](const float4& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
+#pragma unroll
+    for (int jg = 0; jg < TN / JG; ++jg) {
+      float4 b4[BKM ? JG : TN / 4];
+      if constexpr (BKM) {  // [BN][32], 128-byte swizzled rows; thread columns tx + 16 j
+#pragma unroll
+        for (int j = 0; j < JG; ++j) {
+          const int c = tx + 16 * (jg * JG + j);
+          b4[j] = *reinterpret_cast<const float4*>(Bs + c * kBK + 4 * swz_chunk(tx, q));
+        }
+      }
+      if constexpr (P == Pair::kK) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < TM; ++i) {
+            const Acc2 a2 = h == 0 ? pack2(a4[i].x, a4[i].y) : pack2(a4[i].z, a4[i].w);
+#pragma unroll
+            for (int j = 0; j < JG; ++j)
+              fma2(acc.v[i][jg * JG + j], a2,
+                   h == 0 ? pack2(b4[j].x, b4[j].y) : pack2(b4[j].z, b4[j].w));
+          }
+      } else {
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          float4 ak[TM / 4];
+          if constexpr (!A4) load_a(kk, ak);
+          if constexpr (P == Pair::kN) {
+            // [32][BN], 128 columns a box; thread columns 64 g + 4 tx + {0..3}
+#pragma unroll
+            for (int g = 0; g < TN / 4; ++g)
+              b4[g] = *reinterpret_cast<const float4*>(Bs + (g / 2) * 128 * kBK +
+                                                       (4 * q + kk) * BW + 64 * (g % 2) + 4 * tx);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+              const float v = AK ? el(a4[A4 ? i : 0], kk) : el(ak[i / 4], i % 4);
+              const Acc2 a2 = pack2(v, v);
+#pragma unroll
+              for (int j = 0; j < TN / 2; ++j)
+                fma2(acc.v[i][j], a2, j % 2 == 0 ? pack2(b4[j / 2].x, b4[j / 2].y)
+                                                 : pack2(b4[j / 2].z, b4[j / 2].w));
+            }
+          } else {  // Pair::kM: rows from a4, columns broadcast
+#pragma unroll
+            for (int j = 0; j < JG; ++j) {
+              const float v = el(b4[j], kk);
+              const Acc2 b2 = pack2(v, v);
+#pragma unroll
+              for (int i = 0; i < TM / 2; ++i) {
+                const float4& x = a4[A4 ? kk * (TM / 4) + i / 2 : 0];
+                fma2(acc.v[i][jg * JG + j], i % 2 == 0 ? pack2(x.x, x.y) : pack2(x.z, x.w), b2);
+              }
+            }
+          }
+        }
+      }
+    }
+  }
+}
+
+// One BM x BN tile's k loop, consuming the TMA ring from stage counter `it`
+// (which keeps running across the tiles of a persistent CTA).
+template <int TM, int TN, bool AK, bool BKM>
+__device__ __forceinline__ bool simt_mainloop(const uint8_t* smem, uint64_t* full, uint64_t* empty,
+                                              int nkt, uint32_t& it,
+                                              AccTile<TM, TN, pair_of<AK, BKM>()>& acc, int* err) {
+  using S = SimtShape<TM, TN>;
+  const int lane = threadIdx.x & 31;
+  acc.clear();
   for (int kt = 0; kt < nkt; ++kt, ++it) {
     const int s = it % kStages;
-    const uint32_t ph = (it / kStages) & 1;
-    if (!mbar_wait(&full[s], ph, err, kDevTimeoutFull)) return false;
+    if (!mbar_wait(&full[s], (it / kStages) & 1, err, kDevTimeoutFull)) return false;
     const float* As = reinterpret_cast<const float*>(smem + s * S::STAGE_BYTES);
-    const float* Bs = reinterpret_cast<const float*>(smem + s * S::STAGE_BYTES + S::A_BYTES);
-#pragma unroll
-    for (int q = 0; q < kBK / 4; ++q) {
-      float a[TM][4], bf[TN][4];
-      if (AK) {  // As[BM][32], 128-byte swizzled rows; thread rows ty + 16 i
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-          const int r = ty + 16 * i;
-          const float4 v = *reinterpret_cast<const float4*>(As + r * kBK + 4 * swz_chunk(r, q));
-          a[i][0] = v.x; a[i][1] = v.y; a[i][2] = v.z; a[i][3] = v.w;
-        }
-      } else {   // As[32][BM]; thread rows 64 g + 4 ty + {0..3}
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-          for (int g = 0; g < TM / 4; ++g) {
-            const float4 v =
-                *reinterpret_cast<const float4*>(As + (4 * q + kk) * BM + 64 * g + 4 * ty);
-            a[4 * g + 0][kk] = v.x; a[4 * g + 1][kk] = v.y;
-            a[4 * g + 2][kk] = v.z; a[4 * g + 3][kk] = v.w;
-          }
-      }
-      if (BKM) {  // Bs[BN][32], 128-byte swizzled rows; thread cols tx + 16 j
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          const int c = tx + 16 * j;
-          const float4 v = *reinterpret_cast<const float4*>(Bs + c * kBK + 4 * swz_chunk(c, q));
-          bf[j][0] = v.x; bf[j][1] = v.y; bf[j][2] = v.z; bf[j][3] = v.w;
-        }
-      } else {    // Bs[32][BN]; thread cols 64 g + 4 tx + {0..3}
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-          for (int g = 0; g < TN / 4; ++g) {
-            const float4 v =
-                *reinterpret_cast<const float4*>(Bs + (4 * q + kk) * BN + 64 * g + 4 * tx);
-            bf[4 * g + 0][kk] = v.x; bf[4 * g + 1][kk] = v.y;
-            bf[4 * g + 2][kk] = v.z; bf[4 * g + 3][kk] = v.w;
-          }
-      }
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i][kk], bf[j][kk], acc[i][j]);
-    }
+    simt_consume<TM, TN, AK, BKM>(As, As + S::A_BYTES / 4, acc);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   }
   return true;
 }
 
-// One k-slice (kBK deep) of the register-blocked product, consumed from a
-// staged tile pair.  k-contiguous operands are read as float4 of 4 k; the
-// other layout is read per k so only TN (or TM) values are live at a time.
-template <int TM, int TN, bool AK, bool BKM>
-__device__ __forceinline__ void simt_consume(const float* As, const float* Bs, float (&acc)[TM][TN]) {
-  constexpr int BM = 16 * TM, BN = 16 * TN;
-  const int tid = threadIdx.x;
-  const int ty = tid >> 4, tx = tid & 15;
-#pragma unroll
-  for (int q = 0; q < kBK / 4; ++q) {
-    float a[TM][4], bq[BKM ? TN : 1][4];
-    if (AK) {
-#pragma unroll
-      for (int i = 0; i < TM; ++i) {
-        const int r = ty + 16 * i;
-        const float4 v = *reinterpret_cast<const float4*>(As + r * kBK + 4 * swz_chunk(r, q));
-        a[i][0] = v.x; a[i][1] = v.y; a[i][2] = v.z; a[i][3] = v.w;
-      }
-    }
-    if (BKM) {
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const int c = tx + 16 * j;
-        const float4 v = *reinterpret_cast<const float4*>(Bs + c * kBK + 4 * swz_chunk(c, q));
-        bq[j][0] = v.x; bq[j][1] = v.y; bq[j][2] = v.z; bq[j][3] = v.w;
-      }
-    }
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-      float av[TM], bv[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) av[i] = AK ? a[i][kk] : 0.f;
-      if (!AK) {
-#pragma unroll
-        for (int g = 0; g < TM / 4; ++g) {
-          const float4 v = *reinterpret_cast<const float4*>(As + (4 * q + kk) * BM + 64 * g + 4 * ty);
-          av[4 * g] = v.x; av[4 * g + 1] = v.y; av[4 * g + 2] = v.z; av[4 * g + 3] = v.w;
-        }
-      }
-      if (BKM) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j) bv[j] = bq[j][kk];
-      } else {
-#pragma unroll
-        for (int g = 0; g < TN / 4; ++g) {
-          const float4 v = *reinterpret_cast<const float4*>(Bs + (4 * q + kk) * BN + 64 * g + 4 * tx);
-          bv[4 * g] = v.x; bv[4 * g + 1] = v.y; bv[4 * g + 2] = v.z; bv[4 * g + 3] = v.w;
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-    }
-  }
-}
-
 // alpha/beta epilogue of one tile from registers; C is not read when beta == 0.
 template <int TM, int TN, bool AK, bool BKM>
-__device__ __forceinline__ void simt_store(const float (&acc)[TM][TN], float* C, int M, int N,
-                                           int ldc, float alpha, float beta, int m0, int n0,
+__device__ __forceinline__ void simt_store(const AccTile<TM, TN, pair_of<AK, BKM>()>& tile,
+                                           float* C, int M, int N, int ldc, float alpha, float beta, int m0, int n0,
                                            const Epilogue& epi) {
   const int tid = threadIdx.x;
   const int ty = tid >> 4, tx = tid & 15;
@@ -178,12 +207,15 @@ __device__ __forceinline__ void simt_store(const float (&acc)[TM][TN], float* C,
     const int row = m0 + (AK ? ty + 16 * i : 64 * (i / 4) + 4 * ty + (i % 4));
     if (row >= M) continue;
     float* crow = C + static_cast<size_t>(row) * ldc;
+    float acc[TN];
+#pragma unroll
+    for (int j = 0; j < TN; ++j) acc[j] = tile.get(i, j);
     if (BKM) {
 #pragma unroll
       for (int j = 0; j < TN; ++j) {
         const int col = n0 + tx + 16 * j;
         if (col < N) {
-          float v = alpha * acc[i][j];
+          float v = alpha * acc[j];
           if (beta != 0.f) v += beta * crow[col];
           crow[col] = epilogue_apply(v, epi, row);
         }
@@ -193,8 +225,8 @@ __device__ __forceinline__ void simt_store(const float (&acc)[TM][TN], float* C,
       for (int g = 0; g < TN / 4; ++g) {
         const int col = n0 + 64 * g + 4 * tx;
         if (vec && col + 3 < N) {
-          float4 v = make_float4(alpha * acc[i][4 * g], alpha * acc[i][4 * g + 1],
-                                 alpha * acc[i][4 * g + 2], alpha * acc[i][4 * g + 3]);
+          float4 v = make_float4(alpha * acc[4 * g], alpha * acc[4 * g + 1],
+                                 alpha * acc[4 * g + 2], alpha * acc[4 * g + 3]);
           if (beta != 0.f) {
             const float4 o = *reinterpret_cast<const float4*>(crow + col);
             v.x += beta * o.x; v.y += beta * o.y; v.z += beta * o.z; v.w += beta * o.w;
@@ -206,7 +238,7 @@ __device__ __forceinline__ void simt_store(const float (&acc)[TM][TN], float* C,
 #pragma unroll
           for (int jj = 0; jj < 4; ++jj)
             if (col + jj < N) {
-              float v = alpha * acc[i][4 * g + jj];
+              float v = alpha * acc[4 * g + jj];
               if (beta != 0.f) v += beta * crow[col + jj];
               crow[col + jj] = epilogue_apply(v, epi, row);
             }
@@ -226,7 +258,7 @@ __device__ __forceinline__ void raster_tile(int local, int tiles_m, int tiles_n,
 }
 
 template <int TM, int TN, bool AK, bool BKM>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 2)
     simt_sgemm_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB, float* __restrict__ C, int M,
                       int N, int K, int ldc, float alpha, float beta, Epilogue epi, int tiles_m,
@@ -270,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     return;
   }
-  float acc[TM][TN];
+  AccTile<TM, TN, pair_of<AK, BKM>()> acc;
   uint32_t it = 0;
   if (!simt_mainloop<TM, TN, AK, BKM>(smem, full, empty, nkt, it, acc, err)) return;
   simt_store<TM, TN, AK, BKM>(acc, C, M, N, ldc, alpha, beta, m0, n0, epi);
@@ -278,34 +310,39 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // Producer-less variant: 8 warps only.  With no ninth warp every thread may
 // hold up to 255 registers (a ninth warp caps each scheduler's share at 168),
-// room for the 8 x 16 register block that halves shared-memory wavefronts per
-// FMA.  Thread 0 issues the TMA for stage kt + S - 1 once all warps released
-// the stage they consumed at kt - 1.
+// room for the 8 x 16 register block.  Thread 0 issues the TMA for stage
+// kt + S - 1 once all warps released the stage they consumed at kt - 1.
+//
+// What bounds it: a 128-bit shared load costs a warp four wavefronts, so an
+// 8 x 8 block (16 words read for 64 FMAs) keeps the shared-memory pipe as
+// busy as the FMA pipe and both reach about 70%; an 8 x 16 block reads 24
+// words for 128 FMAs, three quarters of that.  128 x 256 tiles are coarse,
+// so the last of them, which would not fill a wave of SMs, run as two
+// 128 x 128 tiles each (CTAs from `wide_tiles` on).
 template <int TM, int TN, bool AK, bool BKM>
-__global__ void __launch_bounds__(kConsumerWarps * 32, 1)
-    simt_sgemm_np_kernel(const __grid_constant__ CUtensorMap tmA,
-                         const __grid_constant__ CUtensorMap tmB, float* __restrict__ C, int M,
-                         int N, int K, int ldc, float alpha, float beta, Epilogue epi,
-                         int tiles_m, int tiles_n, int* err) {
+__device__ __forceinline__ void simt_np_tile(uint8_t* smem, const CUtensorMap& tmA,
+                                             const CUtensorMap& tmB, float* __restrict__ C, int M,
+                                             int N, int K, int ldc, float alpha, float beta,
+                                             const Epilogue& epi, int m0, int n0, int* err) {
   using S = SimtShape<TM, TN>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = align1024(smem_raw);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * S::STAGE_BYTES);
+  using W = SimtShape<8, 16>;  // the ring's layout (and the barriers') is the wide tile's
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * W::STAGE_BYTES);
   uint64_t* empty = full + kStages;
-  int tile_m, tile_n;
-  raster_tile(blockIdx.x, tiles_m, tiles_n, tile_m, tile_n);
-  const int m0 = tile_m * S::BM, n0 = tile_n * S::BN;
   const int nkt = (K + kBK - 1) / kBK;
   const int tid = threadIdx.x, lane = tid & 31;
   auto issue = [&](int kt) {
     const int s = kt % kStages;
-    uint8_t* sa = smem + s * S::STAGE_BYTES;
+    uint8_t* sa = smem + s * W::STAGE_BYTES;
     uint8_t* sb = sa + S::A_BYTES;
     mbar_arrive_expect_tx(&full[s], S::STAGE_BYTES);
     if (AK) tma_load_2d(sa, &tmA, &full[s], kt * kBK, m0);
     else    tma_load_2d(sa, &tmA, &full[s], m0, kt * kBK);
-    if (BKM) tma_load_2d(sb, &tmB, &full[s], kt * kBK, n0);
-    else     tma_load_2d(sb, &tmB, &full[s], n0, kt * kBK);
+    // B's map has boxes of 128 columns, one or two to a tile
+#pragma unroll
+    for (int h = 0; h < S::BN / 128; ++h) {
+      if (BKM) tma_load_2d(sb + h * 128 * kBK * 4, &tmB, &full[s], kt * kBK, n0 + 128 * h);
+      else     tma_load_2d(sb + h * 128 * kBK * 4, &tmB, &full[s], n0 + 128 * h, kt * kBK);
+    }
   };
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -318,11 +355,8 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     for (int kt = 0; kt < min(kStages - 1, nkt); ++kt) issue(kt);  // first use of each stage
   }
   __syncthreads();
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  AccTile<TM, TN, pair_of<AK, BKM>()> acc;
+  acc.clear();
   for (int kt = 0; kt < nkt; ++kt) {
     if (tid == 0) {
       const int kn = kt + kStages - 1;
@@ -334,13 +368,38 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     }
     const int s = kt % kStages;
     if (!mbar_wait(&full[s], (kt / kStages) & 1, err, kDevTimeoutFull)) return;
-    const float* As = reinterpret_cast<const float*>(smem + s * S::STAGE_BYTES);
-    const float* Bs = reinterpret_cast<const float*>(smem + s * S::STAGE_BYTES + S::A_BYTES);
-    simt_consume<TM, TN, AK, BKM>(As, Bs, acc);
+    const float* As = reinterpret_cast<const float*>(smem + s * W::STAGE_BYTES);
+    simt_consume<TM, TN, AK, BKM>(As, As + S::A_BYTES / 4, acc);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   }
   simt_store<TM, TN, AK, BKM>(acc, C, M, N, ldc, alpha, beta, m0, n0, epi);
+}
+
+template <bool AK, bool BKM>
+__global__ void __launch_bounds__(kConsumerWarps * 32, 1)
+    simt_sgemm_np_kernel(const __grid_constant__ CUtensorMap tmA,
+                         const __grid_constant__ CUtensorMap tmB, float* __restrict__ C, int M,
+                         int N, int K, int ldc, float alpha, float beta, Epilogue epi,
+                         int tiles_m, int tiles_n, int wide_tiles, int* err) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = align1024(smem_raw);
+  // tiles_m x tiles_n tiles of 128 x 256 in raster order
+  const int b = blockIdx.x;
+  int tile_m, tile_n;
+  if (b < wide_tiles) {
+    if constexpr (pair_of<AK, BKM>() != Pair::kK) {
+      raster_tile(b, tiles_m, tiles_n, tile_m, tile_n);
+      simt_np_tile<8, 16, AK, BKM>(smem, tmA, tmB, C, M, N, K, ldc, alpha, beta, epi,
+                                   tile_m * 128, tile_n * 256, err);
+    }
+  } else {
+    raster_tile(wide_tiles + (b - wide_tiles) / 2, tiles_m, tiles_n, tile_m, tile_n);
+    const int n0 = tile_n * 256 + ((b - wide_tiles) & 1) * 128;
+    if (n0 < N)
+      simt_np_tile<8, 8, AK, BKM>(smem, tmA, tmB, C, M, N, K, ldc, alpha, beta, epi, tile_m * 128,
+                                  n0, err);
+  }
 }
 
 // Persistent grouped SIMT GEMM: one CTA per SM walks the tiles of all
@@ -410,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     SimtProblem P;
     int p, m0, n0;
     locate(t, P, p, m0, n0);
-    float acc[TM][TN];
+    AccTile<TM, TN, Pair::kN> acc;
     if (!simt_mainloop<TM, TN, false, false>(smem, full, empty, P.nkt, it, acc, err)) return;
     simt_store<TM, TN, false, false>(acc, P.C, P.M, P.N, P.ldc, P.alpha, P.beta, m0, n0, P.epi);
   }
@@ -515,45 +574,86 @@ void stored_b(const Gemm& g, int& rows, int& cols) {
   if (g.tb == 'N') { rows = g.K; cols = g.N; } else { rows = g.N; cols = g.K; }
 }
 
-template <int TM, int TN, bool AK, bool BKM, bool NP>
-ugemm_status launch_t(const Gemm& g, const float* A, int lda, const float* B, int ldb,
-                      int* dev_err, cudaStream_t st) {
-  using S = SimtShape<TM, TN>;
-  CUtensorMap ta, tb;
-  bool ok;
-  if (AK) ok = encode_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, A, g.K, g.M, lda * 4ull,
-                              kBK, S::BM, CU_TENSOR_MAP_SWIZZLE_128B);
-  else    ok = encode_tmap_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, A, g.M, g.K, lda * 4ull,
-                              S::BM, kBK, CU_TENSOR_MAP_SWIZZLE_NONE);
-  if (!ok) return UGEMM_ERR_CUDA;
-  if (BKM) ok = encode_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, B, g.K, g.N, ldb * 4ull,
-                               kBK, S::BN, CU_TENSOR_MAP_SWIZZLE_128B);
-  else     ok = encode_tmap_2d(&tb, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, B, g.N, g.K, ldb * 4ull,
-                               S::BN, kBK, CU_TENSOR_MAP_SWIZZLE_NONE);
-  if (!ok) return UGEMM_ERR_CUDA;
-  void (*kern)(const CUtensorMap, const CUtensorMap, float*, int, int, int, int, float, float,
-               Epilogue, int, int, int*);
-  if constexpr (NP) kern = simt_sgemm_np_kernel<TM, TN, AK, BKM>;
-  else kern = simt_sgemm_kernel<TM, TN, AK, BKM>;
-  const int threads = NP ? kConsumerWarps * 32 : kThreads;
-  static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
-  if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
-  const int tiles_m = cdiv(g.M, S::BM), tiles_n = cdiv(g.N, S::BN);
-  prof_begin(st);
-  kern<<<tiles_m * tiles_n, threads, S::SMEM, st>>>(ta, tb, g.C, g.M, g.N, g.K, g.ldc, g.alpha,
-                                                     g.beta, g.epi, tiles_m, tiles_n, dev_err);
-  prof_end(st, kProfSimt);
-  return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
+int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return 148;
+  return sms;
 }
 
-template <int TM, int TN, bool NP>
-ugemm_status launch_tile(const Gemm& g, const float* A, int lda, const float* B, int ldb,
-                         int* dev_err, cudaStream_t st) {
-  const bool ak = g.ta == 'N', bk = g.tb == 'T';
-  if (ak && !bk) return launch_t<TM, TN, true, false, NP>(g, A, lda, B, ldb, dev_err, st);
-  if (ak && bk) return launch_t<TM, TN, true, true, NP>(g, A, lda, B, ldb, dev_err, st);
-  if (!ak && !bk) return launch_t<TM, TN, false, false, NP>(g, A, lda, B, ldb, dev_err, st);
-  return launch_t<TM, TN, false, true, NP>(g, A, lda, B, ldb, dev_err, st);
+// The producer-less kernel's tiles for an M x N output.  A wave of 128 x 128
+// tiles takes kNarrowCost of a wave of 128 x 256 tiles (97 and 174 us per 1024
+// k; pairs along k have no wide tiles).  Wide tiles fill whole waves of SMs;
+// what is left of them runs as narrow ones when those fit in one wave, and
+// everything runs narrow where that takes fewer waves' time (a right edge that
+// leaves half of the wide tiles empty).
+constexpr double kNarrowCost = 0.56;
+// 64 x 64 tiles, two CTAs to an SM: 69 us per 1024 k and round of two to an SM.
+constexpr double kSmallCost = 0.40, kSmallHalfCost = 0.29;
+struct NpTiles {
+  int tiles_m, tiles_n, wide;  // 128 x 256 tiles, and how many run as such
+  double cost;                 // waves, in wide tiles
+};
+NpTiles np_tiles(int M, int N, bool wide_ok, int sms) {
+  NpTiles t{cdiv(M, 128), cdiv(N, 256), 0, 0};
+  const int total = t.tiles_m * t.tiles_n, rest = total % sms;
+  const bool tail = rest > 0 && 2 * rest <= sms;
+  const double mixed = total / sms + (rest == 0 ? 0.0 : tail ? kNarrowCost : 1.0);
+  const double narrow = kNarrowCost * cdiv(t.tiles_m * cdiv(N, 128), sms);
+  t.wide = !wide_ok || narrow < mixed ? 0 : tail ? total - rest : total;
+  t.cost = wide_ok ? std::min(narrow, mixed) : narrow;
+  return t;
+}
+
+// Boxes of 32 k by rows_a rows of op(A), rows_b columns of op(B).
+template <bool AK, bool BKM>
+bool encode_operands(const Gemm& g, const float* A, int lda, const float* B, int ldb, int rows_a,
+                     int rows_b, CUtensorMap* ta, CUtensorMap* tb) {
+  const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  return (AK ? encode_tmap_2d(ta, f32, 4, A, g.K, g.M, lda * 4ull, kBK, rows_a,
+                              CU_TENSOR_MAP_SWIZZLE_128B)
+             : encode_tmap_2d(ta, f32, 4, A, g.M, g.K, lda * 4ull, rows_a, kBK,
+                              CU_TENSOR_MAP_SWIZZLE_NONE)) &&
+         (BKM ? encode_tmap_2d(tb, f32, 4, B, g.K, g.N, ldb * 4ull, kBK, rows_b,
+                               CU_TENSOR_MAP_SWIZZLE_128B)
+              : encode_tmap_2d(tb, f32, 4, B, g.N, g.K, ldb * 4ull, rows_b, kBK,
+                               CU_TENSOR_MAP_SWIZZLE_NONE));
+}
+
+// tile: kSimt64x64 (a producer warp), or the producer-less kernel.
+template <bool AK, bool BKM>
+ugemm_status launch_t(const Gemm& g, int tile, const float* A, int lda, const float* B, int ldb,
+                      int* dev_err, cudaStream_t st) {
+  CUtensorMap ta, tb;
+  if (tile == kSimt64x64) {
+    using S = SimtShape<4, 4>;
+    if (!encode_operands<AK, BKM>(g, A, lda, B, ldb, S::BM, S::BN, &ta, &tb)) return UGEMM_ERR_CUDA;
+    auto kern = simt_sgemm_kernel<4, 4, AK, BKM>;
+    static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
+    if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
+    const int tiles_m = cdiv(g.M, S::BM), tiles_n = cdiv(g.N, S::BN);
+    prof_begin(st);
+    kern<<<tiles_m * tiles_n, kThreads, S::SMEM, st>>>(ta, tb, g.C, g.M, g.N, g.K, g.ldc, g.alpha,
+                                                       g.beta, g.epi, tiles_m, tiles_n, dev_err);
+  } else {
+    using S = SimtShape<8, 16>;
+    if (!encode_operands<AK, BKM>(g, A, lda, B, ldb, 128, 128, &ta, &tb)) return UGEMM_ERR_CUDA;
+    auto kern = simt_sgemm_np_kernel<AK, BKM>;
+    static std::atomic<uint64_t> attr_done{0};
+    if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
+    constexpr bool wide_ok = pair_of<AK, BKM>() != Pair::kK;
+    NpTiles t = np_tiles(g.M, g.N, wide_ok, sm_count());
+    const int total = t.tiles_m * t.tiles_n;
+    if (tile == kSimt128x128) t.wide = 0;
+    if (tile == kSimt128x256 && wide_ok) t.wide = total;
+    prof_begin(st);
+    kern<<<t.wide + 2 * (total - t.wide), kConsumerWarps * 32, S::SMEM, st>>>(
+        ta, tb, g.C, g.M, g.N, g.K, g.ldc, g.alpha, g.beta, g.epi, t.tiles_m, t.tiles_n, t.wide,
+        dev_err);
+  }
+  prof_end(st, kProfSimt);
+  return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }
 
 }  // namespace
@@ -567,22 +667,20 @@ size_t simt_scratch_bytes(const Gemm& g) {
 }
 
 int simt_pick_tile(const Gemm& g) {
-  int sms = 148;
-  int dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess)
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  static int forced = -2;
-  if (forced == -2) {
+  static const int forced = [] {
     const char* e = std::getenv("UGEMM_SIMT_TILE");
-    forced = e ? std::atoi(e) : -1;
-    if (forced >= kSimtTileCount) forced = -1;
-  }
+    const int v = e ? std::atoi(e) : -1;
+    return v >= 0 && v < kSimtTileCount ? v : -1;
+  }();
   if (forced >= 0) return forced;
-  // Measured on GB300 at 8192^3: the producer-less 128x128 kernel is 3-18%
-  // faster than the one with a producer warp in every transpose pair; 64x64
-  // tiles win when 128x128 tiles cannot fill two waves.
-  const long big = long(cdiv(g.M, 128)) * cdiv(g.N, 128);
-  return big >= 2L * sms ? kSimt128x128np : kSimt64x64;
+  // whichever needs less time by the waves' measured costs (2048^3 NN: 348 us
+  // mixed, 464 in 64x64 tiles; 1024^3: 99 and 74)
+  const int sms = sm_count();
+  const long small = long(cdiv(g.M, 64)) * cdiv(g.N, 64);
+  const double small_cost =
+      small <= sms ? kSmallHalfCost : kSmallCost * ((small + 2 * sms - 1) / (2 * sms));
+  const bool wide_ok = !(g.ta == 'N' && g.tb == 'T');
+  return np_tiles(g.M, g.N, wide_ok, sms).cost < small_cost ? kSimtMixed : kSimt64x64;
 }
 
 ugemm_status simt_launch(const Gemm& g, int tile, Scratch ws, int* dev_err, cudaStream_t st) {
@@ -616,12 +714,11 @@ ugemm_status simt_launch(const Gemm& g, int tile, Scratch ws, int* dev_err, cuda
     prof_end(st, kProfAux);
     B = dst; ldb = ld; used += need;
   }
-  switch (tile) {
-    case kSimt64x64: return launch_tile<4, 4, false>(g, A, lda, B, ldb, dev_err, st);
-    case kSimt128x256: return launch_tile<8, 16, true>(g, A, lda, B, ldb, dev_err, st);
-    case kSimt128x128np: return launch_tile<8, 8, true>(g, A, lda, B, ldb, dev_err, st);
-    default: return launch_tile<8, 8, false>(g, A, lda, B, ldb, dev_err, st);
-  }
+  const bool ak = g.ta == 'N', bk = g.tb == 'T';
+  if (ak && !bk) return launch_t<true, false>(g, tile, A, lda, B, ldb, dev_err, st);
+  if (ak && bk) return launch_t<true, true>(g, tile, A, lda, B, ldb, dev_err, st);
+  if (!ak && !bk) return launch_t<false, false>(g, tile, A, lda, B, ldb, dev_err, st);
+  return launch_t<false, true>(g, tile, A, lda, B, ldb, dev_err, st);
 }
 
 ugemm_status scale_c_launch(const Gemm& g, cudaStream_t st) {
@@ -653,10 +750,7 @@ ugemm_status grouped_t(const CUtensorMap* maps, const SimtProblem* probs, int np
   auto kern = simt_grouped_kernel<TM, TN>;
   static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
   if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
-  int sms = 148, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::max(1, std::min(total, max_ctas > 0 ? max_ctas : sms));
+  const int grid = std::max(1, std::min(total, max_ctas > 0 ? max_ctas : sm_count()));
   prof_begin(st);
   kern<<<grid, kThreads, S::SMEM, st>>>(maps, probs, nprob, total, dev_err);
   prof_end(st, kProfGrouped);
@@ -674,11 +768,8 @@ ugemm_status simt_grouped_launch(int tile, const CUtensorMap* maps, const SimtPr
 
 ugemm_status pack_batched_launch(const PackJob* jobs, int njobs, int total_tiles, cudaStream_t st) {
   if (total_tiles <= 0) return UGEMM_OK;
-  int sms = 148, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   prof_begin(st);
-  pack_kmajor_batched_kernel<<<std::min(total_tiles, sms * 8), 256, 0, st>>>(jobs, njobs,
+  pack_kmajor_batched_kernel<<<std::min(total_tiles, sm_count() * 8), 256, 0, st>>>(jobs, njobs,
                                                                              total_tiles);
   prof_end(st, kProfSplitPrep);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
