@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "split_tc.cuh"
 
 namespace ugemm {
 namespace {
@@ -198,13 +199,28 @@ struct ugemm_conv_stack_s {
     bool direct_dx = false;
     float* wt = nullptr;  // cin x cout*k*k
     ugemm::Im2col dy_im;  // im2col geometry of dY for that GEMM
+    // Layers whose GEMMs read their operands as bf16 pieces written once per
+    // activation (three-piece forms): X and dY as NHWC pieces, from which
+    // TMA's im2col mode reads the im2col matrices of the forward, dX and dW
+    // GEMMs, and the weights in (tap, channel) order.
+    bool tap_fwd = false, tap_bwd = false;
+    void *xp = nullptr, *wp = nullptr, *wbp = nullptr;  // wbp: the backward GEMM's weights
+    ugemm::PieceOperands fwd_q, dw_q, dx_q;
     ugemm_grouped_plan* fwd = nullptr;
     ugemm_grouped_plan* bwd = nullptr;
   };
+  // Split launches of a run: jobs [first, first + njobs) of the device list.
+  struct Phase {
+    int first = 0, njobs = 0, tiles = 0, tiles_first = 0;  // tiles_first: of the first job alone
+    bool taps = false;                                     // has (tap, channel) jobs
+  };
+  std::vector<Phase> split_fwd, split_bwd;  // per layer: X (or col); dY, then X
+  Phase split_w, split_wb;                  // every layer's weights
+  const ugemm::SplitJob* jobs = nullptr;    // in `pieces`
+  void* pieces = nullptr;                   // pieces of X, W, dY; the job list
   std::vector<Layer> layers;
   int batch = 0, form = UGEMM_PREC_BF16X6;
   bool explicit_col = false;  // UGEMM_CONV_IM2COL: materialise col per layer
-  float* dy_last = nullptr;
   void* arena = nullptr;
   double flops_fwd = 0, flops_bwd = 0;
   cudaGraphExec_t exec[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -214,20 +230,37 @@ struct ugemm_conv_stack_s {
 namespace {
 using Stack = ugemm_conv_stack_s;
 
+ugemm_status split_phase(const Stack* s, const Stack::Phase& ph, int njobs,
+                                  cudaStream_t st) {
+  if (njobs == 0) return UGEMM_OK;
+  const ugemm::SplitJob* jobs = s->jobs + ph.first;
+  const int tiles = njobs == ph.njobs ? ph.tiles : ph.tiles_first;
+  return ph.taps ? ugemm::split_taps_launch(jobs, njobs, tiles, st)
+                 : ugemm::split_batched_launch(3, jobs, njobs, tiles, st);
+}
+
 int run_stack(Stack* s, int what, cudaStream_t st) {
   using namespace ugemm;
+  ugemm_status r;
   if (what & UGEMM_CONV_FORWARD) {
-    for (auto& L : s->layers) {
+    r = split_phase(s, s->split_w, s->split_w.njobs, st);
+    if (r != UGEMM_OK) return r;
+    for (size_t l = 0; l < s->layers.size(); ++l) {
+      auto& L = s->layers[l];
       if (s->explicit_col) {
-        ugemm_status r = im2col_launch(L.x, L.d.cin, s->batch, L.d.height, L.d.width, L.d.ksize,
-                                       L.d.pad, L.d.stride, L.col, st);
+        r = im2col_launch(L.x, L.d.cin, s->batch, L.d.height, L.d.width, L.d.ksize, L.d.pad,
+                          L.d.stride, L.col, st);
         if (r != UGEMM_OK) return r;
       }
+      r = split_phase(s, s->split_fwd[l], s->split_fwd[l].njobs, st);
+      if (r != UGEMM_OK) return r;
       int rc = ugemm_grouped_run(L.fwd, st);
       if (rc != UGEMM_OK) return rc;
     }
   }
   if (what & UGEMM_CONV_BACKWARD) {
+    r = split_phase(s, s->split_wb, s->split_wb.njobs, st);
+    if (r != UGEMM_OK) return r;
     for (int l = static_cast<int>(s->layers.size()) - 1; l >= 0; --l) {
       auto& L = s->layers[l];
       if (L.d.act) {  // dY *= LeakyReLU'(Y); dbias = row sums
@@ -238,15 +271,20 @@ int run_stack(Stack* s, int what, cudaStream_t st) {
         prof_end(st, kProfAux);
         if (cudaPeekAtLastError() != cudaSuccess) return UGEMM_ERR_CUDA;
       }
-      if (L.direct_dx) {
-        ugemm_status r = flip_weights_launch(L.w, L.d.cout, L.d.cin, L.d.ksize, L.wt, st);
+      if (L.tap_bwd) {
+        // dY's pieces; X's too unless this run's forward half wrote them
+        const int n = what & UGEMM_CONV_FORWARD ? 1 : s->split_bwd[l].njobs;
+        r = split_phase(s, s->split_bwd[l], n, st);
+        if (r != UGEMM_OK) return r;
+      } else if (L.direct_dx) {
+        r = flip_weights_launch(L.w, L.d.cout, L.d.cin, L.d.ksize, L.wt, st);
         if (r != UGEMM_OK) return r;
       }
       int rc = ugemm_grouped_run(L.bwd, st);
       if (rc != UGEMM_OK) return rc;
       if (!L.direct_dx) {
-        ugemm_status r = col2im_launch(L.dcol, L.d.cin, s->batch, L.d.height, L.d.width,
-                                       L.d.ksize, L.d.pad, L.d.stride, L.dx, st);
+        r = col2im_launch(L.dcol, L.d.cin, s->batch, L.d.height, L.d.width, L.d.ksize, L.d.pad,
+                          L.d.stride, L.dx, st);
         if (r != UGEMM_OK) return r;
       }
     }
@@ -265,7 +303,150 @@ void destroy_stack(Stack* s) {
     if (L.bwd) ugemm_grouped_plan_destroy(L.bwd);
   }
   if (s->arena) cudaFree(s->arena);
+  if (s->pieces) cudaFree(s->pieces);
   delete s;
+}
+
+// Whether C channels, each tap's padded to 32, make an im2col operand worth
+// reading tap by tap (at most half of k' is padding; fewer channels gather
+// from X instead), within the limits of an im2col tensor map.
+bool taps_ok(int C, int k, int pad, int stride) {
+  return 2 * static_cast<int>(ugemm::align_up(C, 32)) <= 3 * C && k <= 16 && pad <= 16 &&
+         stride <= 8;
+}
+
+// Lays out and fills the pieces buffer and the split jobs of the layers that
+// take their operands as pieces, and points their PieceOperands at them.  The
+// forward GEMM's k order, (tap, channel), follows from the layer's sizes alone,
+// so that an explicit stack (which splits the stored im2col matrix in that
+// order) computes the same bits.  dW needs 64-channel blocks (at most half of
+// its columns padding).
+ugemm_status make_pieces(Stack* s) {
+  using namespace ugemm;
+  const int nl = static_cast<int>(s->layers.size());
+  s->split_fwd.resize(nl);
+  s->split_bwd.resize(nl);
+  if (s->form != UGEMM_PREC_BF16X6 && s->form != UGEMM_PREC_BF16X9) return UGEMM_OK;
+  auto pad32 = [](int c) { return static_cast<int>(align_up(c, 32)); };
+  size_t bytes = 0;
+  auto take = [&](long long rows, long long kp) {
+    const size_t o = bytes;
+    bytes += align_up(size_t(3) * rows * kp * 2, 256);
+    return o;
+  };
+  std::vector<size_t> xo(nl, 0), wo(nl, 0), bo(nl, 0);
+  size_t dy_bytes = 0, col_bytes = 0;
+  for (int l = 0; l < nl; ++l) {
+    auto& L = s->layers[l];
+    const auto& d = L.d;
+    const int kk = d.ksize * d.ksize;
+    const long long in_px = static_cast<long long>(s->batch) * d.height * d.width;
+    if (in_px > 0x7fffffffLL) continue;
+    L.tap_fwd = taps_ok(d.cin, d.ksize, d.pad, d.stride);
+    L.tap_bwd = L.tap_fwd && !s->explicit_col && d.cin > 32 &&
+                static_cast<int>(align_up(d.cin, 64)) <= 2 * d.cin &&
+                (!L.direct_dx || taps_ok(d.cout, d.ksize, d.ksize - 1 - d.pad, 1));
+    if (L.tap_fwd) {
+      wo[l] = take(d.cout, static_cast<long long>(kk) * pad32(d.cin));
+      if (s->explicit_col)
+        col_bytes = std::max<size_t>(col_bytes, size_t(6) * L.n * kk * pad32(d.cin));
+      else
+        xo[l] = take(in_px, pad32(d.cin));
+    }
+    if (L.tap_bwd) {
+      bo[l] = L.direct_dx ? take(d.cin, static_cast<long long>(kk) * pad32(d.cout))
+                          : take(L.kdim, pad32(d.cout));
+      dy_bytes = std::max<size_t>(dy_bytes, size_t(6) * L.n * pad32(d.cout));
+    }
+  }
+  const size_t dy_off = bytes;  // dY's (or col's) pieces, one layer's at a time
+  bytes += align_up(std::max(dy_bytes, col_bytes), 256);
+  const size_t jobs_off = bytes;
+  bytes += 5 * size_t(nl) * sizeof(SplitJob);
+  if (jobs_off == 0) return UGEMM_OK;  // no such layer
+  if (cudaMalloc(&s->pieces, bytes) != cudaSuccess) {
+    s->pieces = nullptr;
+    return UGEMM_ERR_ALLOC;
+  }
+  uint8_t* base = static_cast<uint8_t*>(s->pieces);
+  std::vector<SplitJob> jobs;
+  auto add = [&](Stack::Phase& ph, SplitJob j) {
+    if (ph.njobs == 0) ph.first = static_cast<int>(jobs.size());
+    j.tile_start = ph.tiles;
+    ph.tiles += split_job_tiles(j);
+    if (ph.njobs++ == 0) ph.tiles_first = ph.tiles;
+    ph.taps |= j.gather != 0;
+    jobs.push_back(j);
+  };
+  // rows x K as stored with rows contiguous (ld between k): K-major pieces
+  auto rows_job = [&](const float* src, long long ld, int rows, int K, void* dst) {
+    return SplitJob{src, 1, ld, static_cast<__nv_bfloat16*>(dst), rows, K, pad32(K), 0};
+  };
+  auto taps_job = [&](const float* src, long long sr, long long sk, int rows, int chans, int kk,
+                      int flip, void* dst) {
+    const int kp = kk * pad32(chans);
+    SplitJob j{src, sr, sk, static_cast<__nv_bfloat16*>(dst), rows, kp, kp, 0};
+    j.gather = 3;
+    j.kk = kk;
+    j.chans = chans;
+    j.cp = pad32(chans);
+    j.flip = flip;
+    return j;
+  };
+  for (int l = 0; l < nl; ++l) {
+    auto& L = s->layers[l];
+    if (!L.tap_fwd) continue;
+    const int kk = L.d.ksize * L.d.ksize;
+    L.wp = base + wo[l];
+    add(s->split_w, taps_job(L.w, L.kdim, kk, L.d.cout, L.d.cin, kk, 0, L.wp));
+  }
+  for (int l = 0; l < nl; ++l) {
+    auto& L = s->layers[l];
+    if (!L.tap_bwd) continue;
+    const int kk = L.d.ksize * L.d.ksize;
+    L.wbp = base + bo[l];
+    add(s->split_wb, L.direct_dx
+                         ? taps_job(L.w, kk, L.kdim, L.d.cin, L.d.cout, kk, 1, L.wbp)
+                         : rows_job(L.w, L.kdim, L.kdim, L.d.cout, L.wbp));
+  }
+  for (int l = 0; l < nl; ++l) {
+    auto& L = s->layers[l];
+    const auto& d = L.d;
+    const int kk = d.ksize * d.ksize, in_px = s->batch * d.height * d.width;
+    const int n = static_cast<int>(L.n);
+    void* shared = base + dy_off;
+    SplitJob xj{};
+    if (L.tap_fwd && !s->explicit_col) {
+      L.xp = base + xo[l];
+      xj = rows_job(L.x, in_px, in_px, d.cin, L.xp);
+      add(s->split_fwd[l], xj);
+      L.fwd_q = PieceOperands{PieceOperands::kTaps, L.wp, L.xp, kk * pad32(d.cin), L.im};
+    } else if (L.tap_fwd) {
+      SplitJob j{L.col, n, 0, static_cast<__nv_bfloat16*>(shared), n, kk * pad32(d.cin),
+                 kk * pad32(d.cin), 0};
+      j.gather = 4;
+      j.kk = kk;
+      j.chans = d.cin;
+      j.cp = pad32(d.cin);
+      add(s->split_fwd[l], j);
+      L.fwd_q = PieceOperands{PieceOperands::kPlain, L.wp, shared, kk * pad32(d.cin), L.im};
+    }
+    if (L.tap_bwd) {
+      const float* dy = l + 1 < nl ? s->layers[l + 1].dx : L.y;
+      add(s->split_bwd[l], rows_job(dy, n, n, d.cout, shared));
+      add(s->split_bwd[l], xj);
+      L.dw_q = PieceOperands{PieceOperands::kPix, shared, L.xp, 0, L.im};
+      L.dx_q = L.direct_dx ? PieceOperands{PieceOperands::kTaps, L.wbp, shared,
+                                           kk * pad32(d.cout), L.dy_im}
+                           : PieceOperands{PieceOperands::kPlain, L.wbp, shared, pad32(d.cout),
+                                           L.im};
+    }
+  }
+  s->jobs = reinterpret_cast<const SplitJob*>(base + jobs_off);
+  return cudaMemcpy(base + jobs_off, jobs.data(), jobs.size() * sizeof(SplitJob),
+                    cudaMemcpyHostToDevice) == cudaSuccess
+             ? UGEMM_OK
+             : UGEMM_ERR_CUDA;
 }
 }  // namespace
 
@@ -335,7 +516,7 @@ UGEMM_API int ugemm_conv_stack_create(int nlayers, const ugemm_conv_layer* layer
     if (L.n > 0x7fffffffLL) { destroy_stack(s); return UGEMM_ERR_ARG; }
     s->layers.push_back(L);
   }
-  // arena: x0 | per layer {col, w, y, dw, dcol, dx} | dy_last
+  // arena: x0 | per layer {col, w, y, dw, dcol or wt, dx, bias, dbias}
   const size_t x0 = take(size_t(layers[0].cin) * batch * layers[0].height * layers[0].width);
   for (auto& L : s->layers) {
     off.push_back(s->explicit_col ? take(size_t(L.kdim) * L.n) : 0);  // col
@@ -367,15 +548,20 @@ UGEMM_API int ugemm_conv_stack_create(int nlayers, const ugemm_conv_layer* layer
   }
   for (size_t l = 0; l < s->layers.size(); ++l) {
     auto& L = s->layers[l];
-    const float* dy = (l + 1 < s->layers.size()) ? s->layers[l + 1].dx : nullptr;
-    if (!dy) {
-      s->dy_last = L.y;  // the last layer's output buffer doubles as its incoming gradient slot
-      dy = nullptr;
-    }
-    const int M = L.d.cout, N = static_cast<int>(L.n), K = L.kdim;
-    // forward: y = w * col
+    const float* g = l + 1 < s->layers.size() ? s->layers[l + 1].dx : L.y;
     L.im = make_im2col(L.x, L.d.cin, batch, L.d.height, L.d.width, L.d.ksize, L.d.pad,
                        L.d.stride, L.Ho, L.Wo);
+    if (L.direct_dx)
+      L.dy_im = make_im2col(g, L.d.cout, batch, L.Ho, L.Wo, L.d.ksize, L.d.ksize - 1 - L.d.pad, 1,
+                            L.d.height, L.d.width);
+  }
+  {
+    const ugemm_status rc = make_pieces(s);
+    if (rc != UGEMM_OK) { destroy_stack(s); return rc; }
+  }
+  for (size_t l = 0; l < s->layers.size(); ++l) {
+    auto& L = s->layers[l];
+    const int M = L.d.cout, N = static_cast<int>(L.n), K = L.kdim;
     // col = im2col(x): the materialised buffer, or read from x by the
     // GEMMs' operand pass
     const Im2col* im = s->explicit_col ? nullptr : &L.im;
@@ -383,22 +569,25 @@ UGEMM_API int ugemm_conv_stack_create(int nlayers, const ugemm_conv_layer* layer
     Gemm f{'N', 'N', M, N, K, 1.f, 0.f, L.w, K, L.col, N, L.y, N};
     f.epi = Epilogue{L.d.act ? L.bias : nullptr, L.d.act, L.d.slope};
     f.b_im2col = im;
+    if (L.tap_fwd) f.pieces = &L.fwd_q;
     // backward: dw = dy * col^T, and dcol = w^T * dy (dX = col2im(dcol)) or,
     // for a direct layer, dX = wt * im2col(dY; pad k-1-p): the adjoint of a
     // stride-1 convolution is the convolution of dY with the weights
     // transposed in the channels and flipped in the taps
-    const float* g = dy ? dy : L.y;
+    const float* g = l + 1 < s->layers.size() ? s->layers[l + 1].dx : L.y;
     Gemm b[2] = {Gemm{'N', 'T', M, K, N, 1.f, 0.f, g, N, L.col, N, L.dw, K},
                  Gemm{'T', 'N', K, N, M, 1.f, 0.f, L.w, K, g, N, L.dcol, N}};
     b[0].b_im2col = im;
     if (L.direct_dx) {
       const int kk = L.d.ksize * L.d.ksize;
       const int npix = batch * L.d.height * L.d.width;
-      L.dy_im = make_im2col(g, L.d.cout, batch, L.Ho, L.Wo, L.d.ksize, L.d.ksize - 1 - L.d.pad, 1,
-                            L.d.height, L.d.width);
       b[1] = Gemm{'N', 'N', L.d.cin, npix, L.d.cout * kk, 1.f, 0.f, L.wt, L.d.cout * kk, nullptr,
                   npix, L.dx, npix};
       b[1].b_im2col = &L.dy_im;
+    }
+    if (L.tap_bwd) {
+      b[0].pieces = &L.dw_q;
+      b[1].pieces = &L.dx_q;
     }
     ugemm_status rc = grouped_plan_build(&f, 1, s->form, nullptr, 0, &L.fwd);
     if (rc == UGEMM_OK) rc = grouped_plan_build(b, 2, s->form, nullptr, 0, &L.bwd);

@@ -29,14 +29,23 @@ namespace ugemm {
 namespace {
 
 // Split-K reduction: C = sum_s part_s + beta*C (C not read when beta == 0),
-// then the optional bias / activation; slices summed in a fixed order.
+// then the optional bias / activation; slices summed in a fixed order.  Partial
+// tiles whose columns are (tap, channel) are read in their own order and
+// written in C's (channel, tap).
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const ReduceJob* __restrict__ jobs) {
   const ReduceJob J = jobs[blockIdx.y];
-  const long long mn = static_cast<long long>(J.M) * J.N;
+  const int pn = J.kk > 0 ? J.kk * J.cpad : J.N;  // columns of a partial tile
+  const long long mn = static_cast<long long>(J.M) * pn;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < mn; i += 256LL * gridDim.x) {
+    const int m = static_cast<int>(i / pn);
+    int n = static_cast<int>(i - static_cast<long long>(m) * pn);
+    if (J.kk > 0) {
+      const int tap = n / J.cpad, c = n - tap * J.cpad;
+      if (c >= J.chans) continue;
+      n = c * J.kk + tap;
+    }
     float v = 0.f;
     for (int s = 0; s < J.slices; ++s) v += J.part[s * mn + i];
-    const int m = static_cast<int>(i / J.N), n = static_cast<int>(i % J.N);
     float* cp = J.C + static_cast<long long>(m) * J.ldc + n;
     if (J.beta != 0.f) v += J.beta * *cp;
     *cp = epilogue_apply(v, J.epi, m);
@@ -68,6 +77,7 @@ struct ugemm_grouped_plan_s {
   void* scratch = nullptr;  // operand slots
   int* dev_err = nullptr;
   const CUtensorMap* maps = nullptr;
+  const ugemm::ConvGeo* geo = nullptr;  // PieceOperands plans: one per kernel problem
   const void* probs = nullptr;
   const void* jobs = nullptr;
   int njobs = 0, prep_tiles = 0, gemm_tiles = 0;
@@ -122,7 +132,7 @@ ugemm_status launch_plan(ugemm_grouped_plan_s* p, cudaStream_t st) {
   s = split_gemm_launch(p->split, dummy, dummy, single, p->maps,
                         static_cast<const TcProblem*>(p->probs), p->tiles, p->gemm_tiles,
                         split_chunk_stages(p->split.pieces, std::max(1, p->cfg.chunk_k / kTcKB)),
-                        p->grid, p->dev_err, st);
+                        p->grid, p->dev_err, st, p->geo);
   return s == UGEMM_OK ? reduce_launch(p, st) : s;
 }
 
@@ -144,7 +154,7 @@ bool fused_operand_map(const float* base, long long sr, long long sk, int rows, 
 // problem's operands may be empty); implicit im2col gathers take the
 // pre-pass.
 bool fusable(const Gemm& x) {
-  if (x.K == 0 || x.b_im2col) return false;
+  if (x.K == 0 || x.b_im2col || x.pieces) return false;
   long long a_sr, a_sk, b_sr, b_sk;
   split_operand_strides(x, &a_sr, &a_sk, &b_sr, &b_sk);
   auto ok = [](const float* p, long long sr, long long sk) {
@@ -152,6 +162,14 @@ bool fusable(const Gemm& x) {
     return (sr == 1 || sk == 1) && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0;
   };
   return ok(x.A, a_sr, a_sk) && ok(x.B, b_sr, b_sk);
+}
+
+// Columns of C as the kernel computes it: a kPix problem's are (tap, channel)
+// with each tap's channels padded to 64.
+int kernel_cols(const Gemm& x) {
+  return x.pieces && x.pieces->kind == PieceOperands::kPix
+             ? x.pieces->im.k * x.pieces->im.k * static_cast<int>(align_up(x.pieces->im.C, 64))
+             : x.N;
 }
 
 // Padded tile area of an R x C output in 128 x bn tiles whose right-edge
@@ -251,9 +269,10 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     // tiles with the staged epilogue and narrow-N MMAs win (144 vs 162 us).
     if (form != UGEMM_PREC_SIMT) {
       int widest = 0;
-      for (const Gemm& x : g)
-        widest = std::max(widest,
-                          padded_area(x.N, x.M, 128) < padded_area(x.M, x.N, 128) ? x.M : x.N);
+      for (const Gemm& x : g) {
+        const int n = kernel_cols(x);
+        widest = std::max(widest, padded_area(n, x.M, 128) < padded_area(x.M, n, 128) ? x.M : n);
+      }
       if (widest <= 128) p->cfg.block_n = 128;
     }
   }
@@ -282,6 +301,11 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     p->split.block_n = bn;
     p->split.fused = p->cfg.fused != 0;
     pieces = p->split.pieces;
+    p->split.conv = g[0].pieces != nullptr;
+    if (p->split.conv && pieces != 3) {
+      free_plan(p);
+      return plan_fail(UGEMM_ERR_ARG, "operand pieces: three-piece forms only");
+    }
   }
   // Kernel geometry of each problem (in k-depth order j).  The split form
   // computes C^T = op(B)^T op(A)^T when that wastes less of its 128-row
@@ -291,6 +315,7 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     bool swap = false;
     int tiles = 0, nkb = 0;  // output tiles, k-blocks (32 deep)
     int slices = 1, per = 0; // split-K slices and their length in k-blocks
+    bool sliced = false;     // through partial tiles and a reduce
   };
   std::vector<Geo> geo(count);
   double work = 0;
@@ -301,10 +326,12 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       o.tiles = cdiv(x.M, bn) * cdiv(x.N, bn);
       o.nkb = std::max(1, cdiv(x.K, kBK));
     } else {
-      o.swap = p->cfg.transpose == 0 && padded_area(x.N, x.M, bn) < padded_area(x.M, x.N, bn);
-      const int rows = o.swap ? x.N : x.M, cols = o.swap ? x.M : x.N;
+      const int n = kernel_cols(x);
+      o.swap = p->cfg.transpose == 0 && padded_area(n, x.M, bn) < padded_area(x.M, n, bn);
+      const int rows = o.swap ? n : x.M, cols = o.swap ? x.M : n;
       o.tiles = cdiv(rows, kTcBM) * cdiv(cols, bn);
-      o.nkb = split_nkb(pieces, x.K);
+      o.nkb = split_nkb(pieces, x.pieces && x.pieces->kind != PieceOperands::kPix ? x.pieces->kp
+                                                                                   : x.K);
     }
     o.per = o.nkb;
     work += double(o.tiles) * o.nkb;
@@ -326,12 +353,19 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   for (int j = 0; j < count; ++j) {
     const Gemm& x = g[order[j]];
     Geo& o = geo[j];
-    if (x.K == 0 || o.nkb < 2 * min_slice || o.nkb <= fair) continue;
-    const int len = std::max(min_slice, static_cast<int>(fair) + 1);
-    const size_t tile_bytes = size_t(x.M) * x.N * 4;
-    int sl = std::min(cdiv(o.nkb, len), 256);
-    sl = static_cast<int>(std::min<size_t>(sl, (size_t(1) << 30) / tile_bytes));
-    if (sl < 2) continue;
+    // a kPix problem always goes through partial tiles: the reduce puts its
+    // columns in C's order
+    o.sliced = x.pieces && x.pieces->kind == PieceOperands::kPix;
+    const size_t tile_bytes = size_t(x.M) * kernel_cols(x) * 4;
+    int sl = 1;
+    if (x.K != 0 && o.nkb >= 2 * min_slice && o.nkb > fair) {
+      const int len = std::max(min_slice, static_cast<int>(fair) + 1);
+      sl = std::min(cdiv(o.nkb, len), 256);
+      sl = static_cast<int>(std::min<size_t>(sl, (size_t(1) << 30) / tile_bytes));
+    }
+    if (sl >= 2) o.sliced = true;
+    else sl = 1;
+    if (!o.sliced) continue;
     o.per = cdiv(o.nkb, sl);
     o.slices = cdiv(o.nkb, o.per);
     part_off[j] = part_bytes;
@@ -352,8 +386,8 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       scratch += align_up(size_t(std::max(x.K, 1)) * ld_a[j] * 4, 256);
       b_off[j] = scratch;
       scratch += align_up(size_t(std::max(x.K, 1)) * ld_b[j] * 4, 256);
-    } else if (p->split.fused) {
-      b_off[j] = scratch;  // no pieces in memory: the kernel splits the operands
+    } else if (p->split.fused || x.pieces) {
+      b_off[j] = scratch;  // no pieces in memory, or the caller's
     } else {
       scratch += split_operand_bytes(pieces, x.M, x.K);
       b_off[j] = scratch;
@@ -384,6 +418,7 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   int prep = 0;
   for (int j = 0; j < count; ++j) {
     const Gemm& x = g[order[j]];
+    if (x.pieces) continue;  // written by the caller
     long long a_sr, a_sk, b_sr, b_sk;
     split_operand_strides(x, &a_sr, &a_sk, &b_sr, &b_sk);
     // an implicit im2col B: rows of op(B)^T are pixels ('N') or taps ('T');
@@ -424,7 +459,9 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     }
   std::stable_sort(subs.begin(), subs.end(), [](const Sub& a, const Sub& b) { return a.nkb > b.nkb; });
 
-  std::vector<CUtensorMap> maps(2 * subs.size());
+  const bool conv = !simt && p->split.conv;
+  std::vector<CUtensorMap> maps((conv ? 4 : 2) * subs.size());
+  std::vector<ConvGeo> cgeo(conv ? subs.size() : 0);
   std::vector<TcProblem> tprobs;
   std::vector<SimtProblem> sprobs;
   std::vector<ReduceJob> rjobs;
@@ -435,11 +472,12 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     const Gemm& x = g[order[u.j]];
     const Geo& o = geo[u.j];
     // a slice writes alpha * (its partial product) to its partial tile set
-    const bool sliced = o.slices > 1;
+    const bool sliced = o.sliced;
+    const int ncols = kernel_cols(x);
     float* target = sliced ? reinterpret_cast<float*>(base + part_base + part_off[u.j]) +
-                                 size_t(u.slice) * x.M * x.N
+                                 size_t(u.slice) * x.M * ncols
                            : x.C;
-    const int ldt = sliced ? x.N : x.ldc;
+    const int ldt = sliced ? ncols : x.ldc;
     const float beta = sliced ? 0.f : x.beta;
     const Epilogue epi = sliced ? Epilogue{} : x.epi;
     any_epi |= epi.bias != nullptr || epi.act != 0;
@@ -456,7 +494,9 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       sprobs.push_back(sp);
     } else {
       TcProblem tp{};
-      if (p->split.fused) {
+      if (conv) {
+        ok = conv_encode_maps(*x.pieces, x.M, ncols, bn, o.swap, &maps[4 * i], &cgeo[i]);
+      } else if (p->split.fused) {
         // the kernel copies the FP32 operands; its operand a is op(B)^T
         // when the problem is computed transposed
         long long a_sr, a_sk, b_sr, b_sk;
@@ -479,8 +519,8 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
                                         &maps[2 * i + 1]);
       }
       tp.C = target;
-      tp.M = o.swap ? x.N : x.M;
-      tp.N = o.swap ? x.M : x.N;
+      tp.M = o.swap ? ncols : x.M;
+      tp.N = o.swap ? x.M : ncols;
       tp.ldc = ldt;
       tp.alpha = x.alpha;
       tp.beta = beta;
@@ -500,14 +540,20 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       return plan_fail(UGEMM_ERR_CUDA, "tensor map encoding failed");
     }
     if (sliced && u.slice == 0) {
-      rjobs.push_back(ReduceJob{target, x.C, x.M, x.N, x.ldc, o.slices, x.beta, x.epi});
-      p->reduce_max = std::max(p->reduce_max, static_cast<long long>(x.M) * x.N);
+      ReduceJob rj{target, x.C, x.M, x.N, x.ldc, o.slices, x.beta, x.epi};
+      if (conv && x.pieces->kind == PieceOperands::kPix) {
+        rj.kk = x.pieces->im.k * x.pieces->im.k;
+        rj.cpad = ncols / rj.kk;
+        rj.chans = x.pieces->im.C;
+      }
+      rjobs.push_back(rj);
+      p->reduce_max = std::max(p->reduce_max, static_cast<long long>(x.M) * ncols);
     }
   }
   if (!simt) p->split.epi = any_epi;
   p->gemm_tiles = tiles;
   p->prep_tiles = prep;
-  p->njobs = 2 * count;
+  p->njobs = static_cast<int>(simt ? pjobs.size() : sjobs.size());
   p->nsub = static_cast<int>(subs.size());
   p->nreduce = static_cast<int>(rjobs.size());
 
@@ -532,7 +578,9 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   const bool f16 = !simt && p->split.f16;
   std::vector<size_t> word_off(sjobs.size() + 1, 0);
   for (size_t q = 0; q < sjobs.size(); ++q) word_off[q + 1] = word_off[q] + sjobs[q].rows;
-  const size_t off_w = off_t + align_up(std::max<size_t>(rec_bytes, 1), 256);
+  const size_t off_g = off_t + align_up(std::max<size_t>(rec_bytes, 1), 256);
+  const size_t geo_bytes = cgeo.size() * sizeof(ConvGeo);
+  const size_t off_w = off_g + align_up(std::max<size_t>(geo_bytes, 1), 256);
   const size_t total =
       off_w + (f16 ? align_up(std::max<size_t>(word_off.back(), 1) * sizeof(unsigned), 256) : 0);
   e = cudaMalloc(&p->table, total);
@@ -561,12 +609,14 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
               job_bytes);
   if (red_bytes) std::memcpy(host.data() + off_r, rjobs.data(), red_bytes);
   if (rec_bytes) std::memcpy(host.data() + off_t, recs.data(), rec_bytes);
+  if (geo_bytes) std::memcpy(host.data() + off_g, cgeo.data(), geo_bytes);
   e = cudaMemcpy(p->table, host.data(), total, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     free_plan(p);
     return plan_fail(UGEMM_ERR_ALLOC, "grouped plan table upload failed");
   }
   p->maps = reinterpret_cast<const CUtensorMap*>(tb);
+  if (conv) p->geo = reinterpret_cast<const ConvGeo*>(tb + off_g);
   p->probs = tb + off_p;
   p->jobs = tb + off_j;
   p->reduce = tb + off_r;

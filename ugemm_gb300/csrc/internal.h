@@ -72,6 +72,23 @@ inline Im2col make_im2col(const float* x, int C, int B, int H, int W, int k, int
   return g;
 }
 
+// bf16-piece operands that the caller has written (conv.cu), for grouped plans
+// of three pieces.  NHWC pieces: [3][images x H x W][channels rounded up to 32].
+//   kTaps: C[M x pixels] = A * im2col(x): A's pieces [3][M][k'], k' = (tap,
+//          channel), each tap's channels padded to 32; x as NHWC pieces, the
+//          im2col matrix read through TMA's im2col mode, pixel by pixel K-major;
+//   kPix:  C[M x taps] = A * im2col(x)^T with k = pixels: both operands NHWC
+//          pieces (A's channels are C's rows), read MN-major, columns (tap,
+//          channel) with each tap's channels padded to 64;
+//   kPlain: both operands K-major pieces [3][rows][k'].
+struct PieceOperands {
+  enum Kind { kTaps = 1, kPix = 2, kPlain = 3 } kind = kPlain;
+  const void* a = nullptr;
+  const void* b = nullptr;
+  int kp = 0;          // k' of kTaps and kPlain (a multiple of 32)
+  Im2col im;           // kTaps, kPix: the geometry (im.x unused)
+};
+
 struct Gemm {
   char ta, tb;
   int M, N, K;
@@ -86,6 +103,9 @@ struct Gemm {
   // grouped plans only: B is the im2col matrix of b_im2col->x (K x N taps x
   // pixels when tb == 'N', N x K when tb == 'T'); B and ldb are then unused
   const Im2col* b_im2col = nullptr;
+  // grouped plans only: the operands' pieces, already written (A, lda, B and
+  // ldb are then unused)
+  const PieceOperands* pieces = nullptr;
 };
 
 #ifdef __CUDACC__
@@ -159,6 +179,7 @@ struct SplitPlan {
   bool fused = false;  // grouped launches of three bf16 pieces, 128-wide
                        // tiles: the GEMM kernel splits the FP32 operands
                        // itself (no pre-pass, no pieces in memory)
+  bool conv = false;   // grouped launches of PieceOperands problems
 };
 
 // --- tensor maps -------------------------------------------------------
@@ -169,6 +190,11 @@ bool encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dtype, int elem_bytes,
                     const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1,
                     uint64_t stride2, uint32_t b0, uint32_t b1, uint32_t b2,
                     CUtensorMapSwizzle swz);
+
+// One plane of NHWC 16-bit pieces, read by output pixels of a convolution.
+bool encode_tmap_im2col(CUtensorMap* map, const void* base, int channels, int images, int height,
+                        int width, int ksize, int pad, int stride, uint32_t box_channels,
+                        uint32_t box_pixels, CUtensorMapSwizzle swz);
 
 // --- SIMT path ---------------------------------------------------------
 size_t simt_scratch_bytes(const Gemm& g);
@@ -206,12 +232,15 @@ inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 // alpha * (its partial product) to part + s*M*N (row-major, ld N).  The
 // reduce forms C = sum_s part_s + beta*C (C not read when beta == 0), then
 // the optional bias / activation, summing the slices in a fixed order.
+// kk > 0: the partial tiles' columns are (tap, channel) with `cpad` channels
+// a tap, C's are channel * kk + tap (part_n = kk * cpad columns, N = kk * chans).
 struct ReduceJob {
   const float* part;
   float* C;
   int M, N, ldc, slices;
   float beta;
   Epilogue epi;
+  int kk = 0, cpad = 0, chans = 0;
 };
 ugemm_status splitk_reduce_launch(const ReduceJob* jobs, int njobs, long long max_mn,
                                   cudaStream_t st);

@@ -151,6 +151,19 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// im2col mode on a {channels, W, H, images} tensor: the map's pixels-per-column
+// consecutive output pixels from base pixel (w, h, n) on, each read at the
+// offset (ow, oh) from its base -- a kernel tap -- with zeros outside the image.
+__device__ __forceinline__ void tma_load_im2col(void* dst, const CUtensorMap* map, uint64_t* bar,
+                                                int c, int w, int h, int n, int ow, int oh) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c), "r"(w), "r"(h), "r"(n),
+      "h"(static_cast<uint16_t>(ow)), "h"(static_cast<uint16_t>(oh))
+      : "memory");
+}
+
 // ---------------------------------------------------------------- tcgen05
 // TMEM allocation: executed by one whole warp; writes the TMEM base address
 // to shared memory.  `ncols` is a power of two >= 32.
@@ -180,21 +193,26 @@ __device__ __forceinline__ void tc_fence_after() {
 
 // Shared-memory matrix descriptor for tcgen05.mma (K-major operand).
 //   bits  0-13 start address >> 4
-//   bits 16-29 leading-dimension byte offset >> 4 (unused for swizzled K-major)
-//   bits 32-45 stride-dimension byte offset >> 4 (distance between 8-row groups)
+//   bits 16-29 leading-dimension byte offset >> 4 (unused for swizzled K-major;
+//              MN-major: distance between blocks of one swizzle width of rows)
+//   bits 32-45 stride-dimension byte offset >> 4 (distance between 8-row
+//              groups; MN-major: between groups of 8 k)
 //   bits 46-48 fixed 0b001
 //   bits 61-63 swizzle: 0 none, 2 128B, 4 64B, 6 32B
 __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t sbo_bytes,
-                                                   uint32_t swizzle_code) {
+                                                   uint32_t swizzle_code,
+                                                   uint32_t lbo_bytes = 16) {
   uint64_t d = 0;
   d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(1u) << 16;  // LBO (ignored for swizzled K-major)
+  d |= static_cast<uint64_t>((lbo_bytes & 0x3FFFFu) >> 4) << 16;
   d |= static_cast<uint64_t>((sbo_bytes & 0x3FFFFu) >> 4) << 32;
   d |= static_cast<uint64_t>(1u) << 46;
   d |= static_cast<uint64_t>(swizzle_code & 7u) << 61;
   return d;
 }
 
+// Operands MN-major instead of K-major (16-bit types), added to a descriptor.
+constexpr uint32_t kUmmaMnMajor = (1u << 15) | (1u << 16);
 // Instruction descriptor, kind::f16 / kind::tf32 with FP32 accumulation,
 // both operands K-major.  a_fmt/b_fmt: 0 F16, 1 BF16, 2 TF32.
 __host__ __device__ constexpr uint32_t umma_idesc(uint32_t a_fmt, uint32_t b_fmt, uint32_t m,

@@ -321,7 +321,7 @@ __host__ __device__ constexpr uint32_t corr_code(int p) {
 // count is a template parameter, and the chunk position is a counter
 // rather than a remainder (a run-time division cost ~400 cycles per
 // k-block in the issuing thread, a gap in which the tensor pipe drained).
-template <int NP, int BN, bool GROUPED, bool TF32, bool FUSED, int NPROD>
+template <int NP, int BN, bool GROUPED, bool TF32, bool FUSED, bool CONV, int NPROD>
 __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
                                                const TcProblem* __restrict__ probs,
                                                const int4* __restrict__ tiles, int total_tiles,
@@ -329,7 +329,7 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
                                                uint64_t* empty, uint64_t* main_full,
                                                uint64_t* main_empty, uint64_t* tile_full,
                                                uint64_t* tmem_empty, int chunk_kb, int fmt,
-                                               int* err) {
+                                               const ConvGeo* __restrict__ geo, int* err) {
   constexpr bool WIDE = tc_wide(NP, TF32);
   using S = TcShape<NP, BN, WIDE>;
   constexpr int KK = S::KB / 16;  // k steps of 32 bytes per row in a stage
@@ -345,8 +345,13 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
   constexpr bool MERGE = !TF32 && BN == 128 && NPROD >= 3 && corr_code(0) == 0x1;
   const uint32_t idesc_pair = umma_idesc(ifmt, ifmt, kTcBM, 2 * BN);
   const uint32_t base = smem_u32(smem);
-  const uint64_t da0 = umma_smem_desc(base, SBO, SWZ);
-  const uint64_t db0 = umma_smem_desc(base + S::A_BYTES, SBO, SWZ);
+  uint64_t da0 = umma_smem_desc(base, SBO, SWZ);
+  uint64_t db0 = umma_smem_desc(base + S::A_BYTES, SBO, SWZ);
+  // K-major rows: a k step of 16 is 32 bytes on.  MN-major operands (CONV
+  // launches with k = pixels): 64 rows by 8 k to a 1024-byte swizzle atom, the
+  // atoms of a stage's four groups of 8 k one after the other, then the next
+  // 64 rows; the planes lie where the K-major ones would.
+  uint32_t kstep = 32;
   uint32_t s = 0, ph = 0, ntile = 0;
   uint32_t nbound[NB] = {};
   const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
@@ -360,6 +365,19 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       const int n_rem = P.N - tc.n0;
       if (n_rem < BN)
         idesc = umma_idesc(ifmt, ifmt, kTcBM, static_cast<uint32_t>((n_rem + 15) & ~15));
+    }
+    const bool pair_width = idesc == idesc_full;
+    uint32_t idesc2 = idesc_pair;
+    if constexpr (CONV) {
+      const bool mn = geo[tc.p].kind == PieceOperands::kPix;
+      kstep = mn ? 2048 : 32;
+      da0 = mn ? umma_smem_desc(base, 1024, 2, 4096) : umma_smem_desc(base, SBO, SWZ);
+      db0 = mn ? umma_smem_desc(base + S::A_BYTES, 1024, 2, 4096)
+               : umma_smem_desc(base + S::A_BYTES, SBO, SWZ);
+      if (mn) {
+        idesc |= kUmmaMnMajor;
+        idesc2 |= kUmmaMnMajor;
+      }
     }
     const uint32_t buf = NB == 1 ? 0u : ntile % NB, use = ntile / NB;
     const uint32_t t_main = tmem + buf * 2 * BN, t_corr = t_main + BN;
@@ -375,8 +393,8 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
         const uint32_t ia = corr_code(p) >> 2, ib = corr_code(p) & 3;
 #pragma unroll
         for (int kk = 0; kk < KK; ++kk) {
-          const uint64_t a = da + ((ia * S::A_PLANE + kk * 32) >> 4);
-          const uint64_t b = db + ((ib * S::B_PLANE + kk * 32) >> 4);
+          const uint64_t a = da + ((ia * S::A_PLANE + kk * kstep) >> 4);
+          const uint64_t b = db + ((ib * S::B_PLANE + kk * kstep) >> 4);
           if constexpr (TF32) umma_tf32(t_corr, a, b, idesc, (kbi | p | kk) != 0);
           else umma_bf16(t_corr, a, b, idesc, (kbi | p | kk) != 0);
         }
@@ -393,14 +411,14 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       const uint64_t da = da0 + so, db = db0 + so;
 #pragma unroll
       for (int kk = 0; kk < KK; ++kk)
-        umma_bf16(t_main, da + ((kk * 32) >> 4), db + ((kk * 32) >> 4), idesc_pair, true);
+        umma_bf16(t_main, da + ((kk * kstep) >> 4), db + ((kk * kstep) >> 4), idesc2, true);
 #pragma unroll
       for (int p = 1; p < NPROD - 1; ++p) {
         const uint32_t ia = corr_code(p) >> 2, ib = corr_code(p) & 3;
 #pragma unroll
         for (int kk = 0; kk < KK; ++kk)
-          umma_bf16(t_corr, da + ((ia * S::A_PLANE + kk * 32) >> 4),
-                    db + ((ib * S::B_PLANE + kk * 32) >> 4), idesc, true);
+          umma_bf16(t_corr, da + ((ia * S::A_PLANE + kk * kstep) >> 4),
+                    db + ((ib * S::B_PLANE + kk * kstep) >> 4), idesc, true);
       }
     };
     auto main_product = [&](uint32_t st, bool restart) {
@@ -408,13 +426,13 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       const uint64_t da = da0 + so, db = db0 + so;
 #pragma unroll
       for (int kk = 0; kk < KK; ++kk) {
-        const uint64_t a = da + ((kk * 32) >> 4), b = db + ((kk * 32) >> 4);
+        const uint64_t a = da + ((kk * kstep) >> 4), b = db + ((kk * kstep) >> 4);
         if constexpr (TF32) umma_tf32(t_main, a, b, idesc, !(restart && kk == 0));
         else umma_bf16(t_main, a, b, idesc, !(restart && kk == 0));
       }
     };
     int cpos = 0;  // the k-block's position in its chunk
-    const bool pair_ok = MERGE && idesc == idesc_full;
+    const bool pair_ok = MERGE && pair_width;
     for (int kb = 0; kb < P.nkb;) {
       if (!mbar_wait(&full[s], ph, err, kDevTimeoutFull)) return;
       tc_fence_after();
@@ -476,6 +494,69 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
   }
 }
 
+// The producer's copies of one tile of a CONV launch, stage by stage: the tiled
+// operand as everywhere, the im2col operand by TMA's im2col mode, one copy per
+// plane (and, MN-major, per block of 64 channels).  A stage's k is one tap's 32
+// channels (kTaps) or 32 output pixels (kPix), so a base pixel and a tap offset
+// describe every copy; the taps outside the image and the pixels past the last
+// image are zeros that the copy engine writes.
+template <int BN>
+__device__ __forceinline__ bool conv_produce(const ConvGeo G, const TcProblem& P,
+                                             const TileCoord& tc, const CUtensorMap* mp,
+                                             uint8_t* smem, uint64_t* full, uint64_t* empty,
+                                             uint32_t& it, int* err) {
+  using S = TcShape<3, BN, false>;
+  const int row_t = G.im_a ? tc.n0 : tc.m0, row_i = G.im_a ? tc.m0 : tc.n0;
+  const uint32_t off_t = G.im_a ? S::A_BYTES : 0, off_i = G.im_a ? 0 : S::A_BYTES;
+  const uint32_t plane_t = G.im_a ? S::B_PLANE : S::A_PLANE;
+  const uint32_t plane_i = G.im_a ? S::A_PLANE : S::B_PLANE;
+  const int blk_t = (G.im_a ? BN : kTcBM) / 64, blk_i = (G.im_a ? kTcBM : BN) / 64;
+  int n = 0, h = 0, w = 0;  // base pixel in the image's coordinates
+  auto base_pixel = [&](int pix) {
+    n = G.by_hw(pix);
+    const int q = pix - n * G.hw, i = G.by_wo(q);
+    h = i * G.stride - G.pad;
+    w = (q - i * G.wo) * G.stride - G.pad;
+  };
+  if (G.kind == PieceOperands::kTaps) base_pixel(row_i);
+  for (int kb = 0; kb < P.nkb; ++kb, ++it) {
+    const int s = it % S::STAGES;
+    if (!mbar_wait(&empty[s], ((it / S::STAGES) & 1) ^ 1, err, kDevTimeoutEmpty)) return false;
+    uint8_t* st = smem + s * S::STAGE_BYTES;
+    uint64_t* bar = &full[s];
+    mbar_arrive_expect_tx(bar, S::STAGE_BYTES);
+    const int kblk = P.kb0 + kb;
+    if (G.kind != PieceOperands::kPix) {
+      tma_load_3d(st + off_t, mp, bar, kblk * kTcKB, row_t, 0);
+      if (G.kind == PieceOperands::kPlain) {
+        tma_load_3d(st + off_i, mp + 1, bar, kblk * kTcKB, row_i, 0);
+        continue;
+      }
+      const int tap = G.by_blocks(kblk), c = (kblk - tap * G.blocks) * 32;
+      const int ki = G.by_k(tap), kj = tap - ki * G.ks;
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        tma_load_im2col(st + off_i + p * plane_i, mp + 1 + p, bar, c, w, h, n, kj, ki);
+      continue;
+    }
+    for (int q = 0; q < blk_t; ++q)
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        tma_load_3d(st + off_t + p * plane_t + q * 4096, mp, bar, row_t + 64 * q, kblk * kTcKB, p);
+    base_pixel(kblk * kTcKB);
+    for (int q = 0; q < blk_i; ++q) {
+      // the tile's blocks past the last tap repeat it: columns that are not stored
+      const int blk = min(row_i / 64 + q, G.ks * G.ks * G.blocks - 1);
+      const int tap = G.by_blocks(blk), c = (blk - tap * G.blocks) * 64;
+      const int ki = G.by_k(tap), kj = tap - ki * G.ks;
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        tma_load_im2col(st + off_i + p * plane_i + q * 4096, mp + 1 + p, bar, c, w, h, n, kj, ki);
+    }
+  }
+  return true;
+}
+
 // TF32: the TF32x3 form's instantiation (two planes of 32-deep tf32
 // stages, tcgen05 kind::tf32), a template parameter so that the 16-bit
 // instantiations' MMA issue loop carries no branch on the format.
@@ -485,18 +566,22 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
 // piece ring in the layout the piece copies would have had (K-major, 64-byte
 // rows, 64-byte swizzle), so the MMA issuer and the epilogue run unchanged
 // and the results are the same bits.
-template <int NP, int BN, bool GROUPED, bool EPI, bool TF32 = false, bool FUSED = false>
+// CONV (grouped launches of PieceOperands problems): the producer reads the
+// im2col operand of each problem through TMA's im2col mode.
+template <int NP, int BN, bool GROUPED, bool EPI, bool TF32 = false, bool FUSED = false,
+          bool CONV = false>
 __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1)
     split_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ TcProblem single, const CUtensorMap* __restrict__ maps,
                     const TcProblem* __restrict__ probs, const int4* __restrict__ tiles,
                     int total_tiles, int nprod,
-                    int chunk_kb, int fmt, int* err) {
+                    int chunk_kb, int fmt, const ConvGeo* __restrict__ geo, int* err) {
   // fmt: 16-bit piece format, 0 bf16, 1 fp16 (FP16x3); TF32 instantiations
   // read two planes of 32-deep stages with the 128-byte rows of the
   // two-piece 16-bit shape
   static_assert(!TF32 || NP == 2, "TF32 pieces come in two planes");
   static_assert(!FUSED || (NP == 3 && GROUPED && !TF32), "fused: grouped bf16x3-piece launches");
+  static_assert(!CONV || (NP == 3 && GROUPED && !FUSED), "conv: grouped launches on bf16 pieces");
   // 256-wide fused tiles: the epilogue warps are the converters
   constexpr bool DUAL = FUSED && BN == 256;
   constexpr bool WIDE = tc_wide(NP, TF32);
@@ -617,6 +702,12 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
         for (int t = tr.first; ok && t < tr.end; t += tr.step) {
           TcProblem P;
           const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+          if constexpr (CONV) {
+            const CUtensorMap* mp = &maps[4 * P.map];
+            for (int m = 0; m < 4; ++m) fence_tensormap(mp + m);
+            ok = conv_produce<BN>(geo[tc.p], P, tc, mp, smem, full, empty, it, err);
+            continue;
+          }
           const CUtensorMap* ma = GROUPED ? &maps[2 * P.map] : &tmA;
           const CUtensorMap* mb = GROUPED ? &maps[2 * P.map + 1] : &tmB;
           if (GROUPED) {
@@ -646,17 +737,17 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
         // the product count as a compile-time constant: two-piece forms have
         // three products, three-piece ones six (BF16x6) or nine (BF16x9)
         if constexpr (NP == 2)
-          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 3>(single, probs, tiles, total_tiles, smem,
+          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 3>(single, probs, tiles, total_tiles, smem,
                                                           tmem, full, empty, main_full, main_empty,
-                                                          tile_full, tmem_empty, chunk_kb, fmt, err);
+                                                          tile_full, tmem_empty, chunk_kb, fmt, geo, err);
         else if (nprod == 9)
-          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 9>(single, probs, tiles, total_tiles, smem,
+          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 9>(single, probs, tiles, total_tiles, smem,
                                                           tmem, full, empty, main_full, main_empty,
-                                                          tile_full, tmem_empty, chunk_kb, fmt, err);
+                                                          tile_full, tmem_empty, chunk_kb, fmt, geo, err);
         else
-          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, 6>(single, probs, tiles, total_tiles, smem,
+          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 6>(single, probs, tiles, total_tiles, smem,
                                                           tmem, full, empty, main_full, main_empty,
-                                                          tile_full, tmem_empty, chunk_kb, fmt, err);
+                                                          tile_full, tmem_empty, chunk_kb, fmt, geo, err);
       }
       __syncwarp();
     } else if (DUAL) {
@@ -928,8 +1019,43 @@ struct RawTile {
   float v[2][4];
 };
 
+// Chunk of 8 channels that this thread splits in tile `tile` of a weight job
+// (gather 3): the taps of one row (or, flipped, of all rows) lie next to each
+// other in memory, so they vary fastest.
+struct TapChunk { int r, tap, c; };
+__device__ __forceinline__ TapChunk tap_chunk(const SplitJob& j, int tile) {
+  const int idx = tile * 256 + threadIdx.x, cg = j.cp / 8;
+  const int q = idx / j.kk, tap = idx - q * j.kk;
+  return j.flip ? TapChunk{q % j.rows, tap, (q / j.rows) * 8} : TapChunk{q / cg, tap, (q % cg) * 8};
+}
+
+// TAPS: the launch may hold (tap, channel) jobs (gather 3 and 4).  They are an
+// instantiation of their own: compiled into the common one they cost it
+// registers and so resident blocks (256-problem group: 94 -> 120 us).
+template <bool TAPS = false>
 __device__ __forceinline__ void load_raw(const SplitJob& j, int r0, int k0, RawTile& out) {
   const int t = threadIdx.x;
+  if (TAPS && j.gather == 3) {
+    const TapChunk x = tap_chunk(j, r0);
+    const bool ok = x.r < j.rows && x.c < j.cp;
+    const float* src = j.src + x.r * j.sr + (j.flip ? j.kk - 1 - x.tap : x.tap);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      out.v[e / 4][e % 4] = ok && x.c + e < j.chans ? src[(x.c + e) * j.sk] : 0.f;
+    return;
+  }
+  if (TAPS && j.gather == 4) {  // the thread layout of rows contiguous, k' mapped to (c, tap)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int idx = t + 256 * i, kk = idx >> 3, q4 = (idx & 7) * 4, r = r0 + q4, k = k0 + kk;
+      const int tap = k / j.cp, c = k - tap * j.cp;
+      const float* src = j.src + (static_cast<long long>(c) * j.kk + tap) * j.sr;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        out.v[i][e] = (r + e < j.rows && k < j.Kp && c < j.chans) ? src[r + e] : 0.f;
+    }
+    return;
+  }
   if (j.gather) {  // implicit im2col: the same thread layout, gathered from x
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
@@ -1019,8 +1145,14 @@ __device__ __forceinline__ void load_raw(const SplitJob& j, int r0, int k0, RawT
   }
 }
 
+template <bool TAPS = false>
 __device__ __forceinline__ void raw_to_smem(const SplitJob& j, const RawTile& in, float (*tile)[65]) {
   const int t = threadIdx.x;
+  if (TAPS && j.gather == 3) {  // each thread's own chunk, where split_store reads it
+#pragma unroll
+    for (int e = 0; e < 8; ++e) tile[t >> 3][(t & 7) * 8 + e] = in.v[e / 4][e % 4];
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int idx = t + 256 * i;
@@ -1038,11 +1170,16 @@ __device__ __forceinline__ void raw_to_smem(const SplitJob& j, const RawTile& in
 
 // bf16 pieces of one tile from shared memory: 8 consecutive k of one row per
 // thread, one 16-byte store per plane.
-template <int NP, int FMT>
+template <int NP, int FMT, bool TAPS>
 __device__ __forceinline__ void split_store(const SplitJob& j, int r0, int k0, float (*tile)[65]) {
   const int t = threadIdx.x;
   const int rr = t >> 3, g8 = (t & 7) * 8;
-  const int r = r0 + rr, k = k0 + g8;
+  int r = r0 + rr, k = k0 + g8;
+  if (TAPS && j.gather == 3) {
+    const TapChunk x = tap_chunk(j, r0);
+    r = x.r;
+    k = x.c < j.cp ? x.tap * j.cp + x.c : j.Kp;
+  }
   if (r >= j.rows || k >= j.Kp) return;
   const size_t plane = static_cast<size_t>(j.rows) * j.Kp;
   const int ex = FMT == 1 ? f16_row_exp(j.fmax, r) : 0;
@@ -1068,14 +1205,20 @@ __device__ __forceinline__ int find_job(const int* starts, const SplitJob* jobs,
   return lo;
 }
 
+template <bool TAPS = false>
 __device__ __forceinline__ void tile_origin(const SplitJob& j, int b, int& r0, int& k0) {
   const int local = b - j.tile_start;
+  if (TAPS && j.gather == 3) {
+    r0 = local;
+    k0 = 0;
+    return;
+  }
   const int tiles_k = (j.Kp + 63) / 64;
   r0 = (local / tiles_k) * 32;
   k0 = (local % tiles_k) * 64;
 }
 
-template <int NP, int FMT>
+template <int NP, int FMT, bool TAPS>
 __device__ __forceinline__ void split_batched_body(const SplitJob* __restrict__ jobs, int njobs,
                                                    int total_tiles) {
   __shared__ float tile[32][65];
@@ -1087,21 +1230,21 @@ __device__ __forceinline__ void split_batched_body(const SplitJob* __restrict__ 
   if (b >= total_tiles) return;
   SplitJob cur = jobs[find_job(starts, jobs, njobs, b)];
   int r0, k0;
-  tile_origin(cur, b, r0, k0);
+  tile_origin<TAPS>(cur, b, r0, k0);
   RawTile raw;
-  load_raw(cur, r0, k0, raw);
+  load_raw<TAPS>(cur, r0, k0, raw);
   for (; b < total_tiles; b += gridDim.x) {
-    raw_to_smem(cur, raw, tile);
+    raw_to_smem<TAPS>(cur, raw, tile);
     const int nb = b + gridDim.x;
     SplitJob nxt = cur;
     int nr0 = 0, nk0 = 0;
     if (nb < total_tiles) {  // next tile's loads in flight during this tile's stores
       nxt = jobs[find_job(starts, jobs, njobs, nb)];
-      tile_origin(nxt, nb, nr0, nk0);
-      load_raw(nxt, nr0, nk0, raw);
+      tile_origin<TAPS>(nxt, nb, nr0, nk0);
+      load_raw<TAPS>(nxt, nr0, nk0, raw);
     }
     __syncthreads();
-    split_store<NP, FMT>(cur, r0, k0, tile);
+    split_store<NP, FMT, TAPS>(cur, r0, k0, tile);
     __syncthreads();
     cur = nxt;
     r0 = nr0;
@@ -1109,10 +1252,10 @@ __device__ __forceinline__ void split_batched_body(const SplitJob* __restrict__ 
   }
 }
 
-template <int NP, int FMT>
+template <int NP, int FMT, bool TAPS = false>
 __global__ void __launch_bounds__(256) split_pieces_batched_kernel(const SplitJob* __restrict__ jobs,
                                                                    int njobs, int total_tiles) {
-  split_batched_body<NP, FMT>(jobs, njobs, total_tiles);
+  split_batched_body<NP, FMT, TAPS>(jobs, njobs, total_tiles);
 }
 
 // The same for a few operands whose job records travel as the kernel's
@@ -1121,7 +1264,7 @@ __global__ void __launch_bounds__(256) split_pieces_batched_kernel(const SplitJo
 template <int NP, int FMT>
 __global__ void __launch_bounds__(256) split_pieces_param_kernel(
     const __grid_constant__ SplitJobTable t, int njobs, int total_tiles) {
-  split_batched_body<NP, FMT>(t.jobs, njobs, total_tiles);
+  split_batched_body<NP, FMT, false>(t.jobs, njobs, total_tiles);
 }
 
 // FP16x3 form, first step of the split: the largest finite magnitude of
@@ -1742,13 +1885,13 @@ int sm_count() {
   return sms;
 }
 
-template <int NP, int BN, bool GROUPED, bool EPI, bool TF32, bool FUSED = false>
+template <int NP, int BN, bool GROUPED, bool EPI, bool TF32, bool FUSED = false, bool CONV = false>
 ugemm_status launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const TcProblem& single,
                            const CUtensorMap* maps, const TcProblem* probs, const int4* tiles,
                            int total_tiles, int nprod, int chunk_kb, int max_ctas, int fmt,
-                           int* dev_err, cudaStream_t st) {
+                           int* dev_err, cudaStream_t st, const ConvGeo* geo = nullptr) {
   using S = TcShape<NP, BN, tc_wide(NP, TF32)>;
-  auto kern = split_tc_kernel<NP, BN, GROUPED, EPI, TF32, FUSED>;
+  auto kern = split_tc_kernel<NP, BN, GROUPED, EPI, TF32, FUSED, CONV>;
   static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
   constexpr size_t kSmem = FUSED ? S::SMEM_FUSED : S::SMEM;
   static_assert(kSmem <= 232448, "shared memory budget");
@@ -1764,7 +1907,7 @@ ugemm_status launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const T
   const int grid = std::max(1, std::min(total_tiles, max_ctas > 0 ? max_ctas : sm_count()));
   prof_begin(st);
   kern<<<grid, FUSED ? fused_threads(BN) : kTcSplitThreads, kSmem, st>>>(
-      ta, tb, single, maps, probs, tiles, total_tiles, nprod, chunk_kb, fmt, dev_err);
+      ta, tb, single, maps, probs, tiles, total_tiles, nprod, chunk_kb, fmt, geo, dev_err);
   prof_end(st, GROUPED ? kProfGrouped : kProfSplitGemm);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }
@@ -1898,6 +2041,53 @@ bool split_encode_maps(int pieces, int block_n, const void* ap, int M, const voi
          encode_tmap_3d(tb, dt, eb, bp, Kp, N, np, row, row * N, kb, block_n, np, sw);
 }
 
+bool conv_encode_maps(const PieceOperands& q, int M, int N, int block_n, bool swap,
+                      CUtensorMap* maps, ConvGeo* geo) {
+  const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const uint32_t rows_t = swap ? block_n : kTcBM, rows_i = swap ? kTcBM : block_n;
+  geo->kind = q.kind;
+  geo->im_a = swap ? 1 : 0;
+  if (q.kind == PieceOperands::kPlain || q.kind == PieceOperands::kTaps) {
+    const uint64_t row = uint64_t(q.kp) * 2;
+    if (!encode_tmap_3d(&maps[0], bf, 2, q.a, q.kp, M, 3, row, row * M, kTcKB, rows_t, 3,
+                        CU_TENSOR_MAP_SWIZZLE_64B))
+      return false;
+    if (q.kind == PieceOperands::kPlain) {
+      maps[2] = maps[3] = maps[0];
+      return encode_tmap_3d(&maps[1], bf, 2, q.b, q.kp, N, 3, row, row * N, kTcKB, rows_i, 3,
+                            CU_TENSOR_MAP_SWIZZLE_64B);
+    }
+  }
+  const Im2col& g = q.im;
+  const int cp = static_cast<int>(align_up(g.C, 32));
+  const bool taps = q.kind == PieceOperands::kTaps;
+  geo->stride = g.stride;
+  geo->pad = g.pad;
+  geo->ks = g.k;
+  geo->blocks = taps ? cp / 32 : cdiv(g.C, 64);
+  geo->hw = g.Ho * g.Wo;
+  geo->wo = g.Wo;
+  geo->by_hw = g.by_hw;
+  geo->by_wo = g.by_wo;
+  geo->by_k = g.by_k;
+  geo->by_blocks = FastDiv(static_cast<uint32_t>(geo->blocks));
+  if (!taps) {
+    const int mp = static_cast<int>(align_up(M, 32));
+    const uint64_t npix = uint64_t(g.B) * g.Ho * g.Wo, row = uint64_t(mp) * 2;
+    if (!encode_tmap_3d(&maps[0], bf, 2, q.a, mp, npix, 3, row, row * npix, 64, kTcKB, 1,
+                        CU_TENSOR_MAP_SWIZZLE_128B))
+      return false;
+  }
+  const size_t plane = size_t(g.B) * g.H * g.W * cp * 2;
+  for (int p = 0; p < 3; ++p)
+    if (!encode_tmap_im2col(&maps[1 + p], static_cast<const uint8_t*>(q.b) + p * plane, cp, g.B,
+                            g.H, g.W, g.k, g.pad, g.stride, taps ? 32 : 64,
+                            taps ? rows_i : kTcKB,
+                            taps ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B))
+      return false;
+  return true;
+}
+
 TcProblem split_problem(const Gemm& g, int pieces, int block_n, int tile_start) {
   TcProblem P;
   P.C = g.C;
@@ -1954,8 +2144,23 @@ ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const 
                                const TcProblem& single, const CUtensorMap* maps,
                                const TcProblem* probs, const int4* tiles, int total_tiles,
                                int chunk_kb,
-                               int max_ctas, int* dev_err, cudaStream_t st) {
+                               int max_ctas, int* dev_err, cudaStream_t st, const ConvGeo* geo) {
   const bool grouped = probs != nullptr;
+  if (p.conv) {
+    if (p.pieces != 3 || !grouped || geo == nullptr) return UGEMM_ERR_ARG;
+#define UGEMM_CONV_CASE(BN, EPI)                                                                 \
+  if (p.block_n == BN && p.epi == EPI)                                                          \
+    return launch_kernel<3, BN, true, EPI, false, false, true>(ta, tb, single, maps, probs,     \
+                                                               tiles, total_tiles, p.products,  \
+                                                               chunk_kb, max_ctas, 0, dev_err,  \
+                                                               st, geo);
+    UGEMM_CONV_CASE(128, false)
+    UGEMM_CONV_CASE(128, true)
+    UGEMM_CONV_CASE(256, false)
+    UGEMM_CONV_CASE(256, true)
+#undef UGEMM_CONV_CASE
+    return UGEMM_ERR_ARG;
+  }
   if (p.fused) {  // grouped launches of three bf16 pieces only
     if (p.pieces != 3 || !grouped || (p.block_n == 256 && single.chunk_sums == nullptr))
       return UGEMM_ERR_ARG;
@@ -2013,6 +2218,15 @@ ugemm_status split_batched_launch(int pieces, const SplitJob* jobs, int njobs, i
   if (pieces == 3) split_pieces_batched_kernel<3, 0><<<grid, 256, 0, st>>>(jobs, njobs, total_tiles);
   else if (pieces == kPiecesTf32) split_pieces_batched_kernel<2, 2><<<grid, 256, 0, st>>>(jobs, njobs, total_tiles);
   else split_pieces_batched_kernel<2, 0><<<grid, 256, 0, st>>>(jobs, njobs, total_tiles);
+  prof_end(st, kProfSplitPrep);
+  return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
+}
+
+ugemm_status split_taps_launch(const SplitJob* jobs, int njobs, int total_tiles, cudaStream_t st) {
+  if (total_tiles <= 0) return UGEMM_OK;
+  prof_begin(st);
+  split_pieces_batched_kernel<3, 0, true>
+      <<<std::min(total_tiles, sm_count() * 8), 256, 0, st>>>(jobs, njobs, total_tiles);
   prof_end(st, kProfSplitPrep);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }

@@ -172,6 +172,18 @@ struct TcProblem {
   float* chunk_sums = nullptr;
 };
 
+// What the producer of a CONV launch needs to know of a problem; problem p's
+// tensor maps are maps[4p] (the tiled operand) and maps[4p + 1..3] (the planes
+// of the im2col operand; kPlain: maps[4p + 1], the tiled b operand).
+struct ConvGeo {
+  int kind = 0;         // PieceOperands::Kind
+  int im_a = 0;         // the im2col operand is the kernel's a operand
+  int stride = 1, pad = 0, ks = 1;
+  int blocks = 1;       // channel blocks a tap: 32 channels (kTaps) or 64 (kPix)
+  int hw = 1, wo = 1;   // output pixels of an image and of a row
+  FastDiv by_hw, by_wo, by_blocks, by_k;
+};
+
 // One operand to split in the batched pre-pass.
 struct SplitJob {
   const float* src;
@@ -180,14 +192,24 @@ struct SplitJob {
   int rows, K, Kp;
   int tile_start;       // first 32x64 tile index of this job
   // implicit im2col operand (src unused): 1 = rows are pixels and k taps,
-  // 2 = rows are taps and k pixels; 0 = plain strided matrix
+  // 2 = rows are taps and k pixels; 0 = plain strided matrix.  Operands with
+  // k' = (tap, channel), kk taps of cp channels (chans of them real):
+  // 3 = weights, element (r, tap, c) at src[r*sr + c*sk + tap], taps reversed
+  // when flip; 4 = a stored im2col matrix, rows contiguous, element (r, tap, c)
+  // at src[(c*kk + tap)*sr + r]
   int gather = 0;
   Im2col im;
+  int kk = 0, chans = 0, cp = 0, flip = 0;
   // FP16x3 form: `rows` words that receive the largest magnitude of each row
   // (operand_max_batched_kernel), from which each row's power-of-two scale
   // follows; null: bf16 pieces.
   unsigned* fmax = nullptr;
 };
+
+// Tiles of a job in the launch's tile list.
+inline int split_job_tiles(const SplitJob& j) {
+  return j.gather == 3 ? cdiv(j.rows * (j.Kp / 8), 256) : cdiv(j.rows, 32) * cdiv(j.Kp, 64);
+}
 
 int split_kp(int K);
 int split_default_chunk_kb(int K);
@@ -257,7 +279,12 @@ ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail
 ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const CUtensorMap& tb,
                                const TcProblem& single, const CUtensorMap* maps,
                                const TcProblem* probs, const int4* tiles, int total_tiles,
-                               int chunk_kb, int max_ctas, int* dev_err, cudaStream_t st);
+                               int chunk_kb, int max_ctas, int* dev_err, cudaStream_t st,
+                               const ConvGeo* geo = nullptr);
+// The tensor maps of one CONV problem (maps[0..3]) whose C is M x N; swap: the
+// im2col operand (kPlain: B) is the kernel's a.  False if TMA cannot describe it.
+bool conv_encode_maps(const PieceOperands& q, int M, int N, int block_n, bool swap,
+                      CUtensorMap* maps, ConvGeo* geo);
 // The TMA map of a fused launch's FP32 operand stored as R rows x Cc columns
 // (leading dimension ld elements): kcontig, the kernel reads k along the
 // columns (box {box_k, box_rows}; 128-byte swizzle for 32-deep boxes, 64-byte
@@ -286,6 +313,8 @@ ugemm_status split_param_launch(int pieces, const SplitJobTable& t, int njobs, i
                                 cudaStream_t st);
 ugemm_status split_batched_launch(int pieces, const SplitJob* jobs, int njobs, int total_tiles,
                                   cudaStream_t st, unsigned* fmax_words = nullptr, int nwords = 0);
+// Three-piece jobs of every kind, (tap, channel) ones included.
+ugemm_status split_taps_launch(const SplitJob* jobs, int njobs, int total_tiles, cudaStream_t st);
 // Split one operand into its pieces at dst (split_operand_bytes of room).
 // f16: FP16x3 pieces -- the largest magnitude of every row is first found
 // into the operand's trailer words (cleared here), then each row's pieces
