@@ -204,6 +204,7 @@ struct ugemm_conv_stack_s {
     // TMA's im2col mode reads the im2col matrices of the forward, dX and dW
     // GEMMs, and the weights in (tap, channel) order.
     bool tap_fwd = false, tap_bwd = false;
+    bool tap_shape = false;  // tap_bwd but for the stack's explicit_col
     void *xp = nullptr, *wp = nullptr, *wbp = nullptr;  // wbp: the backward GEMM's weights
     ugemm::PieceOperands fwd_q, dw_q, dx_q;
     ugemm_grouped_plan* fwd = nullptr;
@@ -315,6 +316,35 @@ bool taps_ok(int C, int k, int pad, int stride) {
          stride <= 8;
 }
 
+// Tile width and k slices of a layer's backward launch, in which dW and dX
+// (equal flops) share the SMs: the width whose slower half is fastest.  They
+// follow from the implicit formulation's sizes in explicit stacks too, so that
+// dW is cut, and rounds, alike in both.
+void backward_geometry(const Stack* s, const Stack::Layer& L, ugemm::Gemm* b) {
+  using namespace ugemm;
+  const auto& d = L.d;
+  const int kk = d.ksize * d.ksize, npix = static_cast<int>(L.n);
+  const int in_px = s->batch * d.height * d.width;
+  const bool direct = d.stride == 1 && d.pad <= d.ksize - 1;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  double best = 1e300;
+  for (int bn : {64, 128, 256}) {
+    const GeoChoice w = choose_geometry(3, d.cout, kk * static_cast<int>(align_up(d.cin, 64)),
+                                        cdiv(npix, 32), sms / 2.0, bn, true, 256);
+    const GeoChoice x =
+        direct ? choose_geometry(3, d.cin, in_px, kk * cdiv(d.cout, 32), sms / 2.0, bn, true, 256)
+               : choose_geometry(3, L.kdim, npix, cdiv(d.cout, 32), sms / 2.0, bn, true, 256);
+    const double us = std::max(w.us, x.us);
+    if (us >= best) continue;
+    best = us;
+    b[0].block_n = bn;
+    b[0].slices = w.slices;
+    b[1].slices = direct && !L.direct_dx ? 1 : x.slices;  // (an explicit stack's dcol)
+  }
+}
+
 // Lays out and fills the pieces buffer and the split jobs of the layers that
 // take their operands as pieces, and points their PieceOperands at them.  The
 // forward GEMM's k order, (tap, channel), follows from the layer's sizes alone,
@@ -343,9 +373,10 @@ ugemm_status make_pieces(Stack* s) {
     const long long in_px = static_cast<long long>(s->batch) * d.height * d.width;
     if (in_px > 0x7fffffffLL) continue;
     L.tap_fwd = taps_ok(d.cin, d.ksize, d.pad, d.stride);
-    L.tap_bwd = L.tap_fwd && !s->explicit_col && d.cin > 32 &&
-                static_cast<int>(align_up(d.cin, 64)) <= 2 * d.cin &&
-                (!L.direct_dx || taps_ok(d.cout, d.ksize, d.ksize - 1 - d.pad, 1));
+    const bool direct = d.stride == 1 && d.pad <= d.ksize - 1;
+    L.tap_shape = L.tap_fwd && d.cin > 32 && static_cast<int>(align_up(d.cin, 64)) <= 2 * d.cin &&
+                  (!direct || taps_ok(d.cout, d.ksize, d.ksize - 1 - d.pad, 1));
+    L.tap_bwd = L.tap_shape && !s->explicit_col;
     if (L.tap_fwd) {
       wo[l] = take(d.cout, static_cast<long long>(kk) * pad32(d.cin));
       if (s->explicit_col)
@@ -589,6 +620,7 @@ UGEMM_API int ugemm_conv_stack_create(int nlayers, const ugemm_conv_layer* layer
       b[0].pieces = &L.dw_q;
       b[1].pieces = &L.dx_q;
     }
+    if (L.tap_shape) backward_geometry(s, L, b);
     ugemm_status rc = grouped_plan_build(&f, 1, s->form, nullptr, 0, &L.fwd);
     if (rc == UGEMM_OK) rc = grouped_plan_build(b, 2, s->form, nullptr, 0, &L.bwd);
     if (rc != UGEMM_OK) { destroy_stack(s); return rc; }

@@ -172,10 +172,17 @@ int kernel_cols(const Gemm& x) {
              : x.N;
 }
 
+// k-blocks of a split-form problem.
+int kernel_nkb(int pieces, const Gemm& x) {
+  return split_nkb(pieces,
+                   x.pieces && x.pieces->kind != PieceOperands::kPix ? x.pieces->kp : x.K);
+}
+
 // Padded tile area of an R x C output in 128 x bn tiles whose right-edge
 // tile is only as wide as its columns rounded to 16 (the split kernel's
 // narrow-N MMAs).
 double padded_area(int rows, int cols, int bn) {
+  if (bn == 64) return double(align_up(rows, 128)) * align_up(cols, 64);
   return double(align_up(rows, 128)) * ((cols / bn) * bn + align_up(cols % bn, 16));
 }
 
@@ -291,6 +298,18 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   cudaGetDevice(&p->device);
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+  // Untuned plans of three pieces: one problem takes the tile width, the
+  // orientation and the k slices that its measured stage and tile times make
+  // fastest; 64-wide tiles exist for these only.
+  GeoChoice one;
+  if (!config && form != UGEMM_PREC_SIMT && split_plan_for(form, g[0]).pieces == 3) {
+    if (g[0].block_n) {
+      p->cfg.block_n = g[0].block_n;
+    } else if (count == 1 && g[0].K > 0) {
+      one = choose_geometry(3, g[0].M, kernel_cols(g[0]), kernel_nkb(3, g[0]), sms, 0, true, 256);
+      p->cfg.block_n = one.block_n;
+    }
+  }
   for (const Gemm& x : g) p->flops += 2.0 * x.M * x.N * x.K;
 
   const bool simt = form == UGEMM_PREC_SIMT;
@@ -327,11 +346,12 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       o.nkb = std::max(1, cdiv(x.K, kBK));
     } else {
       const int n = kernel_cols(x);
-      o.swap = p->cfg.transpose == 0 && padded_area(n, x.M, bn) < padded_area(x.M, n, bn);
+      o.swap = one.us > 0 ? one.swap
+                          : p->cfg.transpose == 0 &&
+                                padded_area(n, x.M, bn) < padded_area(x.M, n, bn);
       const int rows = o.swap ? n : x.M, cols = o.swap ? x.M : n;
       o.tiles = cdiv(rows, kTcBM) * cdiv(cols, bn);
-      o.nkb = split_nkb(pieces, x.pieces && x.pieces->kind != PieceOperands::kPix ? x.pieces->kp
-                                                                                   : x.K);
+      o.nkb = kernel_nkb(pieces, x);
     }
     o.per = o.nkb;
     work += double(o.tiles) * o.nkb;
@@ -358,7 +378,10 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     o.sliced = x.pieces && x.pieces->kind == PieceOperands::kPix;
     const size_t tile_bytes = size_t(x.M) * kernel_cols(x) * 4;
     int sl = 1;
-    if (x.K != 0 && o.nkb >= 2 * min_slice && o.nkb > fair) {
+    if (one.us > 0 || x.slices > 0) {
+      sl = one.us > 0 ? one.slices : std::min(x.slices, o.nkb);
+      sl = static_cast<int>(std::min<size_t>(sl, std::max<size_t>(1, (size_t(1) << 30) / tile_bytes)));
+    } else if (x.K != 0 && o.nkb >= 2 * min_slice && o.nkb > fair) {
       const int len = std::max(min_slice, static_cast<int>(fair) + 1);
       sl = std::min(cdiv(o.nkb, len), 256);
       sl = static_cast<int>(std::min<size_t>(sl, (size_t(1) << 30) / tile_bytes));

@@ -106,6 +106,9 @@ struct Gemm {
   // grouped plans only: the operands' pieces, already written (A, lda, B and
   // ldb are then unused)
   const PieceOperands* pieces = nullptr;
+  // grouped plans only: tile width of the plan (its first problem's) and k
+  // slices of this problem, chosen by the caller; 0: by the plan
+  int block_n = 0, slices = 0;
 };
 
 #ifdef __CUDACC__

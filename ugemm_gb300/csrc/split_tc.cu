@@ -45,6 +45,7 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <cmath>
 
 #include <algorithm>
 #include <cstdlib>
@@ -361,7 +362,7 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
     // a group's narrow problems and right-edge tiles multiply only the
     // columns that exist (UMMA N in steps of 16)
     uint32_t idesc = idesc_full;
-    if constexpr (GROUPED) {
+    if constexpr (GROUPED && BN != 64) {
       const int n_rem = P.N - tc.n0;
       if (n_rem < BN)
         idesc = umma_idesc(ifmt, ifmt, kTcBM, static_cast<uint32_t>((n_rem + 15) & ~15));
@@ -380,12 +381,41 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       }
     }
     const uint32_t buf = NB == 1 ? 0u : ntile % NB, use = ntile / NB;
-    const uint32_t t_main = tmem + buf * 2 * BN, t_corr = t_main + BN;
+    const uint32_t t_main = tmem + buf * S::ACC_COLS, t_corr = t_main + BN;
     // the epilogue must have read this buffer's previous tile
     if (use > 0 && !mbar_wait(&tmem_empty[buf], (use - 1) & 1, err, kDevTimeoutAccum)) return;
     tc_fence_after();
+    // 64-wide tiles: the B planes lie back to back in the stage, 64 rows each,
+    // so one piece of A times two or three pieces of B is one MMA of N = 128 or
+    // 192 whose results land in adjacent accumulators: A0 [B0; B1; B2] in the
+    // main and the two correction accumulators, A1 [B0; B1] in the latter, A2 B0
+    // in the last.  An MMA of N = 64 takes about as long as one of N = 128 (A is
+    // read from shared memory either way), so this is what makes the narrow tile
+    // as fast per column as the wide ones.  `n`: pieces of B.
+    constexpr bool STACK = BN == 64;
+    auto stacked = [&](uint32_t st, uint32_t d, int ia, int ib, int n, bool keep_first) {
+      const uint64_t so = (st * static_cast<uint32_t>(S::STAGE_BYTES)) >> 4;
+      const uint32_t id = umma_idesc(ifmt, ifmt, kTcBM, 64 * n) | (idesc & kUmmaMnMajor);
+#pragma unroll
+      for (int kk = 0; kk < KK; ++kk)
+        umma_bf16(d, da0 + so + ((ia * S::A_PLANE + kk * kstep) >> 4),
+                  db0 + so + ((ib * S::B_PLANE + kk * kstep) >> 4), id, keep_first || kk != 0);
+    };
+    auto stacked_rest = [&](uint32_t st) {  // everything but A0's products
+      stacked(st, t_corr, 1, 0, 2, true);
+      stacked(st, t_corr + 64, 2, 0, 1, true);
+      if constexpr (NPROD == 9) {
+        stacked(st, t_corr, 1, 2, 1, true);
+        stacked(st, t_corr, 2, 1, 2, true);
+      }
+    };
     // the descriptors of stage st; the MMAs of its corrections and main product
     auto corrections = [&](uint32_t st, int kbi) {
+      if constexpr (STACK) {
+        stacked(st, t_corr, 0, 1, 2, kbi != 0);
+        stacked_rest(st);
+        return;
+      }
       const uint64_t so = (st * static_cast<uint32_t>(S::STAGE_BYTES)) >> 4;
       const uint64_t da = da0 + so, db = db0 + so;
 #pragma unroll
@@ -407,6 +437,11 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
     // one 256-row operand), so A0 is read once for both.  Only where both
     // accumulate (not at a chunk start, not in a tile's first k-block).
     auto merged_first = [&](uint32_t st) {
+      if constexpr (STACK) {
+        stacked(st, t_main, 0, 0, 3, true);
+        stacked_rest(st);
+        return;
+      }
       const uint64_t so = (st * static_cast<uint32_t>(S::STAGE_BYTES)) >> 4;
       const uint64_t da = da0 + so, db = db0 + so;
 #pragma unroll
@@ -432,7 +467,7 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       }
     };
     int cpos = 0;  // the k-block's position in its chunk
-    const bool pair_ok = MERGE && pair_width;
+    const bool pair_ok = STACK || (MERGE && pair_width);
     for (int kb = 0; kb < P.nkb;) {
       if (!mbar_wait(&full[s], ph, err, kDevTimeoutFull)) return;
       tc_fence_after();
@@ -773,7 +808,7 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       TcProblem P;
       const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
       const uint32_t buf = ntile % NB, use = ntile / NB;
-      const uint32_t t_buf = tmem + buf * 2 * BN + lane_base + col_off;
+      const uint32_t t_buf = tmem + buf * S::ACC_COLS + lane_base + col_off;
       if (P.beta != 0.f) prefetch_old_c<BN, GROUPED>(P, tc, ew, warp, lane);
       float acc[HALF];
 #pragma unroll
@@ -801,6 +836,7 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       // last main chunk, then the corrections (one 32-column slice live at a time)
       acc_add_tmem<HALF, GROUPED>(t_buf, acc, n_live);
       acc_add_tmem<HALF, GROUPED>(t_buf + BN, acc, n_live);
+      if constexpr (S::ACCS == 3) acc_add_tmem<HALF, GROUPED>(t_buf + 2 * BN, acc, n_live);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
@@ -1961,6 +1997,50 @@ std::vector<int4> split_tile_table(const TcProblem* probs, int nprob, int block_
   return table;
 }
 
+// Microseconds of one pipeline stage (a 32-deep k-block) of a tile, and of what
+// a tile costs beyond its stages (filling the pipeline, the last drain, and the
+// stores as far as the next tile's MMAs do not hide them: narrower tiles have a
+// second set of accumulators).  Measured on GB300 with all SMs busy; the 64-wide
+// stage is bound by its 36 KB of copies, the others by their MMAs.
+double stage_us(int pieces, int bn) {
+  const double w = bn == 256 ? 0.80 : bn == 128 ? 0.45 : 0.30;
+  return pieces == 3 ? w : w / 2;
+}
+double tile_us(int bn) { return bn == 256 ? 3.0 : bn == 128 ? 1.5 : 1.2; }
+
+GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int block_n,
+                          bool transpose, int max_slices) {
+  GeoChoice best;
+  best.us = 1e300;
+  const double sms = std::max(1.0, share);
+  for (int bn : {64, 128, 256}) {
+    if (block_n ? bn != block_n : bn == 64 && pieces != 3) continue;
+    for (int swap = 0; swap < (transpose ? 2 : 1); ++swap) {
+      const int rows = swap ? N : M, cols = swap ? M : N;
+      const double tiles = double(cdiv(rows, kTcBM)) * cdiv(cols, bn);
+      int last = 0;
+      for (int sl = 1; sl <= max_slices && sl <= nkb; ++sl) {
+        const int per = cdiv(nkb, sl);
+        if (sl > 1 && per < 4) break;
+        if (per == last) continue;
+        last = per;
+        const int n = cdiv(nkb, per);
+        double us = std::ceil(tiles * n / sms) * (per * stage_us(pieces, bn) + tile_us(bn));
+        // partial tiles written and read back (4 TB/s) and a launch to sum them
+        if (n > 1) us += 3.0 + (n + 1.0) * M * N * 4 / 4e6;
+        if (us < best.us - 1e-9) {
+          best.block_n = bn;
+          best.swap = swap != 0;
+          best.slices = n;
+          best.per = per;
+          best.us = us;
+        }
+      }
+    }
+  }
+  return best;
+}
+
 // Depth of the main accumulator's chunks, in 32-deep k-blocks, for a GEMM
 // of depth K (UGEMM_CHUNK_K overrides).  Each chunk is summed in TMEM, whose
 // adds truncate, then drained into FP32 registers with round-to-nearest
@@ -2154,6 +2234,8 @@ ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const 
                                                                tiles, total_tiles, p.products,  \
                                                                chunk_kb, max_ctas, 0, dev_err,  \
                                                                st, geo);
+    UGEMM_CONV_CASE(64, false)
+    UGEMM_CONV_CASE(64, true)
     UGEMM_CONV_CASE(128, false)
     UGEMM_CONV_CASE(128, true)
     UGEMM_CONV_CASE(256, false)
@@ -2187,6 +2269,8 @@ ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const 
   UGEMM_SPLIT_CASE(NP, BN, false, true, T)  \
   UGEMM_SPLIT_CASE(NP, BN, true, false, T)  \
   UGEMM_SPLIT_CASE(NP, BN, true, true, T)
+  UGEMM_SPLIT_CASE(3, 64, true, false, false)
+  UGEMM_SPLIT_CASE(3, 64, true, true, false)
   UGEMM_SPLIT_CASES(3, 256, false)
   UGEMM_SPLIT_CASES(3, 128, false)
   UGEMM_SPLIT_CASES(2, 256, false)

@@ -114,12 +114,12 @@ struct TcShape {
   static constexpr int B_BYTES = NP * B_PLANE;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int FIT = (224 * 1024) / STAGE_BYTES;
-  static constexpr int STAGES = FIT > 4 ? 4 : FIT;
+  static constexpr int STAGES = BN == 64 ? 5 : (FIT > 4 ? 4 : FIT);
   // Each epilogue warp's 32 x 32 output blocks pass through shared memory so
   // that C is written by rows: whole blocks (padded rows) where the stage
   // ring leaves room -- 128-wide tiles, and 256-wide ones of two pieces --,
   // 8 rows at a time for 256-wide tiles of three pieces.
-  static constexpr bool STAGE_C = (BN == 128 || NP == 2);
+  static constexpr bool STAGE_C = (BN <= 128 || NP == 2);
   static constexpr size_t STAGE_C_BYTES = size_t(kTcEpiWarps) * (STAGE_C ? 32 : 8) * 33 * 4;
   static constexpr size_t SMEM =
       1024 + size_t(STAGES) * STAGE_BYTES + 256 + STAGE_C_BYTES;
@@ -131,9 +131,13 @@ struct TcShape {
   static constexpr size_t FUSED_RING =
       size_t(kTcFusedPieceStages) * STAGE_BYTES + size_t(kTcRawStages) * RAW_BYTES;
   static constexpr size_t SMEM_FUSED = 1024 + FUSED_RING + 256 + STAGE_C_BYTES;
-  // main + correction accumulators, double-buffered across tiles when they fit
+  // main + correction accumulators (64-wide tiles: two of those),
+  // double-buffered across tiles when they fit
+  static constexpr int ACCS = BN == 64 ? 3 : 2;
   static constexpr int ACC_BUFS = (4 * BN <= 512) ? 2 : 1;
-  static constexpr uint32_t TMEM_COLS = ACC_BUFS * 2 * BN;
+  static constexpr uint32_t ACC_COLS = ACCS * BN;
+  static constexpr uint32_t TMEM_COLS = BN == 64 ? 512 : ACC_BUFS * ACC_COLS;
+  static_assert(ACC_BUFS * ACC_COLS <= TMEM_COLS, "tensor memory");
   static_assert(STAGES >= 2, "pipeline needs two stages");
   static_assert(SMEM <= 232448, "shared memory budget");
 };
@@ -210,6 +214,20 @@ struct SplitJob {
 inline int split_job_tiles(const SplitJob& j) {
   return j.gather == 3 ? cdiv(j.rows * (j.Kp / 8), 256) : cdiv(j.rows, 32) * cdiv(j.Kp, 64);
 }
+
+// How a problem of C (M x N) with nkb k-blocks is cut for a grouped launch of
+// three-piece operands on `share` of the SMs: tile width, transposition, k
+// slices, and the model's time in microseconds.
+struct GeoChoice {
+  int block_n = 256;
+  bool swap = false;
+  int slices = 1, per = 0;
+  double us = 0;
+};
+// block_n: 0 to choose among the widths that `pieces` has; transpose: whether
+// C^T may be computed instead.
+GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int block_n,
+                          bool transpose, int max_slices);
 
 int split_kp(int K);
 int split_default_chunk_kb(int K);
