@@ -51,6 +51,7 @@
 #include <cstdlib>
 #include <functional>
 #include <queue>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -312,16 +313,16 @@ __host__ __device__ constexpr uint32_t corr_code(int p) {
        : p == 5 ? 0x6 : p == 6 ? 0x9 : 0xA;
 }
 
-// The MMA issuer (one thread).  Per k-block: wait for the stage, issue the
+// The MMA issuer (one warp).  Per k-block: wait for the stage, issue the
 // correction products into their accumulator, the main product into its
 // (restarted at each chunk once the epilogue drained it), commit the stage
-// free; per tile, commit the accumulators full.  Everything per k-block is
-// compile-time but the stage: the descriptors are those of stage 0 plus the
-// stage's offset (the address field counts 16-byte units, and shared
-// memory stays below 256 KB, so the field never carries), the product
-// count is a template parameter, and the chunk position is a counter
-// rather than a remainder (a run-time division cost ~400 cycles per
-// k-block in the issuing thread, a gap in which the tensor pipe drained).
+// free; per tile, commit the accumulators full.  An MMA of 128 columns takes
+// 64 cycles, so the issuing itself counts: the warp runs the loop converged and
+// one lane issues, so that descriptors are uniform values, made by 32-bit adds
+// of compile-time offsets to the stage's (the address field counts 16-byte
+// units, and shared memory stays below 256 KB, so the field never carries);
+// the product count is a template parameter, and the chunk position is a
+// counter rather than a remainder.
 template <int NP, int BN, bool GROUPED, bool TF32, bool FUSED, bool CONV, int NPROD>
 __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
                                                const TcProblem* __restrict__ probs,
@@ -344,90 +345,68 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
   const uint32_t idesc_full = umma_idesc(ifmt, ifmt, kTcBM, BN);
   // 128-wide tiles whose first correction is A0 B1: the pair A0 [B0; B1]
   constexpr bool MERGE = !TF32 && BN == 128 && NPROD >= 3 && corr_code(0) == 0x1;
-  const uint32_t idesc_pair = umma_idesc(ifmt, ifmt, kTcBM, 2 * BN);
+  constexpr bool STACK = BN == 64;
   const uint32_t base = smem_u32(smem);
-  uint64_t da0 = umma_smem_desc(base, SBO, SWZ);
-  uint64_t db0 = umma_smem_desc(base + S::A_BYTES, SBO, SWZ);
-  // K-major rows: a k step of 16 is 32 bytes on.  MN-major operands (CONV
-  // launches with k = pixels): 64 rows by 8 k to a 1024-byte swizzle atom, the
-  // atoms of a stage's four groups of 8 k one after the other, then the next
-  // 64 rows; the planes lie where the K-major ones would.
-  uint32_t kstep = 32;
+  const uint64_t kmajor = umma_smem_desc(base, SBO, SWZ);
+  const uint64_t mnmajor = umma_smem_desc(base, 1024, 2, 4096);
+  const bool leader = elect_one();
   uint32_t s = 0, ph = 0, ntile = 0;
   uint32_t nbound[NB] = {};
-  const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
-  for (int t = tr.first; t < tr.end; t += tr.step, ++ntile) {
-    TcProblem P;
-    const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
-    // a group's narrow problems and right-edge tiles multiply only the
-    // columns that exist (UMMA N in steps of 16)
-    uint32_t idesc = idesc_full;
-    if constexpr (GROUPED && BN != 64) {
-      const int n_rem = P.N - tc.n0;
-      if (n_rem < BN)
-        idesc = umma_idesc(ifmt, ifmt, kTcBM, static_cast<uint32_t>((n_rem + 15) & ~15));
-    }
-    const bool pair_width = idesc == idesc_full;
-    uint32_t idesc2 = idesc_pair;
-    if constexpr (CONV) {
-      const bool mn = geo[tc.p].kind == PieceOperands::kPix;
-      kstep = mn ? 2048 : 32;
-      da0 = mn ? umma_smem_desc(base, 1024, 2, 4096) : umma_smem_desc(base, SBO, SWZ);
-      db0 = mn ? umma_smem_desc(base + S::A_BYTES, 1024, 2, 4096)
-               : umma_smem_desc(base + S::A_BYTES, SBO, SWZ);
-      if (mn) {
-        idesc |= kUmmaMnMajor;
-        idesc2 |= kUmmaMnMajor;
-      }
-    }
-    const uint32_t buf = NB == 1 ? 0u : ntile % NB, use = ntile / NB;
+  auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code));
+  };
+  // One tile.  MN: operands MN-major (CONV launches with k = pixels): 64 rows by
+  // 8 k to a 1024-byte swizzle atom, the atoms of a stage's four groups of 8 k
+  // one after the other, then the next 64 rows; the planes lie where the K-major
+  // ones would.
+  auto tile = [&](auto mn, int nkb, uint32_t idesc, uint32_t buf) -> bool {
+    constexpr bool MN = decltype(mn)::value;
+    constexpr uint32_t KSTEP = MN ? 2048 : 32, MNBITS = MN ? kUmmaMnMajor : 0;
+    const uint64_t desc = MN ? mnmajor : kmajor;
+    const uint32_t lo0 = static_cast<uint32_t>(desc), hi = static_cast<uint32_t>(desc >> 32);
+    const bool pair_ok = STACK || (MERGE && idesc == idesc_full);
+    const uint32_t id = idesc | MNBITS;
+    const uint32_t id_pair = umma_idesc(ifmt, ifmt, kTcBM, BN == 128 ? 256 : BN) | MNBITS;
     const uint32_t t_main = tmem + buf * S::ACC_COLS, t_corr = t_main + BN;
-    // the epilogue must have read this buffer's previous tile
-    if (use > 0 && !mbar_wait(&tmem_empty[buf], (use - 1) & 1, err, kDevTimeoutAccum)) return;
-    tc_fence_after();
+    // A piece ia times B pieces from ib on, k step kk of stage st (its
+    // descriptors' lower word at lo), into d
+    auto mma = [&](uint32_t lo, uint32_t d, int ia, int ib, int kk, uint32_t i, bool keep) {
+      const uint32_t a = lo + ((ia * S::A_PLANE + kk * KSTEP) >> 4);
+      const uint32_t b = lo + ((S::A_BYTES + ib * S::B_PLANE + kk * KSTEP) >> 4);
+      if constexpr (TF32) umma_tf32(d, a, hi, b, hi, i, keep);
+      else umma_bf16(d, a, hi, b, hi, i, keep);
+    };
+    auto stage_lo = [&](uint32_t st) { return lo0 + st * (S::STAGE_BYTES >> 4); };
     // 64-wide tiles: the B planes lie back to back in the stage, 64 rows each,
     // so one piece of A times two or three pieces of B is one MMA of N = 128 or
     // 192 whose results land in adjacent accumulators: A0 [B0; B1; B2] in the
-    // main and the two correction accumulators, A1 [B0; B1] in the latter, A2 B0
-    // in the last.  An MMA of N = 64 takes about as long as one of N = 128 (A is
-    // read from shared memory either way), so this is what makes the narrow tile
-    // as fast per column as the wide ones.  `n`: pieces of B.
-    constexpr bool STACK = BN == 64;
-    auto stacked = [&](uint32_t st, uint32_t d, int ia, int ib, int n, bool keep_first) {
-      const uint64_t so = (st * static_cast<uint32_t>(S::STAGE_BYTES)) >> 4;
-      const uint32_t id = umma_idesc(ifmt, ifmt, kTcBM, 64 * n) | (idesc & kUmmaMnMajor);
-#pragma unroll
-      for (int kk = 0; kk < KK; ++kk)
-        umma_bf16(d, da0 + so + ((ia * S::A_PLANE + kk * kstep) >> 4),
-                  db0 + so + ((ib * S::B_PLANE + kk * kstep) >> 4), id, keep_first || kk != 0);
+    // main one and the next two, A1 [B0; B1] in two more, A2 B0 in the last.
+    auto stacked = [&](uint32_t lo, int kk, uint32_t acc, int ia, int ib, int n, bool keep) {
+      mma(lo, t_main + acc * 64, ia, ib, kk, umma_idesc(ifmt, ifmt, kTcBM, 64 * n) | MNBITS, keep);
     };
-    auto stacked_rest = [&](uint32_t st) {  // everything but A0's products
-      stacked(st, t_corr, 1, 0, 2, true);
-      stacked(st, t_corr + 64, 2, 0, 1, true);
+    auto stacked_rest = [&](uint32_t lo, int kk, bool keep) {  // all but A0's products
+      stacked(lo, kk, 3, 1, 0, 2, keep);
+      stacked(lo, kk, 5, 2, 0, 1, keep);
       if constexpr (NPROD == 9) {
-        stacked(st, t_corr, 1, 2, 1, true);
-        stacked(st, t_corr, 2, 1, 2, true);
+        stacked(lo, kk, 3, 2, 1, 2, true);
+        stacked(lo, kk, 5, 1, 2, 1, true);
       }
     };
-    // the descriptors of stage st; the MMAs of its corrections and main product
     auto corrections = [&](uint32_t st, int kbi) {
+      if (!leader) return;
+      const uint32_t lo = stage_lo(st);
       if constexpr (STACK) {
-        stacked(st, t_corr, 0, 1, 2, kbi != 0);
-        stacked_rest(st);
-        return;
-      }
-      const uint64_t so = (st * static_cast<uint32_t>(S::STAGE_BYTES)) >> 4;
-      const uint64_t da = da0 + so, db = db0 + so;
-#pragma unroll
-      for (int p = 0; p < NPROD - 1; ++p) {
-        const uint32_t ia = corr_code(p) >> 2, ib = corr_code(p) & 3;
 #pragma unroll
         for (int kk = 0; kk < KK; ++kk) {
-          const uint64_t a = da + ((ia * S::A_PLANE + kk * kstep) >> 4);
-          const uint64_t b = db + ((ib * S::B_PLANE + kk * kstep) >> 4);
-          if constexpr (TF32) umma_tf32(t_corr, a, b, idesc, (kbi | p | kk) != 0);
-          else umma_bf16(t_corr, a, b, idesc, (kbi | p | kk) != 0);
+          stacked(lo, kk, 1, 0, 1, 2, (kbi | kk) != 0);
+          stacked_rest(lo, kk, (kbi | kk) != 0);
         }
+      } else {
+#pragma unroll
+        for (int p = 0; p < NPROD - 1; ++p)
+#pragma unroll
+          for (int kk = 0; kk < KK; ++kk)
+            mma(lo, t_corr, corr_code(p) >> 2, corr_code(p) & 3, kk, id, (kbi | p | kk) != 0);
       }
     };
     // A full-width 128-wide tile's main product and first correction, A0 B0
@@ -436,48 +415,45 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
     // B0 and B1 planes are adjacent in the stage (rows 0-127 and 128-255 of
     // one 256-row operand), so A0 is read once for both.  Only where both
     // accumulate (not at a chunk start, not in a tile's first k-block).
-    auto merged_first = [&](uint32_t st) {
+    auto merged = [&](uint32_t st) {
+      if (!leader) return;
+      const uint32_t lo = stage_lo(st);
       if constexpr (STACK) {
-        stacked(st, t_main, 0, 0, 3, true);
-        stacked_rest(st);
-        return;
-      }
-      const uint64_t so = (st * static_cast<uint32_t>(S::STAGE_BYTES)) >> 4;
-      const uint64_t da = da0 + so, db = db0 + so;
 #pragma unroll
-      for (int kk = 0; kk < KK; ++kk)
-        umma_bf16(t_main, da + ((kk * kstep) >> 4), db + ((kk * kstep) >> 4), idesc2, true);
+        for (int kk = 0; kk < KK; ++kk) {
+          stacked(lo, kk, 0, 0, 0, 3, true);
+          stacked_rest(lo, kk, true);
+        }
+      } else {
 #pragma unroll
-      for (int p = 1; p < NPROD - 1; ++p) {
-        const uint32_t ia = corr_code(p) >> 2, ib = corr_code(p) & 3;
+        for (int kk = 0; kk < KK; ++kk) mma(lo, t_main, 0, 0, kk, id_pair, true);
 #pragma unroll
-        for (int kk = 0; kk < KK; ++kk)
-          umma_bf16(t_corr, da + ((ia * S::A_PLANE + kk * kstep) >> 4),
-                    db + ((ib * S::B_PLANE + kk * kstep) >> 4), idesc, true);
+        for (int p = 1; p < NPROD - 1; ++p)
+#pragma unroll
+          for (int kk = 0; kk < KK; ++kk)
+            mma(lo, t_corr, corr_code(p) >> 2, corr_code(p) & 3, kk, id, true);
       }
     };
     auto main_product = [&](uint32_t st, bool restart) {
-      const uint64_t so = (st * static_cast<uint32_t>(S::STAGE_BYTES)) >> 4;
-      const uint64_t da = da0 + so, db = db0 + so;
+      if (!leader) return;
+      const uint32_t lo = stage_lo(st);
 #pragma unroll
-      for (int kk = 0; kk < KK; ++kk) {
-        const uint64_t a = da + ((kk * kstep) >> 4), b = db + ((kk * kstep) >> 4);
-        if constexpr (TF32) umma_tf32(t_main, a, b, idesc, !(restart && kk == 0));
-        else umma_bf16(t_main, a, b, idesc, !(restart && kk == 0));
-      }
+      for (int kk = 0; kk < KK; ++kk) mma(lo, t_main, 0, 0, kk, id, !(restart && kk == 0));
+    };
+    auto commit = [&](uint64_t* bar) {
+      if (leader) umma_commit(bar);
     };
     int cpos = 0;  // the k-block's position in its chunk
-    const bool pair_ok = STACK || (MERGE && pair_width);
-    for (int kb = 0; kb < P.nkb;) {
-      if (!mbar_wait(&full[s], ph, err, kDevTimeoutFull)) return;
+    for (int kb = 0; kb < nkb;) {
+      if (!wait(&full[s], ph, kDevTimeoutFull)) return false;
       tc_fence_after();
       if (pair_ok && cpos != 0) {
-        merged_first(s);
-        umma_commit(&empty[s]);
+        merged(s);
+        commit(&empty[s]);
         ++kb;
         if (++cpos == chunk_kb) {
           cpos = 0;
-          if (kb < P.nkb) umma_commit(&main_full[buf]);
+          if (kb < nkb) commit(&main_full[buf]);
         }
         if (++s == NST) {
           s = 0;
@@ -496,8 +472,9 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       int ahead = 0;
       if (cpos == 0 && kb > 0) {
         uint32_t s2 = s + 1 == NST ? 0 : s + 1, ph2 = s + 1 == NST ? ph ^ 1 : ph;
-        while (ahead < NST - 1 && ahead + 1 < chunk_kb && kb + 1 + ahead < P.nkb &&
-               !mbar_test_wait(&main_empty[buf], nbound[buf] & 1) && mbar_test_wait(&full[s2], ph2)) {
+        while (ahead < NST - 1 && ahead + 1 < chunk_kb && kb + 1 + ahead < nkb &&
+               __all_sync(0xffffffffu, !mbar_test_wait(&main_empty[buf], nbound[buf] & 1) &&
+                                           mbar_test_wait(&full[s2], ph2))) {
           tc_fence_after();
           corrections(s2, kb + 1 + ahead);
           ++ahead;
@@ -506,7 +483,7 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
             ph2 ^= 1;
           }
         }
-        if (!mbar_wait(&main_empty[buf], nbound[buf] & 1, err, kDevTimeoutAccum)) return;
+        if (!wait(&main_empty[buf], nbound[buf] & 1, kDevTimeoutAccum)) return false;
         ++nbound[buf];
         tc_fence_after();
       }
@@ -514,10 +491,10 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       // ahead, each stage released once its MMAs complete
       for (int a = 0; a <= ahead; ++a, ++kb) {
         main_product(s, cpos == 0);
-        umma_commit(&empty[s]);
+        commit(&empty[s]);
         if (++cpos == chunk_kb) {
           cpos = 0;
-          if (kb + 1 < P.nkb) umma_commit(&main_full[buf]);
+          if (kb + 1 < nkb) commit(&main_full[buf]);
         }
         if (++s == NST) {
           s = 0;
@@ -525,7 +502,32 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
         }
       }
     }
-    umma_commit(&tile_full[buf]);
+    commit(&tile_full[buf]);
+    return true;
+  };
+  const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
+  for (int t = tr.first; t < tr.end; t += tr.step, ++ntile) {
+    TcProblem P;
+    const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+    // a group's narrow problems and right-edge tiles multiply only the
+    // columns that exist (UMMA N in steps of 16)
+    uint32_t idesc = idesc_full;
+    if constexpr (GROUPED && BN != 64) {
+      const int n_rem = P.N - tc.n0;
+      if (n_rem < BN)
+        idesc = umma_idesc(ifmt, ifmt, kTcBM, static_cast<uint32_t>((n_rem + 15) & ~15));
+    }
+    const uint32_t buf = NB == 1 ? 0u : ntile % NB, use = ntile / NB;
+    // the epilogue must have read this buffer's previous tile
+    if (use > 0 && !wait(&tmem_empty[buf], (use - 1) & 1, kDevTimeoutAccum)) return;
+    tc_fence_after();
+    bool ok;
+    if constexpr (CONV)
+      ok = geo[tc.p].kind == PieceOperands::kPix
+               ? tile(std::true_type{}, P.nkb, idesc, buf)
+               : tile(std::false_type{}, P.nkb, idesc, buf);
+    else ok = tile(std::false_type{}, P.nkb, idesc, buf);
+    if (!ok) return;
   }
 }
 
@@ -768,22 +770,20 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       }
     } else if (warp == 1) {
       // ------------------------------------------------------ MMA issuer
-      if (lane == 0) {
-        // the product count as a compile-time constant: two-piece forms have
-        // three products, three-piece ones six (BF16x6) or nine (BF16x9)
-        if constexpr (NP == 2)
-          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 3>(single, probs, tiles, total_tiles, smem,
-                                                          tmem, full, empty, main_full, main_empty,
-                                                          tile_full, tmem_empty, chunk_kb, fmt, geo, err);
-        else if (nprod == 9)
-          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 9>(single, probs, tiles, total_tiles, smem,
-                                                          tmem, full, empty, main_full, main_empty,
-                                                          tile_full, tmem_empty, chunk_kb, fmt, geo, err);
-        else
-          mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 6>(single, probs, tiles, total_tiles, smem,
-                                                          tmem, full, empty, main_full, main_empty,
-                                                          tile_full, tmem_empty, chunk_kb, fmt, geo, err);
-      }
+      // the product count as a compile-time constant: two-piece forms have
+      // three products, three-piece ones six (BF16x6) or nine (BF16x9)
+      if constexpr (NP == 2)
+        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 3>(
+            single, probs, tiles, total_tiles, smem, tmem, full, empty, main_full, main_empty,
+            tile_full, tmem_empty, chunk_kb, fmt, geo, err);
+      else if (nprod == 9)
+        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 9>(
+            single, probs, tiles, total_tiles, smem, tmem, full, empty, main_full, main_empty,
+            tile_full, tmem_empty, chunk_kb, fmt, geo, err);
+      else
+        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 6>(
+            single, probs, tiles, total_tiles, smem, tmem, full, empty, main_full, main_empty,
+            tile_full, tmem_empty, chunk_kb, fmt, geo, err);
       __syncwarp();
     } else if (DUAL) {
       // ---------------------------------- epilogue warps that also convert
@@ -836,7 +836,8 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       // last main chunk, then the corrections (one 32-column slice live at a time)
       acc_add_tmem<HALF, GROUPED>(t_buf, acc, n_live);
       acc_add_tmem<HALF, GROUPED>(t_buf + BN, acc, n_live);
-      if constexpr (S::ACCS == 3) acc_add_tmem<HALF, GROUPED>(t_buf + 2 * BN, acc, n_live);
+#pragma unroll
+      for (int c = 2; c < S::ACCS; ++c) acc_add_tmem<HALF, GROUPED>(t_buf + c * BN, acc, n_live);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
@@ -2003,7 +2004,7 @@ std::vector<int4> split_tile_table(const TcProblem* probs, int nprob, int block_
 // second set of accumulators).  Measured on GB300 with all SMs busy; the 64-wide
 // stage is bound by its 36 KB of copies, the others by their MMAs.
 double stage_us(int pieces, int bn) {
-  const double w = bn == 256 ? 0.80 : bn == 128 ? 0.45 : 0.30;
+  const double w = bn == 256 ? 0.80 : bn == 128 ? 0.64 : 0.30;
   return pieces == 3 ? w : w / 2;
 }
 double tile_us(int bn) { return bn == 256 ? 3.0 : bn == 128 ? 1.5 : 1.2; }

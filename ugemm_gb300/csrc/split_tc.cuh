@@ -131,10 +131,10 @@ struct TcShape {
   static constexpr size_t FUSED_RING =
       size_t(kTcFusedPieceStages) * STAGE_BYTES + size_t(kTcRawStages) * RAW_BYTES;
   static constexpr size_t SMEM_FUSED = 1024 + FUSED_RING + 256 + STAGE_C_BYTES;
-  // main + correction accumulators (64-wide tiles: two of those),
-  // double-buffered across tiles when they fit
-  static constexpr int ACCS = BN == 64 ? 3 : 2;
-  static constexpr int ACC_BUFS = (4 * BN <= 512) ? 2 : 1;
+  // main + correction accumulators, double-buffered across tiles when they
+  // fit; 64-wide tiles: the main and five of corrections (mma_issue_loop)
+  static constexpr int ACCS = BN == 64 ? 6 : 2;
+  static constexpr int ACC_BUFS = (BN != 64 && 4 * BN <= 512) ? 2 : 1;
   static constexpr uint32_t ACC_COLS = ACCS * BN;
   static constexpr uint32_t TMEM_COLS = BN == 64 ? 512 : ACC_BUFS * ACC_COLS;
   static_assert(ACC_BUFS * ACC_COLS <= TMEM_COLS, "tensor memory");
