@@ -55,14 +55,13 @@ __device__ __forceinline__ void fma2(Acc2& acc, Acc2 a, Acc2 b) {
 
 // Which dimension a pair of accumulators spans.  The operand whose fragment
 // already lies in register pairs (float4 loads of consecutive rows or columns)
-// is the paired one, and the other is broadcast, which costs nothing; pairs
-// assembled from two loads cost a move each (4096^3 NT: 35 TFLOP/s).  Where
-// both operands are k-contiguous, a pair is an even and an odd k of the same
-// element, added at the end: no moves, but twice the accumulators, so an 8 x 8
-// block is the largest.
-enum class Pair { kN, kM, kK };
+// is the paired one, and the other is broadcast, which costs nothing.  Where
+// both operands are k-contiguous there is none: pairs assembled from two loads
+// cost a move each (4096^3 NT: 35 TFLOP/s, 49 with scalar FMAs), and an even and
+// an odd k of one element, summed apart, would be another order of summation.
+enum class Pair { kN, kM, kNone };
 template <bool AK, bool BKM>
-constexpr Pair pair_of() { return !BKM ? Pair::kN : !AK ? Pair::kM : Pair::kK; }
+constexpr Pair pair_of() { return !BKM ? Pair::kN : !AK ? Pair::kM : Pair::kNone; }
 
 template <int TM, int TN, Pair P>
 struct AccTile {
@@ -77,9 +76,19 @@ struct AccTile {
   __device__ __forceinline__ float get(int i, int j) const {
     float lo, hi;
     unpack2(v[P == Pair::kM ? i / 2 : i][P == Pair::kN ? j / 2 : j], lo, hi);
-    if (P == Pair::kK) return lo + hi;
     return ((P == Pair::kM ? i : j) & 1) ? hi : lo;
   }
+};
+template <int TM, int TN>
+struct AccTile<TM, TN, Pair::kNone> {
+  float v[TM][TN];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) v[i][j] = 0.f;
+  }
+  __device__ __forceinline__ float get(int i, int j) const { return v[i][j]; }
 };
 
 // One k-slice (kBK deep) of the register-blocked product, consumed from a
@@ -125,17 +134,14 @@ __device__ __forceinline__ void simt_consume(const float* As, const float* Bs,
           b4[j] = *reinterpret_cast<const float4*>(Bs + c * kBK + 4 * swz_chunk(tx, q));
         }
       }
-      if constexpr (P == Pair::kK) {
+      if constexpr (P == Pair::kNone) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-          for (int i = 0; i < TM; ++i) {
-            const Acc2 a2 = h == 0 ? pack2(a4[i].x, a4[i].y) : pack2(a4[i].z, a4[i].w);
+          for (int i = 0; i < TM; ++i)
 #pragma unroll
             for (int j = 0; j < JG; ++j)
-              fma2(acc.v[i][jg * JG + j], a2,
-                   h == 0 ? pack2(b4[j].x, b4[j].y) : pack2(b4[j].z, b4[j].w));
-          }
+              acc.v[i][jg * JG + j] = fmaf(el(a4[i], kk), el(b4[j], kk), acc.v[i][jg * JG + j]);
       } else {
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
@@ -258,7 +264,7 @@ __device__ __forceinline__ void raster_tile(int local, int tiles_m, int tiles_n,
 }
 
 template <int TM, int TN, bool AK, bool BKM>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, AK && BKM ? 1 : 2)
     simt_sgemm_kernel(const __grid_constant__ CUtensorMap tmA,
                       const __grid_constant__ CUtensorMap tmB, float* __restrict__ C, int M,
                       int N, int K, int ldc, float alpha, float beta, Epilogue epi, int tiles_m,
@@ -388,7 +394,7 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
   const int b = blockIdx.x;
   int tile_m, tile_n;
   if (b < wide_tiles) {
-    if constexpr (pair_of<AK, BKM>() != Pair::kK) {
+    if constexpr (pair_of<AK, BKM>() != Pair::kNone) {
       raster_tile(b, tiles_m, tiles_n, tile_m, tile_n);
       simt_np_tile<8, 16, AK, BKM>(smem, tmA, tmB, C, M, N, K, ldc, alpha, beta, epi,
                                    tile_m * 128, tile_n * 256, err);
@@ -584,7 +590,7 @@ int sm_count() {
 
 // The producer-less kernel's tiles for an M x N output.  A wave of 128 x 128
 // tiles takes kNarrowCost of a wave of 128 x 256 tiles (97 and 174 us per 1024
-// k; pairs along k have no wide tiles).  Wide tiles fill whole waves of SMs;
+// k; without pairs there are no wide tiles).  Wide tiles fill whole waves of SMs;
 // what is left of them runs as narrow ones when those fit in one wave, and
 // everything runs narrow where that takes fewer waves' time (a right edge that
 // leaves half of the wide tiles empty).
@@ -642,7 +648,7 @@ ugemm_status launch_t(const Gemm& g, int tile, const float* A, int lda, const fl
     auto kern = simt_sgemm_np_kernel<AK, BKM>;
     static std::atomic<uint64_t> attr_done{0};
     if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
-    constexpr bool wide_ok = pair_of<AK, BKM>() != Pair::kK;
+    constexpr bool wide_ok = pair_of<AK, BKM>() != Pair::kNone;
     NpTiles t = np_tiles(g.M, g.N, wide_ok, sm_count());
     const int total = t.tiles_m * t.tiles_n;
     if (tile == kSimt128x128) t.wide = 0;
