@@ -371,9 +371,7 @@ void backward_geometry(const Stack* s, const Stack::Layer& L, ugemm::Gemm* b) {
   const int kk = d.ksize * d.ksize, npix = static_cast<int>(L.n);
   const int in_px = s->batch * d.height * d.width;
   const bool direct = d.stride == 1 && d.pad <= d.ksize - 1;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_sms();
   double best = 1e300;
   for (int bn : {64, 128, 256}) {
     const GeoChoice w = choose_geometry(3, d.cout, kk * static_cast<int>(align_up(d.cin, 64)),

@@ -142,9 +142,8 @@ __device__ __forceinline__ void splitk_reduce_taps(const ReduceJob& J, float* bu
   }
 }
 
-__global__ void __launch_bounds__(256, 6) splitk_reduce_kernel(const ReduceJob* __restrict__ jobs) {
+__device__ __forceinline__ void splitk_reduce_job(const ReduceJob& J) {
   __shared__ float sums[4][256];
-  const ReduceJob J = jobs[blockIdx.y];
   // (with too few such blocks to fill the SMs, as for a 64 x 576 gradient of 30
   // slices, the groups of slices above are faster: 4 us against 8)
   if (J.kk > 0 && J.kk <= kReduceTaps && J.M * ((J.chans + 63) / 64) >= 304) {
@@ -160,16 +159,49 @@ __global__ void __launch_bounds__(256, 6) splitk_reduce_kernel(const ReduceJob* 
     splitk_reduce_body<1>(J, sums);
 }
 
+__global__ void __launch_bounds__(256, 6) splitk_reduce_kernel(const ReduceJob* __restrict__ jobs) {
+  pdl_trigger();
+  pdl_wait();
+  splitk_reduce_job(jobs[blockIdx.y]);
+}
+
+struct ReduceTable {
+  ReduceJob jobs[kMultiMax];
+};
+__global__ void __launch_bounds__(256, 6)
+    splitk_reduce_param_kernel(const __grid_constant__ ReduceTable t) {
+  pdl_trigger();
+  pdl_wait();
+  splitk_reduce_job(t.jobs[blockIdx.y]);
+}
+
+dim3 reduce_grid(long long max_mn, int njobs) {
+  return dim3(static_cast<unsigned>(std::min<long long>((max_mn + 63) / 64, 152LL * 12)), njobs);
+}
+
 }  // namespace
 
 ugemm_status splitk_reduce_launch(const ReduceJob* jobs, int njobs, long long max_mn,
                                   cudaStream_t st) {
   if (njobs <= 0) return UGEMM_OK;
-  const long long blocks = std::min<long long>((max_mn + 63) / 64, 152LL * 12);
   prof_begin(st);
-  splitk_reduce_kernel<<<dim3(static_cast<unsigned>(blocks), njobs), 256, 0, st>>>(jobs);
+  const cudaError_t e =
+      launch_dependent(splitk_reduce_kernel, reduce_grid(max_mn, njobs), 256, 0, st, jobs);
   prof_end(st, kProfAux);
-  return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
+  return e == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
+}
+
+ugemm_status splitk_reduce_param_launch(const ReduceJob* jobs, int njobs, long long max_mn,
+                                        cudaStream_t st) {
+  if (njobs <= 0) return UGEMM_OK;
+  if (njobs > kMultiMax) return UGEMM_ERR_ARG;
+  ReduceTable t{};
+  for (int i = 0; i < njobs; ++i) t.jobs[i] = jobs[i];
+  prof_begin(st);
+  const cudaError_t e =
+      launch_dependent(splitk_reduce_param_kernel, reduce_grid(max_mn, njobs), 256, 0, st, t);
+  prof_end(st, kProfAux);
+  return e == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }
 
 }  // namespace ugemm
@@ -404,8 +436,7 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     if (p->cfg.block_n != 64 && p->cfg.block_n != 128) p->cfg.block_n = 128;
   }
   cudaGetDevice(&p->device);
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+  const int sms = device_sms();
   // Untuned plans of three pieces: one problem takes the tile width, the
   // orientation and the k slices that its measured stage and tile times make
   // fastest; 64-wide tiles exist for these only.

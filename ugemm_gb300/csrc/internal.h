@@ -8,6 +8,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <string>
+#include <utility>
 
 #include "../../include/sgemm_cuda.h"
 
@@ -227,7 +228,54 @@ bool smem_attr_once(Kernel kern, size_t bytes, std::atomic<uint64_t>& done) {
   done.fetch_or(bit, std::memory_order_release);
   return true;
 }
+// SMs of the current device (looked up once per device; 148 if that fails).
+inline int device_sms() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      return 148;
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
 ugemm_status scale_c_launch(const Gemm& g, cudaStream_t st);  // C = beta*C (or 0)
+
+// Programmatic dependent launch: a kernel launched with launch_dependent may
+// start while the kernel before it in the stream still runs, once all of that
+// kernel's blocks have called pdl_trigger (or ended), and every one of its
+// threads calls pdl_wait before it touches global memory: from there on the
+// earlier kernel, and by its own wait all before it, are complete.  Launch
+// latency and the prologue (barriers, tensor memory) then overlap the earlier
+// kernel's end.  A sequence's first kernel is launched normally.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, int threads, size_t smem,
+                             cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  // within a captured graph plain edges are as fast (12-layer stack: 1745 us,
+  // 1829 with programmatic ones)
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  cfg.numAttrs = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+#endif
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
@@ -235,6 +283,7 @@ inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 // alpha * (its partial product) to part + s*M*N (row-major, ld N).  The
 // reduce forms C = sum_s part_s + beta*C (C not read when beta == 0), then
 // the optional bias / activation, summing the slices in a fixed order.
+constexpr int kMultiMax = 4;
 // kk > 0: the partial tiles' columns are (tap, channel) with `cpad` channels
 // a tap, C's are channel * kk + tap (part_n = kk * cpad columns, N = kk * chans).
 struct ReduceJob {
@@ -247,10 +296,12 @@ struct ReduceJob {
 };
 ugemm_status splitk_reduce_launch(const ReduceJob* jobs, int njobs, long long max_mn,
                                   cudaStream_t st);
+// The same for up to kMultiMax jobs in host memory, passed as a parameter.
+ugemm_status splitk_reduce_param_launch(const ReduceJob* jobs, int njobs, long long max_mn,
+                                        cudaStream_t st);
 
 // Up to kMultiMax split-precision GEMMs (and split-K slices of them) in one
 // persistent launch, scratch in the caller's workspace (multi.cu).
-constexpr int kMultiMax = 4;
 bool multi_wanted(const Gemm& g, const SplitPlan& p);  // under-filled, deep k
 size_t multi_scratch_bytes(const Gemm* gs, int n, const SplitPlan& p);
 ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& p, Scratch ws, int* dev_err,

@@ -1,21 +1,21 @@
 // multi.cu -- a few split-precision GEMMs, and split-K slices of them, in one
 // persistent launch of the grouped tensor-core kernel, with all scratch in
 // the caller's workspace: no plan, no allocation, nothing read from host
-// memory at run time (the problem table travels as a kernel parameter), so
+// memory at run time (the problem table is the GEMM kernel's parameter), so
 // it is usable inside stream capture.
 //
 // Used where one GEMM launch at a time leaves SMs idle:
 //   * ugemm_sgemm_backward: dA = alpha dC op(B)^T and dB = alpha op(A)^T dC
 //     share one launch, so the tiles of both fill the GPU together;
-//   * single GEMMs whose output has fewer tiles than the GPU has SMs and
-//     whose k is deep (a weight-gradient shape): cut into k slices whose
-//     FP32 partial tiles one reduce launch sums in a fixed order.
+//   * single GEMMs whose whole tiles leave SMs idle: narrower tiles, or k
+//     slices whose FP32 partial tiles one reduce launch sums in a fixed order.
 // Each GEMM may also be computed transposed (C^T = op(B)^T op(A)^T) when
 // that wastes less of the 128-row tiles, as in grouped plans.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstddef>
 #include <cstring>
 
@@ -25,112 +25,81 @@
 namespace ugemm {
 namespace {
 
-constexpr int kMultiSubs = 24;  // kernel problems (slices) per launch
-constexpr int kMinSlice = 16;   // shortest slice, in 32-deep k-blocks
+static_assert(sizeof(MultiTable) <= 16384, "a kernel parameter, copied at every launch");
 
-// The shortest slice in stages of the kernel's k depth.
-int min_slice(int pieces) { return kMinSlice * kTcKB / split_stage_k(pieces); }
+constexpr int kMinSlice = 16;  // shortest slice of several GEMMs', in k-blocks
 
-// Everything the launch reads from device memory, filled by one small kernel
-// from its by-value parameter (at most 4 KB of parameters).
-struct MultiTable {
-  CUtensorMap maps[2 * kMultiMax];
-  TcProblem probs[kMultiSubs];
-  ReduceJob red[kMultiMax];
-};
-static_assert(sizeof(MultiTable) <= 4000, "multi table must fit the kernel parameter space");
-static_assert(sizeof(MultiTable) % 16 == 0, "multi table copies as 16-byte words");
-
-// Block 0 copies the table; every thread also writes the tile table of a
-// grid of `grid` CTAs: CTA c takes tiles c, c + grid, c + 2 grid, ... (in
-// longest-k-first problem order), stored contiguously after the grid's
-// {first, end} ranges, one {problem, m0, n0, 0} record per tile.
-__global__ void multi_table_kernel(const __grid_constant__ MultiTable t, int nsub, int total_tiles,
-                                   int block_n, int grid, MultiTable* dst, int4* table) {
-  if (blockIdx.x == 0) {
-    const uint4* s = reinterpret_cast<const uint4*>(&t);
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    for (int i = threadIdx.x; i < static_cast<int>(sizeof(MultiTable) / 16); i += blockDim.x)
-      d[i] = s[i];
-    // the GEMM kernel reads the tensor maps through the tensormap proxy
-    asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");
-  }
-  const int per = total_tiles / grid, extra = total_tiles % grid;
-  auto first = [&](int c) { return c * per + (c < extra ? c : extra); };
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < grid; c += gridDim.x * blockDim.x)
-    table[c] = make_int4(first(c), first(c + 1), 0, 0);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total_tiles; i += gridDim.x * blockDim.x) {
-    int p = 0;
-    while (p + 1 < nsub && t.probs[p + 1].tile_start <= i) ++p;
-    const TcProblem& P = t.probs[p];
-    int m0, n0;
-    tc_raster(i - P.tile_start, P.tiles_m, P.tiles_n, block_n, m0, n0);
-    table[grid + first(i % grid) + i / grid] = make_int4(p, m0, n0, 0);
-  }
+MultiTable empty_table() {
+  MultiTable t;
+  std::memset(&t, 0, sizeof t);
+  for (TcProblem& p : t.probs) p.tile_start = INT_MAX;
+  return t;
 }
 
 double padded(int rows, int cols, int bn) {
   return double(align_up(rows, 128)) * ((cols / bn) * bn + align_up(cols % bn, 16));
 }
 
-int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
-struct Geo {
-  bool swap = false;
-  int tiles = 0, nkb = 0, slices = 1, per = 0;
-};
-
 // Scratch layout: per GEMM [A pieces | B pieces], then the partial tiles of
-// the sliced GEMMs, the table and the tile records.
+// the sliced GEMMs.
 struct Layout {
-  Geo geo[kMultiMax];
+  GeoChoice geo[kMultiMax];
   int block_n = 256;
   size_t a_off[kMultiMax], b_off[kMultiMax], part_off[kMultiMax];
-  size_t table_off = 0, recs_off = 0, total = 0;
-  int grid = 1;  // persistent CTAs of the launch
+  size_t total = 0;
+  double us = 0;  // one GEMM: the model's time of the launch and its reduce
 };
 
+// One GEMM: the tile width and slices of the least time by the stage times.
+// Several: 256-wide tiles unless every output is narrow, and slices no longer
+// than half an SM's fair share, which round robin then balances (2048 x 8192 x
+// 1024 backward: 342 us, 435 with whole tiles on each GEMM's share of the SMs).
 Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
   Layout L;
-  // 256-wide tiles unless every output is narrow in its better orientation
-  int widest = 0;
-  for (int i = 0; i < n; ++i) {
-    const Gemm& g = gs[i];
-    const bool swap = padded(g.N, g.M, 256) < padded(g.M, g.N, 256);
-    widest = std::max(widest, swap ? g.M : g.N);
-  }
-  L.block_n = widest > 128 ? 256 : 128;
-  double work = 0;
-  for (int i = 0; i < n; ++i) {
-    const Gemm& g = gs[i];
-    Geo& o = L.geo[i];
-    o.swap = padded(g.N, g.M, L.block_n) < padded(g.M, g.N, L.block_n);
-    const int rows = o.swap ? g.N : g.M, cols = o.swap ? g.M : g.N;
-    o.tiles = cdiv(rows, kTcBM) * cdiv(cols, L.block_n);
-    o.nkb = split_nkb(p.pieces, g.K);
-    o.per = o.nkb;
-    work += double(o.tiles) * o.nkb;
-  }
-  // split-K: tiles no longer than about half an SM's fair share of the work
-  const double fair = work / (2.0 * sms);
-  int subs = n;
-  for (int i = 0; i < n; ++i) {
-    const Gemm& g = gs[i];
-    Geo& o = L.geo[i];
-    if (o.nkb < 2 * min_slice(p.pieces) || o.nkb <= fair) continue;
-    const int len = std::max(min_slice(p.pieces), static_cast<int>(fair) + 1);
-    const size_t tile_bytes = size_t(g.M) * g.N * 4;
-    int sl = std::min(cdiv(o.nkb, len), kMultiSubs - (subs - 1));
-    sl = static_cast<int>(std::min<size_t>(sl, (size_t(512) << 20) / tile_bytes));
-    if (sl < 2) continue;
-    o.per = cdiv(o.nkb, sl);
-    o.slices = cdiv(o.nkb, o.per);
-    subs += o.slices - 1;
+  auto most = [&](const Gemm& g) {  // slices whose partial tiles take 512 MiB
+    return std::max(1, static_cast<int>(std::min(1e9, double(512 << 20) / (double(g.M) * g.N * 4))));
+  };
+  if (n == 1) {
+    L.us = 1e300;
+    for (int bn : {64, 128, 256}) {
+      if (bn == 64 && p.pieces != 3) continue;
+      const GeoChoice c = choose_geometry(p.pieces, gs[0].M, gs[0].N, split_nkb(p.pieces, gs[0].K),
+                                          sms, bn, true, std::min(kMultiSubs, most(gs[0])));
+      if (c.us >= L.us) continue;
+      L.us = c.us;
+      L.block_n = bn;
+      L.geo[0] = c;
+    }
+  } else {
+    int widest = 0;
+    for (int i = 0; i < n; ++i) {
+      const Gemm& g = gs[i];
+      widest = std::max(widest, padded(g.N, g.M, 256) < padded(g.M, g.N, 256) ? g.M : g.N);
+    }
+    L.block_n = widest > 128 ? 256 : 128;
+    double work = 0;
+    int tiles[kMultiMax], nkb[kMultiMax];
+    for (int i = 0; i < n; ++i) {
+      const Gemm& g = gs[i];
+      GeoChoice& o = L.geo[i];
+      o.swap = padded(g.N, g.M, L.block_n) < padded(g.M, g.N, L.block_n);
+      tiles[i] = cdiv(o.swap ? g.N : g.M, kTcBM) * cdiv(o.swap ? g.M : g.N, L.block_n);
+      nkb[i] = split_nkb(p.pieces, g.K);
+      o.per = nkb[i];
+      work += double(tiles[i]) * nkb[i];
+    }
+    const double fair = work / (2.0 * sms);
+    int subs = n;
+    for (int i = 0; i < n; ++i) {
+      GeoChoice& o = L.geo[i];
+      if (nkb[i] < 2 * kMinSlice || nkb[i] <= fair) continue;
+      const int len = std::max(kMinSlice, static_cast<int>(fair) + 1);
+      const int sl = std::min({cdiv(nkb[i], len), kMultiSubs - (subs - 1), most(gs[i])});
+      if (sl < 2) continue;
+      o.per = cdiv(nkb[i], sl);
+      o.slices = cdiv(nkb[i], o.per);
+      subs += o.slices - 1;
+    }
   }
   size_t off = 0;
   for (int i = 0; i < n; ++i) {
@@ -143,12 +112,7 @@ Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
     L.part_off[i] = off;
     if (L.geo[i].slices > 1) off += align_up(size_t(L.geo[i].slices) * gs[i].M * gs[i].N * 4, 256);
   }
-  L.table_off = align_up(off, 256);
-  int tiles = 0;
-  for (int i = 0; i < n; ++i) tiles += L.geo[i].tiles * L.geo[i].slices;
-  L.grid = std::max(1, std::min(tiles, sms));
-  L.recs_off = L.table_off + align_up(sizeof(MultiTable), 256);
-  L.total = L.recs_off + align_up(size_t(L.grid + tiles) * sizeof(int4), 256);
+  L.total = align_up(off, 256);
   return L;
 }
 
@@ -157,10 +121,10 @@ Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
 TailPlan tail_plan(const Gemm& g, const SplitPlan& p) {
   TailPlan t;
   if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return t;
-  const int sms = sm_count();
+  const int sms = device_sms();
   const int tiles_m = cdiv(g.M, kTcBM), tiles_n = cdiv(g.N, p.block_n);
   const int tiles = tiles_m * tiles_n, rem = tiles % sms;
-  if (tiles <= sms || rem == 0 || split_nkb(p.pieces, g.K) < 2 * min_slice(p.pieces)) return t;
+  if (tiles <= sms || rem == 0 || split_nkb(p.pieces, g.K) < 32) return t;
   // the raster order ends with the last group of tile rows, column by column
   const int first_m = ((tiles_m - 1) / kTcRaster) * kTcRaster, rows = tiles_m - first_m;
   const int cols = cdiv(rem, rows);             // whole tile columns of that group
@@ -175,9 +139,7 @@ TailPlan tail_plan(const Gemm& g, const SplitPlan& p) {
 size_t tail_scratch_bytes(const Gemm& g, const SplitPlan& p) {
   const TailPlan t = tail_plan(g, p);
   if (!t.use) return 0;
-  const int tiles = 2 * cdiv(g.M - t.r0, kTcBM) * cdiv(g.N - t.c0, p.block_n);
-  return align_up(2 * size_t(g.M - t.r0) * (g.N - t.c0) * 4, 256) +
-         align_up(sizeof(MultiTable), 256) + align_up(size_t(sm_count() + tiles) * sizeof(int4), 256);
+  return align_up(2 * size_t(g.M - t.r0) * (g.N - t.c0) * 4, 256);
 }
 
 ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail,
@@ -185,12 +147,8 @@ ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail
                          cudaStream_t st) {
   const int Mt = g.M - tail.r0, Nt = g.N - tail.c0, Kp = split_kp(g.K);
   const size_t mn = size_t(Mt) * Nt;
-  uint8_t* base = static_cast<uint8_t*>(scratch);
-  float* part = reinterpret_cast<float*>(base);
-  uint8_t* tab = base + align_up(2 * mn * 4, 256);
-  int4* recs = reinterpret_cast<int4*>(tab + align_up(sizeof(MultiTable), 256));
-  MultiTable t;
-  std::memset(&t, 0, sizeof t);
+  float* part = static_cast<float*>(scratch);
+  MultiTable t = empty_table();
   const size_t row_bytes = size_t(Kp) * piece_bytes(p.pieces);
   const auto* ap = static_cast<const uint8_t*>(a_pieces) + size_t(tail.r0) * row_bytes;
   const auto* bp = static_cast<const uint8_t*>(b_pieces) + size_t(tail.c0) * row_bytes;
@@ -220,13 +178,7 @@ ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail
   }
   Epilogue epi = g.epi;
   if (epi.bias) epi.bias += tail.r0;
-  t.red[0] = ReduceJob{part, g.C + size_t(tail.r0) * g.ldc + tail.c0, Mt, Nt, g.ldc, 2, g.beta, epi};
-  const int grid = std::max(1, std::min(tiles, sm_count()));
-  prof_begin(st);
-  multi_table_kernel<<<std::max(1, std::min(cdiv(tiles, 256), 64)), 256, 0, st>>>(
-      t, 2, tiles, p.block_n, grid, reinterpret_cast<MultiTable*>(tab), recs);
-  prof_end(st, kProfControl);
-  if (cudaPeekAtLastError() != cudaSuccess) return UGEMM_ERR_CUDA;
+  const ReduceJob red{part, g.C + size_t(tail.r0) * g.ldc + tail.c0, Mt, Nt, g.ldc, 2, g.beta, epi};
   SplitPlan q = p;
   q.epi = false;
   CUtensorMap dummy;
@@ -234,24 +186,30 @@ ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail
   TcProblem single{};
   const int chunk =
       split_chunk_stages(p.pieces, p.chunk_kb > 0 ? p.chunk_kb : split_default_chunk_kb(g.K));
-  ugemm_status s = split_gemm_launch(
-      q, dummy, dummy, single, reinterpret_cast<const CUtensorMap*>(tab + offsetof(MultiTable, maps)),
-      reinterpret_cast<const TcProblem*>(tab + offsetof(MultiTable, probs)), recs, tiles, chunk,
-      grid, dev_err, st);
-  if (s != UGEMM_OK) return s;
-  return splitk_reduce_launch(reinterpret_cast<const ReduceJob*>(tab + offsetof(MultiTable, red)),
-                              1, static_cast<long long>(mn), st);
+  const ugemm_status s =
+      split_gemm_launch(q, dummy, dummy, single, nullptr, nullptr, nullptr, tiles, chunk,
+                        std::max(1, std::min(tiles, device_sms())), dev_err, st, nullptr, &t);
+  return s != UGEMM_OK ? s
+                       : splitk_reduce_param_launch(&red, 1, static_cast<long long>(mn), st);
 }
 
+// Whether a GEMM runs here rather than as one launch of whole 256- (or, up to
+// 128 columns, 128-) wide tiles: when narrower tiles or k slices are faster by
+// the stage times, as they are where whole tiles leave SMs idle (1024^3: 32 tiles
+// of 256; 2048^3: one wave of 128 of the 152 SMs).
 bool multi_wanted(const Gemm& g, const SplitPlan& p) {
   if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return false;
+  const int sms = device_sms();
   const int tiles = cdiv(g.M, kTcBM) * cdiv(g.N, p.block_n);
-  return tiles < sm_count() && split_nkb(p.pieces, g.K) >= 2 * min_slice(p.pieces);
+  if (tiles > 4 * sms) return false;
+  const GeoChoice whole = choose_geometry(p.pieces, g.M, g.N, split_nkb(p.pieces, g.K), sms,
+                                          p.block_n, false, 1);
+  return layout_for(&g, 1, p, sms).us < 0.95 * whole.us;
 }
 
 size_t multi_scratch_bytes(const Gemm* gs, int n, const SplitPlan& p) {
   if (n < 1 || n > kMultiMax) return 0;
-  return layout_for(gs, n, p, sm_count()).total;
+  return layout_for(gs, n, p, device_sms()).total;
 }
 
 ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch ws, int* dev_err,
@@ -259,15 +217,15 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
   if (n < 1 || n > kMultiMax) return UGEMM_ERR_ARG;
   for (int i = 0; i < n; ++i)
     if (gs[i].M == 0 || gs[i].N == 0 || gs[i].K == 0 || gs[i].alpha == 0.f) return UGEMM_ERR_ARG;
-  const Layout L = layout_for(gs, n, plan, sm_count());
+  const Layout L = layout_for(gs, n, plan, device_sms());
   if (L.total > ws.bytes) return UGEMM_ERR_ARENA_TOO_SMALL;
   uint8_t* base = static_cast<uint8_t*>(ws.ptr);
   SplitPlan p = plan;
   p.block_n = L.block_n;
   p.epi = false;
 
-  MultiTable t;
-  std::memset(&t, 0, sizeof t);
+  MultiTable t = empty_table();
+  ReduceJob red[kMultiMax];
   SplitJobTable jt{};
   static_assert(2 * kMultiMax <= kSplitTableJobs, "two operands per GEMM");
   int nj = 0, split_tiles = 0;
@@ -275,7 +233,8 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
   long long red_max = 0;
   for (int i = 0; i < n; ++i) {
     const Gemm& g = gs[i];
-    const Geo& o = L.geo[i];
+    const GeoChoice& o = L.geo[i];
+    const int nkb = split_nkb(p.pieces, g.K);
     void* ap = base + L.a_off[i];
     void* bp = base + L.b_off[i];
     long long a_sr, a_sk, b_sr, b_sk;
@@ -309,7 +268,7 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
       tp.alpha = g.alpha;
       tp.beta = sliced ? 0.f : g.beta;
       tp.kb0 = sidx * o.per;
-      tp.nkb = std::min(o.per, o.nkb - tp.kb0);
+      tp.nkb = std::min(o.per, nkb - tp.kb0);
       tp.tiles_m = cdiv(tp.M, kTcBM);
       tp.tiles_n = cdiv(tp.N, p.block_n);
       tp.swap = o.swap ? 1 : 0;
@@ -324,7 +283,7 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
       }
     }
     if (sliced) {
-      t.red[nred++] = ReduceJob{part, g.C, g.M, g.N, g.ldc, o.slices, g.beta, g.epi};
+      red[nred++] = ReduceJob{part, g.C, g.M, g.N, g.ldc, o.slices, g.beta, g.epi};
       red_max = std::max(red_max, static_cast<long long>(g.M) * g.N);
     }
   }
@@ -343,25 +302,15 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
     const ugemm_status s = split_param_launch(p.pieces, jt, nj, split_tiles, st);
     if (s != UGEMM_OK) return s;
   }
-  uint8_t* tab = base + L.table_off;
-  int4* recs = reinterpret_cast<int4*>(base + L.recs_off);
-  prof_begin(st);
-  multi_table_kernel<<<std::max(1, std::min(cdiv(tiles, 256), 64)), 256, 0, st>>>(
-      t, nsub, tiles, p.block_n, L.grid, reinterpret_cast<MultiTable*>(tab), recs);
-  prof_end(st, kProfControl);
-  if (cudaPeekAtLastError() != cudaSuccess) return UGEMM_ERR_CUDA;
   CUtensorMap dummy;
   std::memset(&dummy, 0, sizeof dummy);
   TcProblem single{};
   const int chunk =
       split_chunk_stages(p.pieces, p.chunk_kb > 0 ? p.chunk_kb : split_default_chunk_kb(min_k));
-  ugemm_status s = split_gemm_launch(
-      p, dummy, dummy, single, reinterpret_cast<const CUtensorMap*>(tab + offsetof(MultiTable, maps)),
-      reinterpret_cast<const TcProblem*>(tab + offsetof(MultiTable, probs)), recs, tiles, chunk,
-      L.grid, dev_err, st);
-  if (s != UGEMM_OK || nred == 0) return s;
-  return splitk_reduce_launch(reinterpret_cast<const ReduceJob*>(tab + offsetof(MultiTable, red)),
-                              nred, red_max, st);
+  const ugemm_status s =
+      split_gemm_launch(p, dummy, dummy, single, nullptr, nullptr, nullptr, tiles, chunk,
+                        std::max(1, std::min(tiles, device_sms())), dev_err, st, nullptr, &t);
+  return s != UGEMM_OK ? s : splitk_reduce_param_launch(red, nred, red_max, st);
 }
 
 }  // namespace ugemm

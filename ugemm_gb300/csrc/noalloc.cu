@@ -146,8 +146,12 @@ extern "C" UGEMM_API int ugemm_sgemm_dev_noalloc(char major, char transa, char t
     s = scale_c_launch(g, st);
     return s == UGEMM_OK ? s : fail(s, "scale launch failed");
   }
+  // the same route as the workspace entry point's, unless only whole tiles,
+  // which need no partial ones, fit the array
   const SplitPlan plan = split_plan_for(form, g);
-  const size_t need = split_scratch_bytes(g, plan);
+  const bool multi =
+      multi_wanted(g, plan) && multi_scratch_bytes(&g, 1, plan) <= kNoAllocScratchBytes;
+  const size_t need = multi ? 0 : split_scratch_bytes(g, plan);
   if (need > kNoAllocScratchBytes) {
     char msg[160];
     std::snprintf(msg, sizeof msg,
@@ -163,7 +167,8 @@ extern "C" UGEMM_API int ugemm_sgemm_dev_noalloc(char major, char transa, char t
   prof_end(st, kProfControl);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(UGEMM_ERR_CUDA, cudaGetErrorString(e));
-  s = split_launch(g, plan, Scratch{slot->scratch, kNoAllocScratchBytes}, slot->err, st);
+  const Scratch ws{slot->scratch, kNoAllocScratchBytes};
+  s = multi ? multi_launch(&g, 1, plan, ws, slot->err, st) : split_launch(g, plan, ws, slot->err, st);
   if (s != UGEMM_OK) {
     const cudaError_t le = cudaGetLastError();
     return fail(s, le != cudaSuccess ? cudaGetErrorString(le) : "split launch failed");

@@ -224,41 +224,45 @@ __host__ __device__ constexpr uint32_t umma_idesc(uint32_t a_fmt, uint32_t b_fmt
 }
 
 // Descriptors come as their two words: the upper one is the same for a whole
-// launch, and the lower one is a 32-bit sum.
+// launch, and the lower one is a 32-bit sum.  A converged warp executes the call;
+// the lane whose `issue` is set issues the MMA (a predicate, not a branch: in a
+// branch of one lane the compiler keeps the operands in vector registers).
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint32_t alo, uint32_t ahi,
                                           uint32_t blo, uint32_t bhi, uint32_t idesc,
-                                          uint32_t accumulate) {
+                                          uint32_t accumulate, uint32_t issue) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, i;\n"
       ".reg .b64 a, b;\n"
       "mov.b64 a, {%1, %2};\n"
       "mov.b64 b, {%3, %4};\n"
       "setp.ne.b32 p, %6, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n"
+      "setp.ne.b32 i, %7, 0;\n"
+      "@i tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n"
       "}\n" ::"r"(tmem_d),
-      "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate)
+      "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
 
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint32_t alo, uint32_t ahi,
                                           uint32_t blo, uint32_t bhi, uint32_t idesc,
-                                          uint32_t accumulate) {
+                                          uint32_t accumulate, uint32_t issue) {
   asm volatile(
       "{\n"
-      ".reg .pred p;\n"
+      ".reg .pred p, i;\n"
       ".reg .b64 a, b;\n"
       "mov.b64 a, {%1, %2};\n"
       "mov.b64 b, {%3, %4};\n"
       "setp.ne.b32 p, %6, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %5, p;\n"
+      "setp.ne.b32 i, %7, 0;\n"
+      "@i tcgen05.mma.cta_group::1.kind::tf32 [%0], a, b, %5, p;\n"
       "}\n" ::"r"(tmem_d),
-      "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate)
+      "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate), "r"(issue)
       : "memory");
 }
 
-// One lane of a converged warp, the same one every time.
-__device__ __forceinline__ bool elect_one() {
+// Non-zero in one lane of a converged warp, the same one every time.
+__device__ __forceinline__ uint32_t elect_one() {
   uint32_t ok;
   asm volatile(
       "{\n"
@@ -267,7 +271,7 @@ __device__ __forceinline__ bool elect_one() {
       "selp.u32 %0, 1, 0, p;\n"
       "}\n"
       : "=r"(ok));
-  return ok != 0;
+  return ok;
 }
 
 // Arrive on an mbarrier once all tcgen05 operations issued so far by this

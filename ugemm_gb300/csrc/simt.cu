@@ -580,14 +580,6 @@ void stored_b(const Gemm& g, int& rows, int& cols) {
   if (g.tb == 'N') { rows = g.K; cols = g.N; } else { rows = g.N; cols = g.K; }
 }
 
-int sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return 148;
-  return sms;
-}
-
 // The producer-less kernel's tiles for an M x N output.  A wave of 128 x 128
 // tiles takes kNarrowCost of a wave of 128 x 256 tiles (97 and 174 us per 1024
 // k; without pairs there are no wide tiles).  Wide tiles fill whole waves of SMs;
@@ -649,7 +641,7 @@ ugemm_status launch_t(const Gemm& g, int tile, const float* A, int lda, const fl
     static std::atomic<uint64_t> attr_done{0};
     if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
     constexpr bool wide_ok = pair_of<AK, BKM>() != Pair::kNone;
-    NpTiles t = np_tiles(g.M, g.N, wide_ok, sm_count());
+    NpTiles t = np_tiles(g.M, g.N, wide_ok, device_sms());
     const int total = t.tiles_m * t.tiles_n;
     if (tile == kSimt128x128) t.wide = 0;
     if (tile == kSimt128x256 && wide_ok) t.wide = total;
@@ -681,7 +673,7 @@ int simt_pick_tile(const Gemm& g) {
   if (forced >= 0) return forced;
   // whichever needs less time by the waves' measured costs (2048^3 NN: 348 us
   // mixed, 464 in 64x64 tiles; 1024^3: 99 and 74)
-  const int sms = sm_count();
+  const int sms = device_sms();
   const long small = long(cdiv(g.M, 64)) * cdiv(g.N, 64);
   const double small_cost =
       small <= sms ? kSmallHalfCost : kSmallCost * ((small + 2 * sms - 1) / (2 * sms));
@@ -756,7 +748,7 @@ ugemm_status grouped_t(const CUtensorMap* maps, const SimtProblem* probs, int np
   auto kern = simt_grouped_kernel<TM, TN>;
   static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
   if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
-  const int grid = std::max(1, std::min(total, max_ctas > 0 ? max_ctas : sm_count()));
+  const int grid = std::max(1, std::min(total, max_ctas > 0 ? max_ctas : device_sms()));
   prof_begin(st);
   kern<<<grid, kThreads, S::SMEM, st>>>(maps, probs, nprob, total, dev_err);
   prof_end(st, kProfGrouped);
@@ -775,7 +767,7 @@ ugemm_status simt_grouped_launch(int tile, const CUtensorMap* maps, const SimtPr
 ugemm_status pack_batched_launch(const PackJob* jobs, int njobs, int total_tiles, cudaStream_t st) {
   if (total_tiles <= 0) return UGEMM_OK;
   prof_begin(st);
-  pack_kmajor_batched_kernel<<<std::min(total_tiles, sm_count() * 8), 256, 0, st>>>(jobs, njobs,
+  pack_kmajor_batched_kernel<<<std::min(total_tiles, device_sms() * 8), 256, 0, st>>>(jobs, njobs,
                                                                              total_tiles);
   prof_end(st, kProfSplitPrep);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;

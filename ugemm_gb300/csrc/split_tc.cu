@@ -72,6 +72,12 @@ __device__ __forceinline__ void fence_tensormap(const CUtensorMap* map) {
                : "memory");
 }
 
+// Lane 0's value: the same in every lane already, but known to be so.
+template <typename T>
+__device__ __forceinline__ T uniform(T v) {
+  return __shfl_sync(0xffffffffu, v, 0);
+}
+
 struct TileCoord { int p, m0, n0; };
 
 // Tiles of this CTA: a grouped launch walks its own slice of the planned tile
@@ -79,14 +85,16 @@ struct TileCoord { int p, m0, n0; };
 // ranges), one GEMM strides through its tiles by the grid size.
 struct TileRange { int first, end, step; };
 
-template <bool GROUPED>
+// TABLE: the launch may take its problems from a MultiTable (tiles null).
+template <bool GROUPED, bool TABLE>
 __device__ __forceinline__ TileRange tile_range(const int4* tiles, int total_tiles) {
   if constexpr (GROUPED) {
-    const int4 r = tiles[blockIdx.x];
-    return TileRange{r.x, r.y, 1};
-  } else {
-    return TileRange{static_cast<int>(blockIdx.x), total_tiles, static_cast<int>(gridDim.x)};
+    if (!TABLE || tiles != nullptr) {
+      const int4 r = tiles[blockIdx.x];
+      return TileRange{r.x, r.y, 1};
+    }
   }
+  return TileRange{static_cast<int>(blockIdx.x), total_tiles, static_cast<int>(gridDim.x)};
 }
 
 // Tile t of one GEMM in raster order (tc_raster).  Grouped launches read the
@@ -94,11 +102,18 @@ __device__ __forceinline__ TileRange tile_range(const int4* tiles, int total_til
 // n0} per tile, built when the launch is planned: a persistent CTA then pays
 // two dependent loads per tile instead of a binary search through the
 // problem records (each step an L2 round trip).
-template <int BN, bool GROUPED>
+template <int BN, bool GROUPED, bool TABLE>
 __device__ __forceinline__ TileCoord tile_coord(const TcProblem& single, const TcProblem* probs,
                                                 const int4* tiles, int t, TcProblem& P) {
   TileCoord tc;
   if constexpr (GROUPED) {
+    if (TABLE && tiles == nullptr) {  // at most kMultiSubs problems, in the parameter
+      tc.p = 0;
+      while (tc.p + 1 < kMultiSubs && probs[tc.p + 1].tile_start <= t) ++tc.p;
+      P = probs[tc.p];
+      tc_raster(t - P.tile_start, P.tiles_m, P.tiles_n, BN, tc.m0, tc.n0);
+      return tc;
+    }
     const int4 r = tiles[gridDim.x + t];
     tc.p = r.x;
     tc.m0 = r.y;
@@ -317,9 +332,9 @@ __host__ __device__ constexpr uint32_t corr_code(int p) {
 // correction products into their accumulator, the main product into its
 // (restarted at each chunk once the epilogue drained it), commit the stage
 // free; per tile, commit the accumulators full.  An MMA of 128 columns takes
-// 64 cycles, so the issuing itself counts: the warp runs the loop converged and
-// one lane issues, so that descriptors are uniform values, made by 32-bit adds
-// of compile-time offsets to the stage's (the address field counts 16-byte
+// 64 cycles, so the issuing itself counts: the warp runs the loop converged, on
+// values known to be uniform, and one lane's instructions issue; descriptors are
+// 32-bit sums of compile-time offsets and the stage's (the address field counts 16-byte
 // units, and shared memory stays below 256 KB, so the field never carries);
 // the product count is a template parameter, and the chunk position is a
 // counter rather than a remainder.
@@ -338,6 +353,7 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
   constexpr uint32_t SBO = WIDE ? 1024 : 512, SWZ = WIDE ? 2 : 4;
   constexpr int NST = FUSED ? kTcFusedPieceStages : S::STAGES;
   constexpr int NB = S::ACC_BUFS;
+  constexpr bool TABLE = GROUPED && !FUSED && !CONV;
   // instruction descriptor operand format: bf16 pieces (1), the FP16x3
   // form's fp16 pieces (0) or the TF32x3 form's tf32 pieces (2); one k step
   // is 32 bytes of a row in each: 16 16-bit or 8 tf32 elements
@@ -349,7 +365,7 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
   const uint32_t base = smem_u32(smem);
   const uint64_t kmajor = umma_smem_desc(base, SBO, SWZ);
   const uint64_t mnmajor = umma_smem_desc(base, 1024, 2, 4096);
-  const bool leader = elect_one();
+  const uint32_t leader = elect_one();
   uint32_t s = 0, ph = 0, ntile = 0;
   uint32_t nbound[NB] = {};
   auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
@@ -373,8 +389,8 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
     auto mma = [&](uint32_t lo, uint32_t d, int ia, int ib, int kk, uint32_t i, bool keep) {
       const uint32_t a = lo + ((ia * S::A_PLANE + kk * KSTEP) >> 4);
       const uint32_t b = lo + ((S::A_BYTES + ib * S::B_PLANE + kk * KSTEP) >> 4);
-      if constexpr (TF32) umma_tf32(d, a, hi, b, hi, i, keep);
-      else umma_bf16(d, a, hi, b, hi, i, keep);
+      if constexpr (TF32) umma_tf32(d, a, hi, b, hi, i, keep, leader);
+      else umma_bf16(d, a, hi, b, hi, i, keep, leader);
     };
     auto stage_lo = [&](uint32_t st) { return lo0 + st * (S::STAGE_BYTES >> 4); };
     // 64-wide tiles: the B planes lie back to back in the stage, 64 rows each,
@@ -393,7 +409,6 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       }
     };
     auto corrections = [&](uint32_t st, int kbi) {
-      if (!leader) return;
       const uint32_t lo = stage_lo(st);
       if constexpr (STACK) {
 #pragma unroll
@@ -416,7 +431,6 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
     // one 256-row operand), so A0 is read once for both.  Only where both
     // accumulate (not at a chunk start, not in a tile's first k-block).
     auto merged = [&](uint32_t st) {
-      if (!leader) return;
       const uint32_t lo = stage_lo(st);
       if constexpr (STACK) {
 #pragma unroll
@@ -435,7 +449,6 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
       }
     };
     auto main_product = [&](uint32_t st, bool restart) {
-      if (!leader) return;
       const uint32_t lo = stage_lo(st);
 #pragma unroll
       for (int kk = 0; kk < KK; ++kk) mma(lo, t_main, 0, 0, kk, id, !(restart && kk == 0));
@@ -505,10 +518,12 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
     commit(&tile_full[buf]);
     return true;
   };
-  const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
+  TileRange tr = tile_range<GROUPED, TABLE>(tiles, total_tiles);
+  tr.first = uniform(tr.first);
+  tr.end = uniform(tr.end);
   for (int t = tr.first; t < tr.end; t += tr.step, ++ntile) {
     TcProblem P;
-    const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+    const TileCoord tc = tile_coord<BN, GROUPED, TABLE>(single, probs, tiles, t, P);
     // a group's narrow problems and right-edge tiles multiply only the
     // columns that exist (UMMA N in steps of 16)
     uint32_t idesc = idesc_full;
@@ -523,10 +538,10 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
     tc_fence_after();
     bool ok;
     if constexpr (CONV)
-      ok = geo[tc.p].kind == PieceOperands::kPix
-               ? tile(std::true_type{}, P.nkb, idesc, buf)
-               : tile(std::false_type{}, P.nkb, idesc, buf);
-    else ok = tile(std::false_type{}, P.nkb, idesc, buf);
+      ok = uniform(geo[tc.p].kind) == PieceOperands::kPix
+               ? tile(std::true_type{}, uniform(P.nkb), uniform(idesc), buf)
+               : tile(std::false_type{}, uniform(P.nkb), uniform(idesc), buf);
+    else ok = tile(std::false_type{}, uniform(P.nkb), uniform(idesc), buf);
     if (!ok) return;
   }
 }
@@ -594,6 +609,10 @@ __device__ __forceinline__ bool conv_produce(const ConvGeo G, const TcProblem& P
   return true;
 }
 
+// The table parameter of the instantiations that can take one.
+template <bool TABLE> struct TableParam { MultiTable t; };
+template <> struct TableParam<false> {};
+
 // TF32: the TF32x3 form's instantiation (two planes of 32-deep tf32
 // stages, tcgen05 kind::tf32), a template parameter so that the 16-bit
 // instantiations' MMA issue loop carries no branch on the format.
@@ -612,13 +631,21 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
                     const __grid_constant__ TcProblem single, const CUtensorMap* __restrict__ maps,
                     const TcProblem* __restrict__ probs, const int4* __restrict__ tiles,
                     int total_tiles, int nprod,
-                    int chunk_kb, int fmt, const ConvGeo* __restrict__ geo, int* err) {
+                    int chunk_kb, int fmt, const ConvGeo* __restrict__ geo, int* err,
+                    const __grid_constant__ TableParam<GROUPED && !FUSED && !CONV> table) {
   // fmt: 16-bit piece format, 0 bf16, 1 fp16 (FP16x3); TF32 instantiations
   // read two planes of 32-deep stages with the 128-byte rows of the
   // two-piece 16-bit shape
   static_assert(!TF32 || NP == 2, "TF32 pieces come in two planes");
   static_assert(!FUSED || (NP == 3 && GROUPED && !TF32), "fused: grouped bf16x3-piece launches");
   static_assert(!CONV || (NP == 3 && GROUPED && !FUSED), "conv: grouped launches on bf16 pieces");
+  constexpr bool TABLE = GROUPED && !FUSED && !CONV;
+  if constexpr (TABLE) {
+    if (probs == nullptr) {
+      probs = table.t.probs;
+      maps = table.t.maps;
+    }
+  }
   // 256-wide fused tiles: the epilogue warps are the converters
   constexpr bool DUAL = FUSED && BN == 256;
   constexpr bool WIDE = tc_wide(NP, TF32);
@@ -647,7 +674,7 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
                                              // with the piece stage it parks sums in
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stage_free + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) {
       // a fused piece stage is written by the converter threads, each of
@@ -672,10 +699,12 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
     tmem_alloc(tmem_slot, S::TMEM_COLS);
     tmem_relinquish();
   }
+  pdl_trigger();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = uniform(*tmem_slot);
+  pdl_wait();
   // A 256-wide tile's epilogue holds 128 sums a thread: the four control
   // warps (producer, issuer, two idle) give registers to the eight epilogue
   // warps, instead of 168 each (at 168 the
@@ -698,11 +727,11 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       if (lane == 0) {
         uint32_t it = 0;
         bool ok = true;
-        const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
+        const TileRange tr = tile_range<GROUPED, TABLE>(tiles, total_tiles);
         uint8_t* raw = smem + NST * S::STAGE_BYTES;
         for (int t = tr.first; ok && t < tr.end; t += tr.step) {
           TcProblem P;
-          const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+          const TileCoord tc = tile_coord<BN, GROUPED, TABLE>(single, probs, tiles, t, P);
           const CUtensorMap* ma = &maps[2 * P.map];
           const CUtensorMap* mb = &maps[2 * P.map + 1];
           fence_tensormap(ma);
@@ -735,10 +764,10 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
         }
         uint32_t it = 0;
         bool ok = true;
-        const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
+        const TileRange tr = tile_range<GROUPED, TABLE>(tiles, total_tiles);
         for (int t = tr.first; ok && t < tr.end; t += tr.step) {
           TcProblem P;
-          const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+          const TileCoord tc = tile_coord<BN, GROUPED, TABLE>(single, probs, tiles, t, P);
           if constexpr (CONV) {
             const CUtensorMap* mp = &maps[4 * P.map];
             for (int m = 0; m < 4; ++m) fence_tensormap(mp + m);
@@ -747,7 +776,7 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
           }
           const CUtensorMap* ma = GROUPED ? &maps[2 * P.map] : &tmA;
           const CUtensorMap* mb = GROUPED ? &maps[2 * P.map + 1] : &tmB;
-          if (GROUPED) {
+          if (GROUPED && tiles != nullptr) {  // maps in device memory
             fence_tensormap(ma);
             fence_tensormap(mb);
           }
@@ -803,10 +832,10 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
     uint32_t ntile = 0;
     uint32_t nbound[NB] = {};
     bool ok = true;
-    const TileRange tr = tile_range<GROUPED>(tiles, total_tiles);
+    const TileRange tr = tile_range<GROUPED, TABLE>(tiles, total_tiles);
     for (int t = tr.first; ok && t < tr.end; t += tr.step, ++ntile) {
       TcProblem P;
-      const TileCoord tc = tile_coord<BN, GROUPED>(single, probs, tiles, t, P);
+      const TileCoord tc = tile_coord<BN, GROUPED, TABLE>(single, probs, tiles, t, P);
       const uint32_t buf = ntile % NB, use = ntile / NB;
       const uint32_t t_buf = tmem + buf * S::ACC_COLS + lane_base + col_off;
       if (P.beta != 0.f) prefetch_old_c<BN, GROUPED>(P, tc, ew, warp, lane);
@@ -1260,6 +1289,8 @@ __device__ __forceinline__ void split_batched_body(const SplitJob* __restrict__ 
                                                    int total_tiles) {
   __shared__ float tile[32][65];
   __shared__ int starts[kJobCache];
+  pdl_trigger();
+  pdl_wait();
   const int cached = min(njobs, kJobCache);
   for (int i = threadIdx.x; i < cached; i += blockDim.x) starts[i] = jobs[i].tile_start;
   __syncthreads();
@@ -1911,22 +1942,12 @@ void launch_split(const float* src, long long sr, long long sk, int rows, int K,
   prof_end(st, kProfSplitPrep);
 }
 
-int sm_count() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 148;
-  }
-  return sms;
-}
-
 template <int NP, int BN, bool GROUPED, bool EPI, bool TF32, bool FUSED = false, bool CONV = false>
 ugemm_status launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const TcProblem& single,
                            const CUtensorMap* maps, const TcProblem* probs, const int4* tiles,
                            int total_tiles, int nprod, int chunk_kb, int max_ctas, int fmt,
-                           int* dev_err, cudaStream_t st, const ConvGeo* geo = nullptr) {
+                           int* dev_err, cudaStream_t st, const ConvGeo* geo = nullptr,
+                           const MultiTable* table = nullptr) {
   using S = TcShape<NP, BN, tc_wide(NP, TF32)>;
   auto kern = split_tc_kernel<NP, BN, GROUPED, EPI, TF32, FUSED, CONV>;
   static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
@@ -1941,12 +1962,18 @@ ugemm_status launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const T
       return UGEMM_ERR_CUDA;
   }
   if (!smem_attr_once(kern, kSmem, attr_done)) return UGEMM_ERR_CUDA;
-  const int grid = std::max(1, std::min(total_tiles, max_ctas > 0 ? max_ctas : sm_count()));
+  const int grid = std::max(1, std::min(total_tiles, max_ctas > 0 ? max_ctas : device_sms()));
+  TableParam<GROUPED && !FUSED && !CONV> tp;
+  if constexpr (GROUPED && !FUSED && !CONV) {
+    if (table) tp.t = *table;
+    else if (!probs) return UGEMM_ERR_ARG;
+  }
   prof_begin(st);
-  kern<<<grid, FUSED ? fused_threads(BN) : kTcSplitThreads, kSmem, st>>>(
-      ta, tb, single, maps, probs, tiles, total_tiles, nprod, chunk_kb, fmt, geo, dev_err);
+  const cudaError_t e = launch_dependent(kern, dim3(grid), FUSED ? fused_threads(BN) : kTcSplitThreads,
+                                         kSmem, st, ta, tb, single, maps, probs, tiles, total_tiles,
+                                         nprod, chunk_kb, fmt, geo, dev_err, tp);
   prof_end(st, GROUPED ? kProfGrouped : kProfSplitGemm);
-  return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
+  return e == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }
 
 int kp_of(int K) { return static_cast<int>(align_up(std::max(K, 1), kTcKB)); }
@@ -2005,7 +2032,7 @@ std::vector<int4> split_tile_table(const TcProblem* probs, int nprob, int block_
 // stage is bound by its 36 KB of copies, the others by their MMAs.
 double stage_us(int pieces, int bn) {
   const double w = bn == 256 ? 0.80 : bn == 128 ? 0.64 : 0.30;
-  return pieces == 3 ? w : w / 2;
+  return pieces == 2 ? w / 2 : w;  // three products instead of six
 }
 double tile_us(int bn) { return bn == 256 ? 3.0 : bn == 128 ? 1.5 : 1.2; }
 
@@ -2225,8 +2252,9 @@ ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const 
                                const TcProblem& single, const CUtensorMap* maps,
                                const TcProblem* probs, const int4* tiles, int total_tiles,
                                int chunk_kb,
-                               int max_ctas, int* dev_err, cudaStream_t st, const ConvGeo* geo) {
-  const bool grouped = probs != nullptr;
+                               int max_ctas, int* dev_err, cudaStream_t st, const ConvGeo* geo,
+                               const MultiTable* table) {
+  const bool grouped = probs != nullptr || table != nullptr;
   if (p.conv) {
     if (p.pieces != 3 || !grouped || geo == nullptr) return UGEMM_ERR_ARG;
 #define UGEMM_CONV_CASE(BN, EPI)                                                                 \
@@ -2264,7 +2292,8 @@ ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const 
 #define UGEMM_SPLIT_CASE(NP, BN, GR, EPI, T)                                                     \
   if (kernel_np(p.pieces) == NP && p.block_n == BN && grouped == GR && p.epi == EPI && tf32 == T) \
     return launch_kernel<NP, BN, GR, EPI, T>(ta, tb, single, maps, probs, tiles, total_tiles,     \
-                                             p.products, chunk_kb, max_ctas, fmt, dev_err, st);
+                                             p.products, chunk_kb, max_ctas, fmt, dev_err, st,    \
+                                             nullptr, table);
 #define UGEMM_SPLIT_CASES(NP, BN, T)    \
   UGEMM_SPLIT_CASE(NP, BN, false, false, T) \
   UGEMM_SPLIT_CASE(NP, BN, false, true, T)  \
@@ -2286,7 +2315,7 @@ ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const 
 ugemm_status split_batched_launch(int pieces, const SplitJob* jobs, int njobs, int total_tiles,
                                   cudaStream_t st, unsigned* fmax_words, int nwords) {
   if (total_tiles <= 0) return UGEMM_OK;
-  const int grid = std::min(total_tiles, sm_count() * 8);
+  const int grid = std::min(total_tiles, device_sms() * 8);
   if (fmax_words) {  // FP16x3: the largest magnitude of every job's rows first
     if (pieces != 2) return UGEMM_ERR_ARG;
     if (cudaMemsetAsync(fmax_words, 0, sizeof(unsigned) * nwords, st) != cudaSuccess)
@@ -2311,7 +2340,7 @@ ugemm_status split_taps_launch(const SplitJob* jobs, int njobs, int total_tiles,
   if (total_tiles <= 0) return UGEMM_OK;
   prof_begin(st);
   split_pieces_batched_kernel<3, 0, true>
-      <<<std::min(total_tiles, sm_count() * 8), 256, 0, st>>>(jobs, njobs, total_tiles);
+      <<<std::min(total_tiles, device_sms() * 8), 256, 0, st>>>(jobs, njobs, total_tiles);
   prof_end(st, kProfSplitPrep);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }
@@ -2320,7 +2349,7 @@ ugemm_status split_param_launch(int pieces, const SplitJobTable& t, int njobs, i
                                 cudaStream_t st) {
   if (total_tiles <= 0) return UGEMM_OK;
   if (njobs < 1 || njobs > kSplitTableJobs) return UGEMM_ERR_ARG;
-  const int grid = std::min(total_tiles, sm_count() * 8);
+  const int grid = std::min(total_tiles, device_sms() * 8);
   prof_begin(st);
   if (pieces == 3) split_pieces_param_kernel<3, 0><<<grid, 256, 0, st>>>(t, njobs, total_tiles);
   else if (pieces == kPiecesTf32) split_pieces_param_kernel<2, 2><<<grid, 256, 0, st>>>(t, njobs, total_tiles);
@@ -2376,7 +2405,7 @@ ugemm_status split_operand_launch(int pieces, const float* src, long long sr, lo
       const long long other = kcontig ? sr : sk;
       const bool vec = ((reinterpret_cast<uintptr_t>(src) & 15) == 0) && ((other & 3) == 0);
       const int band = kcontig ? 16 : 256, bands = cdiv(rows, band);
-      const int want_y = std::max(1, std::min(cdiv(K, 256), cdiv(sm_count() * 8, bands)));
+      const int want_y = std::max(1, std::min(cdiv(K, 256), cdiv(device_sms() * 8, bands)));
       const int kper = static_cast<int>(align_up(cdiv(K, want_y), 64));
       const dim3 grid(bands, cdiv(K, kper));
       prof_begin(st);
@@ -2391,7 +2420,7 @@ ugemm_status split_operand_launch(int pieces, const float* src, long long sr, lo
         j.fmax = words;
         const int tiles = cdiv(rows, 32) * cdiv(Kp, 64);
         j.tile_start = 0;
-        operand_max_single_kernel<<<std::min(tiles, sm_count() * 8), 256, 0, st>>>(j, tiles);
+        operand_max_single_kernel<<<std::min(tiles, device_sms() * 8), 256, 0, st>>>(j, tiles);
       }
       prof_end(st, kProfSplitPrep);
     }

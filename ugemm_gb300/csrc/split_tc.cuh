@@ -176,6 +176,16 @@ struct TcProblem {
   float* chunk_sums = nullptr;
 };
 
+// A few GEMMs and their k slices as the parameter of a grouped launch: no table
+// in device memory, so nothing to write before it.  probs: longest k first,
+// tile_start ascending, unused entries at INT_MAX; CTA c takes tiles c, c + grid,
+// ... of the list.
+constexpr int kMultiSubs = 24;  // kernel problems (slices) per launch
+struct MultiTable {
+  CUtensorMap maps[2 * kMultiMax];
+  TcProblem probs[kMultiSubs];
+};
+
 // What the producer of a CONV launch needs to know of a problem; problem p's
 // tensor maps are maps[4p] (the tiled operand) and maps[4p + 1..3] (the planes
 // of the im2col operand; kPlain: maps[4p + 1], the tiled b operand).
@@ -293,12 +303,13 @@ ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail
 // probs/tiles: a grouped launch's problem records and its tile table (from
 // split_tile_table, for a grid of exactly max_ctas CTAs); both null for one
 // GEMM (`single`).
+// table: a grouped launch of these problems (maps, probs and tiles null).
 // p.fused (grouped only): `maps` describe the FP32 operands, not pieces.
 ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const CUtensorMap& tb,
                                const TcProblem& single, const CUtensorMap* maps,
                                const TcProblem* probs, const int4* tiles, int total_tiles,
                                int chunk_kb, int max_ctas, int* dev_err, cudaStream_t st,
-                               const ConvGeo* geo = nullptr);
+                               const ConvGeo* geo = nullptr, const MultiTable* table = nullptr);
 // The tensor maps of one CONV problem (maps[0..3]) whose C is M x N; swap: the
 // im2col operand (kPlain: B) is the kernel's a.  False if TMA cannot describe it.
 bool conv_encode_maps(const PieceOperands& q, int M, int N, int block_n, bool swap,
