@@ -193,10 +193,17 @@ def ugemm_sgemm(major: str, transa: str, transb: str, M: int, N: int, K: int, al
 # Device-pointer API on torch tensors
 # --------------------------------------------------------------------------
 def _stream_ptr(stream) -> int:
-    import torch
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return stream.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        torch.cuda.init()
+        _raw_stream = (torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice)
+    return _raw_stream[0](_raw_stream[1]())  # without a Stream object on the way
+
+
+_raw_stream = None
 
 
 def sgemm_dev(ta: str, tb: str, M: int, N: int, K: int, alpha: float, A, lda: int, B, ldb: int,

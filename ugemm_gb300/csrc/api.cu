@@ -14,6 +14,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "internal.h"
 
@@ -25,17 +26,23 @@ thread_local std::string t_last_msg;
 
 struct DeviceState {
   bool ready = false;
-  // Device-side error words: dev_err[0] is written by the bounded waits of
-  // the kernels of one call (the word the kernels see); dev_err[1] holds the
-  // first code that a device-pointer call left there, until ugemm_check
-  // reads it (error_fold_kernel moves it before the next call's kernels).
-  int* dev_err = nullptr;
+  // Device-side error words, written by the bounded waits of kernels.  Each
+  // call's kernels get a word of their own, words[0, kErrSlots) in turn, so
+  // that a code an earlier call left neither stops a later call's waits nor is
+  // taken for its own; words[kErrSlots] holds the first code found when the
+  // words come round again, until ugemm_check reads it.
+  int* words = nullptr;
+  unsigned calls = 0;
+  // the last fold of all words: a call on another stream waits for it
+  cudaEvent_t folded = nullptr;
+  cudaStream_t fold_stream = nullptr;
+  bool fold_pending = false, fold_due = false;
   void* ws = nullptr;         // workspace of the device-pointer API
   size_t ws_bytes = 0;
   int sms = 0, cc_major = 0, cc_minor = 0;
 };
 
-constexpr int kMaxDevices = 64;
+constexpr int kMaxDevices = 64, kErrSlots = 4096;
 std::mutex g_mu;
 DeviceState g_dev[kMaxDevices];
 
@@ -78,42 +85,73 @@ ugemm_status device_state(DeviceState** out) {
     cudaDeviceGetAttribute(&d.cc_minor, cudaDevAttrComputeCapabilityMinor, dev);
     if (d.cc_major != 10 || d.cc_minor != 3)
       return fail(UGEMM_ERR_UNSUPPORTED, "libugemm_cuda is built for sm_103a (GB300)%s");
-    e = cudaMalloc(&d.dev_err, 2 * sizeof(int));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(error word)");
-    e = cudaMemset(d.dev_err, 0, 2 * sizeof(int));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemset(error word)");
+    e = cudaMalloc(&d.words, (kErrSlots + 1) * sizeof(int));
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(error words)");
+    e = cudaMemset(d.words, 0, (kErrSlots + 1) * sizeof(int));
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d.folded, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+      cudaFree(d.words);
+      d.words = nullptr;
+      return cuda_fail(e, "error words");
+    }
     d.ready = true;
   }
   *out = &d;
   return UGEMM_OK;
 }
 
-// Stream-ordered start of a call on the device path: a code left in the
-// kernels' word by an earlier call moves to the held word (the first one is
-// kept) and the kernels' word is cleared, so a stale timeout neither stops
-// this call's waits early nor is reported as this call's; ugemm_check reports
-// it.  One thread, a few instructions.
-__global__ void error_fold_kernel(int* words) {
-  const int code = words[0];
-  if (code != 0) {
-    if (words[1] == 0) words[1] = code;
-    words[0] = 0;
-  }
-}
-
-ugemm_status begin_call(int* words, cudaStream_t st) {
-  (void)cudaGetLastError();  // a pending error of earlier, unrelated work is not this call's
-  prof_begin(st);
-  error_fold_kernel<<<1, 1, 0, st>>>(words);
-  prof_end(st, kProfControl);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? UGEMM_OK : cuda_fail(e, "error word fold");
-}
-
 bool is_capturing(cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) return false;
   return cs != cudaStreamCaptureStatusNone;
+}
+
+// Moves the first non-zero code of words[0, n) to the held word (if that is
+// free) and clears them.
+__global__ void error_fold_kernel(int* words, int n, int* held) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const int code = words[i];
+    if (code != 0) {
+      atomicCAS(held, 0, code);
+      words[i] = 0;
+    }
+  }
+}
+
+// Start of a call on the device path: its error word.  No launch but once in
+// kErrSlots calls, when the words come round and are folded (a launch of one
+// thread before every call took 2 us of its 13).  A call under capture is
+// replayed any number of times with one word, so its graph folds that word.
+// Caller holds g_mu.
+ugemm_status begin_call(DeviceState& d, cudaStream_t st, int** word) {
+  (void)cudaGetLastError();  // a pending error of earlier, unrelated work is not this call's
+  const unsigned slot = d.calls++ % kErrSlots;
+  *word = d.words + slot;
+  const bool capturing = is_capturing(st);
+  if (slot == 0 && d.calls > 1) d.fold_due = true;
+  const bool fold = d.fold_due && !capturing;
+  cudaError_t e = cudaSuccess;
+  if (capturing || fold) {
+    prof_begin(st);
+    if (fold)
+      error_fold_kernel<<<1, 256, 0, st>>>(d.words, kErrSlots, d.words + kErrSlots);
+    else
+      error_fold_kernel<<<1, 1, 0, st>>>(*word, 1, d.words + kErrSlots);
+    prof_end(st, kProfControl);
+    e = cudaGetLastError();
+    if (e == cudaSuccess && fold) {
+      e = cudaEventRecord(d.folded, st);
+      d.fold_stream = st;
+      d.fold_pending = true;
+      d.fold_due = false;
+    }
+  }
+  if (d.fold_pending && !capturing) {
+    if (cudaEventQuery(d.folded) == cudaSuccess) d.fold_pending = false;
+    else if (st != d.fold_stream && e == cudaSuccess) e = cudaStreamWaitEvent(st, d.folded, 0);
+    (void)cudaGetLastError();  // the query's "not ready"
+  }
+  return e == cudaSuccess ? UGEMM_OK : cuda_fail(e, "error word");
 }
 
 // Grow the device workspace to `need` bytes (never during stream capture).
@@ -215,15 +253,15 @@ ugemm_status launch(const Gemm& g, int form, Scratch ws, int* dev_err, cudaStrea
   return UGEMM_OK;
 }
 
-// Read and clear the device error word (synchronises `st`).
-ugemm_status check_device_error(DeviceState& d, cudaStream_t st) {
+// Read and clear a call's error word (synchronises `st`).
+ugemm_status check_device_error(int* word, cudaStream_t st) {
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
   int code = 0;
-  e = cudaMemcpy(&code, d.dev_err, sizeof(int), cudaMemcpyDeviceToHost);
+  e = cudaMemcpy(&code, word, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(error word)");
   if (code != 0) {
-    cudaMemset(d.dev_err, 0, sizeof(int));
+    cudaMemset(word, 0, sizeof(int));
     char buf[128];
     std::snprintf(buf, sizeof buf, "kernel pipeline wait timed out (code %d)", code);
     set_last_error(UGEMM_ERR_TIMEOUT, buf);
@@ -240,9 +278,10 @@ ugemm_status dev_gemm(const Gemm& g, int precision, cudaStream_t st) {
   const int form = resolve_form(precision, g);
   s = ensure_workspace(*d, scratch_for(g, form), st);
   if (s != UGEMM_OK) return s;
-  s = begin_call(d->dev_err, st);
+  int* word = nullptr;
+  s = begin_call(*d, st, &word);
   if (s != UGEMM_OK) return s;
-  return launch(g, form, Scratch{d->ws, d->ws_bytes}, d->dev_err, st);
+  return launch(g, form, Scratch{d->ws, d->ws_bytes}, word, st);
 }
 
 // Host-pointer GEMM in an arena too small for the 256-byte-aligned layout:
@@ -253,7 +292,7 @@ ugemm_status dev_gemm(const Gemm& g, int precision, cudaStream_t st) {
 // ten times the three matrices (sgemm_test.c:29), which this layout fits for
 // every shape in the SIMT form (at most 3 padding floats per row).
 ugemm_status host_gemm_tight(const Gemm& g, int form, void* arena, size_t arena_bytes,
-                             DeviceState& d, cudaStream_t st) {
+                             int* word, cudaStream_t st) {
   const size_t a_rows = g.ta == 'N' ? g.M : g.K, b_rows = g.tb == 'N' ? g.K : g.N;
   const size_t a_cols = g.ta == 'N' ? g.K : g.M, b_cols = g.tb == 'N' ? g.N : g.K;
   const bool need_ab = g.K > 0 && g.alpha != 0.f;
@@ -288,20 +327,21 @@ ugemm_status host_gemm_tight(const Gemm& g, int form, void* arena, size_t arena_
                           g.N * sizeof(float), g.M, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(e, "copy C to device");
   }
-  ugemm_status s = launch(dg, form, Scratch{base + s_off, arena_bytes - s_off}, d.dev_err, st);
+  ugemm_status s = launch(dg, form, Scratch{base + s_off, arena_bytes - s_off}, word, st);
   if (s != UGEMM_OK) return s;
   e = cudaMemcpy2DAsync(g.C, g.ldc * sizeof(float), dg.C, g.N * sizeof(float), g.N * sizeof(float),
                         g.M, cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return cuda_fail(e, "copy C to host");
-  return check_device_error(d, st);
+  return check_device_error(word, st);
 }
 
 // Host-pointer GEMM through a device arena [A | B | C | scratch].
 ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_bytes,
                        DeviceState& d, cudaStream_t st) {
   if (g.M == 0 || g.N == 0) return UGEMM_OK;
+  int* word = nullptr;
   {
-    ugemm_status bs = begin_call(d.dev_err, st);
+    ugemm_status bs = begin_call(d, st, &word);
     if (bs != UGEMM_OK) return bs;
   }
   const size_t a_rows = g.ta == 'N' ? g.M : g.K, b_rows = g.tb == 'N' ? g.K : g.N;
@@ -311,13 +351,13 @@ ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_b
   const size_t c_bytes = align_up(size_t(g.M) * g.ldc * sizeof(float), 256);
   const int form = resolve_form(precision, g);
   {
-    ugemm_status ps = host_gemm_pipelined(g, form, arena, arena_bytes, d.dev_err, st);
-    if (ps == UGEMM_OK) return check_device_error(d, st);
+    ugemm_status ps = host_gemm_pipelined(g, form, arena, arena_bytes, word, st);
+    if (ps == UGEMM_OK) return check_device_error(word, st);
     if (ps != UGEMM_ERR_UNSUPPORTED) return fail(ps, "pipelined host GEMM failed%s");
   }
   const bool need_ab = g.K > 0 && g.alpha != 0.f;
   const size_t need = (need_ab ? a_bytes + b_bytes : 0) + c_bytes + scratch_for(g, form);
-  if (need > arena_bytes) return host_gemm_tight(g, form, arena, arena_bytes, d, st);
+  if (need > arena_bytes) return host_gemm_tight(g, form, arena, arena_bytes, word, st);
   uint8_t* base = static_cast<uint8_t*>(arena);
   Gemm dg = g;
   size_t off = 0;
@@ -341,7 +381,7 @@ ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_b
     if (e != cudaSuccess) return cuda_fail(e, "copy C to device");
   }
   Scratch ws{base + off + c_bytes, arena_bytes - off - c_bytes};
-  ugemm_status s = launch(dg, form, ws, d.dev_err, st);
+  ugemm_status s = launch(dg, form, ws, word, st);
   if (s != UGEMM_OK) return s;
   // Copy back row by row only when the host C has padding we must not touch.
   if (g.ldc == g.N) {
@@ -351,7 +391,7 @@ ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_b
                           g.N * sizeof(float), g.M, cudaMemcpyDeviceToHost, st);
   }
   if (e != cudaSuccess) return cuda_fail(e, "copy C to host");
-  return check_device_error(d, st);
+  return check_device_error(word, st);
 }
 
 }  // namespace
@@ -586,9 +626,10 @@ int ugemm_sgemm_backward(char transa, char transb, int M, int N, int K, float al
       const SplitPlan p = split_plan_for(form, gs[0]);
       s = ensure_workspace(*d, multi_scratch_bytes(gs, n, p), st);
       if (s != UGEMM_OK) return s;
-      s = begin_call(d->dev_err, st);
+      int* word = nullptr;
+      s = begin_call(*d, st, &word);
       if (s != UGEMM_OK) return s;
-      s = multi_launch(gs, n, p, Scratch{d->ws, d->ws_bytes}, d->dev_err, st);
+      s = multi_launch(gs, n, p, Scratch{d->ws, d->ws_bytes}, word, st);
       if (s == UGEMM_ERR_CUDA) return cuda_fail(cudaGetLastError(), "kernel launch");
       if (s != UGEMM_OK) return fail(s, "launch failed%s");
       return UGEMM_OK;
@@ -625,18 +666,21 @@ int ugemm_check(void* stream) {
   DeviceState* d = nullptr;
   ugemm_status s = device_state(&d);
   if (s != UGEMM_OK) return s;
-  int words[2] = {0, 0}, na[2] = {0, 0};
-  e = cudaMemcpy(words, d->dev_err, sizeof words, cudaMemcpyDeviceToHost);
+  std::vector<int> words(kErrSlots + 1);
+  int na[2] = {0, 0};
+  e = cudaMemcpy(words.data(), d->words, words.size() * sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(error words)");
   int* nw = noalloc_error_words();
   if (nw) {
     e = cudaMemcpy(na, nw, sizeof na, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(error words)");
   }
-  // the first recorded code wins: held codes are older than current ones
-  const int code = words[1] ? words[1] : words[0] ? words[0] : na[1] ? na[1] : na[0];
+  // the first recorded code wins: the held one, then the calls' in their order
+  int code = words[kErrSlots];
+  for (unsigned i = 0; i < kErrSlots && code == 0; ++i) code = words[(d->calls + i) % kErrSlots];
+  if (code != 0) cudaMemset(d->words, 0, words.size() * sizeof(int));
+  if (code == 0) code = na[1] ? na[1] : na[0];
   if (code == 0) return UGEMM_OK;
-  if (words[0] || words[1]) cudaMemset(d->dev_err, 0, sizeof words);
   if (na[0] || na[1]) cudaMemset(nw, 0, sizeof na);
   char buf[160];
   std::snprintf(buf, sizeof buf,
@@ -650,7 +694,10 @@ int ugemm_debug_set_error_word(int which, int code) {
   DeviceState* d = nullptr;
   ugemm_status s = device_state(&d);
   if (s != UGEMM_OK) return s;
-  int* word = which == 0 ? d->dev_err : which == 1 ? noalloc_error_words() : nullptr;
+  // the word of the last device-pointer call
+  int* word = which == 0   ? d->words + (d->calls + kErrSlots - 1) % kErrSlots
+              : which == 1 ? noalloc_error_words()
+                           : nullptr;
   if (!word) return fail(UGEMM_ERR_ARG, "no such error word on this device (yet)%s");
   const cudaError_t e = cudaMemcpy(word, &code, sizeof code, cudaMemcpyHostToDevice);
   return e == cudaSuccess ? UGEMM_OK : cuda_fail(e, "cudaMemcpy(error word)");
