@@ -73,3 +73,27 @@ def test_saxpy_large_and_strided():
     ug.saxpy(1000, 2.0, xs, 3, ys, 2)
     torch.cuda.synchronize()
     assert torch.allclose(ys, ref, atol=1e-6)
+
+
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("M,N,pad,off", [(512, 512, 0, 0), (516, 4097, 0, 0), (2436, 1025, 4, 0),
+                                         (1, 9000, 0, 0), (31, 511, 1, 0), (5000, 2049, 3, 1),
+                                         (640, 8200, 0, 1)])
+def test_gemv_vector_widths_and_shared_columns(trans, M, N, pad, off):
+    """Aligned and unaligned columns, one and several warps (or a cluster) per
+    output.  FP32 sums of N products: within sqrt(N) 2^-24 ~ 6e-6 / 1e3 of FP64
+    normwise; 2e-6 is the suite's bound."""
+    rows, cols = (M, N) if trans == "N" else (N, M)   # column-major rows x cols
+    lda = rows + pad
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    buf = torch.rand((cols * lda + 4,), device="cuda", generator=g) - 0.5
+    A = buf[off:off + cols * lda].view(cols, lda)[:, :rows]
+    x = torch.rand((N,), device="cuda", generator=g) - 0.5
+    y = torch.rand((2 * M,), device="cuda", generator=g)
+    a64 = A.double().T if trans == "N" else A.double()
+    ref = 1.5 * (a64 @ x.double()) + 0.5 * y[::2].double()
+    odd = y[1::2].clone()
+    ug.sgemv(trans, M, N, 1.5, A.data_ptr(), lda, x, 1, 0.5, y, 2)
+    torch.cuda.synchronize()
+    assert float(torch.linalg.norm(y[::2].double() - ref) / torch.linalg.norm(ref)) < 2e-6
+    assert torch.equal(y[1::2], odd)

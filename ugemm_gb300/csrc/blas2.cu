@@ -2,11 +2,14 @@
 // sgemv_cpu, ugemm.h:86-160).  Both are HBM-bound: every element of x / A is
 // read once with coalesced loads; reductions are done in a fixed order, so
 // results are deterministic.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace ugemm {
 namespace {
@@ -31,48 +34,177 @@ __global__ void saxpy_kernel(int n, float alpha, const float* __restrict__ x, in
 }
 
 // 'N': A is column-major M x N (A[m + n*lda]); y[m] = alpha * sum_n A[m,n] x[n]
-// + beta * y[m].  A block owns 32 rows; its 8 warps take every 8th column and
-// the 8 partial sums are added in a fixed order.
-__global__ void __launch_bounds__(256) sgemv_n_kernel(int M, int N, float alpha,
-                                                      const float* __restrict__ A, int lda,
-                                                      const float* __restrict__ x, int incx,
-                                                      float beta, float* __restrict__ y, int incy) {
-  __shared__ float part[8][33];
+// + beta * y[m].  A block owns 32 V rows (V = 4: 16-byte loads, 512 bytes of a
+// column at a time); its 16 warps take every 16th column, several loads in flight
+// each, and the partial sums are added in a fixed order.  HBM-bound: what counts
+// is bytes in flight and long runs of a column, so where row blocks are few a
+// cluster of kGemvCluster blocks shares the columns of each, the sums passing
+// through distributed shared memory in rank order.
+constexpr int kGemvWarps = 16, kGemvCluster = 8;
+template <int V>
+__global__ void __launch_bounds__(kGemvWarps * 32)
+    sgemv_n_kernel(int M, int N, float alpha, const float* __restrict__ A, int lda,
+                   const float* __restrict__ x, int incx, float beta, float* __restrict__ y,
+                   int incy, int share) {
+  __shared__ float part[kGemvWarps][32 * V + 1];
+  __shared__ float sum[32 * V];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int m = blockIdx.x * 32 + lane;
-  float s = 0.f;
-  if (m < M)
-    for (int n = w; n < N; n += 8) s += A[m + static_cast<long long>(n) * lda] * x[static_cast<long long>(n) * incx];
-  part[w][lane] = s;
-  __syncthreads();
-  if (w == 0 && m < M) {
-    float t = 0.f;
+  const int rank = share > 1 ? blockIdx.x % share : 0;
+  const int m0 = (blockIdx.x / share) * 32 * V, m = m0 + lane * V;
+  const int step = kGemvWarps * share;
+  constexpr int U = V == 4 ? 4 : 8;  // loads in flight
+  float s[V];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) t += part[j][lane];
-    float* yp = y + static_cast<long long>(m) * incy;
+  for (int e = 0; e < V; ++e) s[e] = 0.f;
+  if (m < M) {  // (V = 4: M is a multiple of 4)
+    const float* col = A + m;
+    auto load = [&](int n, float (&v)[V]) {
+      const float* p = col + static_cast<long long>(n) * lda;
+      if constexpr (V == 4) {
+        const float4 q = __ldcs(reinterpret_cast<const float4*>(p));
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+      } else {
+        v[0] = *p;
+      }
+    };
+    int n = w * share + rank;
+    for (; n + (U - 1) * step < N; n += U * step) {
+      float v[U][V];
+#pragma unroll
+      for (int u = 0; u < U; ++u) load(n + u * step, v[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float b = x[static_cast<long long>(n + u * step) * incx];
+#pragma unroll
+        for (int e = 0; e < V; ++e) s[e] += v[u][e] * b;
+      }
+    }
+    for (; n < N; n += step) {
+      float v[V];
+      load(n, v);
+      const float b = x[static_cast<long long>(n) * incx];
+#pragma unroll
+      for (int e = 0; e < V; ++e) s[e] += v[e] * b;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < V; ++e) part[w][lane * V + e] = s[e];
+  __syncthreads();
+  const int r = threadIdx.x;  // a row of the block
+  float t = 0.f;
+  if (r < 32 * V) {
+#pragma unroll
+    for (int j = 0; j < kGemvWarps; ++j) t += part[j][r];
+    sum[r] = t;
+  }
+  if (share > 1) {
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    if (rank == 0 && r < 32 * V) {
+      t = 0.f;
+      for (int c = 0; c < share; ++c) t += cl.map_shared_rank(sum, c)[r];
+    }
+    cl.sync();  // the others' shared memory stays until it has been read
+  }
+  if (rank == 0 && r < 32 * V && m0 + r < M) {
+    float* yp = y + static_cast<long long>(m0 + r) * incy;
     *yp = (beta == 0.f) ? alpha * t : alpha * t + beta * *yp;
   }
 }
 
 // 'T': A is column-major N x M (A[n + m*lda]); y[m] = alpha * sum_n A[n,m] x[n]
-// + beta * y[m].  One warp per output, coalesced along the column, reduced by
-// a fixed shuffle tree.
+// + beta * y[m].  WPC warps per output, coalesced along the column: 16-byte
+// loads, eight in flight, where A's columns and x allow them (VEC); reduced by a
+// fixed shuffle tree.  HBM-bound (8192 x 8192: one scalar load in flight 53 us,
+// 5.1 TB/s); few outputs take a block each (WPC = 8).
+template <int WPC, bool VEC>
 __global__ void __launch_bounds__(256) sgemv_t_kernel(int M, int N, float alpha,
                                                       const float* __restrict__ A, int lda,
                                                       const float* __restrict__ x, int incx,
                                                       float beta, float* __restrict__ y, int incy) {
-  const int lane = threadIdx.x & 31;
-  const int m = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (m >= M) return;
-  const float* col = A + static_cast<long long>(m) * lda;
+  __shared__ float part[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int m = blockIdx.x * (8 / WPC) + w / WPC;
+  const int t = (w % WPC) * 32 + lane;  // this thread among the output's
+  constexpr int T = WPC * 32;
   float s = 0.f;
-  for (int n = lane; n < N; n += 32) s += col[n] * x[static_cast<long long>(n) * incx];
+  if (m < M) {
+    const float* col = A + static_cast<long long>(m) * lda;
+    if (VEC) {
+      const float4* c4 = reinterpret_cast<const float4*>(col);
+      const float4* x4 = reinterpret_cast<const float4*>(x);
+      const int n4 = N / 4;
+      int i = t;
+      for (; i + 7 * T < n4; i += 8 * T) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldcs(c4 + i + u * T);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float4 b = x4[i + u * T];
+          s += v[u].x * b.x; s += v[u].y * b.y; s += v[u].z * b.z; s += v[u].w * b.w;
+        }
+      }
+      for (; i < n4; i += T) {
+        const float4 v = c4[i], b = x4[i];
+        s += v.x * b.x; s += v.y * b.y; s += v.z * b.z; s += v.w * b.w;
+      }
+      for (int n = 4 * n4 + t; n < N; n += T) s += col[n] * x[n];
+    } else {
+      int n = t;
+      for (; n + 7 * T < N; n += 8 * T) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = col[n + u * T];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += v[u] * x[static_cast<long long>(n + u * T) * incx];
+      }
+      for (; n < N; n += T) s += col[n] * x[static_cast<long long>(n) * incx];
+    }
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) {
+  if (WPC > 1) {
+    if (lane == 0) part[w] = s;
+    __syncthreads();
+    s = 0.f;
+#pragma unroll
+    for (int j = 0; j < WPC; ++j) s += part[w / WPC * WPC + j];
+  }
+  if (t == 0 && m < M) {
     float* yp = y + static_cast<long long>(m) * incy;
     *yp = (beta == 0.f) ? alpha * s : alpha * s + beta * *yp;
   }
+}
+
+template <int WPC>
+void launch_gemv_t(int M, int N, float alpha, const float* A, int lda, const float* x, int incx,
+                   float beta, float* y, int incy, cudaStream_t st) {
+  const bool vec = (lda & 3) == 0 && incx == 1 &&
+                   ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
+  const int grid = cdiv(M, 8 / WPC);
+  if (vec) sgemv_t_kernel<WPC, true><<<grid, 256, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
+  else sgemv_t_kernel<WPC, false><<<grid, 256, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
+}
+
+// Clusters of blocks share the columns when the row blocks are few.
+template <int V>
+cudaError_t launch_gemv_n(int M, int N, float alpha, const float* A, int lda, const float* x,
+                          int incx, float beta, float* y, int incy, cudaStream_t st) {
+  const int rows = cdiv(M, 32 * V);
+  const int share = rows < 4 * device_sms() && N >= 4 * kGemvWarps * kGemvCluster ? kGemvCluster : 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * share);
+  cfg.blockDim = dim3(kGemvWarps * 32);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = share;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = share > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, sgemv_n_kernel<V>, M, N, alpha, A, lda, x, incx, beta, y, incy,
+                            share);
 }
 
 }  // namespace
@@ -106,8 +238,15 @@ UGEMM_API int ugemm_sgemv(char trans, int M, int N, float alpha, const float* A,
   if (!y || (N > 0 && (!A || !x))) return UGEMM_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   prof_begin(st);
-  if (t) sgemv_t_kernel<<<(M + 7) / 8, 256, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
-  else sgemv_n_kernel<<<(M + 31) / 32, 256, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
+  if (!t && ((M | lda) & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && M >= 512)
+    (void)launch_gemv_n<4>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
+  else if (!t)
+    (void)launch_gemv_n<1>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
+  else if (N > 4096 || M < 16 * device_sms())
+    launch_gemv_t<8>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
+  else if (N > 2048) launch_gemv_t<4>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
+  else if (N > 1024) launch_gemv_t<2>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
+  else launch_gemv_t<1>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
   prof_end(st, kProfAux);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }
