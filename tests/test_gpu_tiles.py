@@ -49,3 +49,30 @@ def test_simt_wide_and_narrow_tiles(ta, tb, M, N, K):
 @pytest.mark.parametrize("beta", [0.0, 0.5])
 def test_split_epilogue_unaligned_rows(prec, M, N, K, pad, beta):
     check("T", "N", M, N, K, prec, beta, pad)
+
+
+@pytest.mark.parametrize("ta,tb", ["NN", "NT", "TN", "TT"])
+@pytest.mark.parametrize("M,N,K", [(100, 6000, 500), (6000, 100, 516), (128, 25088, 96),
+                                   (64, 64, 8192), (1, 4096, 300), (512, 512, 512), (896, 900, 1100)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_split_routes(ta, tb, M, N, K, off):
+    """Outputs with a short side or few tiles: operands that TMA can copy are split
+    inside the GEMM kernel or cut into slices and narrow tiles, others (a base one
+    float off a 16-byte boundary) beforehand; C updated, bias and LeakyReLU fused."""
+    g = torch.Generator(device="cuda").manual_seed(M + 3 * N + 7 * K)
+
+    def mat(r, c):
+        ld = (c + 3) // 4 * 4
+        buf = torch.rand((r * ld + 4,), device="cuda", generator=g) * 2 - 1
+        return buf[off:off + r * ld].view(r, ld)[:, :c]
+
+    A = mat(M, K) if ta == "N" else mat(K, M)
+    B = mat(K, N) if tb == "N" else mat(N, K)
+    C = mat(M, N)
+    bias = torch.randn((M,), device="cuda", generator=g)
+    ref = ug.ref64(ta, tb, A, B, C.contiguous(), 1.5, 0.5) + bias.double()[:, None]
+    ref = torch.where(ref > 0, ref, 0.1 * ref)
+    ug.gemm_ex(A, B, C, bias=bias, act=1, slope=0.1, ta=ta, tb=tb, alpha=1.5, beta=0.5,
+               precision="bf16x6")
+    torch.cuda.synchronize()
+    assert float(torch.linalg.norm(C.double() - ref) / torch.linalg.norm(ref)) < 2e-6

@@ -566,12 +566,18 @@ int ugemm_sgemm_dev_ex(char major, char transa, char transb, int M, int N, int K
 size_t ugemm_workspace_bytes(char major, char transa, char transb, int M, int N, int K, int lda,
                              int ldb, int precision) {
   Gemm g;
-  // Pointers only matter for alignment: assume aligned device buffers.
-  static float dummy[4] __attribute__((aligned(16)));
+  // Pointers only matter for alignment: assume aligned device buffers, but
+  // enough for the split forms' route on others too (the operands of unaligned
+  // buffers are not split inside the GEMM kernel).
+  static float dummy[8] __attribute__((aligned(16)));
   if (make_gemm(major, transa, transb, M, N, K, 1.f, dummy, lda, dummy, ldb, 0.f, dummy,
                 (major == 'R' || major == 'r') ? N : M, &g) != UGEMM_OK)
     return 0;
-  return scratch_for(g, resolve_form(precision, g));
+  const int form = resolve_form(precision, g);
+  const size_t aligned = scratch_for(g, form);
+  if (!is_split_form(form)) return aligned;
+  g.A = g.B = dummy + 1;
+  return std::max(aligned, scratch_for(g, form));
 }
 
 int ugemm_reserve_workspace(size_t bytes) {

@@ -239,6 +239,50 @@ struct ugemm_grouped_plan_s {
 namespace ugemm {
 namespace {
 
+// The FP32 source of one kernel operand of a fused launch (rows of op(A),
+// or of op(B)^T, by k) as a 2-D tensor map: k contiguous (row stride sr) or
+// rows contiguous (k stride sk).  *kc says which.
+bool fused_operand_map(const float* base, long long sr, long long sk, int rows, int K,
+                       int box_rows, int box_k, CUtensorMap* map, int* kc) {
+  if (sk == 1) {
+    *kc = 1;
+    return fused_encode_map(base, sr, rows, K, true, box_rows, box_k, map);
+  }
+  *kc = 0;
+  return sr == 1 && fused_encode_map(base, sk, K, rows, false, box_rows, box_k, map);
+}
+
+}  // namespace
+
+// A fused launch copies the FP32 operands with TMA: each needs a unit
+// stride, a 16-byte aligned base and leading dimension, and k > 0 (a K == 0
+// problem's operands may be empty); implicit im2col gathers take the
+// pre-pass.
+bool fusable(const Gemm& x) {
+  if (x.K == 0 || x.b_im2col || x.pieces) return false;
+  long long a_sr, a_sk, b_sr, b_sk;
+  split_operand_strides(x, &a_sr, &a_sk, &b_sr, &b_sk);
+  auto ok = [](const float* p, long long sr, long long sk) {
+    const long long ld = sk == 1 ? sr : sk;
+    return (sr == 1 || sk == 1) && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0;
+  };
+  return ok(x.A, a_sr, a_sk) && ok(x.B, b_sr, b_sk);
+}
+
+bool fused_encode_problem(const Gemm& x, bool swap, int bn, CUtensorMap* maps, TcProblem* tp) {
+  // operand a is op(B)^T when the problem is computed transposed
+  long long a_sr, a_sk, b_sr, b_sk;
+  split_operand_strides(x, &a_sr, &a_sk, &b_sr, &b_sk);
+  const int bk = fused_raw_k(bn);
+  if (swap)
+    return fused_operand_map(x.B, b_sr, b_sk, x.N, x.K, kTcBM, bk, &maps[0], &tp->kc_a) &&
+           fused_operand_map(x.A, a_sr, a_sk, x.M, x.K, bn, bk, &maps[1], &tp->kc_b);
+  return fused_operand_map(x.A, a_sr, a_sk, x.M, x.K, kTcBM, bk, &maps[0], &tp->kc_a) &&
+         fused_operand_map(x.B, b_sr, b_sk, x.N, x.K, bn, bk, &maps[1], &tp->kc_b);
+}
+
+namespace {
+
 ugemm_status plan_fail(ugemm_status s, const char* msg) {
   set_last_error(s, msg);
   return s;
@@ -274,34 +318,6 @@ ugemm_status launch_plan(ugemm_grouped_plan_s* p, cudaStream_t st) {
                         split_chunk_stages(p->split.pieces, std::max(1, p->cfg.chunk_k / kTcKB)),
                         p->grid, p->dev_err, st, p->geo);
   return s == UGEMM_OK ? reduce_launch(p, st) : s;
-}
-
-// The FP32 source of one kernel operand of a fused launch (rows of op(A),
-// or of op(B)^T, by k) as a 2-D tensor map: k contiguous (row stride sr) or
-// rows contiguous (k stride sk).  *kc says which.
-bool fused_operand_map(const float* base, long long sr, long long sk, int rows, int K,
-                       int box_rows, int box_k, CUtensorMap* map, int* kc) {
-  if (sk == 1) {
-    *kc = 1;
-    return fused_encode_map(base, sr, rows, K, true, box_rows, box_k, map);
-  }
-  *kc = 0;
-  return sr == 1 && fused_encode_map(base, sk, K, rows, false, box_rows, box_k, map);
-}
-
-// A fused launch copies the FP32 operands with TMA: each needs a unit
-// stride, a 16-byte aligned base and leading dimension, and k > 0 (a K == 0
-// problem's operands may be empty); implicit im2col gathers take the
-// pre-pass.
-bool fusable(const Gemm& x) {
-  if (x.K == 0 || x.b_im2col || x.pieces) return false;
-  long long a_sr, a_sk, b_sr, b_sk;
-  split_operand_strides(x, &a_sr, &a_sk, &b_sr, &b_sk);
-  auto ok = [](const float* p, long long sr, long long sk) {
-    const long long ld = sk == 1 ? sr : sk;
-    return (sr == 1 || sk == 1) && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0;
-  };
-  return ok(x.A, a_sr, a_sk) && ok(x.B, b_sr, b_sk);
 }
 
 // Columns of C as the kernel computes it: a kPix problem's are (tap, channel)
@@ -421,6 +437,29 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
         widest = std::max(widest, padded_area(n, x.M, 128) < padded_area(x.M, n, 128) ? x.M : n);
       }
       if (widest <= 128) p->cfg.block_n = 128;
+    }
+  }
+  // Untuned groups of three pieces whose operands TMA can copy: the launch that
+  // splits them itself, or a pre-pass and 256-wide tiles, by the time of their
+  // stages (1.14 us a 128-wide fused one, 0.80 a 256-wide one and 3 a tile, 2.2
+  // for a million elements split beforehand).  256-problem group: 135 and 222 us;
+  // 4096^3: 0.81 and 0.54 ms.
+  if (!config && form != UGEMM_PREC_SIMT && split_plan_for(form, g[0]).pieces == 3 &&
+      g[0].block_n == 0 && std::all_of(g.begin(), g.end(), fusable)) {
+    double fused = 0, whole = 5, elements = 0;
+    for (const Gemm& x : g) {
+      const int nkb = split_nkb(3, x.K);
+      auto tiles = [&](int bn) {
+        const bool sw = padded_area(x.N, x.M, bn) < padded_area(x.M, x.N, bn);
+        return double(cdiv(sw ? x.N : x.M, kTcBM)) * cdiv(sw ? x.M : x.N, bn);
+      };
+      fused += tiles(128) * nkb * 1.14;
+      whole += tiles(256) * (nkb * 0.80 + 3) / device_sms();
+      elements += (double(x.M) + x.N) * x.K;
+    }
+    if (count > 1 && fused / device_sms() < whole + split_pass_us(elements)) {
+      p->cfg.fused = 1;
+      p->cfg.block_n = 128;
     }
   }
   if (form != UGEMM_PREC_SIMT) {
@@ -659,19 +698,7 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       if (conv) {
         ok = conv_encode_maps(*x.pieces, x.M, ncols, bn, o.swap, &maps[4 * i], &cgeo[i]);
       } else if (p->split.fused) {
-        // the kernel copies the FP32 operands; its operand a is op(B)^T
-        // when the problem is computed transposed
-        long long a_sr, a_sk, b_sr, b_sk;
-        split_operand_strides(x, &a_sr, &a_sk, &b_sr, &b_sk);
-        const int bk = fused_raw_k(bn);
-        ok = o.swap ? fused_operand_map(x.B, b_sr, b_sk, x.N, x.K, kTcBM, bk, &maps[2 * i],
-                                        &tp.kc_a) &&
-                          fused_operand_map(x.A, a_sr, a_sk, x.M, x.K, bn, bk, &maps[2 * i + 1],
-                                            &tp.kc_b)
-                    : fused_operand_map(x.A, a_sr, a_sk, x.M, x.K, kTcBM, bk, &maps[2 * i],
-                                        &tp.kc_a) &&
-                          fused_operand_map(x.B, b_sr, b_sk, x.N, x.K, bn, bk, &maps[2 * i + 1],
-                                            &tp.kc_b);
+        ok = fused_encode_problem(x, o.swap, bn, &maps[2 * i], &tp);
       } else {
         const void* da = base + a_off[u.j];
         const void* db = base + b_off[u.j];

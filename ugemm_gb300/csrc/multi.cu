@@ -47,7 +47,8 @@ struct Layout {
   int block_n = 256;
   size_t a_off[kMultiMax], b_off[kMultiMax], part_off[kMultiMax];
   size_t total = 0;
-  double us = 0;  // one GEMM: the model's time of the launch and its reduce
+  double us = 0;       // one GEMM: the model's time of all its launches
+  bool fused = false;  // one GEMM: the operands split inside the GEMM kernel
 };
 
 // One GEMM: the tile width and slices of the least time by the stage times.
@@ -69,6 +70,21 @@ Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
       L.us = c.us;
       L.block_n = bn;
       L.geo[0] = c;
+    }
+    // the pieces' traffic (16 bytes an element) against slower stages: fused
+    // where one side of the output is short
+    L.us += split_pass_us((double(gs[0].M) + gs[0].N) * gs[0].K);
+    if (p.pieces == 3 && p.products == 6 && fusable(gs[0])) {
+      GeoChoice c;
+      c.us = fused_us(gs[0], sms, &c.swap, &c.slices, std::min(kMultiSubs, most(gs[0])));
+      if (c.us < L.us) {
+        const int nkb = split_nkb(3, gs[0].K);
+        c.per = cdiv(nkb, c.slices);
+        L.us = c.us;
+        L.block_n = 128;
+        L.geo[0] = c;
+        L.fused = true;
+      }
     }
   } else {
     int widest = 0;
@@ -103,7 +119,8 @@ Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
   }
   size_t off = 0;
   for (int i = 0; i < n; ++i) {
-    L.a_off[i] = off;
+    L.a_off[i] = L.b_off[i] = off;
+    if (L.fused) continue;  // no pieces in memory
     off += split_operand_bytes(p.pieces, gs[i].M, gs[i].K);
     L.b_off[i] = off;
     off += split_operand_bytes(p.pieces, gs[i].N, gs[i].K);
@@ -204,7 +221,8 @@ bool multi_wanted(const Gemm& g, const SplitPlan& p) {
   if (tiles > 4 * sms) return false;
   const GeoChoice whole = choose_geometry(p.pieces, g.M, g.N, split_nkb(p.pieces, g.K), sms,
                                           p.block_n, false, 1);
-  return layout_for(&g, 1, p, sms).us < 0.95 * whole.us;
+  return layout_for(&g, 1, p, sms).us <
+         0.95 * (whole.us + split_pass_us((double(g.M) + g.N) * g.K));
 }
 
 size_t multi_scratch_bytes(const Gemm* gs, int n, const SplitPlan& p) {
@@ -223,6 +241,7 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
   SplitPlan p = plan;
   p.block_n = L.block_n;
   p.epi = false;
+  p.fused = L.fused;
 
   MultiTable t = empty_table();
   ReduceJob red[kMultiMax];
@@ -239,7 +258,9 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
     void* bp = base + L.b_off[i];
     long long a_sr, a_sk, b_sr, b_sk;
     split_operand_strides(g, &a_sr, &a_sk, &b_sr, &b_sk);
-    if (p.f16) {  // the FP16x3 split needs each operand's row maxima first
+    int kc[2] = {1, 1};
+    if (L.fused) {  // nothing to split beforehand
+    } else if (p.f16) {  // the FP16x3 split needs each operand's row maxima first
       ugemm_status s = split_operand_launch(p.pieces, g.A, a_sr, a_sk, g.M, g.K, ap, st, true);
       if (s == UGEMM_OK) s = split_operand_launch(p.pieces, g.B, b_sr, b_sk, g.N, g.K, bp, st, true);
       if (s != UGEMM_OK) return s;
@@ -252,10 +273,19 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
                                split_tiles};
       split_tiles += cdiv(g.N, 32) * tk;
     }
-    const bool ok = o.swap ? split_encode_maps(p.pieces, p.block_n, bp, g.N, ap, g.M, g.K,
-                                               &t.maps[2 * i], &t.maps[2 * i + 1])
-                           : split_encode_maps(p.pieces, p.block_n, ap, g.M, bp, g.N, g.K,
-                                               &t.maps[2 * i], &t.maps[2 * i + 1]);
+    bool ok;
+    if (L.fused) {
+      TcProblem layouts{};
+      ok = fused_encode_problem(g, o.swap, p.block_n, &t.maps[2 * i], &layouts);
+      kc[0] = layouts.kc_a;
+      kc[1] = layouts.kc_b;
+    } else if (o.swap) {
+      ok = split_encode_maps(p.pieces, p.block_n, bp, g.N, ap, g.M, g.K, &t.maps[2 * i],
+                             &t.maps[2 * i + 1]);
+    } else {
+      ok = split_encode_maps(p.pieces, p.block_n, ap, g.M, bp, g.N, g.K, &t.maps[2 * i],
+                             &t.maps[2 * i + 1]);
+    }
     if (!ok) return UGEMM_ERR_CUDA;
     const bool sliced = o.slices > 1;
     float* part = reinterpret_cast<float*>(base + L.part_off[i]);
@@ -273,6 +303,8 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
       tp.tiles_n = cdiv(tp.N, p.block_n);
       tp.swap = o.swap ? 1 : 0;
       tp.map = i;
+      tp.kc_a = kc[0];
+      tp.kc_b = kc[1];
       tp.epi = sliced ? Epilogue{} : g.epi;
       p.epi |= tp.epi.bias != nullptr || tp.epi.act != 0;
       if (p.f16) {  // kernel operand a is op(B)^T's pieces when swapped

@@ -72,6 +72,11 @@ __device__ __forceinline__ void fence_tensormap(const CUtensorMap* map) {
                : "memory");
 }
 
+// Whether an instantiation can take its problems from a MultiTable, besides the
+// 128-wide fused ones made for it (there the search costs the others' converters
+// 5%: 256-problem group 134 -> 142 us).
+constexpr bool tc_table(bool grouped, bool fused, bool conv) { return grouped && !conv && !fused; }
+
 // Lane 0's value: the same in every lane already, but known to be so.
 template <typename T>
 __device__ __forceinline__ T uniform(T v) {
@@ -308,10 +313,11 @@ __device__ __forceinline__ void acc_add_tmem(uint32_t t, float (&acc)[HALF], int
 }
 
 // The converter warps of a fused launch (defined with the split helpers).
-template <int NP, int BN>
+template <int NP, int BN, bool TABLE>
 __device__ void fused_convert(const TcProblem* __restrict__ probs, const int4* __restrict__ tiles,
-                              uint8_t* pieces, uint8_t* raw, uint64_t* full, uint64_t* empty,
-                              uint64_t* raw_full, uint64_t* raw_empty, int ct, int* err);
+                              int total_tiles, uint8_t* pieces, uint8_t* raw, uint64_t* full,
+                              uint64_t* empty, uint64_t* raw_full, uint64_t* raw_empty, int ct,
+                              int* err);
 // The epilogue warps of a 256-wide fused launch, which also convert.
 template <int NP, int BN, bool EPI>
 __device__ void fused_dual(const TcProblem* __restrict__ probs, const int4* __restrict__ tiles,
@@ -338,7 +344,7 @@ __host__ __device__ constexpr uint32_t corr_code(int p) {
 // units, and shared memory stays below 256 KB, so the field never carries);
 // the product count is a template parameter, and the chunk position is a
 // counter rather than a remainder.
-template <int NP, int BN, bool GROUPED, bool TF32, bool FUSED, bool CONV, int NPROD>
+template <int NP, int BN, bool GROUPED, bool TF32, bool FUSED, bool CONV, bool TABLE, int NPROD>
 __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
                                                const TcProblem* __restrict__ probs,
                                                const int4* __restrict__ tiles, int total_tiles,
@@ -353,7 +359,6 @@ __device__ __forceinline__ void mma_issue_loop(const TcProblem& single,
   constexpr uint32_t SBO = WIDE ? 1024 : 512, SWZ = WIDE ? 2 : 4;
   constexpr int NST = FUSED ? kTcFusedPieceStages : S::STAGES;
   constexpr int NB = S::ACC_BUFS;
-  constexpr bool TABLE = GROUPED && !FUSED && !CONV;
   // instruction descriptor operand format: bf16 pieces (1), the FP16x3
   // form's fp16 pieces (0) or the TF32x3 form's tf32 pieces (2); one k step
   // is 32 bytes of a row in each: 16 16-bit or 8 tf32 elements
@@ -625,21 +630,20 @@ template <> struct TableParam<false> {};
 // CONV (grouped launches of PieceOperands problems): the producer reads the
 // im2col operand of each problem through TMA's im2col mode.
 template <int NP, int BN, bool GROUPED, bool EPI, bool TF32 = false, bool FUSED = false,
-          bool CONV = false>
+          bool CONV = false, bool TABLE = tc_table(GROUPED, FUSED, CONV)>
 __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1)
     split_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ TcProblem single, const CUtensorMap* __restrict__ maps,
                     const TcProblem* __restrict__ probs, const int4* __restrict__ tiles,
                     int total_tiles, int nprod,
                     int chunk_kb, int fmt, const ConvGeo* __restrict__ geo, int* err,
-                    const __grid_constant__ TableParam<GROUPED && !FUSED && !CONV> table) {
+                    const __grid_constant__ TableParam<TABLE> table) {
   // fmt: 16-bit piece format, 0 bf16, 1 fp16 (FP16x3); TF32 instantiations
   // read two planes of 32-deep stages with the 128-byte rows of the
   // two-piece 16-bit shape
   static_assert(!TF32 || NP == 2, "TF32 pieces come in two planes");
   static_assert(!FUSED || (NP == 3 && GROUPED && !TF32), "fused: grouped bf16x3-piece launches");
   static_assert(!CONV || (NP == 3 && GROUPED && !FUSED), "conv: grouped launches on bf16 pieces");
-  constexpr bool TABLE = GROUPED && !FUSED && !CONV;
   if constexpr (TABLE) {
     if (probs == nullptr) {
       probs = table.t.probs;
@@ -719,7 +723,7 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       // threads of warps 12 and 13 first (see fused_convert)
       static_assert(kTcConvWarps == 6 && 2 + kTcEpiWarps == 10, "converter warps 10-15");
       if constexpr (FUSED && !DUAL)
-        fused_convert<NP, BN>(probs, tiles, smem, smem + NST * S::STAGE_BYTES, full, empty,
+        fused_convert<NP, BN, TABLE>(probs, tiles, total_tiles, smem, smem + NST * S::STAGE_BYTES, full, empty,
                               raw_full, raw_empty, ((warp - 2 - kTcEpiWarps + 4) % 6) * 32 + lane,
                               err);
     } else if (FUSED && warp == 0) {
@@ -734,8 +738,10 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
           const TileCoord tc = tile_coord<BN, GROUPED, TABLE>(single, probs, tiles, t, P);
           const CUtensorMap* ma = &maps[2 * P.map];
           const CUtensorMap* mb = &maps[2 * P.map + 1];
-          fence_tensormap(ma);
-          fence_tensormap(mb);
+          if (!TABLE || tiles != nullptr) {
+            fence_tensormap(ma);
+            fence_tensormap(mb);
+          }
           // each piece stage from kTcKB / RAW_K raw stages
           for (int kr = 0; ok && kr < P.nkb * (kTcKB / S::RAW_K); ++kr, ++it) {
             const int s = it % RST;
@@ -802,15 +808,15 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       // the product count as a compile-time constant: two-piece forms have
       // three products, three-piece ones six (BF16x6) or nine (BF16x9)
       if constexpr (NP == 2)
-        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 3>(
+        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, TABLE, 3>(
             single, probs, tiles, total_tiles, smem, tmem, full, empty, main_full, main_empty,
             tile_full, tmem_empty, chunk_kb, fmt, geo, err);
       else if (nprod == 9)
-        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 9>(
+        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, TABLE, 9>(
             single, probs, tiles, total_tiles, smem, tmem, full, empty, main_full, main_empty,
             tile_full, tmem_empty, chunk_kb, fmt, geo, err);
       else
-        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, 6>(
+        mma_issue_loop<NP, BN, GROUPED, TF32, FUSED, CONV, TABLE, 6>(
             single, probs, tiles, total_tiles, smem, tmem, full, empty, main_full, main_empty,
             tile_full, tmem_empty, chunk_kb, fmt, geo, err);
       __syncwarp();
@@ -1549,10 +1555,11 @@ __global__ void __launch_bounds__(256) operand_max_batched_kernel(const SplitJob
 // SM sub-partitions 2, 3, 0, 1, 2, 3: the caller numbers the threads of
 // warps 12 and 13, alone on theirs, first, so that the chunks left over
 // after five rounds (threads 0-63 take a sixth) fall to them (140 -> 137 us).
-template <int NP, int BN>
+template <int NP, int BN, bool TABLE>
 __device__ void fused_convert(const TcProblem* __restrict__ probs, const int4* __restrict__ tiles,
-                              uint8_t* pieces, uint8_t* raw, uint64_t* full, uint64_t* empty,
-                              uint64_t* raw_full, uint64_t* raw_empty, int ct, int* err) {
+                              int total_tiles, uint8_t* pieces, uint8_t* raw, uint64_t* full,
+                              uint64_t* empty, uint64_t* raw_full, uint64_t* raw_empty, int ct,
+                              int* err) {
   using S = TcShape<NP, BN, false>;
   constexpr int CH_A = kTcBM * (kTcKB / 8);
   constexpr int CH = CH_A + BN * (kTcKB / 8);
@@ -1562,12 +1569,13 @@ __device__ void fused_convert(const TcProblem* __restrict__ probs, const int4* _
   static_assert(kTcKB == 32 && S::RAW_K == kTcKB,
                 "32-deep stages: 128-byte raw rows, 64-byte piece rows");
   static_assert(S::RAW_A % 32 == 0, "bit 4 of a raw offset is bit 0 of its 16-byte unit");
-  const int4 range = tiles[blockIdx.x];
+  const TileRange tr = tile_range<true, TABLE>(tiles, total_tiles);
   uint32_t it = 0;
-  for (int t = range.x; t < range.y; ++t) {
-    const int4 rec = tiles[gridDim.x + t];
-    const TcProblem& P = probs[rec.x];
-    const int nkb = P.nkb, kc_a = P.kc_a, kc_b = P.kc_b;
+  for (int t = tr.first; t < tr.end; t += tr.step) {
+    int p = 0;  // the tile's problem, of which the converters read three fields
+    if (!TABLE || tiles != nullptr) p = tiles[gridDim.x + t].x;
+    else while (p + 1 < kMultiSubs && probs[p + 1].tile_start <= t) ++p;
+    const int nkb = probs[p].nkb, kc_a = probs[p].kc_a, kc_b = probs[p].kc_b;
     // this tile's chunk offsets: raw bytes from the raw stage (for a
     // [rows][32] tile the first of its two units; the second is at bit 4
     // flipped: unit (2c + 1) ^ (r & 7) = ((2c) ^ (r & 7)) ^ 1) and piece bytes
@@ -1942,14 +1950,15 @@ void launch_split(const float* src, long long sr, long long sk, int rows, int K,
   prof_end(st, kProfSplitPrep);
 }
 
-template <int NP, int BN, bool GROUPED, bool EPI, bool TF32, bool FUSED = false, bool CONV = false>
+template <int NP, int BN, bool GROUPED, bool EPI, bool TF32, bool FUSED = false, bool CONV = false,
+          bool TABLE = tc_table(GROUPED, FUSED, CONV)>
 ugemm_status launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const TcProblem& single,
                            const CUtensorMap* maps, const TcProblem* probs, const int4* tiles,
                            int total_tiles, int nprod, int chunk_kb, int max_ctas, int fmt,
                            int* dev_err, cudaStream_t st, const ConvGeo* geo = nullptr,
                            const MultiTable* table = nullptr) {
   using S = TcShape<NP, BN, tc_wide(NP, TF32)>;
-  auto kern = split_tc_kernel<NP, BN, GROUPED, EPI, TF32, FUSED, CONV>;
+  auto kern = split_tc_kernel<NP, BN, GROUPED, EPI, TF32, FUSED, CONV, TABLE>;
   static std::atomic<uint64_t> attr_done{0};  // per instantiation and device
   constexpr size_t kSmem = FUSED ? S::SMEM_FUSED : S::SMEM;
   static_assert(kSmem <= 232448, "shared memory budget");
@@ -1963,8 +1972,8 @@ ugemm_status launch_kernel(const CUtensorMap& ta, const CUtensorMap& tb, const T
   }
   if (!smem_attr_once(kern, kSmem, attr_done)) return UGEMM_ERR_CUDA;
   const int grid = std::max(1, std::min(total_tiles, max_ctas > 0 ? max_ctas : device_sms()));
-  TableParam<GROUPED && !FUSED && !CONV> tp;
-  if constexpr (GROUPED && !FUSED && !CONV) {
+  TableParam<TABLE> tp;
+  if constexpr (TABLE) {
     if (table) tp.t = *table;
     else if (!probs) return UGEMM_ERR_ARG;
   }
@@ -2063,6 +2072,33 @@ GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int b
           best.per = per;
           best.us = us;
         }
+      }
+    }
+  }
+  return best;
+}
+
+double split_pass_us(double elements) { return 3.0 + 2.2e-6 * elements; }
+
+// A fused stage of a 128 x 128 tile takes 1.14 us with all SMs busy.
+double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_slices) {
+  const int nkb = split_nkb(3, g.K);
+  double best = 1e300;
+  for (int sw = 0; sw < 2; ++sw) {
+    const double tiles = double(cdiv(sw ? g.N : g.M, kTcBM)) * cdiv(sw ? g.M : g.N, 128);
+    int last = 0;
+    for (int sl = 1; sl <= max_slices && sl <= nkb; ++sl) {
+      const int per = cdiv(nkb, sl);
+      if (sl > 1 && per < 4) break;
+      if (per == last) continue;
+      last = per;
+      const int n = cdiv(nkb, per);
+      double us = std::ceil(tiles * n / std::max(1.0, share)) * (per * 1.14 + 3.0);
+      if (n > 1) us += 3.0 + (n + 1.0) * g.M * g.N * 4 / 4e6;
+      if (us < best - 1e-9) {
+        best = us;
+        *swap = sw != 0;
+        *slices = n;
       }
     }
   }
@@ -2275,15 +2311,17 @@ ugemm_status split_gemm_launch(const SplitPlan& p, const CUtensorMap& ta, const 
   if (p.fused) {  // grouped launches of three bf16 pieces only
     if (p.pieces != 3 || !grouped || (p.block_n == 256 && single.chunk_sums == nullptr))
       return UGEMM_ERR_ARG;
-#define UGEMM_FUSED_CASE(BN, EPI)                                                                \
-  if (p.block_n == BN && p.epi == EPI)                                                          \
-    return launch_kernel<3, BN, true, EPI, false, true>(ta, tb, single, maps, probs, tiles,     \
-                                                        total_tiles, p.products, chunk_kb,      \
-                                                        max_ctas, 0, dev_err, st);
-    UGEMM_FUSED_CASE(128, false)
-    UGEMM_FUSED_CASE(128, true)
-    UGEMM_FUSED_CASE(256, false)
-    UGEMM_FUSED_CASE(256, true)
+#define UGEMM_FUSED_CASE(BN, EPI, TAB)                                                           \
+  if (p.block_n == BN && p.epi == EPI && (table != nullptr) == TAB)                             \
+    return launch_kernel<3, BN, true, EPI, false, true, false, TAB>(                            \
+        ta, tb, single, maps, probs, tiles, total_tiles, p.products, chunk_kb, max_ctas, 0,     \
+        dev_err, st, nullptr, table);
+    UGEMM_FUSED_CASE(128, false, false)
+    UGEMM_FUSED_CASE(128, true, false)
+    UGEMM_FUSED_CASE(128, false, true)
+    UGEMM_FUSED_CASE(128, true, true)
+    UGEMM_FUSED_CASE(256, false, false)
+    UGEMM_FUSED_CASE(256, true, false)
 #undef UGEMM_FUSED_CASE
     return UGEMM_ERR_ARG;
   }

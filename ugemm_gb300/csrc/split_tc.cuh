@@ -239,6 +239,15 @@ struct GeoChoice {
 GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int block_n,
                           bool transpose, int max_slices);
 
+// The same for a fused launch (128-wide tiles; operands copied as FP32), and what
+// splitting `elements` operand elements beforehand takes.
+double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_slices);
+double split_pass_us(double elements);
+// Whether a fused launch can copy the operands.
+bool fusable(const Gemm& g);
+// The raw-tile maps and layouts of a fused problem.
+bool fused_encode_problem(const Gemm& g, bool swap, int block_n, CUtensorMap* maps, TcProblem* p);
+
 int split_kp(int K);
 int split_default_chunk_kb(int K);
 // Bytes of one operand's pieces [pieces][rows][Kp]; two-piece operands also
