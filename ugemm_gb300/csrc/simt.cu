@@ -96,12 +96,13 @@ struct AccTile<TM, TN, Pair::kNone> {
 // columns are k-contiguous (tb == 'T').  k-contiguous operands are read as
 // float4 of 4 k, eight columns of B at a time; the other layout is read per
 // k, so few fragment values are live beside the accumulators.
-template <int TM, int TN, bool AK, bool BKM>
+// BOX: columns of B to a box of its map, [32][BOX] in the stage.
+template <int TM, int TN, bool AK, bool BKM, int BOX>
 __device__ __forceinline__ void simt_consume(const float* As, const float* Bs,
                                              AccTile<TM, TN, pair_of<AK, BKM>()>& acc) {
   constexpr Pair P = pair_of<AK, BKM>();
-  constexpr int BM = 16 * TM, BW = TN > 8 ? 128 : 16 * TN;  // BW: columns of a B box
-  constexpr int JG = BKM && TN > 8 ? 8 : TN;  // columns of a B fragment
+  constexpr int BM = 16 * TM;
+  constexpr int JG = BKM && TN > 8 ? (TN % 8 ? 4 : 8) : TN;  // columns of a B fragment
   constexpr bool A4 = AK || BKM;              // A's fragment covers the 4 k of a step
   const int tid = threadIdx.x;
   const int ty = tid >> 4, tx = tid & 15;
@@ -148,11 +149,11 @@ __device__ __forceinline__ void simt_consume(const float* As, const float* Bs,
           float4 ak[TM / 4];
           if constexpr (!A4) load_a(kk, ak);
           if constexpr (P == Pair::kN) {
-            // [32][BN], 128 columns a box; thread columns 64 g + 4 tx + {0..3}
+            // thread columns 64 g + 4 tx + {0..3}
 #pragma unroll
             for (int g = 0; g < TN / 4; ++g)
-              b4[g] = *reinterpret_cast<const float4*>(Bs + (g / 2) * 128 * kBK +
-                                                       (4 * q + kk) * BW + 64 * (g % 2) + 4 * tx);
+              b4[g] = *reinterpret_cast<const float4*>(
+                  Bs + 64 * g / BOX * BOX * kBK + (4 * q + kk) * BOX + 64 * g % BOX + 4 * tx);
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
               const float v = AK ? el(a4[A4 ? i : 0], kk) : el(ak[i / 4], i % 4);
@@ -193,7 +194,7 @@ __device__ __forceinline__ bool simt_mainloop(const uint8_t* smem, uint64_t* ful
     const int s = it % kStages;
     if (!mbar_wait(&full[s], (it / kStages) & 1, err, kDevTimeoutFull)) return false;
     const float* As = reinterpret_cast<const float*>(smem + s * S::STAGE_BYTES);
-    simt_consume<TM, TN, AK, BKM>(As, As + S::A_BYTES / 4, acc);
+    simt_consume<TM, TN, AK, BKM, S::BN>(As, As + S::A_BYTES / 4, acc);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   }
@@ -324,8 +325,9 @@ __global__ void __launch_bounds__(kThreads, AK && BKM ? 1 : 2)
 // busy as the FMA pipe and both reach about 70%; an 8 x 16 block reads 24
 // words for 128 FMAs, three quarters of that.  128 x 256 tiles are coarse,
 // so the last of them, which would not fill a wave of SMs, run as two
-// 128 x 128 tiles each (CTAs from `wide_tiles` on).
-template <int TM, int TN, bool AK, bool BKM>
+// 128 x 128 tiles each (CTAs from `wide_tiles` on); 8 x 12 blocks, 128 x 192
+// tiles, fill the waves of some outputs better (np_tiles).
+template <int TM, int TN, bool AK, bool BKM, int BOX>
 __device__ __forceinline__ void simt_np_tile(uint8_t* smem, const CUtensorMap& tmA,
                                              const CUtensorMap& tmB, float* __restrict__ C, int M,
                                              int N, int K, int ldc, float alpha, float beta,
@@ -343,11 +345,10 @@ __device__ __forceinline__ void simt_np_tile(uint8_t* smem, const CUtensorMap& t
     mbar_arrive_expect_tx(&full[s], S::STAGE_BYTES);
     if (AK) tma_load_2d(sa, &tmA, &full[s], kt * kBK, m0);
     else    tma_load_2d(sa, &tmA, &full[s], m0, kt * kBK);
-    // B's map has boxes of 128 columns, one or two to a tile
 #pragma unroll
-    for (int h = 0; h < S::BN / 128; ++h) {
-      if (BKM) tma_load_2d(sb + h * 128 * kBK * 4, &tmB, &full[s], kt * kBK, n0 + 128 * h);
-      else     tma_load_2d(sb + h * 128 * kBK * 4, &tmB, &full[s], n0 + 128 * h, kt * kBK);
+    for (int h = 0; h < S::BN / BOX; ++h) {
+      if (BKM) tma_load_2d(sb + h * BOX * kBK * 4, &tmB, &full[s], kt * kBK, n0 + BOX * h);
+      else     tma_load_2d(sb + h * BOX * kBK * 4, &tmB, &full[s], n0 + BOX * h, kt * kBK);
     }
   };
   if (tid == 0) {
@@ -375,14 +376,14 @@ __device__ __forceinline__ void simt_np_tile(uint8_t* smem, const CUtensorMap& t
     const int s = kt % kStages;
     if (!mbar_wait(&full[s], (kt / kStages) & 1, err, kDevTimeoutFull)) return;
     const float* As = reinterpret_cast<const float*>(smem + s * W::STAGE_BYTES);
-    simt_consume<TM, TN, AK, BKM>(As, As + S::A_BYTES / 4, acc);
+    simt_consume<TM, TN, AK, BKM, BOX>(As, As + S::A_BYTES / 4, acc);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[s]);
   }
   simt_store<TM, TN, AK, BKM>(acc, C, M, N, ldc, alpha, beta, m0, n0, epi);
 }
 
-template <bool AK, bool BKM>
+template <bool AK, bool BKM, int WT>
 __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     simt_sgemm_np_kernel(const __grid_constant__ CUtensorMap tmA,
                          const __grid_constant__ CUtensorMap tmB, float* __restrict__ C, int M,
@@ -390,21 +391,23 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
                          int tiles_m, int tiles_n, int wide_tiles, int* err) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  // tiles_m x tiles_n tiles of 128 x 256 in raster order
+  // tiles_m x tiles_n tiles of 128 x W in raster order
+  constexpr int W = 16 * WT, BOX = W % 128 == 0 ? 128 : 64;
   const int b = blockIdx.x;
   int tile_m, tile_n;
   if (b < wide_tiles) {
     if constexpr (pair_of<AK, BKM>() != Pair::kNone) {
       raster_tile(b, tiles_m, tiles_n, tile_m, tile_n);
-      simt_np_tile<8, 16, AK, BKM>(smem, tmA, tmB, C, M, N, K, ldc, alpha, beta, epi,
-                                   tile_m * 128, tile_n * 256, err);
+      simt_np_tile<8, WT, AK, BKM, BOX>(smem, tmA, tmB, C, M, N, K, ldc, alpha, beta, epi,
+                                   tile_m * 128, tile_n * W, err);
     }
   } else {
     raster_tile(wide_tiles + (b - wide_tiles) / 2, tiles_m, tiles_n, tile_m, tile_n);
-    const int n0 = tile_n * 256 + ((b - wide_tiles) & 1) * 128;
-    if (n0 < N)
-      simt_np_tile<8, 8, AK, BKM>(smem, tmA, tmB, C, M, N, K, ldc, alpha, beta, epi, tile_m * 128,
-                                  n0, err);
+    const int n0 = tile_n * W + ((b - wide_tiles) & 1) * 128;
+    const int n1 = min(N, (tile_n + 1) * W);  // the next tile's columns are not this one's
+    if (n0 < n1)
+      simt_np_tile<8, 8, AK, BKM, BOX>(smem, tmA, tmB, C, M, n1, K, ldc, alpha, beta, epi,
+                                  tile_m * 128, n0, err);
   }
 }
 
@@ -586,22 +589,33 @@ void stored_b(const Gemm& g, int& rows, int& cols) {
 // what is left of them runs as narrow ones when those fit in one wave, and
 // everything runs narrow where that takes fewer waves' time (a right edge that
 // leaves half of the wide tiles empty).
-constexpr double kNarrowCost = 0.56;
+constexpr double kNarrowCost = 0.56, kMiddleCost = 0.78;  // 128 and 192 wide
 // 64 x 64 tiles, two CTAs to an SM: 69 us per 1024 k and round of two to an SM.
 constexpr double kSmallCost = 0.40, kSmallHalfCost = 0.29;
 struct NpTiles {
-  int tiles_m, tiles_n, wide;  // 128 x 256 tiles, and how many run as such
-  double cost;                 // waves, in wide tiles
+  int width = 256;             // of the wide tiles
+  int tiles_m = 0, tiles_n = 0, wide = 0;  // wide tiles, and how many run as such
+  double cost = 0;             // waves, in 256-wide tiles
 };
 NpTiles np_tiles(int M, int N, bool wide_ok, int sms) {
-  NpTiles t{cdiv(M, 128), cdiv(N, 256), 0, 0};
-  const int total = t.tiles_m * t.tiles_n, rest = total % sms;
-  const bool tail = rest > 0 && 2 * rest <= sms;
-  const double mixed = total / sms + (rest == 0 ? 0.0 : tail ? kNarrowCost : 1.0);
-  const double narrow = kNarrowCost * cdiv(t.tiles_m * cdiv(N, 128), sms);
-  t.wide = !wide_ok || narrow < mixed ? 0 : tail ? total - rest : total;
-  t.cost = wide_ok ? std::min(narrow, mixed) : narrow;
-  return t;
+  NpTiles best;
+  best.tiles_m = cdiv(M, 128);
+  best.tiles_n = cdiv(N, 256);
+  best.cost = kNarrowCost * cdiv(best.tiles_m * cdiv(N, 128), sms);
+  for (int width : {256, 192}) {
+    if (!wide_ok) break;
+    NpTiles t;
+    t.width = width;
+    t.tiles_m = cdiv(M, 128);
+    t.tiles_n = cdiv(N, width);
+    const int total = t.tiles_m * t.tiles_n, rest = total % sms;
+    const bool tail = rest > 0 && 2 * rest <= sms;
+    const double wave = width == 256 ? 1.0 : kMiddleCost;
+    t.wide = tail ? total - rest : total;
+    t.cost = wave * (total / sms) + (rest == 0 ? 0.0 : tail ? kNarrowCost : wave);
+    if (t.cost < best.cost) best = t;
+  }
+  return best;
 }
 
 // Boxes of 32 k by rows_a rows of op(A), rows_b columns of op(B).
@@ -636,15 +650,19 @@ ugemm_status launch_t(const Gemm& g, int tile, const float* A, int lda, const fl
                                                        g.beta, g.epi, tiles_m, tiles_n, dev_err);
   } else {
     using S = SimtShape<8, 16>;
-    if (!encode_operands<AK, BKM>(g, A, lda, B, ldb, 128, 128, &ta, &tb)) return UGEMM_ERR_CUDA;
-    auto kern = simt_sgemm_np_kernel<AK, BKM>;
-    static std::atomic<uint64_t> attr_done{0};
-    if (!smem_attr_once(kern, S::SMEM, attr_done)) return UGEMM_ERR_CUDA;
     constexpr bool wide_ok = pair_of<AK, BKM>() != Pair::kNone;
     NpTiles t = np_tiles(g.M, g.N, wide_ok, device_sms());
+    if (tile != kSimtMixed) {
+      t.width = 256;
+      t.tiles_n = cdiv(g.N, 256);
+      t.wide = tile == kSimt128x256 && wide_ok ? t.tiles_m * t.tiles_n : 0;
+    }
+    if (!encode_operands<AK, BKM>(g, A, lda, B, ldb, 128, t.width == 192 ? 64 : 128, &ta, &tb))
+      return UGEMM_ERR_CUDA;
+    auto kern = t.width == 192 ? simt_sgemm_np_kernel<AK, BKM, 12> : simt_sgemm_np_kernel<AK, BKM, 16>;
+    static std::atomic<uint64_t> attr_done[2];  // per instantiation and device
+    if (!smem_attr_once(kern, S::SMEM, attr_done[t.width == 192])) return UGEMM_ERR_CUDA;
     const int total = t.tiles_m * t.tiles_n;
-    if (tile == kSimt128x128) t.wide = 0;
-    if (tile == kSimt128x256 && wide_ok) t.wide = total;
     prof_begin(st);
     kern<<<t.wide + 2 * (total - t.wide), kConsumerWarps * 32, S::SMEM, st>>>(
         ta, tb, g.C, g.M, g.N, g.K, g.ldc, g.alpha, g.beta, g.epi, t.tiles_m, t.tiles_n, t.wide,
