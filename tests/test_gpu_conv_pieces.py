@@ -63,6 +63,18 @@ def test_layer_against_fp64(prec, layer, batch, separate):
     stack.close()
 
 
+# edges of the weight split's tiles (72 taps x rows, 64 / 32 / 16 channels of up
+# to 72 / 144 / 256 taps): ragged rows and channels, one tap, even kernels, and
+# kernels on both sides of each limit
+@pytest.mark.parametrize("layer,batch", [
+    ((22, 33, 9, 9, 1, 3, 1), 2), ((70, 65, 9, 9, 1, 3, 1), 1), ((64, 33, 8, 8, 2, 1, 0), 2),
+    ((40, 47, 9, 9, 1, 2, 1), 1), ((72, 40, 10, 10, 1, 8, 4), 1), ((44, 70, 10, 10, 1, 9, 4), 1),
+    ((64, 44, 13, 13, 1, 12, 6), 1), ((44, 23, 14, 14, 1, 13, 6), 1),
+    ((64, 64, 17, 17, 1, 16, 8), 1)])
+def test_weight_split_tiles(layer, batch):
+    test_layer_against_fp64("bf16x6", layer, batch, False)
+
+
 def test_backward_alone_reads_the_inputs_it_is_given():
     """A backward run splits X itself: writing X between the two runs counts."""
     layer, batch = (64, 64, 8, 8, 1, 3, 1), 2

@@ -258,7 +258,7 @@ struct ugemm_conv_stack_s {
   // Split launches of a run: jobs [first, first + njobs) of the device list.
   struct Phase {
     int first = 0, njobs = 0, tiles = 0, tiles_first = 0;  // tiles_first: of the first job alone
-    bool taps = false;                                     // has (tap, channel) jobs
+    bool taps = false, col = false;  // weights by tap; a stored im2col matrix
   };
   std::vector<Phase> split_fwd, split_bwd;  // per layer: X (or col); dY, then X
   Phase split_w, split_wb;                  // every layer's weights
@@ -281,8 +281,9 @@ ugemm_status split_phase(const Stack* s, const Stack::Phase& ph, int njobs,
   if (njobs == 0) return UGEMM_OK;
   const ugemm::SplitJob* jobs = s->jobs + ph.first;
   const int tiles = njobs == ph.njobs ? ph.tiles : ph.tiles_first;
-  return ph.taps ? ugemm::split_taps_launch(jobs, njobs, tiles, st)
-                 : ugemm::split_batched_launch(3, jobs, njobs, tiles, st);
+  return ph.taps  ? ugemm::split_taps_launch(jobs, njobs, tiles, st)
+         : ph.col ? ugemm::split_col_launch(jobs, njobs, tiles, st)
+                  : ugemm::split_batched_launch(3, jobs, njobs, tiles, st);
 }
 
 int run_stack(Stack* s, int what, cudaStream_t st) {
@@ -449,7 +450,8 @@ ugemm_status make_pieces(Stack* s) {
     j.tile_start = ph.tiles;
     ph.tiles += split_job_tiles(j);
     if (ph.njobs++ == 0) ph.tiles_first = ph.tiles;
-    ph.taps |= j.gather != 0;
+    ph.taps |= j.gather == 3;
+    ph.col |= j.gather == 4;
     jobs.push_back(j);
   };
   // rows x K as stored with rows contiguous (ld between k): K-major pieces

@@ -1091,32 +1091,14 @@ struct RawTile {
   float v[2][4];
 };
 
-// Chunk of 8 channels that this thread splits in tile `tile` of a weight job
-// (gather 3): the taps of one row (or, flipped, of all rows) lie next to each
-// other in memory, so they vary fastest.
-struct TapChunk { int r, tap, c; };
-__device__ __forceinline__ TapChunk tap_chunk(const SplitJob& j, int tile) {
-  const int idx = tile * 256 + threadIdx.x, cg = j.cp / 8;
-  const int q = idx / j.kk, tap = idx - q * j.kk;
-  return j.flip ? TapChunk{q % j.rows, tap, (q / j.rows) * 8} : TapChunk{q / cg, tap, (q % cg) * 8};
-}
-
-// TAPS: the launch may hold (tap, channel) jobs (gather 3 and 4).  They are an
-// instantiation of their own: compiled into the common one they cost it
-// registers and so resident blocks (256-problem group: 94 -> 120 us).
-template <bool TAPS = false>
+// COL: the launch may hold a stored im2col matrix (gather 4); GATHER: it may
+// hold implicit im2col operands (gather 1 and 2).  Instantiations of their own:
+// compiled into the common one, gather 4 cost it registers and so resident
+// blocks (256-problem group: 94 -> 120 us).
+template <bool COL = false, bool GATHER = true>
 __device__ __forceinline__ void load_raw(const SplitJob& j, int r0, int k0, RawTile& out) {
   const int t = threadIdx.x;
-  if (TAPS && j.gather == 3) {
-    const TapChunk x = tap_chunk(j, r0);
-    const bool ok = x.r < j.rows && x.c < j.cp;
-    const float* src = j.src + x.r * j.sr + (j.flip ? j.kk - 1 - x.tap : x.tap);
-#pragma unroll
-    for (int e = 0; e < 8; ++e)
-      out.v[e / 4][e % 4] = ok && x.c + e < j.chans ? src[(x.c + e) * j.sk] : 0.f;
-    return;
-  }
-  if (TAPS && j.gather == 4) {  // the thread layout of rows contiguous, k' mapped to (c, tap)
+  if (COL && j.gather == 4) {  // the thread layout of rows contiguous, k' mapped to (c, tap)
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int idx = t + 256 * i, kk = idx >> 3, q4 = (idx & 7) * 4, r = r0 + q4, k = k0 + kk;
@@ -1128,7 +1110,7 @@ __device__ __forceinline__ void load_raw(const SplitJob& j, int r0, int k0, RawT
     }
     return;
   }
-  if (j.gather) {  // implicit im2col: the same thread layout, gathered from x
+  if (GATHER && j.gather) {  // implicit im2col: the same thread layout, gathered from x
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int idx = t + 256 * i;
@@ -1217,14 +1199,8 @@ __device__ __forceinline__ void load_raw(const SplitJob& j, int r0, int k0, RawT
   }
 }
 
-template <bool TAPS = false>
 __device__ __forceinline__ void raw_to_smem(const SplitJob& j, const RawTile& in, float (*tile)[65]) {
   const int t = threadIdx.x;
-  if (TAPS && j.gather == 3) {  // each thread's own chunk, where split_store reads it
-#pragma unroll
-    for (int e = 0; e < 8; ++e) tile[t >> 3][(t & 7) * 8 + e] = in.v[e / 4][e % 4];
-    return;
-  }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int idx = t + 256 * i;
@@ -1242,16 +1218,11 @@ __device__ __forceinline__ void raw_to_smem(const SplitJob& j, const RawTile& in
 
 // bf16 pieces of one tile from shared memory: 8 consecutive k of one row per
 // thread, one 16-byte store per plane.
-template <int NP, int FMT, bool TAPS>
+template <int NP, int FMT>
 __device__ __forceinline__ void split_store(const SplitJob& j, int r0, int k0, float (*tile)[65]) {
   const int t = threadIdx.x;
   const int rr = t >> 3, g8 = (t & 7) * 8;
-  int r = r0 + rr, k = k0 + g8;
-  if (TAPS && j.gather == 3) {
-    const TapChunk x = tap_chunk(j, r0);
-    r = x.r;
-    k = x.c < j.cp ? x.tap * j.cp + x.c : j.Kp;
-  }
+  const int r = r0 + rr, k = k0 + g8;
   if (r >= j.rows || k >= j.Kp) return;
   const size_t plane = static_cast<size_t>(j.rows) * j.Kp;
   const int ex = FMT == 1 ? f16_row_exp(j.fmax, r) : 0;
@@ -1277,20 +1248,14 @@ __device__ __forceinline__ int find_job(const int* starts, const SplitJob* jobs,
   return lo;
 }
 
-template <bool TAPS = false>
 __device__ __forceinline__ void tile_origin(const SplitJob& j, int b, int& r0, int& k0) {
   const int local = b - j.tile_start;
-  if (TAPS && j.gather == 3) {
-    r0 = local;
-    k0 = 0;
-    return;
-  }
   const int tiles_k = (j.Kp + 63) / 64;
   r0 = (local / tiles_k) * 32;
   k0 = (local % tiles_k) * 64;
 }
 
-template <int NP, int FMT, bool TAPS>
+template <int NP, int FMT, bool COL>
 __device__ __forceinline__ void split_batched_body(const SplitJob* __restrict__ jobs, int njobs,
                                                    int total_tiles) {
   __shared__ float tile[32][65];
@@ -1304,21 +1269,21 @@ __device__ __forceinline__ void split_batched_body(const SplitJob* __restrict__ 
   if (b >= total_tiles) return;
   SplitJob cur = jobs[find_job(starts, jobs, njobs, b)];
   int r0, k0;
-  tile_origin<TAPS>(cur, b, r0, k0);
+  tile_origin(cur, b, r0, k0);
   RawTile raw;
-  load_raw<TAPS>(cur, r0, k0, raw);
+  load_raw<COL>(cur, r0, k0, raw);
   for (; b < total_tiles; b += gridDim.x) {
-    raw_to_smem<TAPS>(cur, raw, tile);
+    raw_to_smem(cur, raw, tile);
     const int nb = b + gridDim.x;
     SplitJob nxt = cur;
     int nr0 = 0, nk0 = 0;
     if (nb < total_tiles) {  // next tile's loads in flight during this tile's stores
       nxt = jobs[find_job(starts, jobs, njobs, nb)];
-      tile_origin<TAPS>(nxt, nb, nr0, nk0);
-      load_raw<TAPS>(nxt, nr0, nk0, raw);
+      tile_origin(nxt, nb, nr0, nk0);
+      load_raw<COL>(nxt, nr0, nk0, raw);
     }
     __syncthreads();
-    split_store<NP, FMT, TAPS>(cur, r0, k0, tile);
+    split_store<NP, FMT>(cur, r0, k0, tile);
     __syncthreads();
     cur = nxt;
     r0 = nr0;
@@ -1326,10 +1291,10 @@ __device__ __forceinline__ void split_batched_body(const SplitJob* __restrict__ 
   }
 }
 
-template <int NP, int FMT, bool TAPS = false>
+template <int NP, int FMT, bool COL = false>
 __global__ void __launch_bounds__(256) split_pieces_batched_kernel(const SplitJob* __restrict__ jobs,
                                                                    int njobs, int total_tiles) {
-  split_batched_body<NP, FMT, TAPS>(jobs, njobs, total_tiles);
+  split_batched_body<NP, FMT, COL>(jobs, njobs, total_tiles);
 }
 
 // The same for a few operands whose job records travel as the kernel's
@@ -1339,6 +1304,78 @@ template <int NP, int FMT>
 __global__ void __launch_bounds__(256) split_pieces_param_kernel(
     const __grid_constant__ SplitJobTable t, int njobs, int total_tiles) {
   split_batched_body<NP, FMT, false>(t.jobs, njobs, total_tiles);
+}
+
+// Weights as (tap, channel) pieces (gather 3), tap_rows rows x tap_chans
+// channels x all taps a tile, with plain operands between them.  The taps of
+// one weight lie next to each other in memory and a whole plane row apart in
+// the pieces, so whichever way threads read or write without a tile, one side
+// of the copy is one element a line: reading 36 bytes apart and writing 16-byte
+// chunks, the 12 layers' 7.8 M weights took 28.6 us and, flipped, 34.6.  Through
+// shared memory both sides are runs (reads of tap_rows or tap_chans times kk
+// floats, writes of 128 bytes): 18.1 and 23.3 us (4.3 TB/s; the bytes need 11.5).
+// One tile at a time, five blocks an SM for the loads in flight.
+constexpr int kTapTile = 4608 + 64;  // tap_rows * tap_chans * kk at most, and a word a run
+
+__device__ __forceinline__ void split_taps_tile(const SplitJob& j, int local, float* s) {
+  const int kk = j.kk, cw = tap_chans(kk), rw = tap_rows(kk), ncb = (j.cp + cw - 1) / cw;
+  const int rb = local / ncb, r0 = rb * rw, c0 = (local - rb * ncb) * cw;
+  const int nr = min(rw, j.rows - r0), nc = min(cw, j.cp - c0);  // nc: 64, 32 or 16
+  const int real = max(0, min(nc, j.chans - c0));                 // channels that exist
+  // a run of consecutive floats: a row's (channel, tap), or, transposed (flip),
+  // a channel's (row, tap), at an odd pitch that spreads the channels over the banks
+  const bool by_row = j.sk == kk;
+  const int pitch = by_row ? cw * kk : (rw * kk) | 1;
+  const float* __restrict__ src = j.src + r0 * j.sr + c0 * j.sk;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (by_row) {
+    for (int run = warp; run < nr; run += 8)
+#pragma unroll 6
+      for (int p = lane; p < real * kk; p += 32) s[run * pitch + p] = __ldg(src + run * j.sr + p);
+  } else {
+    for (int p = lane; p < nr * kk; p += 32)
+#pragma unroll 8
+      for (int run = warp; run < real; run += 8) s[run * pitch + p] = __ldg(src + run * j.sk + p);
+  }
+  __syncthreads();
+  const int sh = nc == 64 ? 3 : (nc == 32 ? 2 : 1), chunks = (nr * kk) << sh;
+  const size_t plane = static_cast<size_t>(j.rows) * j.Kp;
+  const int step = by_row ? kk : pitch;
+  for (int i = threadIdx.x; i < chunks; i += 256) {
+    const int c8 = (i & ((1 << sh) - 1)) * 8, q = i >> sh, r = q / kk, tap = q - r * kk;
+    const int st = j.flip ? kk - 1 - tap : tap;
+    const float* w = s + (by_row ? r * pitch : r * kk) + c8 * step + st;
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = c8 + e < real ? w[e * step] : 0.f;
+    store_pieces8<3, 0>(j.dst, plane,
+                        static_cast<size_t>(r0 + r) * j.Kp + tap * j.cp + c0 + c8, v, 0);
+  }
+}
+
+__global__ void __launch_bounds__(256, 5) split_taps_kernel(const SplitJob* __restrict__ jobs,
+                                                            int njobs, int total_tiles) {
+  __shared__ float tile[kTapTile];
+  __shared__ int starts[kJobCache];
+  const int cached = min(njobs, kJobCache);
+  for (int i = threadIdx.x; i < cached; i += blockDim.x) starts[i] = jobs[i].tile_start;
+  __syncthreads();
+  for (int b = blockIdx.x; b < total_tiles; b += gridDim.x) {
+    const SplitJob& j = jobs[find_job(starts, jobs, njobs, b)];
+    if (j.gather == 3) {
+      split_taps_tile(j, b - j.tile_start, tile);
+    } else {
+      auto* t = reinterpret_cast<float(*)[65]>(tile);
+      int r0, k0;
+      RawTile raw;
+      tile_origin(j, b, r0, k0);
+      load_raw<false, false>(j, r0, k0, raw);
+      raw_to_smem(j, raw, t);
+      __syncthreads();
+      split_store<3, 0>(j, r0, k0, t);
+    }
+    __syncthreads();
+  }
 }
 
 // FP16x3 form, first step of the split: the largest finite magnitude of
@@ -2374,11 +2411,20 @@ ugemm_status split_batched_launch(int pieces, const SplitJob* jobs, int njobs, i
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }
 
-ugemm_status split_taps_launch(const SplitJob* jobs, int njobs, int total_tiles, cudaStream_t st) {
+ugemm_status split_col_launch(const SplitJob* jobs, int njobs, int total_tiles, cudaStream_t st) {
   if (total_tiles <= 0) return UGEMM_OK;
   prof_begin(st);
   split_pieces_batched_kernel<3, 0, true>
       <<<std::min(total_tiles, device_sms() * 8), 256, 0, st>>>(jobs, njobs, total_tiles);
+  prof_end(st, kProfSplitPrep);
+  return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
+}
+
+ugemm_status split_taps_launch(const SplitJob* jobs, int njobs, int total_tiles, cudaStream_t st) {
+  if (total_tiles <= 0) return UGEMM_OK;
+  prof_begin(st);
+  split_taps_kernel<<<std::min(total_tiles, device_sms() * 5), 256, 0, st>>>(jobs, njobs,
+                                                                              total_tiles);
   prof_end(st, kProfSplitPrep);
   return cudaPeekAtLastError() == cudaSuccess ? UGEMM_OK : UGEMM_ERR_CUDA;
 }

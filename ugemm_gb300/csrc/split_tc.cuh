@@ -220,9 +220,18 @@ struct SplitJob {
   unsigned* fmax = nullptr;
 };
 
+// Rows and channels of a gather-3 job's tile: 64 channels, so that a row's tap
+// is a 128-byte run, and what then fits 4608 elements; fewer channels beyond 72
+// taps (8 x 8 kernels; 256 taps at most).
+__host__ __device__ inline int tap_rows(int kk) {
+  return kk > 72 ? 1 : (kk < 3 ? 32 : 72 / kk);
+}
+__host__ __device__ inline int tap_chans(int kk) { return kk > 144 ? 16 : (kk > 72 ? 32 : 64); }
+
 // Tiles of a job in the launch's tile list.
 inline int split_job_tiles(const SplitJob& j) {
-  return j.gather == 3 ? cdiv(j.rows * (j.Kp / 8), 256) : cdiv(j.rows, 32) * cdiv(j.Kp, 64);
+  return j.gather == 3 ? cdiv(j.rows, tap_rows(j.kk)) * cdiv(j.cp, tap_chans(j.kk))
+                       : cdiv(j.rows, 32) * cdiv(j.Kp, 64);
 }
 
 // How a problem of C (M x N) with nkb k-blocks is cut for a grouped launch of
@@ -353,6 +362,8 @@ ugemm_status split_batched_launch(int pieces, const SplitJob* jobs, int njobs, i
                                   cudaStream_t st, unsigned* fmax_words = nullptr, int nwords = 0);
 // Three-piece jobs of every kind, (tap, channel) ones included.
 ugemm_status split_taps_launch(const SplitJob* jobs, int njobs, int total_tiles, cudaStream_t st);
+// The same for a stored im2col matrix (gather 4).
+ugemm_status split_col_launch(const SplitJob* jobs, int njobs, int total_tiles, cudaStream_t st);
 // Split one operand into its pieces at dst (split_operand_bytes of room).
 // f16: FP16x3 pieces -- the largest magnitude of every row is first found
 // into the operand's trailer words (cleared here), then each row's pieces
