@@ -211,21 +211,26 @@ __device__ __forceinline__ void epi_store(const TcProblem& P, const TileCoord& t
     return;
   }
   // Each 32 x 32 block is transposed through shared memory, so that a store
-  // instruction writes one 128-byte row segment: all 32 rows at once where
-  // the ring leaves 32 x 33 floats a warp (STAGE_C), else 8 rows at a time
-  // (lanes 8p..8p+7 hold rows 8p..8p+7).  A batch of rows' old values is read
-  // together before any store: one at a time, each read waited for the store
-  // before it (C may alias itself as far as the compiler knows), and storing
-  // straight from registers, a row per lane, touched 32 lines per instruction
-  // (4095 x 4097 x 1023, beta = 0.5: 459 -> 166 us of GEMM kernel).  Grouped
-  // launches keep the row loops rolled: their tiles are short, and unrolled
-  // this code, which runs once a tile, missed the instruction cache (5 to 10
-  // us a tile); one GEMM's long tiles rather want many reads in flight
-  // (8192^3 FP16x3: 1.84 ms unrolled, 1.97 rolled).
-  constexpr int SROWS = S::STAGE_C ? 32 : 8, BATCH = GROUPED || SROWS == 8 ? 8 : 16;
-  constexpr int kUnroll = GROUPED ? 1 : 4;
-  float* stage = stage_base + ew * SROWS * 33;
+  // instruction writes whole row segments: all 32 rows at once where the ring
+  // leaves 32 x 32 floats a warp (STAGE_C), else 8 rows at a time (lanes
+  // 8p..8p+7 hold rows 8p..8p+7); the 16-byte units of a row are swizzled by
+  // the row, so no access has bank conflicts.  Old values are read GB rows at a
+  // time before any store: one at a time, each read waited for the store before
+  // it (C may alias itself as far as the compiler knows).  While a tile is
+  // stored nothing drains the next tile's chunks, so after one chunk the tensor
+  // pipe waits: what counts is the number of instructions.  Blocks inside the
+  // matrix therefore have no bounds tests and store four floats a lane (four
+  // rows an instruction) where C's rows are 16-byte aligned, one otherwise;
+  // with a test, a 64-bit product and a select at each of 128 row stores this
+  // took 28 500 cycles a 128 x 256 tile, now 10 700 (19 000 with unaligned rows
+  // and old values): 3072 x 4864 x 1024 in BF16x6 215 000 -> 171 000 cycles.
+  // Grouped launches roll the row loops: their tiles are short and unrolled
+  // code, run once a tile, misses the instruction cache.
+  constexpr int SROWS = S::STAGE_C ? 32 : 8;
+  constexpr int GB = GROUPED ? 8 : 32, SUB = GB < SROWS ? GB : SROWS;
+  float* stage = stage_base + ew * SROWS * 32;
   const int row0 = tc.m0 + q * 32;
+  const bool vec = (reinterpret_cast<uintptr_t>(P.C) & 15) == 0 && (P.ldc & 3) == 0;
   float bl = 0.f;  // lane l: the bias of row row0 + l
   if constexpr (EPI) {
     if (P.epi.bias != nullptr && row0 + lane < P.M) bl = __ldg(P.epi.bias + row0 + lane);
@@ -233,46 +238,99 @@ __device__ __forceinline__ void epi_store(const TcProblem& P, const TileCoord& t
 #pragma unroll
   for (int c32 = 0; c32 < HALF / 32; ++c32) {
     if (GROUPED && c32 * 32 >= n_live) break;
-    const int cc = tc.n0 + col_off + c32 * 32 + lane;
-    const bool live = cc < P.N;
-#pragma unroll kUnroll
-    for (int pass = 0; pass < 32 / SROWS; ++pass) {
-      if (row0 + pass * SROWS >= P.M) break;
-      float old[BATCH];
-      auto load_old = [&](int lr) {
-        const int rows = P.M - (row0 + lr);
-        const float* cp = P.C + static_cast<size_t>(row0 + lr) * P.ldc + cc;
+    const int c0 = tc.n0 + col_off + c32 * 32;
+    // rows [row, row + SROWS) of the block to the staging area
+    auto put = [&](int row) {
+      __syncwarp();
+      if (SROWS == 32 || (lane >> 3) == (row >> 3)) {
+        const int r = lane & (SROWS - 1);
 #pragma unroll
-        for (int rr = 0; rr < BATCH; ++rr) old[rr] = 0.f;
+        for (int u = 0; u < 8; ++u)
+          *reinterpret_cast<float4*>(stage + r * 32 + ((u ^ (r & 7)) * 4)) =
+              make_float4(acc[c32 * 32 + u * 4], acc[c32 * 32 + u * 4 + 1],
+                          acc[c32 * 32 + u * 4 + 2], acc[c32 * 32 + u * 4 + 3]);
+      }
+      __syncwarp();
+    };
+    auto value = [&](float sum, float old, int row) {
+      float x = scaled_sum(P, sum, old);
+      if constexpr (EPI) {
+        const float b = __shfl_sync(0xffffffffu, bl, row);
+        if (has_epi) x = epilogue_value(x, b, P.epi);
+      }
+      return x;
+    };
+    // a block inside the matrix: W floats of RPI rows an instruction
+    auto inside = [&](auto w) {
+      constexpr int W = decltype(w)::value, RPI = W;
+      using T = std::conditional_t<W == 4, float4, float>;
+      const int lr = W == 4 ? lane >> 3 : 0, lc = W == 4 ? (lane & 7) * 4 : lane;
+      const size_t step = static_cast<size_t>(RPI) * P.ldc;
+      float* cp = P.C + static_cast<size_t>(row0 + lr) * P.ldc + c0 + lc;
+#pragma unroll(GROUPED ? 1 : 4)
+      for (int g = 0; g < 32; g += GB) {
+        float old[GB / RPI][W];
+#pragma unroll
+        for (int i = 0; i < GB / RPI; ++i)
+#pragma unroll
+          for (int e = 0; e < W; ++e) old[i][e] = 0.f;
         if (P.beta != 0.f) {
+          const float* op = cp;
 #pragma unroll
-          for (int rr = 0; rr < BATCH; ++rr)
-            if (live && rr < rows) old[rr] = cp[static_cast<size_t>(rr) * P.ldc];
-        }
-      };
-      if (!GROUPED && BATCH == SROWS) load_old(pass * SROWS);
-      if (SROWS == 32 || (lane >> 3) == pass) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) stage[(lane & (SROWS - 1)) * 33 + j] = acc[c32 * 32 + j];
-      }
-      __syncwarp();
-#pragma unroll kUnroll
-      for (int g = 0; g < SROWS; g += BATCH) {
-        const int lr = pass * SROWS + g, rows = P.M - (row0 + lr);
-        if (rows <= 0) break;
-        if (GROUPED || BATCH != SROWS) load_old(lr);
-        float* cp = P.C + static_cast<size_t>(row0 + lr) * P.ldc + cc;
-#pragma unroll
-        for (int rr = 0; rr < BATCH; ++rr) {
-          float x = scaled_sum(P, stage[(g + rr) * 33 + lane], old[rr]);
-          if constexpr (EPI) {
-            const float b = __shfl_sync(0xffffffffu, bl, lr + rr);
-            if (has_epi) x = epilogue_value(x, b, P.epi);
+          for (int i = 0; i < GB / RPI; ++i, op += step) {
+            const T o = *reinterpret_cast<const T*>(op);
+            if constexpr (W == 4) {
+              old[i][0] = o.x; old[i][1] = o.y; old[i][2] = o.z; old[i][3] = o.w;
+            } else {
+              old[i][0] = o;
+            }
           }
-          if (live && rr < rows) cp[static_cast<size_t>(rr) * P.ldc] = x;
+        }
+#pragma unroll
+        for (int h = 0; h < GB; h += SUB) {
+          if (((g + h) & (SROWS - 1)) == 0) put(g + h);
+#pragma unroll
+          for (int i = 0; i < SUB / RPI; ++i, cp += step) {
+            const int row = g + h + i * RPI + lr, r = row & (SROWS - 1), o = h / RPI + i;
+            const T x = *reinterpret_cast<const T*>(stage + r * 32 + (lc ^ ((r & 7) * 4)));
+            if constexpr (W == 4) {
+              *reinterpret_cast<float4*>(cp) =
+                  make_float4(value(x.x, old[o][0], row), value(x.y, old[o][1], row),
+                              value(x.z, old[o][2], row), value(x.w, old[o][3], row));
+            } else {
+              *cp = value(x, old[o][0], row);
+            }
+          }
         }
       }
-      __syncwarp();
+    };
+    if (row0 + 32 <= P.M && c0 + 32 <= P.N) {
+      if (vec) inside(std::integral_constant<int, 4>{});
+      else inside(std::integral_constant<int, 1>{});
+      continue;
+    }
+    // the matrix's edge: 8 rows at a time, every element tested
+    const bool live = c0 + lane < P.N;
+#pragma unroll 1
+    for (int row = 0; row < 32; row += 8) {
+      const int rows = P.M - (row0 + row);
+      if (rows <= 0) break;
+      if ((row & (SROWS - 1)) == 0) put(row);
+      float* cp = P.C + static_cast<size_t>(row0 + row) * P.ldc + c0 + lane;
+      float old[8];
+#pragma unroll
+      for (int rr = 0; rr < 8; ++rr) old[rr] = 0.f;
+      if (P.beta != 0.f) {
+#pragma unroll
+        for (int rr = 0; rr < 8; ++rr)
+          if (live && rr < rows) old[rr] = cp[static_cast<size_t>(rr) * P.ldc];
+      }
+#pragma unroll
+      for (int rr = 0; rr < 8; ++rr) {
+        const int r = (row + rr) & (SROWS - 1);
+        const float x = value(stage[r * 32 + (lane ^ (rr * 4))], old[rr], row + rr);
+        if (live && rr < rows) cp[static_cast<size_t>(rr) * P.ldc] = x;
+      }
     }
   }
 }

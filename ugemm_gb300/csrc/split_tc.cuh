@@ -116,11 +116,11 @@ struct TcShape {
   static constexpr int FIT = (224 * 1024) / STAGE_BYTES;
   static constexpr int STAGES = BN == 64 ? 5 : (FIT > 4 ? 4 : FIT);
   // Each epilogue warp's 32 x 32 output blocks pass through shared memory so
-  // that C is written by rows: whole blocks (padded rows) where the stage
+  // that C is written by rows: whole blocks (swizzled rows) where the stage
   // ring leaves room -- 128-wide tiles, and 256-wide ones of two pieces --,
   // 8 rows at a time for 256-wide tiles of three pieces.
   static constexpr bool STAGE_C = (BN <= 128 || NP == 2);
-  static constexpr size_t STAGE_C_BYTES = size_t(kTcEpiWarps) * (STAGE_C ? 32 : 8) * 33 * 4;
+  static constexpr size_t STAGE_C_BYTES = size_t(kTcEpiWarps) * (STAGE_C ? 32 : 8) * 32 * 4;
   static constexpr size_t SMEM =
       1024 + size_t(STAGES) * STAGE_BYTES + 256 + STAGE_C_BYTES;
   // fused launches: kTcFusedPieceStages piece stages, then kTcRawStages raw
