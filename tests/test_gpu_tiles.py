@@ -76,3 +76,27 @@ def test_split_routes(ta, tb, M, N, K, off):
                precision="bf16x6")
     torch.cuda.synchronize()
     assert float(torch.linalg.norm(C.double() - ref) / torch.linalg.norm(ref)) < 2e-6
+
+
+# values in [1, 2) have scale exponent 14: 63 and 64 are reached at 2^-49 and
+# 2^-50, -63 and -64 at 2^77 and 2^78
+@pytest.mark.parametrize("a_exp,b_exp", [(77, 0), (78, 0), (0, 77), (0, 78), (77, -49), (78, -50),
+                                         (-49, 0), (-50, 0), (0, -49), (0, -50), (-49, -49)])
+def test_fp16x3_scale_limits(a_exp, b_exp):
+    """A row of A (a column of B) times 2^e has its scale exponent moved by e and the
+    same pieces, so C's row (column) is the plain result times 2^e to the bit, on
+    both sides of the exponents (+-63) up to which one product undoes both scales."""
+    M, N, K = 200, 330, 96
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A = torch.rand((M, K), device="cuda", generator=g) + 0.5
+    B = torch.rand((K, N), device="cuda", generator=g) + 0.5
+    A[:, 0], B[0] = 1.75, 1.75
+    plain = ug.gemm(A, B, torch.empty((M, N), device="cuda"), precision="fp16x3").clone()
+    A2, B2 = A.clone(), B.clone()
+    A2[5] *= 2.0 ** a_exp
+    B2[:, 7] *= 2.0 ** b_exp
+    out = ug.gemm(A2, B2, torch.empty((M, N), device="cuda"), precision="fp16x3")
+    want = plain.clone()
+    want[5] *= 2.0 ** a_exp
+    want[:, 7] *= 2.0 ** b_exp
+    assert torch.equal(out, want)

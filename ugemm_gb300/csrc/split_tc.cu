@@ -164,9 +164,26 @@ __device__ __forceinline__ void epi_store(const TcProblem& P, const TileCoord& t
         const int col = tc.n0 + col_off + c32 * 32 + lane;
         eb[c32] = col < P.N ? f16_scale_exp(P.fmax_b[col]) : 0;
       }
+      // exponents within +-63 (values of 2^-49 to 2^77) add up to a normal power
+      // of two, the product of theirs: a shuffle and two multiplications an
+      // element, the same bits as scale_pow2's one multiplication (8192^3: 2304 ->
+      // 2272 us)
+      bool near = ea >= -63 && ea <= 63;
 #pragma unroll
-      for (int j = 0; j < HALF; ++j)
-        acc[j] = scale_pow2(acc[j], -(ea + __shfl_sync(0xffffffffu, eb[j / 32], j % 32)));
+      for (int c = 0; c < HALF / 32; ++c) near = near && eb[c] >= -63 && eb[c] <= 63;
+      if (__all_sync(0xffffffffu, near)) {
+        const float fa = pow2f(-ea);
+#pragma unroll
+        for (int c = 0; c < HALF / 32; ++c) {
+          const float fb = pow2f(-eb[c]);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) acc[c * 32 + j] *= fa * __shfl_sync(0xffffffffu, fb, j);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < HALF; ++j)
+          acc[j] = scale_pow2(acc[j], -(ea + __shfl_sync(0xffffffffu, eb[j / 32], j % 32)));
+      }
     }
   }
   // alpha/beta epilogue (C not read when beta == 0).  The bias /
