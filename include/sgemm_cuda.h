@@ -123,12 +123,12 @@ UGEMM_API int ugemm_sgemm_dev(char major, char transa, char transb, int M, int N
  * loop where an allocation could stall or fail -- and it calls no
  * cudaMalloc, cudaFree or allocating routine.  The split pieces of A and B
  * live in a fixed 64 MiB array in the library's device memory, held by every
- * GPU that loads the library until the process exits; calls whose scratch
- * exceeds it return UGEMM_ERR_ARENA_TOO_SMALL.  The scratch of a call is
- * exactly ugemm_workspace_bytes with the same arguments: about
- * 6 * (M + N) * roundup(K, 32) bytes of pieces for the three-piece forms,
- * plus, when the last wave of output tiles runs as the wave-tail launch, its
- * partial tiles.  The first call on a device looks up the array's device
+ * GPU that loads the library until the process exits; calls whose operands'
+ * pieces exceed it -- about 6 * (M + N) * roundup(K, 32) bytes for the
+ * three-piece forms, plus, when the last wave of whole output tiles is short,
+ * its FP32 partial tiles -- return UGEMM_ERR_ARENA_TOO_SMALL.  The route is
+ * ugemm_sgemm_dev's where that one's scratch fits the array too, else
+ * whole tiles.  The first call on a device looks up the array's device
  * address (with that device current); make that first call before any stream
  * capture.  All calls share the array: calls that overlap on the GPU (other
  * streams or host threads) race on it.  A kernel wait that gives up is
@@ -172,20 +172,20 @@ UGEMM_API int ugemm_sgemm_backward(char transa, char transb, int M, int N, int K
  * counterpart: the reference reports no device errors).  The calls above are
  * stream-ordered and return before their kernels run, so a bounded wait that
  * gives up (UGEMM_ERR_TIMEOUT on the host-pointer calls) cannot be returned
- * by them; it is recorded in a per-device error word instead.  This call
- * synchronises `stream`, reads the word of ugemm_sgemm_dev, _dev_ex,
+ * by them; it is recorded in an error word of the device instead.  This call
+ * synchronises `stream`, reads the words of ugemm_sgemm_dev, _dev_ex,
  * ugemm_sgemm_backward and ugemm_sgemm_dev_noalloc on the current device,
- * clears it and returns UGEMM_ERR_TIMEOUT (with the code in the last-error
+ * clears them and returns UGEMM_ERR_TIMEOUT (with the code in the last-error
  * message) if any of their kernels gave up since the last check, else
- * UGEMM_OK.  A stale code never disturbs a later call: each call moves it
- * aside before its own kernels run.  The word is per device, shared by all
- * streams.  (Grouped plans have their own word: ugemm_grouped_check.) */
+ * UGEMM_OK.  A stale code never disturbs a later call: calls take their words
+ * in turn, and a word's code is moved aside before it is used again.  The
+ * words are per device, shared by all streams.  (Grouped plans have their own word: ugemm_grouped_check.) */
 UGEMM_API int ugemm_check(void *stream);
 
 /* Test hook for the error reporting above (no reference counterpart): writes
  * `code` into an error word of the current device with a synchronous host
- * copy, as a timed-out kernel wait would -- which 0: the device-pointer
- * calls' word, 1: the allocation-free entry point's (after its first call
+ * copy, as a timed-out kernel wait would -- which 0: the word of the last
+ * device-pointer call, 1: the allocation-free entry point's (after its first call
  * on the device).  Launches nothing; for tests of ugemm_check only. */
 UGEMM_API int ugemm_debug_set_error_word(int which, int code);
 
@@ -295,8 +295,9 @@ UGEMM_API int ugemm_col2im(const float *col, int channels, int batch, int height
  *   backward dW_l = dY_l * col_l^T, dcol_l = W_l^T * dY_l (one grouped launch),
  *            dX_l = col2im(dcol_l) = dY_{l-1}
  * with X_{l+1} = Y_l.  By default the GEMMs read col_l = im2col(X_l)
- * implicitly: the operand pass of the forward and dW GEMMs gathers it from
- * X_l, and no col buffer exists; in the split forms a stride-1 layer's dX is
+ * implicitly and no col buffer exists: in BF16X6 and BF16X9 from pieces of X_l
+ * with channels innermost, split once a run, otherwise gathered from X_l by the
+ * operand pass.  In the split forms a stride-1 layer's dX is
  * then one GEMM, dX_l = Wt_l * im2col(dY_l, pad k-1-p) with Wt_l the weights
  * transposed in the channels and flipped in the taps, and has no dcol
  * buffer.  UGEMM_CONV_IM2COL materialises col_l with an im2col pass first
@@ -364,8 +365,8 @@ UGEMM_API int ugemm_sgemv(char trans, int M, int N, float alpha, const float *A,
  * kernel launch is bracketed by CUDA events on its own stream.  collect()
  * synchronises, returns the summed milliseconds and launch counts per kind
  * (0 SIMT GEMM, 1 split pre-pass, 2 split tcgen05 GEMM, 3 auxiliary, 4 grouped
- * GEMM, 5 control: the one-thread error-word fold that starts each
- * device-pointer call, 6 copy: the copy kernels that read pageable host
+ * GEMM, 5 control: the folds of the device-pointer calls' error words,
+ * 6 copy: the copy kernels that read pageable host
  * buffers) and clears the record. */
 UGEMM_API int ugemm_profile_enable(int on);
 UGEMM_API int ugemm_profile_collect(double *ms_per_kind, int *launches_per_kind, int nkinds);

@@ -100,3 +100,24 @@ def test_fp16x3_scale_limits(a_exp, b_exp):
     want[5] *= 2.0 ** a_exp
     want[:, 7] *= 2.0 ** b_exp
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 4096), (320, 1000, 2048)])
+def test_arena_for_whole_tiles_alone(M, N, K):
+    """k slices need partial tiles beside the pieces; an arena that only holds the
+    pieces is still enough, for whole tiles."""
+    import numpy as np
+    pieces = 6 * (M + N) * K
+    assert ug.workspace_bytes("N", "N", M, N, K, K, N, "bf16x6") > pieces + 4096
+    rng = np.random.default_rng(1)
+    A, B = rng.random((M, K), np.float32) - 0.5, rng.random((K, N), np.float32) - 0.5
+    C = np.zeros((M, N), np.float32)
+    ug.sgemm_cuda_init(size=4 * (M * K + K * N + M * N) + pieces + 4096)
+    try:
+        ug.set_precision("bf16x6")
+        ug.sgemm_cuda("N", "N", M, N, K, 1.0, A, B, 0.0, C)
+    finally:
+        ug.set_precision("auto")
+        ug.sgemm_cuda_finish()
+    ref = A.astype(np.float64) @ B.astype(np.float64)
+    assert np.linalg.norm(C - ref) / np.linalg.norm(ref) < 2e-6

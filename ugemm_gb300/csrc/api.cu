@@ -231,7 +231,15 @@ size_t scratch_for(const Gemm& g, int form) {
   return split_scratch_bytes(g, p);
 }
 
-// Launch one GEMM on `st` using `ws` as scratch.
+// The least scratch it can run in: whole tiles need no partial ones.
+size_t scratch_least(const Gemm& g, int form) {
+  const size_t want = scratch_for(g, form);
+  if (want == 0 || !is_split_form(form)) return want;
+  return std::min(want, split_scratch_bytes(g, split_plan_for(form, g)));
+}
+
+// Launch one GEMM on `st` using `ws` as scratch: on narrower tiles or slices
+// where that is faster and their scratch fits.
 ugemm_status launch(const Gemm& g, int form, Scratch ws, int* dev_err, cudaStream_t st) {
   if (g.M == 0 || g.N == 0) return UGEMM_OK;
   if (g.K == 0 || g.alpha == 0.f) return scale_c_launch(g, st);
@@ -240,8 +248,8 @@ ugemm_status launch(const Gemm& g, int form, Scratch ws, int* dev_err, cudaStrea
     s = simt_launch(g, simt_pick_tile(g), ws, dev_err, st);
   } else if (is_split_form(form)) {
     const SplitPlan p = split_plan_for(form, g);
-    s = multi_wanted(g, p) ? multi_launch(&g, 1, p, ws, dev_err, st)
-                           : split_launch(g, p, ws, dev_err, st);
+    const bool multi = multi_wanted(g, p) && multi_scratch_bytes(&g, 1, p) <= ws.bytes;
+    s = multi ? multi_launch(&g, 1, p, ws, dev_err, st) : split_launch(g, p, ws, dev_err, st);
   } else {
     return fail(UGEMM_ERR_ARG, "unknown precision%s");
   }
@@ -276,7 +284,10 @@ ugemm_status dev_gemm(const Gemm& g, int precision, cudaStream_t st) {
   ugemm_status s = device_state(&d);
   if (s != UGEMM_OK) return s;
   const int form = resolve_form(precision, g);
-  s = ensure_workspace(*d, scratch_for(g, form), st);
+  const size_t want = scratch_for(g, form);
+  // a graph is captured in the workspace there is, if the call fits it at all
+  if (want <= d->ws_bytes || !is_capturing(st) || scratch_least(g, form) > d->ws_bytes)
+    s = ensure_workspace(*d, want, st);
   if (s != UGEMM_OK) return s;
   int* word = nullptr;
   s = begin_call(*d, st, &word);
@@ -309,7 +320,7 @@ ugemm_status host_gemm_tight(const Gemm& g, int form, void* arena, size_t arena_
   dg.lda = lda4;
   dg.ldb = ldb4;
   dg.ldc = g.N;
-  const size_t scratch = scratch_for(dg, form);
+  const size_t scratch = scratch_least(dg, form);
   const size_t s_off = scratch ? align_up(a_bytes + b_bytes + c_bytes, 256) : a_bytes + b_bytes + c_bytes;
   if (s_off + scratch > arena_bytes)
     return fail(UGEMM_ERR_ARENA_TOO_SMALL, "device arena too small for this call%s");

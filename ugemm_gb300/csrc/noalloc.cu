@@ -151,7 +151,8 @@ extern "C" UGEMM_API int ugemm_sgemm_dev_noalloc(char major, char transa, char t
   const SplitPlan plan = split_plan_for(form, g);
   const bool multi =
       multi_wanted(g, plan) && multi_scratch_bytes(&g, 1, plan) <= kNoAllocScratchBytes;
-  const size_t need = multi ? 0 : split_scratch_bytes(g, plan);
+  // what is refused follows from whole tiles on pieces, whatever the route
+  const size_t need = split_scratch_bytes(g, plan);
   if (need > kNoAllocScratchBytes) {
     char msg[160];
     std::snprintf(msg, sizeof msg,
