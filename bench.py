@@ -223,7 +223,7 @@ def conv_forms(ug, torch, stream, steps):
     from ugemm_gb300 import workloads
     batch = 32
     layers = workloads.conv_layers(batch)
-    out = {"layers": len(layers), "batch": batch, "im2col": "implicit (gathered in the operand pass)"}
+    out = {"layers": len(layers), "batch": batch, "im2col": "implicit (TMA im2col mode; gathered in the operand pass by fp16x3 and simt)"}
     for name, prec, explicit in (("bf16x6", "bf16x6", False), ("fp16x3", "fp16x3", False),
                                  ("simt", "simt", False), ("bf16x6_explicit_im2col", "bf16x6", True)):
         st = ug.ConvStack(layers, batch, precision=prec, graph=True, im2col=explicit)

@@ -31,10 +31,11 @@
 //   2. GEMM kernel, 12 warps (a fused launch: 10 or 16, without idle ones):
 //        warp 0   TMA producer: one 3-D TMA per operand per stage brings all
 //                 pieces of a 32-deep k slice (64-byte swizzle; TF32
-//                 pieces: 128-byte rows and swizzle) into a 3-4 stage ring
+//                 pieces: 128-byte rows and swizzle) into a 3-5 stage ring
 //                 (mbarrier full/empty pairs);
-//        warp 1   allocates TMEM (2 x BN columns: main + corrections) and,
-//                 from one thread, issues the tcgen05.mma stream;
+//        warp 1   allocates TMEM (2 x BN columns: main + corrections; six
+//                 accumulators of a 64-wide tile) and, converged, one lane
+//                 issuing, runs the tcgen05.mma stream;
 //        warps 4-11 epilogue: chunk drains, then alpha/beta and the store of
 //                 the 128 x BN tile (one TMEM lane per row; two warps per
 //                 lane quarter, each owning half of the columns).
@@ -2373,7 +2374,7 @@ void split_operand_strides(const Gemm& g, long long* a_sr, long long* a_sk, long
 ugemm_status split_launch(const Gemm& g, const SplitPlan& p, Scratch ws, int* dev_err,
                           cudaStream_t st) {
   if (split_scratch_bytes(g, p) > ws.bytes) return UGEMM_ERR_ARENA_TOO_SMALL;
-  // scratch: [A pieces | B pieces | wave-tail partial tiles and table]
+  // scratch: [A pieces | B pieces | wave-tail partial tiles]
   uint8_t* ap = static_cast<uint8_t*>(ws.ptr);
   uint8_t* bp = ap + split_operand_bytes(p.pieces, g.M, g.K);
   uint8_t* tail_scratch = bp + split_operand_bytes(p.pieces, g.N, g.K);
