@@ -376,16 +376,21 @@ void backward_geometry(const Stack* s, const Stack::Layer& L, ugemm::Gemm* b) {
   double best = 1e300;
   for (int bn : {64, 128, 256}) {
     const GeoChoice w = choose_geometry(3, d.cout, kk * static_cast<int>(align_up(d.cin, 64)),
-                                        cdiv(npix, 32), sms / 2.0, bn, true, 256);
+                                        cdiv(npix, 32), sms / 2.0, bn, true, 256, kPlanSum);
     const GeoChoice x =
-        direct ? choose_geometry(3, d.cin, in_px, kk * cdiv(d.cout, 32), sms / 2.0, bn, true, 256)
-               : choose_geometry(3, L.kdim, npix, cdiv(d.cout, 32), sms / 2.0, bn, true, 256);
+        direct ? choose_geometry(3, d.cin, in_px, kk * cdiv(d.cout, 32), sms / 2.0, bn, true, 256,
+                                 kPlanSum)
+               : choose_geometry(3, L.kdim, npix, cdiv(d.cout, 32), sms / 2.0, bn, true, 256,
+                                 kPlanSum);
     const double us = std::max(w.us, x.us);
     if (us >= best) continue;
     best = us;
     b[0].block_n = bn;
+    const bool dcol = direct && !L.direct_dx;  // an explicit stack's
     b[0].slices = w.slices;
-    b[1].slices = direct && !L.direct_dx ? 1 : x.slices;  // (an explicit stack's dcol)
+    b[0].sum = w.sum;
+    b[1].slices = dcol ? 1 : x.slices;
+    b[1].sum = dcol ? 0 : x.sum;
   }
 }
 

@@ -342,6 +342,37 @@ double padded_area(int rows, int cols, int bn) {
   return double(align_up(rows, 128)) * ((cols / bn) * bn + align_up(cols % bn, 16));
 }
 
+// Tile width of an untuned launch on pieces: 256, or 128 when no problem is wider
+// than 128 columns in the orientation the kernel computes it (a transposed
+// problem's width is its M).
+int whole_tile_width(const Gemm* gs, int n) {
+  int widest = 0;
+  for (int i = 0; i < n; ++i) {
+    const Gemm& x = gs[i];
+    widest = std::max(widest, padded_area(x.N, x.M, 128) < padded_area(x.M, x.N, 128) ? x.M : x.N);
+  }
+  return widest <= 128 ? 128 : 256;
+}
+
+// Half an SM's share of such a launch's stages.
+double whole_fair(const Gemm* gs, int n) {
+  const int bn = whole_tile_width(gs, n);
+  double work = 0;
+  for (int i = 0; i < n; ++i) {
+    const Gemm& x = gs[i];
+    const bool sw = padded_area(x.N, x.M, bn) < padded_area(x.M, x.N, bn);
+    work += double(cdiv(sw ? x.N : x.M, kTcBM)) * cdiv(sw ? x.M : x.N, bn) * split_nkb(3, x.K);
+  }
+  return work / (2.0 * device_sms());
+}
+
+constexpr int kMaxSlices = 256;
+// k slices whose partial tiles take 1 GiB.
+int most_slices(size_t tile_bytes) {
+  return static_cast<int>(std::min<size_t>(
+      kMaxSlices, std::max<size_t>(1, (size_t(1) << 30) / std::max<size_t>(1, tile_bytes))));
+}
+
 void free_plan(ugemm_grouped_plan_s* p) {
   if (!p) return;
   if (p->exec) cudaGraphExecDestroy(p->exec);
@@ -426,18 +457,7 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     p->cfg = *config;
   } else {
     p->cfg = default_grouped_config(form);
-    // Untuned split plans: 128-wide tiles only when no problem is wider than
-    // 128 columns in the orientation the kernel computes it (a transposed
-    // problem's width is its M); measured on the 256-problem set, 256-wide
-    // tiles with the staged epilogue and narrow-N MMAs win (144 vs 162 us).
-    if (form != UGEMM_PREC_SIMT) {
-      int widest = 0;
-      for (const Gemm& x : g) {
-        const int n = kernel_cols(x);
-        widest = std::max(widest, padded_area(n, x.M, 128) < padded_area(x.M, n, 128) ? x.M : n);
-      }
-      if (widest <= 128) p->cfg.block_n = 128;
-    }
+    if (form != UGEMM_PREC_SIMT) p->cfg.block_n = whole_tile_width(g.data(), count);
   }
   // Untuned groups of three pieces whose operands TMA can copy: the launch that
   // splits them itself, or a pre-pass and 256-wide tiles, by the time of their
@@ -478,15 +498,21 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   const int sms = device_sms();
   // Untuned plans of three pieces: one problem takes the tile width, the
   // orientation and the k slices that its measured stage and tile times make
-  // fastest; 64-wide tiles exist for these only.
+  // fastest; 64-wide tiles exist for these only.  Their k slices are fewer and
+  // longer than a fair share's, which adds roundings, so their chunks are kPlanChunk
+  // deep where other plans' are twice that (12-layer training step: 1599 ->
+  // 1620 us, and 0.56 of the error).
   GeoChoice one;
   if (!config && form != UGEMM_PREC_SIMT && split_plan_for(form, g[0]).pieces == 3) {
     if (g[0].block_n) {
       p->cfg.block_n = g[0].block_n;
     } else if (count == 1 && g[0].K > 0) {
-      one = choose_geometry(3, g[0].M, kernel_cols(g[0]), kernel_nkb(3, g[0]), sms, 0, true, 256);
+      one = choose_geometry(3, g[0].M, kernel_cols(g[0]), kernel_nkb(3, g[0]), sms, 0, true, 256,
+                            kPlanSum);
       p->cfg.block_n = one.block_n;
     }
+    if (g[0].block_n || one.us > 0)
+      p->cfg.chunk_k = std::min(split_default_chunk_kb(1 << 30), kPlanChunk) * kTcKB;
   }
   for (const Gemm& x : g) p->flops += 2.0 * x.M * x.N * x.K;
 
@@ -539,13 +565,14 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   // gradient: small output, k = batch x pixels) would leave most SMs idle,
   // so it is cut into slices of about that length, at least min_slice
   // k-blocks, and at most 1 GiB of partial tiles.
-  // (stages: 16 k-blocks of 32 in the SIMT form and the three-piece split
-  // form, 8 of 64 for two-piece operands)
-  const int min_slice = 16 * kTcKB / (simt ? kTcKB : split_stage_k(pieces));
   // (the threshold divisor is the configuration's split_k: 0 means 2,
   // negative disables split-K)
+  // An untuned fused launch takes the slices of a launch on pieces: no longer,
+  // and so no further from FP64.
   const double fair = p->cfg.split_k < 0 ? 1e300
-                                          : work / ((p->cfg.split_k > 0 ? p->cfg.split_k : 2) * sms);
+                      : !config && !simt && p->split.fused
+                          ? whole_fair(g.data(), count)
+                          : work / ((p->cfg.split_k > 0 ? p->cfg.split_k : 2) * sms);
   std::vector<size_t> part_off(count, 0);
   size_t part_bytes = 0;
   for (int j = 0; j < count; ++j) {
@@ -555,20 +582,15 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     // columns in C's order
     o.sliced = x.pieces && x.pieces->kind == PieceOperands::kPix;
     const size_t tile_bytes = size_t(x.M) * kernel_cols(x) * 4;
-    int sl = 1;
-    if (one.us > 0 || x.slices > 0) {
-      sl = one.us > 0 ? one.slices : std::min(x.slices, o.nkb);
-      sl = static_cast<int>(std::min<size_t>(sl, std::max<size_t>(1, (size_t(1) << 30) / tile_bytes)));
-    } else if (x.K != 0 && o.nkb >= 2 * min_slice && o.nkb > fair) {
-      const int len = std::max(min_slice, static_cast<int>(fair) + 1);
-      sl = std::min(cdiv(o.nkb, len), 256);
-      sl = static_cast<int>(std::min<size_t>(sl, (size_t(1) << 30) / tile_bytes));
-    }
-    if (sl >= 2) o.sliced = true;
-    else sl = 1;
-    if (!o.sliced) continue;
-    o.per = cdiv(o.nkb, sl);
+    o.per = o.nkb;
+    if (one.us > 0 || x.slices > 0)
+      o.per = cdiv(o.nkb, std::min({one.us > 0 ? one.slices : x.slices, o.nkb,
+                                    most_slices(tile_bytes)}));
+    else if (x.K != 0)
+      o.per = slice_blocks(o.nkb, fair, most_slices(tile_bytes));
     o.slices = cdiv(o.nkb, o.per);
+    o.sliced |= o.slices > 1;
+    if (!o.sliced) continue;
     part_off[j] = part_bytes;
     part_bytes += align_up(size_t(o.slices) * tile_bytes, 256);
   }
@@ -719,6 +741,7 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       tp.tile_start = tiles;
       tp.kb0 = u.kb0;
       tp.swap = o.swap ? 1 : 0;
+      tp.sum_kb = one.us > 0 ? one.sum : x.sum;
       tp.map = static_cast<int>(i);
       tp.epi = epi;
       tiles += tp.tiles_m * tp.tiles_n;

@@ -110,6 +110,7 @@ struct Gemm {
   // grouped plans only: tile width of the plan (its first problem's) and k
   // slices of this problem, chosen by the caller; 0: by the plan
   int block_n = 0, slices = 0;
+  int sum = 0;  // with block_n 64: TcProblem::sum_kb
 };
 
 #ifdef __CUDACC__
@@ -302,7 +303,8 @@ ugemm_status splitk_reduce_param_launch(const ReduceJob* jobs, int njobs, long l
 
 // Up to kMultiMax split-precision GEMMs (and split-K slices of them) in one
 // persistent launch, scratch in the caller's workspace (multi.cu).
-bool multi_wanted(const Gemm& g, const SplitPlan& p);  // under-filled, deep k
+bool multi_wanted(const Gemm& g, const SplitPlan& p);  // rather than whole tiles
+bool multi_faster(const Gemm& g, const SplitPlan& p);
 size_t multi_scratch_bytes(const Gemm* gs, int n, const SplitPlan& p);
 ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& p, Scratch ws, int* dev_err,
                           cudaStream_t st);

@@ -27,8 +27,6 @@ namespace {
 
 static_assert(sizeof(MultiTable) <= 16384, "a kernel parameter, copied at every launch");
 
-constexpr int kMinSlice = 16;  // shortest slice of several GEMMs', in k-blocks
-
 MultiTable empty_table() {
   MultiTable t;
   std::memset(&t, 0, sizeof t);
@@ -47,25 +45,64 @@ struct Layout {
   int block_n = 256;
   size_t a_off[kMultiMax], b_off[kMultiMax], part_off[kMultiMax];
   size_t total = 0;
+  int longest = 0;     // one GEMM: choose_geometry's `longest`
   double us = 0;       // one GEMM: the model's time of all its launches
   bool fused = false;  // one GEMM: the operands split inside the GEMM kernel
 };
 
+// Slices whose partial tiles take 512 MiB.
+int most_slices(const Gemm& g) {
+  return std::max(1, static_cast<int>(std::min(1e9, double(512 << 20) / (double(g.M) * g.N * 4))));
+}
+
+// The tiles that several GEMMs share an SM's time by: 256-wide unless every
+// output is narrow in its better orientation.
+struct Shared {
+  int block_n = 256;
+  bool swap[kMultiMax];
+  int nkb[kMultiMax];
+  double fair = 0;  // half an SM's share of the stages
+};
+Shared shared_tiles(const Gemm* gs, int n, int pieces, int sms) {
+  Shared h;
+  int widest = 0;
+  for (int i = 0; i < n; ++i) {
+    const Gemm& g = gs[i];
+    widest = std::max(widest, padded(g.N, g.M, 256) < padded(g.M, g.N, 256) ? g.M : g.N);
+  }
+  h.block_n = widest > 128 ? 256 : 128;
+  for (int i = 0; i < n; ++i) {
+    const Gemm& g = gs[i];
+    const bool sw = h.swap[i] = padded(g.N, g.M, h.block_n) < padded(g.M, g.N, h.block_n);
+    h.nkb[i] = split_nkb(pieces, g.K);
+    h.fair += double(cdiv(sw ? g.N : g.M, kTcBM)) * cdiv(sw ? g.M : g.N, h.block_n) * h.nkb[i];
+  }
+  h.fair /= 2.0 * sms;
+  return h;
+}
+
+// The longest chain of FP32 sums of one GEMM (choose_geometry): its slice, were
+// it cut so that its tiles are half an SM's share each.
+int longest_sum(const Gemm& g, int pieces, int sms) {
+  const Shared h = shared_tiles(&g, 1, pieces, sms);
+  return slice_blocks(h.nkb[0], h.fair, std::min(kMultiSubs, most_slices(g)));
+}
+
 // One GEMM: the tile width and slices of the least time by the stage times.
-// Several: 256-wide tiles unless every output is narrow, and slices no longer
-// than half an SM's fair share, which round robin then balances (2048 x 8192 x
-// 1024 backward: 342 us, 435 with whole tiles on each GEMM's share of the SMs).
+// Several: slices no longer than half an SM's fair share, which round robin
+// then balances (2048 x 8192 x 1024 backward: 342 us, 435 with whole tiles on
+// each GEMM's share of the SMs).
 Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
   Layout L;
-  auto most = [&](const Gemm& g) {  // slices whose partial tiles take 512 MiB
-    return std::max(1, static_cast<int>(std::min(1e9, double(512 << 20) / (double(g.M) * g.N * 4))));
-  };
   if (n == 1) {
+    const int slices = std::min(kMultiSubs, most_slices(gs[0]));
+    const int nkb = split_nkb(p.pieces, gs[0].K);
+    const int longest = L.longest = longest_sum(gs[0], p.pieces, sms);
     L.us = 1e300;
     for (int bn : {64, 128, 256}) {
       if (bn == 64 && p.pieces != 3) continue;
-      const GeoChoice c = choose_geometry(p.pieces, gs[0].M, gs[0].N, split_nkb(p.pieces, gs[0].K),
-                                          sms, bn, true, std::min(kMultiSubs, most(gs[0])));
+      const GeoChoice c = choose_geometry(p.pieces, gs[0].M, gs[0].N, nkb, sms, bn, true, slices,
+                                          longest);
       if (c.us >= L.us) continue;
       L.us = c.us;
       L.block_n = bn;
@@ -76,9 +113,8 @@ Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
     L.us += split_pass_us((double(gs[0].M) + gs[0].N) * gs[0].K);
     if (p.pieces == 3 && p.products == 6 && fusable(gs[0])) {
       GeoChoice c;
-      c.us = fused_us(gs[0], sms, &c.swap, &c.slices, std::min(kMultiSubs, most(gs[0])));
+      c.us = fused_us(gs[0], sms, &c.swap, &c.slices, slices, longest);
       if (c.us < L.us) {
-        const int nkb = split_nkb(3, gs[0].K);
         c.per = cdiv(nkb, c.slices);
         L.us = c.us;
         L.block_n = 128;
@@ -87,33 +123,14 @@ Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
       }
     }
   } else {
-    int widest = 0;
-    for (int i = 0; i < n; ++i) {
-      const Gemm& g = gs[i];
-      widest = std::max(widest, padded(g.N, g.M, 256) < padded(g.M, g.N, 256) ? g.M : g.N);
-    }
-    L.block_n = widest > 128 ? 256 : 128;
-    double work = 0;
-    int tiles[kMultiMax], nkb[kMultiMax];
-    for (int i = 0; i < n; ++i) {
-      const Gemm& g = gs[i];
-      GeoChoice& o = L.geo[i];
-      o.swap = padded(g.N, g.M, L.block_n) < padded(g.M, g.N, L.block_n);
-      tiles[i] = cdiv(o.swap ? g.N : g.M, kTcBM) * cdiv(o.swap ? g.M : g.N, L.block_n);
-      nkb[i] = split_nkb(p.pieces, g.K);
-      o.per = nkb[i];
-      work += double(tiles[i]) * nkb[i];
-    }
-    const double fair = work / (2.0 * sms);
+    const Shared h = shared_tiles(gs, n, p.pieces, sms);
+    L.block_n = h.block_n;
     int subs = n;
     for (int i = 0; i < n; ++i) {
       GeoChoice& o = L.geo[i];
-      if (nkb[i] < 2 * kMinSlice || nkb[i] <= fair) continue;
-      const int len = std::max(kMinSlice, static_cast<int>(fair) + 1);
-      const int sl = std::min({cdiv(nkb[i], len), kMultiSubs - (subs - 1), most(gs[i])});
-      if (sl < 2) continue;
-      o.per = cdiv(nkb[i], sl);
-      o.slices = cdiv(nkb[i], o.per);
+      o.swap = h.swap[i];
+      o.per = slice_blocks(h.nkb[i], h.fair, std::min(kMultiSubs - (subs - 1), most_slices(gs[i])));
+      o.slices = cdiv(h.nkb[i], o.per);
       subs += o.slices - 1;
     }
   }
@@ -141,7 +158,7 @@ TailPlan tail_plan(const Gemm& g, const SplitPlan& p) {
   const int sms = device_sms();
   const int tiles_m = cdiv(g.M, kTcBM), tiles_n = cdiv(g.N, p.block_n);
   const int tiles = tiles_m * tiles_n, rem = tiles % sms;
-  if (tiles <= sms || rem == 0 || split_nkb(p.pieces, g.K) < 32) return t;
+  if (tiles <= sms || rem == 0 || split_nkb(p.pieces, g.K) < 2 * kMinSlice) return t;
   // the raster order ends with the last group of tile rows, column by column
   const int first_m = ((tiles_m - 1) / kTcRaster) * kTcRaster, rows = tiles_m - first_m;
   const int cols = cdiv(rem, rows);             // whole tile columns of that group
@@ -210,19 +227,30 @@ ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail
                        : splitk_reduce_param_launch(&red, 1, static_cast<long long>(mn), st);
 }
 
-// Whether a GEMM runs here rather than as one launch of whole 256- (or, up to
-// 128 columns, 128-) wide tiles: when narrower tiles or k slices are faster by
-// the stage times, as they are where whole tiles leave SMs idle (1024^3: 32 tiles
-// of 256; 2048^3: one wave of 128 of the 152 SMs).
-bool multi_wanted(const Gemm& g, const SplitPlan& p) {
+// Whether narrower tiles or k slices are faster than one launch of whole 256-
+// (or, up to 128 columns, 128-) wide tiles by the stage times, as they are where
+// whole tiles leave SMs idle (1024^3: 32 tiles of 256).
+bool multi_faster(const Gemm& g, const SplitPlan& p) {
   if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return false;
   const int sms = device_sms();
   const int tiles = cdiv(g.M, kTcBM) * cdiv(g.N, p.block_n);
   if (tiles > 4 * sms) return false;
-  const GeoChoice whole = choose_geometry(p.pieces, g.M, g.N, split_nkb(p.pieces, g.K), sms,
-                                          p.block_n, false, 1);
+  const int nkb = split_nkb(p.pieces, g.K);
+  const GeoChoice whole = choose_geometry(p.pieces, g.M, g.N, nkb, sms, p.block_n, false, 1, nkb);
   return layout_for(&g, 1, p, sms).us <
          0.95 * (whole.us + split_pass_us((double(g.M) + g.N) * g.K));
+}
+
+// Whether a GEMM runs here: where that is faster, and where its tiles are fewer
+// than the SMs and k is deep, so that slices or sums of sums (choose_geometry's
+// `longest`) cost little and are nearer FP64 (2048^3 in BF16x6: one wave of 128
+// whole tiles is 1.29e-7 from it, sums of a third of k each 1.16e-7).
+bool multi_wanted(const Gemm& g, const SplitPlan& p) {
+  if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return false;
+  const int sms = device_sms();
+  return (cdiv(g.M, kTcBM) * cdiv(g.N, p.block_n) < sms &&
+          longest_sum(g, p.pieces, sms) < split_nkb(p.pieces, g.K)) ||
+         multi_faster(g, p);
 }
 
 size_t multi_scratch_bytes(const Gemm* gs, int n, const SplitPlan& p) {
@@ -302,6 +330,7 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
       tp.tiles_m = cdiv(tp.M, kTcBM);
       tp.tiles_n = cdiv(tp.N, p.block_n);
       tp.swap = o.swap ? 1 : 0;
+      tp.sum_kb = o.sum;
       tp.map = i;
       tp.kc_a = kc[0];
       tp.kc_b = kc[1];
@@ -337,8 +366,10 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch 
   CUtensorMap dummy;
   std::memset(&dummy, 0, sizeof dummy);
   TcProblem single{};
-  const int chunk =
+  int chunk =
       split_chunk_stages(p.pieces, p.chunk_kb > 0 ? p.chunk_kb : split_default_chunk_kb(min_k));
+  // chunks no deeper than those of the longest sum on average (its last may be short)
+  if (n == 1) chunk = std::max(1, L.longest / cdiv(L.longest, chunk));
   const ugemm_status s =
       split_gemm_launch(p, dummy, dummy, single, nullptr, nullptr, nullptr, tiles, chunk,
                         std::max(1, std::min(tiles, device_sms())), dev_err, st, nullptr, &t);

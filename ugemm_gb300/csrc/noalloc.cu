@@ -146,11 +146,11 @@ extern "C" UGEMM_API int ugemm_sgemm_dev_noalloc(char major, char transa, char t
     s = scale_c_launch(g, st);
     return s == UGEMM_OK ? s : fail(s, "scale launch failed");
   }
-  // the same route as the workspace entry point's, unless only whole tiles,
-  // which need no partial ones, fit the array
+  // the workspace entry point's route where that is faster and its partial
+  // tiles fit the array, else whole tiles
   const SplitPlan plan = split_plan_for(form, g);
   const bool multi =
-      multi_wanted(g, plan) && multi_scratch_bytes(&g, 1, plan) <= kNoAllocScratchBytes;
+      multi_faster(g, plan) && multi_scratch_bytes(&g, 1, plan) <= kNoAllocScratchBytes;
   // what is refused follows from whole tiles on pieces, whatever the route
   const size_t need = split_scratch_bytes(g, plan);
   if (need > kNoAllocScratchBytes) {

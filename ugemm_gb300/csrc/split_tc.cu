@@ -927,6 +927,15 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
       const int nchunks = (P.nkb + chunk_kb - 1) / chunk_kb;
       // columns of this warp's half that hold results (grouped: narrow tiles)
       const int n_live = GROUPED ? P.N - tc.n0 - col_off : HALF;
+      // 64-wide tiles have the registers for sums of sums (P.sum_kb)
+      constexpr bool SUMS = BN == 64;
+      float total[SUMS ? HALF : 1];
+      int per_sum = 0, left = 0;
+      if constexpr (SUMS) {
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) total[j] = 0.f;
+        per_sum = left = P.sum_kb > 0 ? max(1, P.sum_kb / chunk_kb) : nchunks;
+      }
       for (int c = 0; c + 1 < nchunks; ++c) {
         if (!__all_sync(0xffffffffu,
                         mbar_wait(&main_full[buf], nbound[buf] & 1, err, kDevTimeoutAccum))) {
@@ -939,6 +948,16 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&main_empty[buf]);
+        if constexpr (SUMS) {
+          if (--left == 0) {
+            left = per_sum;
+#pragma unroll
+            for (int j = 0; j < HALF; ++j) {
+              total[j] += acc[j];
+              acc[j] = 0.f;
+            }
+          }
+        }
       }
       if (!ok) break;
       if (!__all_sync(0xffffffffu, mbar_wait(&tile_full[buf], use & 1, err, kDevTimeoutAccum)))
@@ -960,6 +979,10 @@ __global__ void __launch_bounds__(FUSED ? fused_threads(BN) : kTcSplitThreads, 1
           acc_add_tmem<HALF, GROUPED>(t_buf + c * BN, corr, n_live);
 #pragma unroll
         for (int j = 0; j < HALF; ++j) acc[j] += corr[j];
+      }
+      if constexpr (SUMS) {
+#pragma unroll
+        for (int j = 0; j < HALF; ++j) acc[j] += total[j];
       }
       tc_fence_before();
       __syncwarp();
@@ -2170,8 +2193,14 @@ double stage_us(int pieces, int bn) {
 }
 double tile_us(int bn) { return bn == 256 ? 3.0 : bn == 128 ? 1.5 : 1.2; }
 
+int slice_blocks(int nkb, double fair, int max_slices) {
+  if (nkb < 2 * kMinSlice || nkb <= fair) return nkb;
+  const int n = std::min(cdiv(nkb, std::max(kMinSlice, static_cast<int>(fair) + 1)), max_slices);
+  return n < 2 ? nkb : cdiv(nkb, n);
+}
+
 GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int block_n,
-                          bool transpose, int max_slices) {
+                          bool transpose, int max_slices, int longest) {
   GeoChoice best;
   best.us = 1e300;
   const double sms = std::max(1.0, share);
@@ -2186,6 +2215,7 @@ GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int b
         if (sl > 1 && per < 4) break;
         if (per == last) continue;
         last = per;
+        if (bn != 64 && per > longest) continue;
         const int n = cdiv(nkb, per);
         double us = std::ceil(tiles * n / sms) * (per * stage_us(pieces, bn) + tile_us(bn));
         // partial tiles written and read back (4 TB/s) and a launch to sum them
@@ -2195,6 +2225,7 @@ GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int b
           best.swap = swap != 0;
           best.slices = n;
           best.per = per;
+          best.sum = per > longest ? longest : 0;
           best.us = us;
         }
       }
@@ -2206,7 +2237,8 @@ GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int b
 double split_pass_us(double elements) { return 3.0 + 2.2e-6 * elements; }
 
 // A fused stage of a 128 x 128 tile takes 1.14 us with all SMs busy.
-double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_slices) {
+double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_slices,
+                int longest) {
   const int nkb = split_nkb(3, g.K);
   double best = 1e300;
   for (int sw = 0; sw < 2; ++sw) {
@@ -2217,6 +2249,7 @@ double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_sl
       if (sl > 1 && per < 4) break;
       if (per == last) continue;
       last = per;
+      if (per > longest) continue;
       const int n = cdiv(nkb, per);
       double us = std::ceil(tiles * n / std::max(1.0, share)) * (per * 1.14 + 3.0);
       if (n > 1) us += 3.0 + (n + 1.0) * g.M * g.N * 4 / 4e6;

@@ -158,6 +158,8 @@ struct TcProblem {
   int tile_start;       // first global tile index of this problem
   int kb0 = 0;
   int swap = 0;
+  int sum_kb = 0;       // 64-wide tiles: stages that one FP32 sum takes before it is
+                        // added to the total; 0: all
   int map = 0;          // tensor maps of this problem: maps[2 * map], maps[2 * map + 1]
   Epilogue epi;
   // FP16x3 form: the largest magnitude of every kernel row (fmax_a[r], a row
@@ -241,16 +243,32 @@ struct GeoChoice {
   int block_n = 256;
   bool swap = false;
   int slices = 1, per = 0;
+  int sum = 0;  // TcProblem::sum_kb
   double us = 0;
 };
+// Stages of one k slice where slices are as long as `fair`, at least kMinSlice
+// stages, and at most max_slices of them: nkb itself where k is not cut.
+constexpr int kMinSlice = 16;
+int slice_blocks(int nkb, double fair, int max_slices);
+// Plans whose geometry choose_geometry picks: depth of a chunk and the longest chain of
+// their sums, in stages.  Chunks of 128 k in chains of 4096 are nearer FP64 than the
+// other plans' chunks of 256 in chains as short as a slice of 512 (chains of 8192 are
+// not: 2048 x 2048 x 8192 in BF16x9 2.21e-7, 2.07e-7).
+constexpr int kPlanChunk = 4, kPlanSum = 128;
 // block_n: 0 to choose among the widths that `pieces` has; transpose: whether
 // C^T may be computed instead.
+// longest: stages that one chain of FP32 sums may take.  A chain rounds at every
+// chunk it adds, so longer ones are further from FP64 (1024^3 in BF16x6: 8.7e-8 as
+// two halves, 9.9e-8 as one chain); 128- and 256-wide tiles have no registers for
+// a second level of sums and take slices no longer than that, 64-wide ones
+// sum within (GeoChoice::sum).
 GeoChoice choose_geometry(int pieces, int M, int N, int nkb, double share, int block_n,
-                          bool transpose, int max_slices);
+                          bool transpose, int max_slices, int longest);
 
 // The same for a fused launch (128-wide tiles; operands copied as FP32), and what
 // splitting `elements` operand elements beforehand takes.
-double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_slices);
+double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_slices,
+                int longest);
 double split_pass_us(double elements);
 // Whether a fused launch can copy the operands.
 bool fusable(const Gemm& g);
