@@ -100,3 +100,12 @@ def test_convolution_layer():
     dx = torch.nn.functional.fold(dcol, (n, n), 3, padding=1, stride=2).permute(1, 0, 2, 3)
     assert rel(st.tensor(0, "dx", (cin, batch, n, n)), dx) < SAMPLE * 3.37e-7
     st.close()
+
+
+@pytest.mark.parametrize("M,N,bound", [(8192, 16, 6.74e-8), (40000, 64, 7.9e-8)])
+def test_gemv_partial_sums(M, N, bound):
+    """Few columns: what adds the warps' sums rounds as much as the sums themselves."""
+    At, x, y = mat(N, M, 3), mat(1, N, 4).reshape(-1), torch.zeros((M,), device="cuda")
+    ug.sgemv("N", M, N, 1.0, At, M, x, 1, 0.0, y, 1)
+    ref = torch.mv(At.double().T, x.double())
+    assert rel(y, ref) < SAMPLE * bound
