@@ -97,3 +97,38 @@ def test_gemv_vector_widths_and_shared_columns(trans, M, N, pad, off):
     torch.cuda.synchronize()
     assert float(torch.linalg.norm(y[::2].double() - ref) / torch.linalg.norm(ref)) < 2e-6
     assert torch.equal(y[1::2], odd)
+
+
+def graph_us(f, n=20):
+    """Microseconds a call of f takes on the device, in a graph of n."""
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    f()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=s):
+        for _ in range(n):
+            f()
+    e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    best = 1e9
+    for _ in range(8):
+        e[0].record()
+        g.replay()
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]))
+    return best * 1000 / n
+
+
+def gemv_us(trans, M, N, pad):
+    lda, cols = (M + pad, N) if trans == "N" else (N + pad, M)
+    A = torch.rand((lda * cols,), device="cuda")
+    x, y = torch.rand((N,), device="cuda"), torch.zeros((M,), device="cuda")
+    return graph_us(lambda: ug.sgemv(trans, M, N, 1.0, A, lda, x, 1, 0.0, y, 1))
+
+
+def test_gemv_time_follows_the_size():
+    """Blocks and warps that share an output must not cost more than they bring:
+    unaligned columns in four-byte loads take less than twice the 16-byte ones (2.5
+    times in clusters of eight), and 2000 short outputs no longer than 2600 (1.7
+    times in eight warps each; 1.35 leaves room for the clock)."""
+    assert gemv_us("N", 16384, 1024, 1) < 2 * gemv_us("N", 16384, 1024, 0)
+    assert gemv_us("T", 2000, 100, 0) < 1.35 * gemv_us("T", 2600, 100, 0)
