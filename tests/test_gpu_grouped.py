@@ -193,3 +193,30 @@ def test_autotuner_caches_its_choice(tmp_path, monkeypatch):
     assert simt_best["block_n"] in (64, 128)
     simt_line = json.loads(cache.read_text().splitlines()[-1])
     assert min(c[7] for c in simt_line["candidates"]) == pytest.approx(simt_line["ms"], rel=1e-6)
+
+
+def test_reduce_of_many_sliced_products_is_short():
+    """The launch that sums the k slices takes a sixth of the GEMM's time with a product of
+    200 x 200 x 3000 and 99 smaller ones (two thirds when each has the blocks of the
+    largest)."""
+    K = 3000
+    shapes = [(200, 200)] + [(100, 101)] * 99
+    ops = [(torch.rand((M, K), device="cuda"), torch.rand((K, N), device="cuda"),
+            torch.empty((M, N), device="cuda")) for M, N in shapes]
+    p = ug.GroupedPlan([dict(ta="N", tb="N", M=A.shape[0], N=B.shape[1], K=K, alpha=1.0, beta=0.0,
+                             A=A, lda=K, B=B, ldb=B.shape[1], C=C, ldc=B.shape[1])
+                        for A, B, C in ops], precision="tf32x3")
+    for _ in range(3):
+        p.run()
+    ug.profile_enable(True)
+    ug.profile_collect()
+    try:
+        for _ in range(5):
+            p.run()
+        r = ug.profile_collect()
+    finally:
+        ug.profile_enable(False)
+    assert r["aux"][1] == 5 and r["aux"][0] < r["grouped"][0] / 3
+    for A, B, C in ops[:3]:
+        assert torch.allclose(C.double(), A.double() @ B.double(), rtol=1e-5)
+    p.close()
