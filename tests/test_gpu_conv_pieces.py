@@ -93,3 +93,17 @@ def test_backward_alone_reads_the_inputs_it_is_given():
     torch.cuda.synchronize()
     assert torch.equal(two, 2 * stack.tensor(0, "dw", (64, 576)))
     stack.close()
+
+
+def test_small_input_is_split_with_the_weights():
+    """One launch splits the weights of all layers and a small first input."""
+    stack = ug.ConvStack([(96, 96, 14, 14, 1, 1, 0)], 1, precision="bf16x6", graph=False)
+    stack.run(ug.CONV_FORWARD)
+    ug.profile_enable(True)
+    ug.profile_collect()
+    try:
+        stack.run(ug.CONV_FORWARD)
+        assert ug.profile_collect()["split_prepass"][1] == 1
+    finally:
+        ug.profile_enable(False)
+        stack.close()

@@ -481,6 +481,17 @@ ugemm_status make_pieces(Stack* s) {
     L.wp = base + wo[l];
     add(s->split_w, taps_job(L.w, L.kdim, kk, L.d.cout, L.d.cin, kk, 0, L.wp));
   }
+  // the first layer's input with them where it is small: one launch less (a
+  // 96 -> 96 channel 1 x 1 layer on one 14 x 14 image: 14.4 us, 12.5 so)
+  auto x_job = [&](int l) {
+    auto& L = s->layers[l];
+    const int in_px = s->batch * L.d.height * L.d.width;
+    L.xp = base + xo[l];
+    return rows_job(L.x, in_px, in_px, L.d.cin, L.xp);
+  };
+  const bool x_with_w = s->layers[0].tap_fwd && !s->explicit_col &&
+                        split_job_tiles(x_job(0)) <= 5 * device_sms();
+  if (x_with_w) add(s->split_w, x_job(0));
   for (int l = 0; l < nl; ++l) {
     auto& L = s->layers[l];
     if (!L.tap_bwd) continue;
@@ -498,9 +509,8 @@ ugemm_status make_pieces(Stack* s) {
     void* shared = base + dy_off;
     SplitJob xj{};
     if (L.tap_fwd && !s->explicit_col) {
-      L.xp = base + xo[l];
-      xj = rows_job(L.x, in_px, in_px, d.cin, L.xp);
-      add(s->split_fwd[l], xj);
+      xj = x_job(l);
+      if (l > 0 || !x_with_w) add(s->split_fwd[l], xj);
       L.fwd_q = PieceOperands{PieceOperands::kTaps, L.wp, L.xp, kk * pad32(d.cin), L.im};
     } else if (L.tap_fwd) {
       SplitJob j{L.col, n, 0, static_cast<__nv_bfloat16*>(shared), n, kk * pad32(d.cin),
