@@ -30,19 +30,27 @@ struct DeviceState {
   // call's kernels get a word of their own, words[0, kErrSlots) in turn, so
   // that a code an earlier call left neither stops a later call's waits nor is
   // taken for its own; words[kErrSlots] holds the first code found when the
-  // words come round again, until ugemm_check reads it.
+  // words come round again, until ugemm_check reads it.  A captured call's word
+  // goes to no eager call: its graph keeps it for life and folds it at every
+  // replay.  Host-pointer calls, one at a time, have a word that each reads and
+  // clears.
   int* words = nullptr;
-  unsigned calls = 0;
+  unsigned calls = 0, captured = 0;
+  int* last_word = nullptr;  // of the last device-pointer call
+  bool host_dirty = false;   // a host-pointer call ended without reading its word
   // the last fold of all words: a call on another stream waits for it
   cudaEvent_t folded = nullptr;
   cudaStream_t fold_stream = nullptr;
-  bool fold_pending = false, fold_due = false;
+  bool fold_pending = false;
   void* ws = nullptr;         // workspace of the device-pointer API
   size_t ws_bytes = 0;
   int sms = 0, cc_major = 0, cc_minor = 0;
 };
 
-constexpr int kMaxDevices = 64, kErrSlots = 4096;
+constexpr int kMaxDevices = 64, kErrSlots = 4096, kCaptured = 1024;
+// words: the calls' ring, the held word, the captured calls', the host-pointer calls'
+constexpr int kCapturedWord = kErrSlots + 1, kHostWord = kCapturedWord + kCaptured;
+constexpr int kWords = kHostWord + 1;
 std::mutex g_mu;
 DeviceState g_dev[kMaxDevices];
 
@@ -85,15 +93,16 @@ ugemm_status device_state(DeviceState** out) {
     cudaDeviceGetAttribute(&d.cc_minor, cudaDevAttrComputeCapabilityMinor, dev);
     if (d.cc_major != 10 || d.cc_minor != 3)
       return fail(UGEMM_ERR_UNSUPPORTED, "libugemm_cuda is built for sm_103a (GB300)%s");
-    e = cudaMalloc(&d.words, (kErrSlots + 1) * sizeof(int));
+    e = cudaMalloc(&d.words, kWords * sizeof(int));
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(error words)");
-    e = cudaMemset(d.words, 0, (kErrSlots + 1) * sizeof(int));
+    e = cudaMemset(d.words, 0, kWords * sizeof(int));
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d.folded, cudaEventDisableTiming);
     if (e != cudaSuccess) {
       cudaFree(d.words);
       d.words = nullptr;
       return cuda_fail(e, "error words");
     }
+    d.last_word = d.words + kErrSlots - 1;
     d.ready = true;
   }
   *out = &d;
@@ -120,38 +129,51 @@ __global__ void error_fold_kernel(int* words, int n, int* held) {
 
 // Start of a call on the device path: its error word.  No launch but once in
 // kErrSlots calls, when the words come round and are folded (a launch of one
-// thread before every call took 2 us of its 13).  A call under capture is
-// replayed any number of times with one word, so its graph folds that word.
-// Caller holds g_mu.
+// thread before every call took 2 us of its 13).  A call under capture takes one
+// of the captured calls' words and folds it in its graph.  Caller holds g_mu.
 ugemm_status begin_call(DeviceState& d, cudaStream_t st, int** word) {
   (void)cudaGetLastError();  // a pending error of earlier, unrelated work is not this call's
-  const unsigned slot = d.calls++ % kErrSlots;
-  *word = d.words + slot;
-  const bool capturing = is_capturing(st);
-  if (slot == 0 && d.calls > 1) d.fold_due = true;
-  const bool fold = d.fold_due && !capturing;
   cudaError_t e = cudaSuccess;
-  if (capturing || fold) {
+  if (is_capturing(st)) {
+    *word = d.last_word = d.words + kCapturedWord + d.captured++ % kCaptured;
     prof_begin(st);
-    if (fold)
-      error_fold_kernel<<<1, 256, 0, st>>>(d.words, kErrSlots, d.words + kErrSlots);
-    else
-      error_fold_kernel<<<1, 1, 0, st>>>(*word, 1, d.words + kErrSlots);
+    error_fold_kernel<<<1, 1, 0, st>>>(*word, 1, d.words + kErrSlots);
     prof_end(st, kProfControl);
     e = cudaGetLastError();
-    if (e == cudaSuccess && fold) {
+    return e == cudaSuccess ? UGEMM_OK : cuda_fail(e, "error word");
+  }
+  const unsigned slot = d.calls++ % kErrSlots;
+  *word = d.last_word = d.words + slot;
+  if (slot == 0 && d.calls > 1) {
+    prof_begin(st);
+    error_fold_kernel<<<1, 256, 0, st>>>(d.words, kErrSlots, d.words + kErrSlots);
+    prof_end(st, kProfControl);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) {
       e = cudaEventRecord(d.folded, st);
       d.fold_stream = st;
       d.fold_pending = true;
-      d.fold_due = false;
     }
   }
-  if (d.fold_pending && !capturing) {
+  if (d.fold_pending) {
     if (cudaEventQuery(d.folded) == cudaSuccess) d.fold_pending = false;
     else if (st != d.fold_stream && e == cudaSuccess) e = cudaStreamWaitEvent(st, d.folded, 0);
     (void)cudaGetLastError();  // the query's "not ready"
   }
   return e == cudaSuccess ? UGEMM_OK : cuda_fail(e, "error word");
+}
+
+// The same for a host-pointer call, which ends with check_device_error.
+ugemm_status begin_host_call(DeviceState& d, int** word) {
+  (void)cudaGetLastError();
+  *word = d.words + kHostWord;
+  if (d.host_dirty) {  // kernels of a call that failed half-way may still run
+    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemset(*word, 0, sizeof(int));
+    if (e != cudaSuccess) return cuda_fail(e, "error word");
+  }
+  d.host_dirty = true;
+  return UGEMM_OK;
 }
 
 // Grow the device workspace to `need` bytes (never during stream capture).
@@ -261,15 +283,16 @@ ugemm_status launch(const Gemm& g, int form, Scratch ws, int* dev_err, cudaStrea
   return UGEMM_OK;
 }
 
-// Read and clear a call's error word (synchronises `st`).
-ugemm_status check_device_error(int* word, cudaStream_t st) {
+// Read and clear the host-pointer calls' error word (synchronises `st`).
+ugemm_status check_device_error(DeviceState& d, cudaStream_t st) {
+  int* word = d.words + kHostWord;
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
   int code = 0;
   e = cudaMemcpy(&code, word, sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(error word)");
+  d.host_dirty = code != 0 && cudaMemset(word, 0, sizeof(int)) != cudaSuccess;
   if (code != 0) {
-    cudaMemset(word, 0, sizeof(int));
     char buf[128];
     std::snprintf(buf, sizeof buf, "kernel pipeline wait timed out (code %d)", code);
     set_last_error(UGEMM_ERR_TIMEOUT, buf);
@@ -303,7 +326,7 @@ ugemm_status dev_gemm(const Gemm& g, int precision, cudaStream_t st) {
 // ten times the three matrices (sgemm_test.c:29), which this layout fits for
 // every shape in the SIMT form (at most 3 padding floats per row).
 ugemm_status host_gemm_tight(const Gemm& g, int form, void* arena, size_t arena_bytes,
-                             int* word, cudaStream_t st) {
+                             DeviceState& d, int* word, cudaStream_t st) {
   const size_t a_rows = g.ta == 'N' ? g.M : g.K, b_rows = g.tb == 'N' ? g.K : g.N;
   const size_t a_cols = g.ta == 'N' ? g.K : g.M, b_cols = g.tb == 'N' ? g.N : g.K;
   const bool need_ab = g.K > 0 && g.alpha != 0.f;
@@ -343,7 +366,7 @@ ugemm_status host_gemm_tight(const Gemm& g, int form, void* arena, size_t arena_
   e = cudaMemcpy2DAsync(g.C, g.ldc * sizeof(float), dg.C, g.N * sizeof(float), g.N * sizeof(float),
                         g.M, cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return cuda_fail(e, "copy C to host");
-  return check_device_error(word, st);
+  return check_device_error(d, st);
 }
 
 // Host-pointer GEMM through a device arena [A | B | C | scratch].
@@ -352,7 +375,7 @@ ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_b
   if (g.M == 0 || g.N == 0) return UGEMM_OK;
   int* word = nullptr;
   {
-    ugemm_status bs = begin_call(d, st, &word);
+    ugemm_status bs = begin_host_call(d, &word);
     if (bs != UGEMM_OK) return bs;
   }
   const size_t a_rows = g.ta == 'N' ? g.M : g.K, b_rows = g.tb == 'N' ? g.K : g.N;
@@ -363,12 +386,12 @@ ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_b
   const int form = resolve_form(precision, g);
   {
     ugemm_status ps = host_gemm_pipelined(g, form, arena, arena_bytes, word, st);
-    if (ps == UGEMM_OK) return check_device_error(word, st);
+    if (ps == UGEMM_OK) return check_device_error(d, st);
     if (ps != UGEMM_ERR_UNSUPPORTED) return fail(ps, "pipelined host GEMM failed%s");
   }
   const bool need_ab = g.K > 0 && g.alpha != 0.f;
   const size_t need = (need_ab ? a_bytes + b_bytes : 0) + c_bytes + scratch_for(g, form);
-  if (need > arena_bytes) return host_gemm_tight(g, form, arena, arena_bytes, word, st);
+  if (need > arena_bytes) return host_gemm_tight(g, form, arena, arena_bytes, d, word, st);
   uint8_t* base = static_cast<uint8_t*>(arena);
   Gemm dg = g;
   size_t off = 0;
@@ -402,7 +425,7 @@ ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_b
                           g.N * sizeof(float), g.M, cudaMemcpyDeviceToHost, st);
   }
   if (e != cudaSuccess) return cuda_fail(e, "copy C to host");
-  return check_device_error(word, st);
+  return check_device_error(d, st);
 }
 
 }  // namespace
@@ -683,7 +706,7 @@ int ugemm_check(void* stream) {
   DeviceState* d = nullptr;
   ugemm_status s = device_state(&d);
   if (s != UGEMM_OK) return s;
-  std::vector<int> words(kErrSlots + 1);
+  std::vector<int> words(kWords);
   int na[2] = {0, 0};
   e = cudaMemcpy(words.data(), d->words, words.size() * sizeof(int), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(error words)");
@@ -695,6 +718,7 @@ int ugemm_check(void* stream) {
   // the first recorded code wins: the held one, then the calls' in their order
   int code = words[kErrSlots];
   for (unsigned i = 0; i < kErrSlots && code == 0; ++i) code = words[(d->calls + i) % kErrSlots];
+  for (int i = 0; i < kCaptured && code == 0; ++i) code = words[kCapturedWord + i];
   if (code != 0) cudaMemset(d->words, 0, words.size() * sizeof(int));
   if (code == 0) code = na[1] ? na[1] : na[0];
   if (code == 0) return UGEMM_OK;
@@ -712,7 +736,7 @@ int ugemm_debug_set_error_word(int which, int code) {
   ugemm_status s = device_state(&d);
   if (s != UGEMM_OK) return s;
   // the word of the last device-pointer call
-  int* word = which == 0   ? d->words + (d->calls + kErrSlots - 1) % kErrSlots
+  int* word = which == 0   ? d->last_word
               : which == 1 ? noalloc_error_words()
                            : nullptr;
   if (!word) return fail(UGEMM_ERR_ARG, "no such error word on this device (yet)%s");
