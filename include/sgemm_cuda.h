@@ -177,9 +177,13 @@ UGEMM_API int ugemm_sgemm_backward(char transa, char transb, int M, int N, int K
  * ugemm_sgemm_backward and ugemm_sgemm_dev_noalloc on the current device,
  * clears them and returns UGEMM_ERR_TIMEOUT (with the code in the last-error
  * message) if any of their kernels gave up since the last check, else
- * UGEMM_OK.  A stale code never disturbs a later call: calls take their words
- * in turn, and a word's code is moved aside before it is used again.  The
- * words are per device, shared by all streams.  (Grouped plans have their own word: ugemm_grouped_check.) */
+ * UGEMM_OK.  A stale code never disturbs a later call: the calls on a stream
+ * take its words in turn, a word's code is moved aside on that stream before the
+ * word is used again, and a captured call's word, which its graph keeps, goes to
+ * no other call (to another captured one after 1024) and is folded at every
+ * replay.  Beyond 64 streams calls share a word, folded before each.  (Host-pointer
+ * calls report their own waits.  Grouped plans have their own word:
+ * ugemm_grouped_check.) */
 UGEMM_API int ugemm_check(void *stream);
 
 /* Test hook for the error reporting above (no reference counterpart): writes

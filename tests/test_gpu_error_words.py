@@ -64,6 +64,28 @@ def test_words_come_round_without_their_codes():
     reported(3)
 
 
+def test_more_streams_than_rings():
+    calls = Calls(200, *[torch.cuda.ExternalStream(s.cuda_stream) for s in
+                         (torch.cuda.Stream(priority=p) for p in (0, -1) * 50)])
+    calls.run()
+    calls.check()
+    ug.check()
+
+
+def test_calls_beside_a_capture_on_another_stream():
+    """Eager calls make nothing that a global-mode capture forbids."""
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    calls, inside = Calls(5000, two), Calls(1, one)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=one):
+        inside.run()
+        calls.run()
+    calls.check()
+    g.replay()
+    inside.check()
+    ug.check()
+
+
 def test_captured_calls_keep_their_word():
     M, K = 1100, 1500
     A, B = torch.rand((M, K), device="cuda"), torch.rand((K, M), device="cuda")

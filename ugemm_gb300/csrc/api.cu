@@ -24,33 +24,39 @@ namespace {
 thread_local int t_last_status = UGEMM_OK;
 thread_local std::string t_last_msg;
 
+constexpr int kRings = 64, kRing = 64, kCaptured = 1024;
+constexpr int kCapturedWord = kRings * kRing, kHostWord = kCapturedWord + kCaptured;
+constexpr int kSharedWord = kHostWord + 1, kHeldWord = kSharedWord + 1, kWords = kHeldWord + 1;
+
 struct DeviceState {
   bool ready = false;
-  // Device-side error words, written by the bounded waits of kernels.  Each
-  // call's kernels get a word of their own, words[0, kErrSlots) in turn, so
-  // that a code an earlier call left neither stops a later call's waits nor is
-  // taken for its own; words[kErrSlots] holds the first code found when the
-  // words come round again, until ugemm_check reads it.  A captured call's word
-  // goes to no eager call: its graph keeps it for life and folds it at every
-  // replay.  Host-pointer calls, one at a time, have a word that each reads and
-  // clears.
+  // Device-side error words, written by the bounded waits of kernels and polled
+  // by them, so that no call may find an earlier call's code in its word:
+  //   kRings rings of kRing words: the calls on one stream take a ring's words
+  //     in turn.  When they come round, a fold on that stream, which is after all
+  //     their users and before the next ones, moves a code to the held word;
+  //   kCaptured words for captured calls, whose graphs keep theirs for life and
+  //     fold it before the call's kernels at every replay;
+  //   the host-pointer calls' (one runs at a time, reads and clears it);
+  //   the word of calls on streams that found no ring, each after a fold of its own;
+  //   the held word: the first code folded, until ugemm_check reads it.
   int* words = nullptr;
-  unsigned calls = 0, captured = 0;
-  int* last_word = nullptr;  // of the last device-pointer call
-  bool host_dirty = false;   // a host-pointer call ended without reading its word
-  // the last fold of all words: a call on another stream waits for it
-  cudaEvent_t folded = nullptr;
-  cudaStream_t fold_stream = nullptr;
-  bool fold_pending = false;
+  struct Ring {
+    unsigned long long stream = 0;  // cudaStreamGetId
+    unsigned next = 0;
+    bool round = false;  // the words have been used before
+  };
+  Ring rings[kRings];
+  int nrings = 0, last_ring = 0;
+  unsigned captured = 0;
+  int* last_word = nullptr;    // of the last device-pointer call
+  bool host_dirty = false;     // a host-pointer call ended without reading its word
   void* ws = nullptr;         // workspace of the device-pointer API
   size_t ws_bytes = 0;
   int sms = 0, cc_major = 0, cc_minor = 0;
 };
 
-constexpr int kMaxDevices = 64, kErrSlots = 4096, kCaptured = 1024;
-// words: the calls' ring, the held word, the captured calls', the host-pointer calls'
-constexpr int kCapturedWord = kErrSlots + 1, kHostWord = kCapturedWord + kCaptured;
-constexpr int kWords = kHostWord + 1;
+constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 DeviceState g_dev[kMaxDevices];
 
@@ -94,15 +100,13 @@ ugemm_status device_state(DeviceState** out) {
     if (d.cc_major != 10 || d.cc_minor != 3)
       return fail(UGEMM_ERR_UNSUPPORTED, "libugemm_cuda is built for sm_103a (GB300)%s");
     e = cudaMalloc(&d.words, kWords * sizeof(int));
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(error words)");
-    e = cudaMemset(d.words, 0, kWords * sizeof(int));
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d.folded, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMemset(d.words, 0, kWords * sizeof(int));
     if (e != cudaSuccess) {
       cudaFree(d.words);
       d.words = nullptr;
       return cuda_fail(e, "error words");
     }
-    d.last_word = d.words + kErrSlots - 1;
+    d.last_word = d.words + kSharedWord;
     d.ready = true;
   }
   *out = &d;
@@ -119,47 +123,44 @@ bool is_capturing(cudaStream_t st) {
 // free) and clears them.
 __global__ void error_fold_kernel(int* words, int n, int* held) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int code = words[i];
-    if (code != 0) {
-      atomicCAS(held, 0, code);
-      words[i] = 0;
-    }
+    const int code = words[i] != 0 ? atomicExch(words + i, 0) : 0;
+    if (code != 0) atomicCAS(held, 0, code);
   }
 }
 
-// Start of a call on the device path: its error word.  No launch but once in
-// kErrSlots calls, when the words come round and are folded (a launch of one
-// thread before every call took 2 us of its 13).  A call under capture takes one
-// of the captured calls' words and folds it in its graph.  Caller holds g_mu.
+// Start of a device-pointer call: its error word.  No launch but once in kRing
+// calls on a stream (a launch of one thread before every call took 2 us of its
+// 13), no event, no query.  Caller holds g_mu.
 ugemm_status begin_call(DeviceState& d, cudaStream_t st, int** word) {
   (void)cudaGetLastError();  // a pending error of earlier, unrelated work is not this call's
-  cudaError_t e = cudaSuccess;
+  int first = kSharedWord, n = 1;  // the words to fold; n == 0: none
   if (is_capturing(st)) {
-    *word = d.last_word = d.words + kCapturedWord + d.captured++ % kCaptured;
-    prof_begin(st);
-    error_fold_kernel<<<1, 1, 0, st>>>(*word, 1, d.words + kErrSlots);
-    prof_end(st, kProfControl);
-    e = cudaGetLastError();
-    return e == cudaSuccess ? UGEMM_OK : cuda_fail(e, "error word");
-  }
-  const unsigned slot = d.calls++ % kErrSlots;
-  *word = d.last_word = d.words + slot;
-  if (slot == 0 && d.calls > 1) {
-    prof_begin(st);
-    error_fold_kernel<<<1, 256, 0, st>>>(d.words, kErrSlots, d.words + kErrSlots);
-    prof_end(st, kProfControl);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) {
-      e = cudaEventRecord(d.folded, st);
-      d.fold_stream = st;
-      d.fold_pending = true;
+    first = kCapturedWord + d.captured++ % kCaptured;
+    *word = d.words + first;
+  } else {
+    *word = d.words + kSharedWord;
+    unsigned long long id = 0;
+    const bool known = cudaStreamGetId(st, &id) == cudaSuccess;
+    int r = d.last_ring;
+    if (known && (r >= d.nrings || d.rings[r].stream != id)) {
+      for (r = 0; r < d.nrings && d.rings[r].stream != id;) ++r;
+      if (r == d.nrings && r < kRings) d.rings[d.nrings++].stream = id;
+    }
+    if (known && r < kRings) {
+      DeviceState::Ring& ring = d.rings[d.last_ring = r];
+      *word = d.words + r * kRing + ring.next;
+      first = r * kRing;
+      n = ring.next == 0 && ring.round ? kRing : 0;
+      ring.next = (ring.next + 1) % kRing;
+      ring.round = true;
     }
   }
-  if (d.fold_pending) {
-    if (cudaEventQuery(d.folded) == cudaSuccess) d.fold_pending = false;
-    else if (st != d.fold_stream && e == cudaSuccess) e = cudaStreamWaitEvent(st, d.folded, 0);
-    (void)cudaGetLastError();  // the query's "not ready"
-  }
+  d.last_word = *word;
+  if (n == 0) return UGEMM_OK;
+  prof_begin(st);
+  error_fold_kernel<<<1, n, 0, st>>>(d.words + first, n, d.words + kHeldWord);
+  prof_end(st, kProfControl);
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? UGEMM_OK : cuda_fail(e, "error word");
 }
 
@@ -715,10 +716,10 @@ int ugemm_check(void* stream) {
     e = cudaMemcpy(na, nw, sizeof na, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(error words)");
   }
-  // the first recorded code wins: the held one, then the calls' in their order
-  int code = words[kErrSlots];
-  for (unsigned i = 0; i < kErrSlots && code == 0; ++i) code = words[(d->calls + i) % kErrSlots];
-  for (int i = 0; i < kCaptured && code == 0; ++i) code = words[kCapturedWord + i];
+  // the first recorded code wins: the held one is older than the calls'
+  words[kHostWord] = 0;  // reported by its own call
+  int code = words[kHeldWord];
+  for (int i = 0; i < kHeldWord && code == 0; ++i) code = words[i];
   if (code != 0) cudaMemset(d->words, 0, words.size() * sizeof(int));
   if (code == 0) code = na[1] ? na[1] : na[0];
   if (code == 0) return UGEMM_OK;
@@ -735,7 +736,7 @@ int ugemm_debug_set_error_word(int which, int code) {
   DeviceState* d = nullptr;
   ugemm_status s = device_state(&d);
   if (s != UGEMM_OK) return s;
-  // the word of the last device-pointer call
+  // (no call yet: a word that is folded before it is used)
   int* word = which == 0   ? d->last_word
               : which == 1 ? noalloc_error_words()
                            : nullptr;
