@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "split_tc.cuh"
 
 namespace ugemm {
 
@@ -245,34 +246,46 @@ bool is_split_form(int form) {
          form == UGEMM_PREC_FP16X3 || form == UGEMM_PREC_TF32X3;
 }
 
-size_t scratch_for(const Gemm& g, int form) {
-  if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return 0;
-  if (form == UGEMM_PREC_SIMT) return simt_scratch_bytes(g);
-  const SplitPlan p = split_plan_for(form, g);
-  // an under-filled GEMM with deep k runs as split-K slices (multi.cu)
-  if (multi_wanted(g, p)) return multi_scratch_bytes(&g, 1, p);
-  return split_scratch_bytes(g, p);
+// How a GEMM runs and the scratch that takes, found once a call.
+struct Route {
+  size_t scratch = 0;
+  SplitPlan plan;      // split forms
+  bool multi = false;  // narrow tiles or k slices (multi.cu)
+  MultiLayout layout;
+};
+Route route_for(const Gemm& g, int form) {
+  Route r;
+  if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return r;
+  if (form == UGEMM_PREC_SIMT) {
+    r.scratch = simt_scratch_bytes(g);
+  } else if (is_split_form(form)) {
+    r.plan = split_plan_for(form, g);
+    r.multi = multi_wanted(g, r.plan, &r.layout);
+    r.scratch = r.multi ? r.layout.total : split_scratch_bytes(g, r.plan);
+  }
+  return r;
 }
 
+size_t scratch_for(const Gemm& g, int form) { return route_for(g, form).scratch; }
+
 // The least scratch it can run in: whole tiles need no partial ones.
-size_t scratch_least(const Gemm& g, int form) {
-  const size_t want = scratch_for(g, form);
-  if (want == 0 || !is_split_form(form)) return want;
-  return std::min(want, split_scratch_bytes(g, split_plan_for(form, g)));
+size_t scratch_least(const Gemm& g, const Route& r) {
+  return r.multi ? std::min(r.scratch, split_scratch_bytes(g, r.plan)) : r.scratch;
 }
 
 // Launch one GEMM on `st` using `ws` as scratch: on narrower tiles or slices
-// where that is faster and their scratch fits.
-ugemm_status launch(const Gemm& g, int form, Scratch ws, int* dev_err, cudaStream_t st) {
+// where that is its route and their scratch fits.
+ugemm_status launch(const Gemm& g, int form, const Route& r, Scratch ws, int* dev_err,
+                    cudaStream_t st) {
   if (g.M == 0 || g.N == 0) return UGEMM_OK;
   if (g.K == 0 || g.alpha == 0.f) return scale_c_launch(g, st);
   ugemm_status s;
   if (form == UGEMM_PREC_SIMT) {
     s = simt_launch(g, simt_pick_tile(g), ws, dev_err, st);
   } else if (is_split_form(form)) {
-    const SplitPlan p = split_plan_for(form, g);
-    const bool multi = multi_wanted(g, p) && multi_scratch_bytes(&g, 1, p) <= ws.bytes;
-    s = multi ? multi_launch(&g, 1, p, ws, dev_err, st) : split_launch(g, p, ws, dev_err, st);
+    s = r.multi && r.scratch <= ws.bytes
+            ? multi_launch(&g, 1, r.plan, r.layout, ws, dev_err, st)
+            : split_launch(g, r.plan, ws, dev_err, st);
   } else {
     return fail(UGEMM_ERR_ARG, "unknown precision%s");
   }
@@ -308,15 +321,15 @@ ugemm_status dev_gemm(const Gemm& g, int precision, cudaStream_t st) {
   ugemm_status s = device_state(&d);
   if (s != UGEMM_OK) return s;
   const int form = resolve_form(precision, g);
-  const size_t want = scratch_for(g, form);
+  const Route r = route_for(g, form);
   // a graph is captured in the workspace there is, if the call fits it at all
-  if (want <= d->ws_bytes || !is_capturing(st) || scratch_least(g, form) > d->ws_bytes)
-    s = ensure_workspace(*d, want, st);
+  if (r.scratch <= d->ws_bytes || !is_capturing(st) || scratch_least(g, r) > d->ws_bytes)
+    s = ensure_workspace(*d, r.scratch, st);
   if (s != UGEMM_OK) return s;
   int* word = nullptr;
   s = begin_call(*d, st, &word);
   if (s != UGEMM_OK) return s;
-  return launch(g, form, Scratch{d->ws, d->ws_bytes}, word, st);
+  return launch(g, form, r, Scratch{d->ws, d->ws_bytes}, word, st);
 }
 
 // Host-pointer GEMM in an arena too small for the 256-byte-aligned layout:
@@ -344,7 +357,8 @@ ugemm_status host_gemm_tight(const Gemm& g, int form, void* arena, size_t arena_
   dg.lda = lda4;
   dg.ldb = ldb4;
   dg.ldc = g.N;
-  const size_t scratch = scratch_least(dg, form);
+  const Route r = route_for(dg, form);
+  const size_t scratch = scratch_least(dg, r);
   const size_t s_off = scratch ? align_up(a_bytes + b_bytes + c_bytes, 256) : a_bytes + b_bytes + c_bytes;
   if (s_off + scratch > arena_bytes)
     return fail(UGEMM_ERR_ARENA_TOO_SMALL, "device arena too small for this call%s");
@@ -362,7 +376,7 @@ ugemm_status host_gemm_tight(const Gemm& g, int form, void* arena, size_t arena_
                           g.N * sizeof(float), g.M, cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(e, "copy C to device");
   }
-  ugemm_status s = launch(dg, form, Scratch{base + s_off, arena_bytes - s_off}, word, st);
+  ugemm_status s = launch(dg, form, r, Scratch{base + s_off, arena_bytes - s_off}, word, st);
   if (s != UGEMM_OK) return s;
   e = cudaMemcpy2DAsync(g.C, g.ldc * sizeof(float), dg.C, g.N * sizeof(float), g.N * sizeof(float),
                         g.M, cudaMemcpyDeviceToHost, st);
@@ -416,7 +430,7 @@ ugemm_status host_gemm(const Gemm& g, int precision, void* arena, size_t arena_b
     if (e != cudaSuccess) return cuda_fail(e, "copy C to device");
   }
   Scratch ws{base + off + c_bytes, arena_bytes - off - c_bytes};
-  ugemm_status s = launch(dg, form, ws, word, st);
+  ugemm_status s = launch(dg, form, route_for(dg, form), ws, word, st);
   if (s != UGEMM_OK) return s;
   // Copy back row by row only when the host C has padding we must not touch.
   if (g.ldc == g.N) {
@@ -665,12 +679,13 @@ int ugemm_sgemm_backward(char transa, char transb, int M, int N, int K, float al
       ugemm_status s = device_state(&d);
       if (s != UGEMM_OK) return s;
       const SplitPlan p = split_plan_for(form, gs[0]);
-      s = ensure_workspace(*d, multi_scratch_bytes(gs, n, p), st);
+      const MultiLayout layout = multi_layout(gs, n, p);
+      s = ensure_workspace(*d, layout.total, st);
       if (s != UGEMM_OK) return s;
       int* word = nullptr;
       s = begin_call(*d, st, &word);
       if (s != UGEMM_OK) return s;
-      s = multi_launch(gs, n, p, Scratch{d->ws, d->ws_bytes}, word, st);
+      s = multi_launch(gs, n, p, layout, Scratch{d->ws, d->ws_bytes}, word, st);
       if (s == UGEMM_ERR_CUDA) return cuda_fail(cudaGetLastError(), "kernel launch");
       if (s != UGEMM_OK) return fail(s, "launch failed%s");
       return UGEMM_OK;

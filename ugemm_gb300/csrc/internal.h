@@ -301,13 +301,6 @@ ugemm_status splitk_reduce_launch(const ReduceJob* jobs, int njobs, long long ma
 ugemm_status splitk_reduce_param_launch(const ReduceJob* jobs, int njobs, long long max_mn,
                                         cudaStream_t st);
 
-// Up to kMultiMax split-precision GEMMs (and split-K slices of them) in one
-// persistent launch, scratch in the caller's workspace (multi.cu).
-bool multi_wanted(const Gemm& g, const SplitPlan& p);  // rather than whole tiles
-bool multi_faster(const Gemm& g, const SplitPlan& p);
-size_t multi_scratch_bytes(const Gemm* gs, int n, const SplitPlan& p);
-ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& p, Scratch ws, int* dev_err,
-                          cudaStream_t st);
 
 // Grouped plans: the builder behind ugemm_grouped_plan_create (validated
 // problems, longest k first inside), default tile configuration and the

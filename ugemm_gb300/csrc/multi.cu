@@ -38,18 +38,6 @@ double padded(int rows, int cols, int bn) {
   return double(align_up(rows, 128)) * ((cols / bn) * bn + align_up(cols % bn, 16));
 }
 
-// Scratch layout: per GEMM [A pieces | B pieces], then the partial tiles of
-// the sliced GEMMs.
-struct Layout {
-  GeoChoice geo[kMultiMax];
-  int block_n = 256;
-  size_t a_off[kMultiMax], b_off[kMultiMax], part_off[kMultiMax];
-  size_t total = 0;
-  int longest = 0;     // one GEMM: choose_geometry's `longest`
-  double us = 0;       // one GEMM: the model's time of all its launches
-  bool fused = false;  // one GEMM: the operands split inside the GEMM kernel
-};
-
 // Slices whose partial tiles take 512 MiB.
 int most_slices(const Gemm& g) {
   return std::max(1, static_cast<int>(std::min(1e9, double(512 << 20) / (double(g.M) * g.N * 4))));
@@ -88,12 +76,15 @@ int longest_sum(const Gemm& g, int pieces, int sms) {
   return slice_blocks(h.nkb[0], h.fair, std::min(kMultiSubs, most_slices(g)));
 }
 
+}  // namespace
+
 // One GEMM: the tile width and slices of the least time by the stage times.
 // Several: slices no longer than half an SM's fair share, which round robin
 // then balances (2048 x 8192 x 1024 backward: 342 us, 435 with whole tiles on
 // each GEMM's share of the SMs).
-Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
-  Layout L;
+MultiLayout multi_layout(const Gemm* gs, int n, const SplitPlan& p) {
+  MultiLayout L;
+  const int sms = device_sms();
   if (n == 1) {
     const int slices = std::min(kMultiSubs, most_slices(gs[0]));
     const int nkb = split_nkb(p.pieces, gs[0].K);
@@ -149,8 +140,6 @@ Layout layout_for(const Gemm* gs, int n, const SplitPlan& p, int sms) {
   L.total = align_up(off, 256);
   return L;
 }
-
-}  // namespace
 
 TailPlan tail_plan(const Gemm& g, const SplitPlan& p) {
   TailPlan t;
@@ -227,43 +216,50 @@ ugemm_status tail_launch(const Gemm& g, const SplitPlan& p, const TailPlan& tail
                        : splitk_reduce_param_launch(&red, 1, static_cast<long long>(mn), st);
 }
 
-// Whether narrower tiles or k slices are faster than one launch of whole 256-
-// (or, up to 128 columns, 128-) wide tiles by the stage times, as they are where
-// whole tiles leave SMs idle (1024^3: 32 tiles of 256).
-bool multi_faster(const Gemm& g, const SplitPlan& p) {
-  if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return false;
-  const int sms = device_sms();
-  const int tiles = cdiv(g.M, kTcBM) * cdiv(g.N, p.block_n);
-  if (tiles > 4 * sms) return false;
+namespace {
+
+// Whether L's narrower tiles or k slices are faster than one launch of whole
+// 256- (or, up to 128 columns, 128-) wide tiles by the stage times, as they are
+// where whole tiles leave SMs idle (1024^3: 32 tiles of 256).
+bool faster_than_whole(const Gemm& g, const SplitPlan& p, const MultiLayout& L) {
   const int nkb = split_nkb(p.pieces, g.K);
-  const GeoChoice whole = choose_geometry(p.pieces, g.M, g.N, nkb, sms, p.block_n, false, 1, nkb);
-  return layout_for(&g, 1, p, sms).us <
-         0.95 * (whole.us + split_pass_us((double(g.M) + g.N) * g.K));
+  const GeoChoice whole =
+      choose_geometry(p.pieces, g.M, g.N, nkb, device_sms(), p.block_n, false, 1, nkb);
+  return L.us < 0.95 * (whole.us + split_pass_us((double(g.M) + g.N) * g.K));
 }
 
-// Whether a GEMM runs here: where that is faster, and where its tiles are fewer
-// than the SMs and k is deep, so that slices or sums of sums (choose_geometry's
-// `longest`) cost little and are nearer FP64 (2048^3 in BF16x6: one wave of 128
-// whole tiles is 1.29e-7 from it, sums of a third of k each 1.16e-7).
-bool multi_wanted(const Gemm& g, const SplitPlan& p) {
-  if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return false;
-  const int sms = device_sms();
-  return (cdiv(g.M, kTcBM) * cdiv(g.N, p.block_n) < sms &&
-          longest_sum(g, p.pieces, sms) < split_nkb(p.pieces, g.K)) ||
-         multi_faster(g, p);
+// Whole tiles of g, or 0 if it does not run here at all.
+int whole_tiles(const Gemm& g, const SplitPlan& p) {
+  if (g.M == 0 || g.N == 0 || g.K == 0 || g.alpha == 0.f) return 0;
+  const double tiles = double(cdiv(g.M, kTcBM)) * cdiv(g.N, p.block_n);
+  return tiles > 4 * device_sms() ? 0 : static_cast<int>(tiles);
 }
 
-size_t multi_scratch_bytes(const Gemm* gs, int n, const SplitPlan& p) {
-  if (n < 1 || n > kMultiMax) return 0;
-  return layout_for(gs, n, p, device_sms()).total;
+}  // namespace
+
+bool multi_faster(const Gemm& g, const SplitPlan& p, MultiLayout* L) {
+  if (whole_tiles(g, p) == 0) return false;
+  *L = multi_layout(&g, 1, p);
+  return faster_than_whole(g, p, *L);
 }
 
-ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, Scratch ws, int* dev_err,
-                          cudaStream_t st) {
+// Where that is faster, and where the tiles are fewer than the SMs and k is deep,
+// so that slices or sums of sums (choose_geometry's `longest`) cost little and are
+// nearer FP64 (2048^3 in BF16x6: one wave of 128 whole tiles is 1.29e-7 from
+// it, sums of a third of k each 1.16e-7).
+bool multi_wanted(const Gemm& g, const SplitPlan& p, MultiLayout* L) {
+  const int tiles = whole_tiles(g, p);
+  if (tiles == 0) return false;
+  *L = multi_layout(&g, 1, p);
+  return (tiles < device_sms() && L->longest < split_nkb(p.pieces, g.K)) ||
+         faster_than_whole(g, p, *L);
+}
+
+ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, const MultiLayout& L,
+                          Scratch ws, int* dev_err, cudaStream_t st) {
   if (n < 1 || n > kMultiMax) return UGEMM_ERR_ARG;
   for (int i = 0; i < n; ++i)
     if (gs[i].M == 0 || gs[i].N == 0 || gs[i].K == 0 || gs[i].alpha == 0.f) return UGEMM_ERR_ARG;
-  const Layout L = layout_for(gs, n, plan, device_sms());
   if (L.total > ws.bytes) return UGEMM_ERR_ARENA_TOO_SMALL;
   uint8_t* base = static_cast<uint8_t*>(ws.ptr);
   SplitPlan p = plan;

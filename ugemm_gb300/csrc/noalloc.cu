@@ -28,6 +28,7 @@
 #include <mutex>
 
 #include "internal.h"
+#include "split_tc.cuh"
 
 namespace ugemm {
 namespace {
@@ -149,8 +150,8 @@ extern "C" UGEMM_API int ugemm_sgemm_dev_noalloc(char major, char transa, char t
   // the workspace entry point's route where that is faster and its partial
   // tiles fit the array, else whole tiles
   const SplitPlan plan = split_plan_for(form, g);
-  const bool multi =
-      multi_faster(g, plan) && multi_scratch_bytes(&g, 1, plan) <= kNoAllocScratchBytes;
+  MultiLayout layout;
+  const bool multi = multi_faster(g, plan, &layout) && layout.total <= kNoAllocScratchBytes;
   // what is refused follows from whole tiles on pieces, whatever the route
   const size_t need = split_scratch_bytes(g, plan);
   if (need > kNoAllocScratchBytes) {
@@ -169,7 +170,8 @@ extern "C" UGEMM_API int ugemm_sgemm_dev_noalloc(char major, char transa, char t
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(UGEMM_ERR_CUDA, cudaGetErrorString(e));
   const Scratch ws{slot->scratch, kNoAllocScratchBytes};
-  s = multi ? multi_launch(&g, 1, plan, ws, slot->err, st) : split_launch(g, plan, ws, slot->err, st);
+  s = multi ? multi_launch(&g, 1, plan, layout, ws, slot->err, st)
+            : split_launch(g, plan, ws, slot->err, st);
   if (s != UGEMM_OK) {
     const cudaError_t le = cudaGetLastError();
     return fail(s, le != cudaSuccess ? cudaGetErrorString(le) : "split launch failed");

@@ -275,6 +275,26 @@ bool fusable(const Gemm& g);
 // The raw-tile maps and layouts of a fused problem.
 bool fused_encode_problem(const Gemm& g, bool swap, int block_n, CUtensorMap* maps, TcProblem* p);
 
+// Up to kMultiMax split-precision GEMMs (and split-K slices of them) in one
+// persistent launch, scratch in the caller's workspace (multi.cu): per GEMM
+// [A pieces | B pieces], then the partial tiles of the sliced GEMMs.
+struct MultiLayout {
+  GeoChoice geo[kMultiMax];
+  int block_n = 256;
+  size_t a_off[kMultiMax], b_off[kMultiMax], part_off[kMultiMax];
+  size_t total = 0;    // bytes of scratch
+  int longest = 0;     // one GEMM: choose_geometry's `longest`
+  double us = 0;       // one GEMM: the model's time of all its launches
+  bool fused = false;  // one GEMM: the operands split inside the GEMM kernel
+};
+MultiLayout multi_layout(const Gemm* gs, int n, const SplitPlan& p);
+// Whether one GEMM runs here rather than as whole tiles, and its layout if so;
+// multi_faster: by time alone.
+bool multi_wanted(const Gemm& g, const SplitPlan& p, MultiLayout* L);
+bool multi_faster(const Gemm& g, const SplitPlan& p, MultiLayout* L);
+ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& p, const MultiLayout& L,
+                          Scratch ws, int* dev_err, cudaStream_t st);
+
 int split_kp(int K);
 int split_default_chunk_kb(int K);
 // Bytes of one operand's pieces [pieces][rows][Kp]; two-piece operands also
