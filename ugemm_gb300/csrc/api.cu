@@ -679,7 +679,10 @@ int ugemm_sgemm_backward(char transa, char transb, int M, int N, int K, float al
       ugemm_status s = device_state(&d);
       if (s != UGEMM_OK) return s;
       const SplitPlan p = split_plan_for(form, gs[0]);
-      const MultiLayout layout = multi_layout(gs, n, p);
+      MultiLayout layout = multi_layout(gs, n, p);
+      // a graph is captured in the workspace there is, if one gradient's pieces fit it
+      if (n == 1 && layout.total > d->ws_bytes && is_capturing(st))
+        layout = multi_layout(gs, n, p, true);
       s = ensure_workspace(*d, layout.total, st);
       if (s != UGEMM_OK) return s;
       int* word = nullptr;

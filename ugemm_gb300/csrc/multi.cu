@@ -82,13 +82,15 @@ int longest_sum(const Gemm& g, int pieces, int sms) {
 // Several: slices no longer than half an SM's fair share, which round robin
 // then balances (2048 x 8192 x 1024 backward: 342 us, 435 with whole tiles on
 // each GEMM's share of the SMs).
-MultiLayout multi_layout(const Gemm* gs, int n, const SplitPlan& p) {
+MultiLayout multi_layout(const Gemm* gs, int n, const SplitPlan& p, bool whole_k) {
   MultiLayout L;
   const int sms = device_sms();
   if (n == 1) {
-    const int slices = std::min(kMultiSubs, most_slices(gs[0]));
+    const int slices = whole_k ? 1 : std::min(kMultiSubs, most_slices(gs[0]));
     const int nkb = split_nkb(p.pieces, gs[0].K);
-    const int longest = L.longest = longest_sum(gs[0], p.pieces, sms);
+    // (without slices, only 64-wide tiles, three pieces', keep the sums short)
+    const int longest = L.longest =
+        whole_k && p.pieces != 3 ? nkb : longest_sum(gs[0], p.pieces, sms);
     L.us = 1e300;
     for (int bn : {64, 128, 256}) {
       if (bn == 64 && p.pieces != 3) continue;

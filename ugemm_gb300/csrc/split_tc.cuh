@@ -287,7 +287,8 @@ struct MultiLayout {
   double us = 0;       // one GEMM: the model's time of all its launches
   bool fused = false;  // one GEMM: the operands split inside the GEMM kernel
 };
-MultiLayout multi_layout(const Gemm* gs, int n, const SplitPlan& p);
+// whole_k: one GEMM without k slices, whose scratch is its pieces at most.
+MultiLayout multi_layout(const Gemm* gs, int n, const SplitPlan& p, bool whole_k = false);
 // Whether one GEMM runs here rather than as whole tiles, and its layout if so;
 // multi_faster: by time alone.
 bool multi_wanted(const Gemm& g, const SplitPlan& p, MultiLayout* L);
