@@ -109,3 +109,19 @@ def test_gemv_partial_sums(M, N, bound):
     ug.sgemv("N", M, N, 1.0, At, M, x, 1, 0.0, y, 1)
     ref = torch.mv(At.double().T, x.double())
     assert rel(y, ref) < SAMPLE * bound
+
+
+@pytest.mark.parametrize("prec", ["bf16x6", "bf16x9"])
+@pytest.mark.parametrize("what,M,N,K,bound", [
+    ("gemm", 1024, 1024, 672, 8.99e-8), ("gradient", 2048, 2048, 672, 8.98e-8),
+    ("gradient", 1000, 3000, 928, 9.79e-8)])
+def test_chunks_of_an_odd_depth(what, prec, M, N, K, bound):
+    """21 and 29 stages: chunks of two and one of one, not 21 or 29 of one."""
+    A, B = mat(M, K, 1), mat(K, N, 2)
+    if what == "gemm":
+        C = ug.gemm(A, B, precision=prec)
+    else:  # C as the gradient of X in Y = X W, A that of Y
+        C, W = torch.empty((M, N), device="cuda"), B.t().contiguous()
+        ug.sgemm_backward("N", "N", M, K, N, 1.0, 0, N, W, K, A, K, 0.0, C, N, 0.0, None, K,
+                          precision=prec)
+    assert rel(C, ug.ref64("N", "N", A, B)) < SAMPLE * bound

@@ -366,8 +366,12 @@ ugemm_status multi_launch(const Gemm* gs, int n, const SplitPlan& plan, const Mu
   TcProblem single{};
   int chunk =
       split_chunk_stages(p.pieces, p.chunk_kb > 0 ? p.chunk_kb : split_default_chunk_kb(min_k));
-  // chunks no deeper than those of the longest sum on average (its last may be short)
-  if (n == 1) chunk = std::max(1, L.longest / cdiv(L.longest, chunk));
+  // chunks no deeper than those of the longest sum on average (its last may be
+  // short); three pieces' not of a single stage for that, as twice the sums round
+  // more than they save (2048 x 2048 x 928: 1.09e-7 of FP64, 9.7e-8 in twos), and
+  // as they are where k is not to be cut
+  if (n == 1 && !(p.pieces == 3 && L.longest >= split_nkb(3, min_k)))
+    chunk = std::max(p.pieces == 3 ? std::min(chunk, 2) : 1, L.longest / cdiv(L.longest, chunk));
   const ugemm_status s =
       split_gemm_launch(p, dummy, dummy, single, nullptr, nullptr, nullptr, tiles, chunk,
                         std::max(1, std::min(tiles, device_sms())), dev_err, st, nullptr, &t);
