@@ -121,3 +121,34 @@ def test_arena_for_whole_tiles_alone(M, N, K):
         ug.sgemm_cuda_finish()
     ref = A.astype(np.float64) @ B.astype(np.float64)
     assert np.linalg.norm(C - ref) / np.linalg.norm(ref) < 2e-6
+
+
+@pytest.mark.parametrize("ta,tb", ["NN", "NT", "TN", "TT"])
+@pytest.mark.parametrize("M,N,K", [(2500, 2300, 270),   # the sizes above, deep enough for wide tiles
+                                   (20000, 129, 257), (2049, 2561, 300), (19457, 300, 260),
+                                   (128, 25088, 290),   # one wave of 128 x 192
+                                   (6000, 6000, 33), (1025, 4097, 31), (4096, 4096, 8)])  # narrow ones
+def test_simt_tiles_by_depth(ta, tb, M, N, K):
+    check(ta, tb, M, N, K, "simt", pad=3)
+
+
+def simt_us(ta, tb, M, N, K):
+    A = torch.rand((M, K) if ta == "N" else (K, M), device="cuda")
+    B = torch.rand((K, N) if tb == "N" else (N, K), device="cuda")
+    C = torch.empty((M, N), device="cuda")
+    e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    best = 1e9
+    for _ in range(8):
+        e[0].record()
+        for _ in range(10):
+            ug.gemm(A, B, C, ta=ta, tb=tb, precision="simt")
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]))
+    return best * 100
+
+
+def test_simt_shallow_time():
+    """A product of one k stage is bound by its stores: it takes as long in every layout
+    (in wide tiles, which NT has none of, 1.26 times as long)."""
+    assert simt_us("N", "N", 6000, 6000, 32) < 1.12 * simt_us("N", "T", 6000, 6000, 32)

@@ -583,25 +583,34 @@ void stored_b(const Gemm& g, int& rows, int& cols) {
   if (g.tb == 'N') { rows = g.K; cols = g.N; } else { rows = g.N; cols = g.K; }
 }
 
-// The producer-less kernel's tiles for an M x N output.  A wave of 128 x 128
-// tiles takes kNarrowCost of a wave of 128 x 256 tiles (97 and 174 us per 1024
-// k; without pairs there are no wide tiles).  Wide tiles fill whole waves of SMs;
-// what is left of them runs as narrow ones when those fit in one wave, and
-// everything runs narrow where that takes fewer waves' time (a right edge that
-// leaves half of the wide tiles empty).
-constexpr double kNarrowCost = 0.56, kMiddleCost = 0.78;  // 128 and 192 wide
-// 64 x 64 tiles, two CTAs to an SM: 69 us per 1024 k and round of two to an SM.
-constexpr double kSmallCost = 0.40, kSmallHalfCost = 0.29;
+// The producer-less kernel's tiles for an M x N output.  Costs in k of a full wave
+// of 128 x 256 tiles (174 us per 1024), K in whole stages: each width's share per k,
+// and what a wave takes beside (prologue, stores; less of it in the first wave, whose
+// stores go to L2), fitted to ten outputs at K = 8 to 1024.  Shallow products are bound by
+// the latter: 4096 x 4096 x 32 takes 47 us in 128 x 128 tiles and 56 in wide ones,
+// 6000 x 6000 x 32 101 and 129.  Without pairs there are no wide tiles.  Wide
+// tiles fill whole waves of SMs; what is left of them runs as narrow ones when
+// those fit in one wave, and everything runs narrow where that takes less time (a
+// right edge that leaves half of the wide tiles empty).
+constexpr double kWideFixed = 100, kWideFirst = 0.42;
+constexpr double kNarrowCost = 0.56, kNarrowFixed = 27.5;  // 128 wide
+constexpr double kMiddleCost = 0.78, kMiddleFixed = 55;  // 192 wide
+// 64 x 64 tiles, two CTAs to an SM: a round of two to an SM, or of one at most;
+// slower where both operands are k-contiguous (4096 x 4096 x 32: 84 us, 49 otherwise)
+constexpr double kSmallCost = 0.375, kSmallHalfCost = 0.29, kSmallFixed = 11.4;
+constexpr double kSmallCostNT = 0.40, kSmallFixedNT = 21.5;
 struct NpTiles {
   int width = 256;             // of the wide tiles
   int tiles_m = 0, tiles_n = 0, wide = 0;  // wide tiles, and how many run as such
-  double cost = 0;             // waves, in 256-wide tiles
+  double cost = 0;
 };
-NpTiles np_tiles(int M, int N, bool wide_ok, int sms) {
+NpTiles np_tiles(int M, int N, int K, bool wide_ok, int sms) {
+  K = cdiv(K, kBK) * kBK;
+  const double narrow = kNarrowCost * K + kNarrowFixed;  // a wave of 128 x 128 tiles
   NpTiles best;
   best.tiles_m = cdiv(M, 128);
   best.tiles_n = cdiv(N, 256);
-  best.cost = kNarrowCost * cdiv(best.tiles_m * cdiv(N, 128), sms);
+  best.cost = narrow * cdiv(best.tiles_m * cdiv(N, 128), sms);
   for (int width : {256, 192}) {
     if (!wide_ok) break;
     NpTiles t;
@@ -610,9 +619,11 @@ NpTiles np_tiles(int M, int N, bool wide_ok, int sms) {
     t.tiles_n = cdiv(N, width);
     const int total = t.tiles_m * t.tiles_n, rest = total % sms;
     const bool tail = rest > 0 && 2 * rest <= sms;
-    const double wave = width == 256 ? 1.0 : kMiddleCost;
+    const double fixed = width == 256 ? kWideFixed : kMiddleFixed;
+    const double wave = (width == 256 ? 1.0 : kMiddleCost) * K + fixed;
+    const int waves = total / sms + (rest > 0 && !tail ? 1 : 0);
     t.wide = tail ? total - rest : total;
-    t.cost = wave * (total / sms) + (rest == 0 ? 0.0 : tail ? kNarrowCost : wave);
+    t.cost = wave * waves + (tail ? narrow : 0.0) - (waves > 0 ? kWideFirst * fixed : 0.0);
     if (t.cost < best.cost) best = t;
   }
   return best;
@@ -651,7 +662,7 @@ ugemm_status launch_t(const Gemm& g, int tile, const float* A, int lda, const fl
   } else {
     using S = SimtShape<8, 16>;
     constexpr bool wide_ok = pair_of<AK, BKM>() != Pair::kNone;
-    NpTiles t = np_tiles(g.M, g.N, wide_ok, device_sms());
+    NpTiles t = np_tiles(g.M, g.N, g.K, wide_ok, device_sms());
     if (tile != kSimtMixed) {
       t.width = 256;
       t.tiles_n = cdiv(g.N, 256);
@@ -693,10 +704,13 @@ int simt_pick_tile(const Gemm& g) {
   // mixed, 464 in 64x64 tiles; 1024^3: 99 and 74)
   const int sms = device_sms();
   const long small = long(cdiv(g.M, 64)) * cdiv(g.N, 64);
-  const double small_cost =
-      small <= sms ? kSmallHalfCost : kSmallCost * ((small + 2 * sms - 1) / (2 * sms));
   const bool wide_ok = !(g.ta == 'N' && g.tb == 'T');
-  return np_tiles(g.M, g.N, wide_ok, sms).cost < small_cost ? kSimtMixed : kSimt64x64;
+  const double fixed = wide_ok ? kSmallFixed : kSmallFixedNT, k = cdiv(g.K, kBK) * kBK;
+  const double small_cost =
+      small <= sms ? kSmallHalfCost * k + fixed
+                   : ((wide_ok ? kSmallCost : kSmallCostNT) * k + fixed) *
+                         ((small + 2 * sms - 1) / (2 * sms));
+  return np_tiles(g.M, g.N, g.K, wide_ok, sms).cost < small_cost ? kSimtMixed : kSimt64x64;
 }
 
 ugemm_status simt_launch(const Gemm& g, int tile, Scratch ws, int* dev_err, cudaStream_t st) {
