@@ -132,3 +132,39 @@ def test_gemv_time_follows_the_size():
     times in eight warps each; 1.35 leaves room for the clock)."""
     assert gemv_us("N", 16384, 1024, 1) < 2 * gemv_us("N", 16384, 1024, 0)
     assert gemv_us("T", 2000, 100, 0) < 1.35 * gemv_us("T", 2600, 100, 0)
+
+
+@pytest.mark.parametrize("M,N", [(1, 1), (127, 8), (129, 3), (2432 * 128 + 4, 5), (2432 * 128 + 5, 8),
+                                 (33, 9), (9728, 96), (9732, 97), (19457, 31), (19456, 256),
+                                 (78000, 17), (77825, 255), (300, 257), (1, 256)])
+@pytest.mark.parametrize("pad", [0, 1, 4])
+def test_gemv_few_columns(M, N, pad):
+    """Threads with rows to themselves, and blocks of four to sixteen warps: the edges of
+    each, strided vectors, y updated or (NaN in it) not read.  The products' rounding and
+    a sum of N: within 2e-6 normwise, as elsewhere."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    lda, incx, incy = M + pad, 1 + pad % 3, 2
+    A = torch.rand((N, lda), device="cuda", generator=g) * 2 - 1
+    x = torch.rand((N * incx,), device="cuda", generator=g) + 0.5
+    y = torch.rand((M * incy,), device="cuda", generator=g)
+    ref = A[:, :M].double().T @ x[::incx].double()
+    z, old = torch.full_like(y, float("nan")), y.clone()
+    ug.sgemv("N", M, N, 1.5, A, lda, x, incx, 0.5, y, incy)
+    ug.sgemv("N", M, N, 1.0, A, lda, x, incx, 0.0, z, incy)
+    torch.cuda.synchronize()
+    assert float(torch.linalg.norm(z[::incy].double() - ref) / torch.linalg.norm(ref)) < 2e-6
+    want = 1.5 * ref + 0.5 * old[::incy].double()
+    assert float(torch.linalg.norm(y[::incy].double() - want) / torch.linalg.norm(want)) < 2e-6
+    assert torch.equal(y[1::incy], old[1::incy]) and bool(torch.isnan(z[1::incy]).all())
+
+
+def test_gemv_time_of_few_columns():
+    """One column is no more than a saxpy of as many elements (with eight warps to 32
+    rows 6 times that; 3 leaves room), and loads in flight do not cost the warps that
+    short columns live by: aligned ones take no longer than others (1.2 times with eight
+    16-byte loads), and 96 floats in four-byte loads 1.1 times the aligned ones (1.45 with
+    eight in flight)."""
+    x, y = torch.rand((1000000,), device="cuda"), torch.rand((1000000,), device="cuda")
+    assert gemv_us("N", 1000000, 1, 0) < 3 * graph_us(lambda: ug.saxpy(1000000, 0.5, x, 1, y, 1))
+    assert gemv_us("T", 144896, 416, 0) < 1.1 * gemv_us("T", 144896, 416, 1)
+    assert gemv_us("T", 94016, 96, 1) < 1.28 * gemv_us("T", 94016, 96, 0)

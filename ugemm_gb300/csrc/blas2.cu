@@ -41,15 +41,16 @@ __global__ void saxpy_kernel(int n, float alpha, const float* __restrict__ x, in
 // cluster of kGemvCluster blocks shares the columns of each, the sums passing
 // through distributed shared memory in rank order.
 constexpr int kGemvCluster = 8;
-template <int V, int W, int U>
+template <int V, int W, int U, bool CLUSTER>
 __global__ void __launch_bounds__(W * 32)
     sgemv_n_kernel(int M, int N, float alpha, const float* __restrict__ A, int lda,
                    const float* __restrict__ x, int incx, float beta, float* __restrict__ y,
-                   int incy, int share) {
+                   int incy, int cluster) {
+  const int share = CLUSTER ? cluster : 1;
   __shared__ float part[W][32 * V + 1];
   __shared__ float sum[32 * V];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int rank = share > 1 ? blockIdx.x % share : 0;
+  const int rank = CLUSTER ? blockIdx.x % share : 0;
   const int m0 = (blockIdx.x / share) * 32 * V, m = m0 + lane * V;
   const int step = W * share;
   float s[V];
@@ -66,17 +67,35 @@ __global__ void __launch_bounds__(W * 32)
         v[0] = *p;
       }
     };
+    // U columns' products: one after the other, or, where few warps make long
+    // chains, in pairs first
+    auto add = [&](const float (&v)[U][V], const float (&b)[U]) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        if constexpr (W >= 8) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) s[e] += v[u][e] * b[u];
+        } else {
+          float p[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) p[u] = v[u][e] * b[u];
+#pragma unroll
+          for (int d = U / 2; d > 0; d /= 2)
+#pragma unroll
+            for (int u = 0; u < d; ++u) p[u] += p[u + d];
+          s[e] += p[0];
+        }
+      }
+    };
     int n = w * share + rank;
     for (; n + (U - 1) * step < N; n += U * step) {
       float v[U][V];
 #pragma unroll
       for (int u = 0; u < U; ++u) load(n + u * step, v[u]);
+      float b[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float b = x[static_cast<long long>(n + u * step) * incx];
-#pragma unroll
-        for (int e = 0; e < V; ++e) s[e] += v[u][e] * b;
-      }
+      for (int u = 0; u < U; ++u) b[u] = x[static_cast<long long>(n + u * step) * incx];
+      add(v, b);
     }
     if (n < N) {  // fewer than U: together all the same, beyond N zeros
       float v[U][V];
@@ -86,12 +105,11 @@ __global__ void __launch_bounds__(W * 32)
         for (int e = 0; e < V; ++e) v[u][e] = 0.f;
         if (n + u * step < N) load(n + u * step, v[u]);
       }
+      float b[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float b = n + u * step < N ? x[static_cast<long long>(n + u * step) * incx] : 0.f;
-#pragma unroll
-        for (int e = 0; e < V; ++e) s[e] += v[u][e] * b;
-      }
+      for (int u = 0; u < U; ++u)
+        b[u] = n + u * step < N ? x[static_cast<long long>(n + u * step) * incx] : 0.f;
+      add(v, b);
     }
   }
 #pragma unroll
@@ -110,9 +128,9 @@ __global__ void __launch_bounds__(W * 32)
 #pragma unroll
       for (int j = 0; j < d; ++j) p[j] += p[j + d];
     t = p[0];
-    sum[r] = t;
+    if (CLUSTER) sum[r] = t;
   }
-  if (share > 1) {
+  if constexpr (CLUSTER) {
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
     if (rank == 0 && r < 32 * V) {
@@ -124,6 +142,52 @@ __global__ void __launch_bounds__(W * 32)
   if (rank == 0 && r < 32 * V && m0 + r < M) {
     float* yp = y + static_cast<long long>(m0 + r) * incy;
     *yp = (beta == 0.f) ? alpha * t : alpha * t + beta * *yp;
+  }
+}
+
+// The same for at most kGemvColumns columns: a thread has V rows to itself, all
+// its loads in flight, and adds the products in pairs.  Nothing is shared, so
+// the blocks are bound by the loads alone (1000000 x 1: 3.6 us, 21 where eight
+// warps share a block's rows; 100000 x 8: 1.8 and 4.2).
+constexpr int kGemvColumns = 8;
+template <int V>
+__global__ void __launch_bounds__(128)
+    sgemv_rows_kernel(int M, int N, float alpha, const float* __restrict__ A, int lda,
+                      const float* __restrict__ x, int incx, float beta, float* __restrict__ y,
+                      int incy) {
+  const long long m = (blockIdx.x * 128LL + threadIdx.x) * V;
+  if (m >= M) return;  // (V = 4: M is a multiple of 4)
+  float p[kGemvColumns][V];
+#pragma unroll
+  for (int n = 0; n < kGemvColumns; ++n) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) p[n][e] = 0.f;
+    if (n < N) {
+      const float* c = A + m + static_cast<long long>(n) * lda;
+      if constexpr (V == 4) {
+        const float4 q = __ldcs(reinterpret_cast<const float4*>(c));
+        p[n][0] = q.x; p[n][1] = q.y; p[n][2] = q.z; p[n][3] = q.w;
+      } else {
+        p[n][0] = __ldcs(c);
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < kGemvColumns; ++n) {
+    const float b = n < N ? x[static_cast<long long>(n) * incx] : 0.f;
+#pragma unroll
+    for (int e = 0; e < V; ++e) p[n][e] *= b;
+  }
+#pragma unroll
+  for (int d = kGemvColumns / 2; d > 0; d /= 2)
+#pragma unroll
+    for (int n = 0; n < d; ++n)
+#pragma unroll
+      for (int e = 0; e < V; ++e) p[n][e] += p[n + d][e];
+#pragma unroll
+  for (int e = 0; e < V; ++e) {
+    float* yp = y + (m + e) * incy;
+    *yp = (beta == 0.f) ? alpha * p[0][e] : alpha * p[0][e] + beta * *yp;
   }
 }
 
@@ -213,8 +277,15 @@ void launch_gemv_t(int M, int N, float alpha, const float* A, int lda, const flo
   const bool vec = (lda & 3) == 0 && incx == 1 &&
                    ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
   const int grid = cdiv(M, 8 / WPC);
-  auto kern = !vec ? (N <= 64 * WPC ? sgemv_t_kernel<WPC, false, 2> : sgemv_t_kernel<WPC, false, 8>)
-              : N <= 256 * WPC ? sgemv_t_kernel<WPC, true, 2> : sgemv_t_kernel<WPC, true, 8>;
+  // eight loads in flight leave fewer warps an SM: where one warp an output makes
+  // many blocks, two 16-byte ones are faster (144896 x 416: 43 us, 51); of four bytes
+  // as many as a short column has (94016 x 96: four 10.0 us, eight 13.1)
+  const bool many = grid > 5 * device_sms();
+  auto kern = vec ? sgemv_t_kernel<WPC, true, 8> : sgemv_t_kernel<WPC, false, 8>;
+  if constexpr (WPC == 1) {
+    if (vec && (N <= 256 || many)) kern = sgemv_t_kernel<1, true, 2>;
+    else if (!vec && N <= 96) kern = N <= 32 ? sgemv_t_kernel<1, false, 2> : sgemv_t_kernel<1, false, 4>;
+  }
   kern<<<grid, 256, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
 }
 
@@ -236,21 +307,45 @@ cudaError_t launch_gemv_nw(int M, int N, float alpha, const float* A, int lda, c
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = share > 1 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, sgemv_n_kernel<V, W, U>, M, N, alpha, A, lda, x, incx, beta, y, incy,
-                            share);
+  auto kern = share > 1 ? sgemv_n_kernel<V, W, U, true> : sgemv_n_kernel<V, W, U, false>;
+  return cudaLaunchKernelEx(&cfg, kern, M, N, alpha, A, lda, x, incx, beta, y, incy, share);
 }
 
-template <int V>
+// vec: 16-byte loads are possible.
 cudaError_t launch_gemv_n(int M, int N, float alpha, const float* A, int lda, const float* x,
-                          int incx, float beta, float* y, int incy, cudaStream_t st) {
-  const int rows = cdiv(M, 32 * V), sms = device_sms();
+                          int incx, float beta, float* y, int incy, bool vec, cudaStream_t st) {
+  const int sms = device_sms(), blocks = cdiv(M, 128);  // of 128 rows, by 16-byte loads
+  if (N <= kGemvColumns) {
+    if (vec && blocks >= 16 * sms)
+      sgemv_rows_kernel<4><<<cdiv(M, 512), 128, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
+    else
+      sgemv_rows_kernel<1><<<blocks, 128, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
+    return cudaPeekAtLastError();
+  }
+  if (N <= 256) {
+    // few columns: no clusters, whose barriers take longer than the columns (1312 x 160
+    // 2.3 us alone, 3.0 in twos); 16-byte loads where their blocks reach most SMs
+    // (16384 x 256 3.5 us, 4.5 without; 4096 x 256 3.3 and 2.6); fewer warps a block where
+    // there are many blocks, whose sums then cost more than the loads (100000 x 100 5.1
+    // us in fours, 6.0 in sixteens; 134571 x 48, unaligned, 6.6 and 13.8; 952 x 32 1.45 in
+    // eights, 1.69)
+    if (vec && blocks >= 4 * sms)
+      return launch_gemv_nw<4, 4, 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
+    if (vec && 2 * blocks >= sms)
+      return launch_gemv_nw<4, 16, 4>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
+    if (blocks >= sms)
+      return launch_gemv_nw<1, 4, 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
+    if (N <= 96)
+      return launch_gemv_nw<1, 8, 4>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
+    return launch_gemv_nw<1, 16, 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
+  }
+  const bool wide = vec && M >= 512;
+  const int rows = wide ? blocks : cdiv(M, 32);
   int share = kGemvCluster;
   while (share > 1 && (2LL * rows * share > 5LL * sms || N < 64 * share)) share /= 2;
-  // few columns of many rows: 8 warps a block, whose sums are half the work
-  // (40000 x 64, unaligned: 5.4 us with 16, 3.6)
-  if (V == 1 && N <= 256 && rows >= 4 * sms)
-    return launch_gemv_nw<1, 8, 4>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
-  return launch_gemv_nw<V, 16, V == 4 ? 4 : 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, share, st);
+  if (wide)
+    return launch_gemv_nw<4, 16, 4>(M, N, alpha, A, lda, x, incx, beta, y, incy, share, st);
+  return launch_gemv_nw<1, 16, 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, share, st);
 }
 
 }  // namespace
@@ -284,14 +379,10 @@ UGEMM_API int ugemm_sgemv(char trans, int M, int N, float alpha, const float* A,
   if (!y || (N > 0 && (!A || !x))) return UGEMM_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   prof_begin(st);
-  // 16-byte loads, but where columns are few and blocks of 32 rows share the SMs more
-  // evenly than blocks of 128 (100000 x 100: 8.1 us, 8.7)
-  const bool even = N <= 256 && cdiv(M, 128) >= 4 * device_sms();
-  if (!t && ((M | lda) & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && M >= 512 && !even)
-    (void)launch_gemv_n<4>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
-  else if (!t)
-    (void)launch_gemv_n<1>(M, N, alpha, A, lda, x, incx, beta, y, incy, st);
-  else {
+  if (!t) {
+    const bool vec = ((M | lda) & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    (void)launch_gemv_n(M, N, alpha, A, lda, x, incx, beta, y, incy, vec, st);
+  } else {
     // warps an output: one up to 2048 long where the outputs fill the SMs, and up to
     // 1024 where they do not, so that no thread has fewer than 16 products and its
     // share of the tree (2000 x 100: 3.3 us in eights, 1.9)
