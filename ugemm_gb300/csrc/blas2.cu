@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "internal.h"
 
@@ -33,6 +34,28 @@ __global__ void saxpy_kernel(int n, float alpha, const float* __restrict__ x, in
   for (; i < n; i += stride) y[i * incy] += alpha * x[i * incx];
 }
 
+// Four floats of A.  A matrix that L2 cannot hold streams past what it does
+// hold (8192 x 8192: 41 us, 43 without); a smaller one stays for the next call, which
+// finds it there (16384 x 1024 transposed: 8.2 us, 14.4 when it may not stay).
+template <bool STREAM>
+__device__ __forceinline__ float4 load_a4(const float4* p) {
+  return STREAM ? __ldcs(p) : __ldg(p);
+}
+
+// Whether A is larger than the current device's L2 (looked up once per device).
+bool beyond_l2(int M, int N) {
+  static std::atomic<int> cached[64];
+  int dev = 0, bytes = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  bytes = cached[dev].load(std::memory_order_relaxed);
+  if (bytes == 0) {
+    if (cudaDeviceGetAttribute(&bytes, cudaDevAttrL2CacheSize, dev) != cudaSuccess || bytes <= 0)
+      return false;
+    cached[dev].store(bytes, std::memory_order_relaxed);
+  }
+  return 4LL * M * N > bytes;
+}
+
 // 'N': A is column-major M x N (A[m + n*lda]); y[m] = alpha * sum_n A[m,n] x[n]
 // + beta * y[m].  A block owns 32 V rows (V = 4: 16-byte loads, 512 bytes of a
 // column at a time); its W warps take every Wth column, U loads in flight
@@ -41,7 +64,7 @@ __global__ void saxpy_kernel(int n, float alpha, const float* __restrict__ x, in
 // cluster of kGemvCluster blocks shares the columns of each, the sums passing
 // through distributed shared memory in rank order.
 constexpr int kGemvCluster = 8;
-template <int V, int W, int U, bool CLUSTER>
+template <int V, int W, int U, bool CLUSTER, bool STREAM>
 __global__ void __launch_bounds__(W * 32)
     sgemv_n_kernel(int M, int N, float alpha, const float* __restrict__ A, int lda,
                    const float* __restrict__ x, int incx, float beta, float* __restrict__ y,
@@ -61,7 +84,7 @@ __global__ void __launch_bounds__(W * 32)
     auto load = [&](int n, float (&v)[V]) {
       const float* p = col + static_cast<long long>(n) * lda;
       if constexpr (V == 4) {
-        const float4 q = __ldcs(reinterpret_cast<const float4*>(p));
+        const float4 q = load_a4<STREAM>(reinterpret_cast<const float4*>(p));
         v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
       } else {
         v[0] = *p;
@@ -165,10 +188,10 @@ __global__ void __launch_bounds__(128)
     if (n < N) {
       const float* c = A + m + static_cast<long long>(n) * lda;
       if constexpr (V == 4) {
-        const float4 q = __ldcs(reinterpret_cast<const float4*>(c));
+        const float4 q = load_a4<false>(reinterpret_cast<const float4*>(c));
         p[n][0] = q.x; p[n][1] = q.y; p[n][2] = q.z; p[n][3] = q.w;
       } else {
-        p[n][0] = __ldcs(c);
+        p[n][0] = *c;
       }
     }
   }
@@ -197,7 +220,7 @@ __global__ void __launch_bounds__(128)
 // bytes; reduced by a fixed tree.  HBM-bound (8192 x 8192: one scalar
 // load in flight 53 us, 5.1 TB/s; now 41); short columns by the loads' latency
 // and the warps in flight, which U = 8 halves.
-template <int WPC, bool VEC, int U>
+template <int WPC, bool VEC, int U, bool STREAM>
 __global__ void __launch_bounds__(256) sgemv_t_kernel(int M, int N, float alpha,
                                                       const float* __restrict__ A, int lda,
                                                       const float* __restrict__ x, int incx,
@@ -221,14 +244,14 @@ __global__ void __launch_bounds__(256) sgemv_t_kernel(int M, int N, float alpha,
       for (; i + (U - 1) * T < n4; i += U * T) {
         float4 v[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = __ldcs(c4 + i + u * T);
+        for (int u = 0; u < U; ++u) v[u] = load_a4<STREAM>(c4 + i + u * T);
 #pragma unroll
         for (int u = 0; u < U; ++u) add(v[u], x4[i + u * T]);
       }
       if constexpr (U <= 2) {
-        if (i < n4) add(__ldcs(c4 + i), x4[i]);
+        if (i < n4) add(load_a4<STREAM>(c4 + i), x4[i]);
       } else {
-        for (; i < n4; i += T) add(c4[i], x4[i]);
+        for (; i < n4; i += T) add(load_a4<STREAM>(c4 + i), x4[i]);
       }
       for (int n = 4 * n4 + t; n < N; n += T) s += col[n] * x[n];
     } else {
@@ -281,10 +304,15 @@ void launch_gemv_t(int M, int N, float alpha, const float* A, int lda, const flo
   // many blocks, two 16-byte ones are faster (144896 x 416: 43 us, 51); of four bytes
   // as many as a short column has (94016 x 96: four 10.0 us, eight 13.1)
   const bool many = grid > 5 * device_sms();
-  auto kern = vec ? sgemv_t_kernel<WPC, true, 8> : sgemv_t_kernel<WPC, false, 8>;
+  const bool stream = vec && beyond_l2(M, N);
+  auto kern = stream ? sgemv_t_kernel<WPC, true, 8, true>
+              : vec  ? sgemv_t_kernel<WPC, true, 8, false>
+                     : sgemv_t_kernel<WPC, false, 8, false>;
   if constexpr (WPC == 1) {
-    if (vec && (N <= 256 || many)) kern = sgemv_t_kernel<1, true, 2>;
-    else if (!vec && N <= 96) kern = N <= 32 ? sgemv_t_kernel<1, false, 2> : sgemv_t_kernel<1, false, 4>;
+    if (vec && (N <= 256 || many))
+      kern = stream ? sgemv_t_kernel<1, true, 2, true> : sgemv_t_kernel<1, true, 2, false>;
+    else if (!vec && N <= 96)
+      kern = N <= 32 ? sgemv_t_kernel<1, false, 2, false> : sgemv_t_kernel<1, false, 4, false>;
   }
   kern<<<grid, 256, 0, st>>>(M, N, alpha, A, lda, x, incx, beta, y, incy);
 }
@@ -307,7 +335,10 @@ cudaError_t launch_gemv_nw(int M, int N, float alpha, const float* A, int lda, c
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = share > 1 ? 1 : 0;
-  auto kern = share > 1 ? sgemv_n_kernel<V, W, U, true> : sgemv_n_kernel<V, W, U, false>;
+  auto kern = share > 1 ? sgemv_n_kernel<V, W, U, true, false> : sgemv_n_kernel<V, W, U, false, false>;
+  if constexpr (V == 4)
+    if (beyond_l2(M, N))
+      kern = share > 1 ? sgemv_n_kernel<4, W, U, true, true> : sgemv_n_kernel<4, W, U, false, true>;
   return cudaLaunchKernelEx(&cfg, kern, M, N, alpha, A, lda, x, incx, beta, y, incy, share);
 }
 
