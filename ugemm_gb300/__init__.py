@@ -199,8 +199,12 @@ def _stream_ptr(stream) -> int:
     if _raw_stream is None:
         import torch
         torch.cuda.init()
-        _raw_stream = (torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice)
-    return _raw_stream[0](_raw_stream[1]())  # without a Stream object on the way
+        try:  # without a Stream object on the way (not in torch's public interface)
+            raw, device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+            _raw_stream = lambda: raw(device())  # noqa: E731
+        except AttributeError:
+            _raw_stream = lambda: torch.cuda.current_stream().cuda_stream  # noqa: E731
+    return _raw_stream()
 
 
 _raw_stream = None
