@@ -687,8 +687,10 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   std::stable_sort(subs.begin(), subs.end(), [](const Sub& a, const Sub& b) { return a.nkb > b.nkb; });
 
   const bool conv = !simt && p->split.conv;
-  std::vector<CUtensorMap> maps((conv ? 4 : 2) * subs.size());
+  const size_t nm = conv ? 4 : 2;  // maps of a kernel problem, the same for all slices of one product
+  std::vector<CUtensorMap> maps(nm * subs.size());
   std::vector<ConvGeo> cgeo(conv ? subs.size() : 0);
+  std::vector<int> mapped(count, -1);  // the kernel problem that has a product's maps already
   std::vector<TcProblem> tprobs;
   std::vector<SimtProblem> sprobs;
   std::vector<ReduceJob> rjobs;
@@ -708,12 +710,16 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
     const float beta = sliced ? 0.f : x.beta;
     const Epilogue epi = sliced ? Epilogue{} : x.epi;
     any_epi |= epi.bias != nullptr || epi.act != 0;
-    bool ok;
+    bool ok = true;
+    const int same = mapped[u.j];
+    if (same < 0) mapped[u.j] = static_cast<int>(i);
+    else std::copy_n(maps.begin() + nm * same, nm, maps.begin() + nm * i);
     if (simt) {
       const float* da = reinterpret_cast<const float*>(base + a_off[u.j]);
       const float* db = reinterpret_cast<const float*>(base + b_off[u.j]);
-      ok = simt_encode_grouped(bn == 64 ? kSimt64x64 : kSimt128x128, da, x.M, db, x.N, x.K,
-                               ld_a[u.j], ld_b[u.j], &maps[2 * i], &maps[2 * i + 1]);
+      if (same < 0)
+        ok = simt_encode_grouped(bn == 64 ? kSimt64x64 : kSimt128x128, da, x.M, db, x.N, x.K,
+                                 ld_a[u.j], ld_b[u.j], &maps[2 * i], &maps[2 * i + 1]);
       SimtProblem sp{target, x.M, x.N, ldt, x.alpha, beta, u.nkb, cdiv(x.M, bn), cdiv(x.N, bn),
                      tiles, epi};
       sp.kt0 = u.kb0;
@@ -721,7 +727,11 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
       sprobs.push_back(sp);
     } else {
       TcProblem tp{};
-      if (conv) {
+      if (same >= 0) {
+        if (conv) cgeo[i] = cgeo[same];
+        tp.kc_a = tprobs[same].kc_a;
+        tp.kc_b = tprobs[same].kc_b;
+      } else if (conv) {
         ok = conv_encode_maps(*x.pieces, x.M, ncols, bn, o.swap, &maps[4 * i], &cgeo[i]);
       } else if (p->split.fused) {
         ok = fused_encode_problem(x, o.swap, bn, &maps[2 * i], &tp);
