@@ -615,17 +615,17 @@ int ugemm_sgemm_dev_ex(char major, char transa, char transb, int M, int N, int K
 size_t ugemm_workspace_bytes(char major, char transa, char transb, int M, int N, int K, int lda,
                              int ldb, int precision) {
   Gemm g;
-  // Pointers only matter for alignment: assume aligned device buffers, but
-  // enough for the split forms' route on others too (the operands of unaligned
-  // buffers are not split inside the GEMM kernel).
-  static float dummy[8] __attribute__((aligned(16)));
-  if (make_gemm(major, transa, transb, M, N, K, 1.f, dummy, lda, dummy, ldb, 0.f, dummy,
+  // Pointers only matter for alignment and for sharing memory: assume aligned
+  // buffers apart from each other, but enough for the split forms' route on others
+  // too (whose operands are not split inside the GEMM kernel).
+  auto at = [](uintptr_t i) { return reinterpret_cast<float*>(i << 48); };
+  if (make_gemm(major, transa, transb, M, N, K, 1.f, at(1), lda, at(2), ldb, 0.f, at(3),
                 (major == 'R' || major == 'r') ? N : M, &g) != UGEMM_OK)
     return 0;
   const int form = resolve_form(precision, g);
   const size_t aligned = scratch_for(g, form);
   if (!is_split_form(form)) return aligned;
-  g.A = g.B = dummy + 1;
+  g.A = at(1) + 1;
   return std::max(aligned, scratch_for(g, form));
 }
 

@@ -19,6 +19,7 @@
 #include <cstdio>
 #include <cstring>
 #include <numeric>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -273,6 +274,34 @@ bool fusable(const Gemm& x) {
   return ok(x.A, a_sr, a_sk) && ok(x.B, b_sr, b_sk);
 }
 
+// A launch on pieces has read every operand before it writes any C; a fused one
+// reads them while it writes, so not for a product into (or beside) its own operand.
+bool writes_operands(const Gemm* gs, int n) {
+  using Span = std::pair<uintptr_t, uintptr_t>;  // [first, last byte]
+  auto span = [](const float* p, int rows, int cols, int ld) {
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(p);
+    return Span{lo, lo + (size_t(std::max(rows, 1) - 1) * ld + std::max(cols, 1)) * 4 - 1};
+  };
+  std::vector<Span> written(n);
+  for (int i = 0; i < n; ++i) written[i] = span(gs[i].C, gs[i].M, gs[i].N, gs[i].ldc);
+  std::sort(written.begin(), written.end());
+  for (int i = 1; i < n; ++i)  // the furthest end so far
+    written[i].second = std::max(written[i].second, written[i - 1].second);
+  auto hit = [&](const Span& r) {
+    auto it = std::upper_bound(written.begin(), written.end(), r.second,
+                               [](uintptr_t v, const Span& w) { return v < w.first; });
+    return it != written.begin() && std::prev(it)->second >= r.first;
+  };
+  for (int i = 0; i < n; ++i) {
+    const Gemm& g = gs[i];
+    const bool ta = g.ta != 'N', tb = g.tb != 'N';
+    if (hit(span(g.A, ta ? g.K : g.M, ta ? g.M : g.K, g.lda)) ||
+        hit(span(g.B, tb ? g.N : g.K, tb ? g.K : g.N, g.ldb)))
+      return true;
+  }
+  return false;
+}
+
 bool fused_encode_problem(const Gemm& x, bool swap, int bn, CUtensorMap* maps, TcProblem* tp) {
   // operand a is op(B)^T when the problem is computed transposed
   long long a_sr, a_sk, b_sr, b_sk;
@@ -469,7 +498,8 @@ ugemm_status grouped_plan_build(const Gemm* gs, int count, int form,
   // for a million elements split beforehand).  256-problem group: 135 and 222 us;
   // 4096^3: 0.81 and 0.54 ms.
   if (!config && form != UGEMM_PREC_SIMT && split_plan_for(form, g[0]).pieces == 3 &&
-      g[0].block_n == 0 && std::all_of(g.begin(), g.end(), fusable)) {
+      g[0].block_n == 0 && std::all_of(g.begin(), g.end(), fusable) &&
+      !writes_operands(g.data(), count)) {
     double fused = 0, whole = 5, elements = 0;
     for (const Gemm& x : g) {
       const int nkb = split_nkb(3, x.K);

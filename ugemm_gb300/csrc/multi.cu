@@ -104,7 +104,7 @@ MultiLayout multi_layout(const Gemm* gs, int n, const SplitPlan& p, bool whole_k
     // the pieces' traffic (16 bytes an element) against slower stages: fused
     // where one side of the output is short
     L.us += split_pass_us((double(gs[0].M) + gs[0].N) * gs[0].K);
-    if (p.pieces == 3 && p.products == 6 && fusable(gs[0])) {
+    if (p.pieces == 3 && p.products == 6 && fusable(gs[0]) && !writes_operands(gs, 1)) {
       GeoChoice c;
       c.us = fused_us(gs[0], sms, &c.swap, &c.slices, slices, longest);
       if (c.us < L.us) {

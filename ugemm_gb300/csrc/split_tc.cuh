@@ -272,6 +272,8 @@ double fused_us(const Gemm& g, double share, bool* swap, int* slices, int max_sl
 double split_pass_us(double elements);
 // Whether a fused launch can copy the operands.
 bool fusable(const Gemm& g);
+// Whether some C shares memory with an operand.
+bool writes_operands(const Gemm* gs, int n);
 // The raw-tile maps and layouts of a fused problem.
 bool fused_encode_problem(const Gemm& g, bool swap, int block_n, CUtensorMap* maps, TcProblem* p);
 
