@@ -245,7 +245,9 @@ typedef struct {
                     pre-pass launch writes the pieces first.  Taken only when
                     every problem has k > 0, unit-stride operands and 16-byte aligned bases
                     and leading dimensions (implicit im2col operands take the pre-pass);
-                    the plan's config reports whether it was */
+                    the plan's config reports whether it was.  Reads operands while it
+                    writes: not for a C that shares memory with an operand (a plan without
+                    a configuration sees to that) */
 } ugemm_tile_config;
 
 typedef struct ugemm_grouped_plan_s ugemm_grouped_plan;

@@ -391,7 +391,7 @@ UGEMM_API int ugemm_saxpy(int N, float alpha, const float* x, int incx, float* y
   if (N < 0 || incx <= 0 || incy <= 0) return UGEMM_ERR_ARG;
   if (N == 0) return UGEMM_OK;
   if (!x || !y) return UGEMM_ERR_ARG;
-  const int grid = static_cast<int>(std::min<long long>((N + 1023) / 1024, 152LL * 16));
+  const int grid = static_cast<int>(std::min<long long>((N + 1023) / 1024, 16LL * device_sms()));
   prof_begin(static_cast<cudaStream_t>(stream));
   saxpy_kernel<<<std::max(grid, 1), 256, 0, static_cast<cudaStream_t>(stream)>>>(N, alpha, x, incx,
                                                                                 y, incy);

@@ -214,7 +214,7 @@ ugemm_status col2im_launch(const float* col, int C, int B, int H, int W, int k, 
   prof_begin(st);
   if (k == 3 && stride == 2 && pad == 1 && blocks <= 0x7fffffffLL) {
     const uint32_t bw = (W + 1) / 2, bhbw = (H + 1) / 2 * bw;
-    col2im_3x3s2_kernel<<<static_cast<unsigned>(std::min<long long>((blocks + 255) / 256, 152 * 32)),
+    col2im_3x3s2_kernel<<<static_cast<unsigned>(std::min<long long>((blocks + 255) / 256, 32 * device_sms())),
                           256, 0, st>>>(col, blocks, B, H, W, Ho, Wo, FastDiv(bw), FastDiv(bhbw),
                                         dx);
   } else if (k == 3 && stride == 1)

@@ -145,7 +145,7 @@ __device__ __forceinline__ void splitk_reduce_taps(const ReduceJob& J, float* bu
 
 __device__ __forceinline__ void splitk_reduce_job(const ReduceJob& J) {
   __shared__ float sums[4][256];
-  // (with too few such blocks to fill the SMs, as for a 64 x 576 gradient of 30
+  // (with fewer such blocks than two an SM, as for a 64 x 576 gradient of 30
   // slices, the groups of slices above are faster: 4 us against 8)
   if (J.kk > 0 && J.kk <= kReduceTaps && J.M * ((J.chans + 63) / 64) >= 304) {
     static_assert(64 * kReduceTaps <= 4 * 256, "shared buffer");

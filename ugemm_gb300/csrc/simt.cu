@@ -3,8 +3,11 @@
 // Replaces the reference's OpenCL gemm_rnn (sgemm_ocl2.h:17-90: 16x16 tile,
 // one output per work-item, two local-memory loads per FMA) and its separate
 // transpose pass (sgemm_ocl2.h:95-128, :180-199).  Here:
-//   * one CTA computes a BM x BN tile of C; 8 consumer warps (16 x 16 threads)
-//     each hold a TM x TN register block; a ninth warp is the TMA producer;
+//   * one CTA computes a tile of C: 128 x 256 or 128 x 192 (8 x 16 or 8 x 12
+//     registers of a thread, packed FP32 FMAs), 128 x 128 for the columns and the
+//     last wave that those leave, or 64 x 64 for small outputs (np_tiles,
+//     simt_pick_tile); 16 x 16 compute threads, whose thread 0 issues the copies
+//     (64 x 64 and grouped tiles: a ninth warp does);
 //   * A and B k-slices (BK = 32) are staged by TMA into a 4-deep shared-memory
 //     ring guarded by mbarriers; k-contiguous tiles use the 128-byte swizzle
 //     so the float4 fragment reads are bank-conflict free;

@@ -2185,11 +2185,14 @@ std::vector<int4> split_tile_table(const TcProblem* probs, int nprob, int block_
 // Microseconds of one pipeline stage (a 32-deep k-block) of a tile, and of what
 // a tile costs beyond its stages (filling the pipeline, the last drain, and the
 // stores as far as the next tile's MMAs do not hide them: narrower tiles have a
-// second set of accumulators).  Measured on GB300 with all SMs busy; the 64-wide
-// stage is bound by its 36 KB of copies, the others by their MMAs.
+// second set of accumulators).  BF16x6's, measured on GB300 with all SMs busy; the
+// 64-wide stage is bound by its 36 KB of copies, the others by their MMAs.  They serve
+// the other forms too: with those forms' own (BF16x9 1.2 to 1.4 times as long, TF32x3
+// 1.25, two 16-bit pieces 0.6 and 0.8) 2700 products, groups and stacks took 0.999 of
+// the time, and FP16x3's single products 1.016.
 double stage_us(int pieces, int bn) {
   const double w = bn == 256 ? 0.80 : bn == 128 ? 0.64 : 0.30;
-  return pieces == 2 ? w / 2 : w;  // three products instead of six
+  return pieces == 2 ? w / 2 : w;
 }
 double tile_us(int bn) { return bn == 256 ? 3.0 : bn == 128 ? 1.5 : 1.2; }
 
