@@ -247,3 +247,57 @@ def test_slices_share_their_products_maps(prec, align):
     for C, ref, _, _ in keep:
         assert float(torch.linalg.norm(C.double() - ref) / torch.linalg.norm(ref)) < 2e-6
     p.close()
+
+
+def test_reduce_of_odd_columns_is_short():
+    """Eight and more slices of a large output whose rows are no multiple of four columns:
+    the call takes no more than 1.1 times one of two columns more (1.2 where four groups of
+    threads share the slices, a column a thread)."""
+    M, K = 480, 8000
+    us, e = [], [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+    for N in (3534, 3536):
+        A, B = torch.rand((M, K), device="cuda") - 0.5, torch.rand((K, N), device="cuda") - 0.5
+        C = torch.empty((M, N), device="cuda")
+        best = 1e9
+        for _ in range(8):
+            e[0].record()
+            for _ in range(10):
+                ug.gemm(A, B, C, precision="bf16x6")
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        us.append(best)
+        ref = A.double() @ B.double()
+        assert float(torch.linalg.norm(C.double() - ref) / torch.linalg.norm(ref)) < 2e-6
+    assert us[0] < 1.1 * us[1]
+
+
+@pytest.mark.parametrize("M,N", [(64, 1), (32, 2), (52, 3), (4, 3), (96, 70), (101, 71), (255, 257),
+                                 (260, 1030), (300, 2001)])
+@pytest.mark.parametrize("prec", ["bf16x6", "fp16x3", "simt"])
+def test_reduce_rows_of_any_length(M, N, prec):
+    """k slices of outputs whose rows are and are not multiples of four columns, added to a
+    padded C with bias and LeakyReLU: a plan, and single calls in the forms that slice them
+    (SIMT's have one chain of all k), within 2e-6 of FP64."""
+    K = 12000
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    A = torch.rand((M, K), device="cuda", generator=g) - 0.5
+    B = torch.rand((K, N), device="cuda", generator=g) - 0.5
+    bias = torch.rand((M,), device="cuda", generator=g) - 0.5
+    C0 = torch.rand((M, N + 1), device="cuda", generator=g)
+    ref = 1.5 * (A.double() @ B.double()) + 0.5 * C0[:, :N].double() + bias.double()[:, None]
+    ref = torch.where(ref > 0, ref, ref * 0.1)
+    two = C0.clone()
+    outs = [two]
+    if prec != "simt":
+        outs.append(C0.clone())
+        ug.gemm_ex(A, B, outs[1][:, :N], bias=bias, act=1, slope=0.1, alpha=1.5, beta=0.5,
+                   precision=prec)
+    p = ug.GroupedPlan([dict(ta="N", tb="N", M=M, N=N, K=K, alpha=1.5, beta=0.5, A=A, lda=K, B=B,
+                             ldb=N, C=two, ldc=N + 1, bias=bias, act=1, slope=0.1)], precision=prec)
+    p.run()
+    p.check()
+    for out in outs:
+        assert float(torch.linalg.norm(out[:, :N].double() - ref) / torch.linalg.norm(ref)) < 2e-6
+        assert torch.equal(out[:, N], C0[:, N])
+    p.close()

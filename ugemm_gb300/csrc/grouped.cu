@@ -30,20 +30,23 @@ namespace ugemm {
 namespace {
 
 // Split-K reduction: C = sum_s part_s + beta*C (C not read when beta == 0),
-// then the optional bias / activation; slices summed in a fixed order.  Partial
-// tiles whose columns are (tap, channel) are read in their own order and
-// written in C's (channel, tap).  HBM- (or L2-) bound where the output is large:
-// four columns a thread, several slices in flight.  A small output of many
-// slices (a weight gradient) is bound by the loads' latency: there four groups
-// of threads take a quarter of the slices each, added in group order.
+// then the optional bias / activation; slices summed in a fixed order, eight or more
+// in four quarters.  Partial tiles whose columns are (tap, channel) are read in their
+// own order and written in C's (channel, tap).  HBM- (or L2-) bound where the output
+// is large: four columns a thread, four slices in flight.  A small output of many
+// slices (a weight gradient) is bound by the loads' latency: there four groups of
+// threads take a quarter each.  (The line: 256 x 256 of 13 slices takes 3.2 us
+// either way, of 64 4.3 in groups and 6.7 without; 1024 x 1024 of 13 11.2 and 6.8;
+// 480 x 3534 of 8, 35 in groups and a column a thread, 8.9.)
 template <int V>
 __device__ __forceinline__ void splitk_reduce_body(const ReduceJob& J, float (*sums)[256]) {
   const int pn = J.kk > 0 ? J.kk * J.cpad : J.N;  // columns of a partial tile
   const long long mn = static_cast<long long>(J.M) * pn;
-  const int groups = J.slices >= 8 ? 4 : 1, cols = 256 / groups;  // threads along the columns
+  const int quarters = J.slices >= 8 ? 4 : 1, per = (J.slices + quarters - 1) / quarters;
+  const int groups = quarters == 4 && mn <= 2500LL * V * J.slices ? 4 : 1;
+  const int cols = 256 / groups;  // threads along the columns
   const int g = threadIdx.x / cols, t = threadIdx.x % cols;
-  const int per = (J.slices + groups - 1) / groups;
-  const int s0 = g * per, s1 = min(J.slices, s0 + per);
+  const int s0 = g * per, s1 = groups > 1 ? min(J.slices, s0 + per) : J.slices;
   const long long step = static_cast<long long>(cols) * V * gridDim.x;
   for (long long base = static_cast<long long>(blockIdx.x) * cols * V; base < mn; base += step) {
     const long long i = base + t * V;
@@ -52,16 +55,49 @@ __device__ __forceinline__ void splitk_reduce_body(const ReduceJob& J, float (*s
 #pragma unroll
     for (int e = 0; e < V; ++e) v[e] = 0.f;
     if (ok) {
+      constexpr int U = 4;  // slices in flight
       const float* p = J.part + s0 * mn + i;
-#pragma unroll 4
-      for (int s = s0; s < s1; ++s, p += mn) {
-        if constexpr (V == 4) {
-          const float4 x = *reinterpret_cast<const float4*>(p);
-          v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-        } else {
-          v[0] += *p;
+      float a[V];  // a quarter's sum
+#pragma unroll
+      for (int e = 0; e < V; ++e) a[e] = 0.f;
+      int left = per;
+      auto next = [&](const float (&x)[V]) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) a[e] += x[e];
+        if (--left == 0) {
+          left = per;
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            v[e] += a[e];
+            a[e] = 0.f;
+          }
         }
+      };
+      auto load = [&](float (&x)[V]) {
+        if constexpr (V == 4) {
+          const float4 q = *reinterpret_cast<const float4*>(p);
+          x[0] = q.x; x[1] = q.y; x[2] = q.z; x[3] = q.w;
+        } else {
+          x[0] = *p;
+        }
+        p += mn;
+      };
+      int s = s0;
+      for (; s + U <= s1; s += U) {
+        float x[U][V];
+#pragma unroll
+        for (int u = 0; u < U; ++u) load(x[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) next(x[u]);
       }
+#pragma unroll 1
+      for (; s < s1; ++s) {
+        float x[V];
+        load(x);
+        next(x);
+      }
+#pragma unroll
+      for (int e = 0; e < V; ++e) v[e] += a[e];
     }
     if (groups > 1) {
 #pragma unroll
@@ -84,15 +120,15 @@ __device__ __forceinline__ void splitk_reduce_body(const ReduceJob& J, float (*s
       n = c * J.kk + tap;
       stride = J.kk;
     }
-    float* cp = J.C + static_cast<long long>(m) * J.ldc + n;
-    const float bias = J.epi.bias ? J.epi.bias[m] : 0.f;
     if constexpr (V == 4) {
-      if (stride == 1 && (J.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(J.C) & 15) == 0) {
+      if (stride == 1 && ((pn | J.ldc) & 3) == 0 && (reinterpret_cast<uintptr_t>(J.C) & 15) == 0) {
+        float* cp = J.C + static_cast<long long>(m) * J.ldc + n;
         if (J.beta != 0.f) {
           const float4 o = *reinterpret_cast<const float4*>(cp);
           v[0] += J.beta * o.x; v[1] += J.beta * o.y; v[2] += J.beta * o.z; v[3] += J.beta * o.w;
         }
         if (J.epi.bias || J.epi.act) {
+          const float bias = J.epi.bias ? J.epi.bias[m] : 0.f;
 #pragma unroll
           for (int e = 0; e < 4; ++e) v[e] = epilogue_value(v[e], bias, J.epi);
         }
@@ -100,15 +136,17 @@ __device__ __forceinline__ void splitk_reduce_body(const ReduceJob& J, float (*s
         continue;
       }
     }
-    float old[V];
-#pragma unroll
-    for (int e = 0; e < V; ++e)
-      old[e] = J.beta != 0.f && n + e * stride < J.N ? cp[e * stride] : 0.f;
 #pragma unroll
     for (int e = 0; e < V; ++e) {
-      if (J.beta != 0.f) v[e] += J.beta * old[e];
-      if (J.epi.bias || J.epi.act) v[e] = epilogue_value(v[e], bias, J.epi);
-      if (n + e * stride < J.N) cp[e * stride] = v[e];
+      int me = m, ne = n + e * stride;
+      if (V == 4 && J.kk == 0)  // rows of any length: the four may end in the next ones
+        for (; ne >= J.N; ne -= J.N) ++me;
+      if (ne >= J.N) break;  // channels that pad the last tap's
+      float* cp = J.C + static_cast<long long>(me) * J.ldc + ne;
+      if (J.beta != 0.f) v[e] += J.beta * *cp;
+      if (J.epi.bias || J.epi.act)
+        v[e] = epilogue_value(v[e], J.epi.bias ? J.epi.bias[me] : 0.f, J.epi);
+      *cp = v[e];
     }
   }
 }
@@ -152,9 +190,11 @@ __device__ __forceinline__ void splitk_reduce_job(const ReduceJob& J) {
     splitk_reduce_taps(J, &sums[0][0]);
     return;
   }
-  // four columns at a time: a row's columns and the partial tiles' 16-byte
-  // alignment allow it (a tap's channels are a multiple of 64)
-  if (((J.kk > 0 ? J.cpad : J.N) & 3) == 0 && (reinterpret_cast<uintptr_t>(J.part) & 15) == 0)
+  // four columns at a time: the partial tiles' sizes and 16-byte alignment allow it (a
+  // tap's channels are a multiple of 64; rows of any length follow one another:
+  // 480 x 3534 of 8 slices a column at a time 14.8 us)
+  const long long unit = J.kk > 0 ? J.cpad : static_cast<long long>(J.M) * J.N;
+  if ((unit & 3) == 0 && (reinterpret_cast<uintptr_t>(J.part) & 15) == 0)
     splitk_reduce_body<4>(J, sums);
   else
     splitk_reduce_body<1>(J, sums);
