@@ -366,8 +366,10 @@ cudaError_t launch_gemv_n(int M, int N, float alpha, const float* A, int lda, co
       return launch_gemv_nw<4, 16, 4>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
     if (blocks >= sms)
       return launch_gemv_nw<1, 4, 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
-    if (N <= 96)
+    if (N <= 32 || (N <= 96 && 2 * blocks >= sms))
       return launch_gemv_nw<1, 8, 4>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
+    if (N <= 96)  // few blocks: most of a warp's columns in flight (64 x 64 1.67 us, 1.76 in fours)
+      return launch_gemv_nw<1, 8, 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
     return launch_gemv_nw<1, 16, 8>(M, N, alpha, A, lda, x, incx, beta, y, incy, 1, st);
   }
   const bool wide = vec && M >= 512;
